@@ -11,8 +11,8 @@
 //     E = sum_rest conj(t[a, rest]) psi[c, rest]   (FP32 per thread and
 //                      across a warp's lanes, FP64 across the warps, in
 //                      fixed order),
-//     W = polar(E)     thread 0, polar_sweep (FP32 Jacobi, null directions
-//                      towards the current gate), G <- conj(W),
+//     W = polar(E)     warp 0 (warp_polar.cuh; null directions towards the
+//                      current gate), G <- conj(W),
 //     t <- G^H t;
 //   the sweep fidelity nuc / ||target||, the sweep count, the stop at
 //   stop_fidelity.
@@ -21,26 +21,24 @@
 // store's layout, <target|C|0> = sum_ac G[a, c] E[a, c] for every gate),
 // the gates stay as they are and no fidelity is written.
 // On a 1024-amplitude state the grouped sweep is bound by launches and its
-// FP64 window algebra (about 130 launches per sweep); here a step is a few
-// block-wide passes over shared memory and one FP32 polar factor.
-#include "device_common.cuh"
+// window algebra (about 130 launches per sweep); here a step is a few
+// block-wide passes over shared memory and one warp's polar factor, which
+// bounds it: peeling the next gate from psi does not depend on the new
+// gate, so the other warps do it meanwhile.
+// Measured (10 qubits, 15 layers, 4 sweeps, 600 steps): 29.1 ms with
+// a single-thread factor and the peel on the chain, 6.7 ms now (11 us a step).
+#include "warp_polar.cuh"
 
-// one state's gate, or its adjoint, as complex64 in shared memory
-__device__ __forceinline__ void fused_load_gate(const double2* g, int m, int adjoint, float2* gs) {
-  if (threadIdx.x < m * m) {
-    const int r = threadIdx.x / m, c = threadIdx.x % m;
-    const double2 v = adjoint ? cconj(g[c * m + r]) : g[r * m + c];
-    gs[threadIdx.x] = cf((float)v.x, (float)v.y);
-  }
-}
+__device__ __forceinline__ bool fused_valid(int k, int site, int n) { return k == 1 || (k == 2 && site <= n - 2); }
 
-__device__ __forceinline__ void fused_apply(float2* v, int n, int q, int k, const float2* gs) {
+// v <- g v (row-major, complex64 in shared memory) on qubit q (and q + 1)
+// by threads tid, tid + step, ... of the block.
+__device__ __forceinline__ void fused_apply(float2* v, int n, int q, int k, const float2* gs, int tid, int step) {
   if (k == 2) {
-    const int slo = n - 2 - q;
-    const int64_t dlo = (int64_t)1 << slo, dhi = dlo << 1;
-    for (int64_t r = threadIdx.x; r < ipow2(n - 2); r += blockDim.x) {
-      const int64_t i0 = quad_base(r, slo);
-      const int64_t idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
+    const int slo = n - 2 - q, dlo = 1 << slo, dhi = dlo << 1;
+    for (int r = tid; r < (1 << (n - 2)); r += step) {
+      const int i0 = (int)quad_base(r, slo);
+      const int idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
       float2 x[4];
 #pragma unroll
       for (int a = 0; a < 4; ++a) x[a] = v[idx[a]];
@@ -53,10 +51,9 @@ __device__ __forceinline__ void fused_apply(float2* v, int n, int q, int k, cons
       }
     }
   } else {
-    const int bit = n - 1 - q;
-    const int64_t d = (int64_t)1 << bit;
-    for (int64_t r = threadIdx.x; r < ipow2(n - 1); r += blockDim.x) {
-      const int64_t i0 = pair_base(r, bit);
+    const int bit = n - 1 - q, d = 1 << bit;
+    for (int r = tid; r < (1 << (n - 1)); r += step) {
+      const int i0 = (int)pair_base(r, bit);
       const float2 x0 = v[i0], x1 = v[i0 + d];
       v[i0] = fmac(fmac(cf(0.f, 0.f), gs[0], x0), gs[1], x1);
       v[i0 + d] = fmac(fmac(cf(0.f, 0.f), gs[2], x0), gs[3], x1);
@@ -64,29 +61,16 @@ __device__ __forceinline__ void fused_apply(float2* v, int n, int q, int k, cons
   }
 }
 
-// Per-warp sum of 16 complex FP32 accumulators by a fixed FP32 butterfly;
-// lane i < 16 writes entry i in FP64.  A lane holds one to four quads of a
-// state of at most 13 qubits, so the FP32 sum over 32 lanes rounds at
-// about 3e-7 of the entry; the FP64 butterfly it replaces held GB300's two
-// FP64 units for about 1300 warp instructions per gate step.
-__device__ __forceinline__ void warp_partial16_f32(const float2 (&e)[16], double2* out) {
-  const int lane = threadIdx.x & 31;
-  double2 mine = czero();
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    float re = e[i].x, im = e[i].y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      re += __shfl_xor_sync(0xffffffffu, re, o);
-      im += __shfl_xor_sync(0xffffffffu, im, o);
-    }
-    if (lane == i) mine = cd((double)re, (double)im);
-  }
-  if (lane < 16) out[lane] = mine;
+// acc += conj(a) b, real and imaginary part separately
+__device__ __forceinline__ void conj_mac(float& re, float& im, float2 a, float2 b) {
+  re = fmaf(a.x, b.x, fmaf(a.y, b.y, re));
+  im = fmaf(a.x, b.y, fmaf(-a.y, b.x, im));
 }
 
-__device__ __forceinline__ float2 conj_mul(float2 a, float2 b) {   // conj(a) b
-  return cf(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
+// entry e of an m x m gate (or its adjoint) as complex64
+__device__ __forceinline__ float2 fused_entry(const double2* g, int m, int adjoint, int e) {
+  const double2 v = adjoint ? cconj(g[(e % m) * m + e / m]) : g[e];
+  return cf((float)v.x, (float)v.y);
 }
 
 __global__ void __launch_bounds__(BLOCK_THREADS) k_sweep_fused(BatchDev bd, const float2* target, double2* gates,
@@ -95,142 +79,160 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_sweep_fused(BatchDev bd, cons
                                                                double stop_fid, double* sweep_fid,
                                                                int* sweeps_done, double2* env_out) {
   extern __shared__ float2 fsm[];
-  __shared__ float2 gs[16];
-  __shared__ double2 wred[WARPS][16];
+  __shared__ float2 gs[2][16];       // the gate to apply (rebuild), or to peel
+  __shared__ float2 gt[16];          // the new gate's adjoint
+  __shared__ double2 gd[2][16];      // the step's gate and the next step's
+  __shared__ double wred[WARPS][32];
   __shared__ double2 env[16];
-  __shared__ double s_nuc;
+  __shared__ WarpPolar wp;
   const int b = blockIdx.x;
   if (b >= bd.B) return;
   const int n = bd.n[b];
-  const int64_t N = ipow2(n);
+  const int N = 1 << n;
   float2* psi = fsm;
   float2* tt = fsm + N;
   const int L = nlayers[b];
   const int G = L * n;
-  const int warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const signed char* ar = arity + bd.gate_off[b] / 16;
   double2* gb = gates + bd.gate_off[b];
-  if (threadIdx.x == 0) s_nuc = 0.0;
+  double nuc = 0.0;   // warp 0
+  // the first step at or after j whose gate is valid (G if none); invalid
+  // slots raise the error flag and are skipped
+  auto next_step = [&](int j, bool forward, int& slot, int& site, int& k) {
+    for (; j < G; ++j) {
+      const int l = forward ? L - 1 - j / n : j / n;
+      site = forward ? j % n : n - 1 - j % n;
+      slot = l * n + site;
+      k = ar[slot];
+      if (fused_valid(k, site, n)) break;
+      if (tid == 0) atomicOr(bd.err, KERR_BAD_GATE);
+    }
+    return j;
+  };
   for (int sw = 0; sw < num_sweeps; ++sw) {
     __syncthreads();
     if (!active[b]) break;
-    for (int64_t i = threadIdx.x; i < N; i += blockDim.x) psi[i] = cf(i == 0 ? 1.f : 0.f, 0.f);
-    for (int j = 0; j < G; ++j) {
-      const int l = L - 1 - j / n, sidx = j % n, k = ar[l * n + sidx];
-      if (!((k == 1) || (k == 2 && sidx <= n - 2))) {
-        if (threadIdx.x == 0) atomicOr(bd.err, KERR_BAD_GATE);
-        continue;
-      }
-      __syncthreads();
-      fused_load_gate(gb + ((int64_t)l * n + sidx) * 16, 1 << k, 0, gs);
-      __syncthreads();
-      fused_apply(psi, n, sidx, k, gs);
+    for (int i = tid; i < N; i += BLOCK_THREADS) {
+      psi[i] = cf(i == 0 ? 1.f : 0.f, 0.f);
+      tt[i] = target[bd.vec_off[b] + i];
     }
-    for (int64_t i = threadIdx.x; i < N; i += blockDim.x) tt[i] = target[bd.vec_off[b] + i];
-    for (int j = 0; j < G; ++j) {
-      const int l = j / n, sidx = n - 1 - j % n, k = ar[l * n + sidx];
-      if (!((k == 1) || (k == 2 && sidx <= n - 2))) {
-        if (threadIdx.x == 0) atomicOr(bd.err, KERR_BAD_GATE);
-        continue;
-      }
-      const int m = 1 << k;
-      double2* gptr = gb + ((int64_t)l * n + sidx) * 16;
+    // C|0>; the next gate is fetched while one is applied
+    int slot, site, k;
+    int j = next_step(0, true, slot, site, k);
+    if (j < G && tid < (1 << (2 * k))) gs[0][tid] = fused_entry(gb + (int64_t)slot * 16, 1 << k, 0, tid);
+    for (int buf = 0; j < G; buf ^= 1) {
       __syncthreads();
-      fused_load_gate(gptr, m, 1, gs);
-      __syncthreads();
-      float2 e[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) e[i] = cf(0.f, 0.f);
-      if (k == 2) {
-        const int slo = n - 2 - sidx;
-        const int64_t dlo = (int64_t)1 << slo, dhi = dlo << 1;
-        for (int64_t r = threadIdx.x; r < ipow2(n - 2); r += blockDim.x) {
-          const int64_t i0 = quad_base(r, slo);
-          const int64_t idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
-          float2 x[4], y[4], tv[4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) x[a] = psi[idx[a]];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            float2 acc = cf(0.f, 0.f);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc = fmac(acc, gs[a * 4 + c], x[c]);
-            y[a] = acc;
-            psi[idx[a]] = acc;
-            tv[a] = tt[idx[a]];
-          }
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const float2 p = conj_mul(tv[a], y[c]);
-              e[a * 4 + c].x += p.x;
-              e[a * 4 + c].y += p.y;
-            }
-        }
-      } else {
-        const int bit = n - 1 - sidx;
-        const int64_t d = (int64_t)1 << bit;
-        for (int64_t r = threadIdx.x; r < ipow2(n - 1); r += blockDim.x) {
-          const int64_t i0 = pair_base(r, bit);
-          const float2 x0 = psi[i0], x1 = psi[i0 + d];
-          const float2 y0 = fmac(fmac(cf(0.f, 0.f), gs[0], x0), gs[1], x1);
-          const float2 y1 = fmac(fmac(cf(0.f, 0.f), gs[2], x0), gs[3], x1);
-          psi[i0] = y0;
-          psi[i0 + d] = y1;
-          const float2 t0 = tt[i0], t1 = tt[i0 + d];
-          const float2 p0 = conj_mul(t0, y0), p1 = conj_mul(t0, y1), p2 = conj_mul(t1, y0), p3 = conj_mul(t1, y1);
-          e[0].x += p0.x;
-          e[0].y += p0.y;
-          e[1].x += p1.x;
-          e[1].y += p1.y;
-          e[2].x += p2.x;
-          e[2].y += p2.y;
-          e[3].x += p3.x;
-          e[3].y += p3.y;
-        }
-      }
-      warp_partial16_f32(e, &wred[warp][0]);
-      __syncthreads();
-      if (threadIdx.x < 16) {
-        double2 sum = czero();
-        for (int w = 0; w < WARPS; ++w) sum = cadd(sum, wred[w][threadIdx.x]);
-        env[threadIdx.x] = sum;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double2 ee[16], w[16], wprev[16];
-        bool finite = true;
-        for (int i = 0; i < m * m; ++i) {
-          ee[i] = env[i];
-          finite = finite && isfinite(ee[i].x) && isfinite(ee[i].y);
-        }
-        if (!finite) {
-          atomicOr(bd.err, KERR_NONFINITE);
-        } else if (env_out) {
-          double2* eo = env_out + bd.gate_off[b] + ((int64_t)l * n + sidx) * 16;
-          for (int i = 0; i < m * m; ++i) eo[i] = ee[i];
-        } else {
-          for (int i = 0; i < m * m; ++i) wprev[i] = cconj(gptr[i]);
-          const double nn = polar_sweep(ee, m, w, wprev);
-          for (int i = 0; i < m * m; ++i) gptr[i] = cconj(w[i]);
-          s_nuc = nn;
-        }
-      }
-      __syncthreads();
-      fused_load_gate(gptr, m, 1, gs);   // t <- G_new^H t
-      __syncthreads();
-      fused_apply(tt, n, sidx, k, gs);
+      int slot2 = 0, site2 = 0, k2 = 0;
+      const int j2 = next_step(j + 1, true, slot2, site2, k2);
+      float2 pre = cf(0.f, 0.f);
+      const bool fetch = j2 < G && tid < (1 << (2 * k2));
+      if (fetch) pre = fused_entry(gb + (int64_t)slot2 * 16, 1 << k2, 0, tid);
+      fused_apply(psi, n, site, k, gs[buf], tid, BLOCK_THREADS);
+      if (fetch) gs[buf ^ 1][tid] = pre;
+      j = j2;
+      slot = slot2;
+      site = site2;
+      k = k2;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && !env_out) {
-      const double f = s_nuc / sqrt(tnorm2[b].x);
+    // backward sweep: the first gate is peeled here, every later one while
+    // its predecessor's polar factor is computed
+    j = next_step(0, false, slot, site, k);
+    if (j < G) {
+      if (tid < (1 << (2 * k))) {
+        gd[0][tid] = gb[(int64_t)slot * 16 + tid];
+        gs[0][tid] = fused_entry(gb + (int64_t)slot * 16, 1 << k, 1, tid);
+      }
+      __syncthreads();
+      fused_apply(psi, n, site, k, gs[0], tid, BLOCK_THREADS);
+    }
+    for (int buf = 0; j < G; buf ^= 1) {
+      __syncthreads();
+      const int m = 1 << k;
+      int slot2 = 0, site2 = 0, k2 = 0;
+      const int j2 = next_step(j + 1, false, slot2, site2, k2);
+      double2 pre = czero();
+      const bool fetch = j2 < G && tid < (1 << (2 * k2));
+      if (fetch) pre = gb[(int64_t)slot2 * 16 + tid];
+      // environment: value 2 i is Re E_i, 2 i + 1 Im E_i
+      float e[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) e[i] = 0.f;
+      if (k == 2) {
+        const int slo = n - 2 - site, dlo = 1 << slo, dhi = dlo << 1;
+        for (int r = tid; r < (N >> 2); r += BLOCK_THREADS) {
+          const int i0 = (int)quad_base(r, slo);
+          const int idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
+          float2 y[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) y[a] = psi[idx[a]];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const float2 tv = tt[idx[a]];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) conj_mac(e[2 * (a * 4 + c)], e[2 * (a * 4 + c) + 1], tv, y[c]);
+          }
+        }
+      } else {
+        const int bit = n - 1 - site, d = 1 << bit;
+        for (int r = tid; r < (N >> 1); r += BLOCK_THREADS) {
+          const int i0 = (int)pair_base(r, bit);
+          const float2 y0 = psi[i0], y1 = psi[i0 + d], t0 = tt[i0], t1 = tt[i0 + d];
+          conj_mac(e[0], e[1], t0, y0);
+          conj_mac(e[2], e[3], t0, y1);
+          conj_mac(e[4], e[5], t1, y0);
+          conj_mac(e[6], e[7], t1, y1);
+        }
+      }
+      // over a warp's lanes in FP32 (a lane holds one to eight quads), over
+      // the warps in FP64
+      wred[warp][lane] = (double)warp_sum32(e);
+      if (fetch) {
+        gd[buf ^ 1][tid] = pre;
+        gs[buf ^ 1][(tid % (1 << k2)) * (1 << k2) + tid / (1 << k2)] = cf((float)pre.x, -(float)pre.y);
+      }
+      __syncthreads();
+      if (warp == 0) {
+        double v[WARPS];
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) v[w] = wred[w][lane];
+        reinterpret_cast<double*>(env)[lane] =
+            ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        __syncwarp();
+        bool finite = true;
+        double2* g = gd[buf];
+        if (env_out) {
+          const bool mine = lane < m * m;
+          const double2 ev = mine ? env[lane] : czero();
+          finite = __all_sync(0xffffffffu, isfinite(ev.x) && isfinite(ev.y));
+          if (mine && finite) env_out[bd.gate_off[b] + (int64_t)slot * 16 + lane] = ev;
+        } else {
+          const double nn = warp_polar(wp, env, g, m, j2 >= G, &finite);
+          if (finite && j2 >= G) nuc = nn;
+          if (finite && lane < m * m) gb[(int64_t)slot * 16 + lane] = g[lane];
+        }
+        if (!finite && lane == 0) atomicOr(bd.err, KERR_NONFINITE);
+        if (lane < m * m) gt[lane] = fused_entry(g, m, 1, lane);
+      } else if (j2 < G) {
+        fused_apply(psi, n, site2, k2, gs[buf ^ 1], tid - 32, BLOCK_THREADS - 32);
+      }
+      __syncthreads();
+      if (j2 < G) fused_apply(tt, n, site, k, gt, tid, BLOCK_THREADS);   // t <- G_new^H t
+      j = j2;
+      slot = slot2;
+      site = site2;
+      k = k2;
+    }
+    if (tid == 0 && !env_out) {
+      const double f = nuc / sqrt(tnorm2[b].x);
       sweep_fid[(int64_t)b * num_sweeps + sw] = f;
       sweeps_done[b] = sw + 1;
       if (stop_fid > 0.0 && f >= stop_fid) active[b] = 0;
     }
   }
 }
+static_assert(WARPS == 8, "the environment's sum over the warps is written out for eight");
 
 int launch_sweep_fused(const BatchDev& bd, int max_n, const float2* target, double2* gates, const signed char* arity,
                        const int* nlayers, int* active, const double2* tnorm2, int num_sweeps, double stop_fid,

@@ -25,15 +25,17 @@
 //                  chunk of GCHUNK tiles, fp64 across the block, one
 //                  partial per chunk)
 //   k_group_polar  one block per state: sum the chunk partials in chunk
-//                  order, then run the group's steps on M in fp64 (target
-//                  update, peel, partial trace, polar factor), keeping the
-//                  replaced gates for the next pass
+//                  order, then run the group's steps on M (target update,
+//                  peel, partial trace, polar factor), keeping the replaced
+//                  gates for the next pass
 // Group 0 only reads (x = C|0>, z = the target); group 1 reads the target
 // and writes t, so the target is never copied.  After the last group the
 // vectors are not needed: the sweep's fidelity is the last step's trace.
 #include <cuda_fp16.h>
 
+#include "dfloat.cuh"
 #include "tile_layout.h"
+#include "warp_polar.cuh"
 #include "window.cuh"
 
 // Gate of state b at backward step j: generated layer j / n, site
@@ -884,100 +886,111 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_rebuild_pa
 
 // ---- per-group polar kernel ------------------------------------------------------
 
-// M <- G^T M on the rows of gate bits (h, l): the target-side update z <- P z
-// with P = G^H maps M to conj(P) M = G^T M.
-__device__ void m_rows(double2* M, int D, const double2* G, int k, int h, int l) {
-  if (k == 2) {
-    const int items = D * (D / 4);
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int col = it % D, o = it / D;
-      int ob = 0, kk = 0;
-      for (int bit = 0; (1 << bit) < D; ++bit) {
-        if (bit == h || bit == l) continue;
-        ob |= ((o >> kk) & 1) << bit;
-        ++kk;
-      }
-      const int idx[4] = {ob, ob | (1 << l), ob | (1 << h), ob | (1 << h) | (1 << l)};
-      double2 x[4], y[4];
-      for (int r = 0; r < 4; ++r) x[r] = M[idx[r] * GM + col];
-      for (int r = 0; r < 4; ++r) {
-        double2 s = czero();
-        for (int rp = 0; rp < 4; ++rp) s = cadd(s, cmul(G[rp * 4 + r], x[rp]));
-        y[r] = s;
-      }
-      for (int r = 0; r < 4; ++r) M[idx[r] * GM + col] = y[r];
-    }
-  } else {
-    const int items = D * (D / 2);
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int col = it % D, o = it / D;
-      const int ob = ((o >> h) << (h + 1)) | (o & ((1 << h) - 1));
-      const double2 x0 = M[ob * GM + col], x1 = M[(ob | (1 << h)) * GM + col];
-      M[ob * GM + col] = cadd(cmul(G[0], x0), cmul(G[2], x1));
-      M[(ob | (1 << h)) * GM + col] = cadd(cmul(G[1], x0), cmul(G[3], x1));
-    }
+// The cross matrix is held in double-float (float4, dfloat.cuh): a 16 x 16
+// update is 4096 complex multiply-adds, which the SM's two FP64 units need
+// about 1 us for and the FP32 pipes, at 2^-46 of relative error on sums whose
+// terms carry FP32 rounding, a third of that.
+
+// index of the o-th combination of the bits other than h (and l)
+__device__ __forceinline__ int spread_bits(int o, int k, int h, int l) {
+  if (k == 1) return ((o >> h) << (h + 1)) | (o & ((1 << h) - 1));
+  const int t = ((o >> l) << (l + 1)) | (o & ((1 << l) - 1));   // l < h
+  return ((t >> h) << (h + 1)) | (t & ((1 << h) - 1));
+}
+
+// value of window index i with the gate bits cleared, and those bits
+__device__ __forceinline__ int gate_bits(int i, int k, int h, int l) {
+  return k == 2 ? (((i >> h) & 1) << 1) | ((i >> l) & 1) : (i >> h) & 1;
+}
+__device__ __forceinline__ int gate_place(int v, int k, int h, int l) {
+  return k == 2 ? (((v >> 1) & 1) << h) | ((v & 1) << l) : v << h;
+}
+
+// dst <- G^T src on the rows of gate bits (h, l): the target-side update
+// z <- P z with P = G^H maps M to conj(P) M = G^T M.
+__device__ __forceinline__ void m_rows(const xc* src, xc* dst, int D, const xc* G, int k, int h, int l, int tid,
+                                       int step) {
+  const int m = 1 << k, clear = ~gate_place(m - 1, k, h, l);
+  for (int e = tid; e < D * D; e += step) {
+    const int i = e / D, c = e % D, r = gate_bits(i, k, h, l), base = i & clear;
+    XA acc = xa_zero();
+    for (int rp = 0; rp < m; ++rp) xa_mac(acc, G[rp * m + r], src[(base | gate_place(rp, k, h, l)) * GM + c]);
+    dst[i * GM + c] = xa_round(acc);
   }
 }
 
-// M <- M Q^T on the columns of gate bits (h, l), Q = G^H: the circuit-side
-// peel x <- Q x.  (M Q^T)[i][c] = sum_c' M[i][c'] conj(G[c'][c]).
-__device__ void m_cols(double2* M, int D, const double2* G, int k, int h, int l) {
-  if (k == 2) {
-    const int items = D * (D / 4);
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int row = it % D, o = it / D;
-      int ob = 0, kk = 0;
-      for (int bit = 0; (1 << bit) < D; ++bit) {
-        if (bit == h || bit == l) continue;
-        ob |= ((o >> kk) & 1) << bit;
-        ++kk;
-      }
-      const int idx[4] = {ob, ob | (1 << l), ob | (1 << h), ob | (1 << h) | (1 << l)};
-      double2 x[4], y[4];
-      for (int c = 0; c < 4; ++c) x[c] = M[row * GM + idx[c]];
-      for (int c = 0; c < 4; ++c) {
-        double2 s = czero();
-        for (int cp = 0; cp < 4; ++cp) s = cadd(s, cmul(cconj(G[cp * 4 + c]), x[cp]));
-        y[c] = s;
-      }
-      for (int c = 0; c < 4; ++c) M[row * GM + idx[c]] = y[c];
-    }
-  } else {
-    const int items = D * (D / 2);
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int row = it % D, o = it / D;
-      const int ob = ((o >> h) << (h + 1)) | (o & ((1 << h) - 1));
-      const double2 x0 = M[row * GM + ob], x1 = M[row * GM + (ob | (1 << h))];
-      M[row * GM + ob] = cadd(cmul(cconj(G[0]), x0), cmul(cconj(G[2]), x1));
-      M[row * GM + (ob | (1 << h))] = cadd(cmul(cconj(G[1]), x0), cmul(cconj(G[3]), x1));
-    }
+// dst <- src Q^T on the columns of gate bits (h, l), Q = G^H: the
+// circuit-side peel x <- Q x.  (M Q^T)[i][c] = sum_c' M[i][c'] conj(G[c'][c]).
+__device__ __forceinline__ void m_cols(const xc* src, xc* dst, int D, const xc* G, int k, int h, int l, int tid,
+                                       int step) {
+  const int m = 1 << k, clear = ~gate_place(m - 1, k, h, l);
+  for (int e = tid; e < D * D; e += step) {
+    const int i = e / D, c = e % D, r = gate_bits(c, k, h, l), base = c & clear;
+    XA acc = xa_zero();
+    for (int cp = 0; cp < m; ++cp)
+      xa_mac(acc, xc_conj(G[cp * m + r]), src[i * GM + (base | gate_place(cp, k, h, l))]);
+    dst[i * GM + c] = xa_round(acc);
   }
 }
 
-// One block per state and group.  The polar factor of each step is the
-// sweep polar of small_linalg.h: singular values of E at most 1e-6 of the
+// One block per state and group.  The polar factor of each step is
+// warp_polar (warp_polar.cuh): singular values of E at most 1e-6 of the
 // largest count as zero, and on that null space (inputs the circuit never
 // feeds the gate, such as fresh |0> qubits) every completion is optimal, so
 // the kernel keeps the one nearest to the current gate; structured gates
 // stay structured under fp32 rounding.  nuc[b] receives Re Tr(W^H E) of the
-// last step, |<t|new|psi>| after the update.
-#define POLAR_THREADS 64
+// sweep's last step, |<t|new|psi>| after the update.
+//
+// A step is a chain (the environment, its polar factor, the update of M's
+// rows), and a group's steps follow one another; the columns' update of the
+// next step commutes with the rows' and runs on the other warps while warp
+// 0 computes the polar factor.
+// Measured on a 20-qubit state (three steps per group): 170 us per launch with
+// a single-thread factor and FP64 updates by 64 threads, 39 us now.
+#define POLAR_THREADS 256
 
 __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, GroupDev gd, int g, double2* gates,
                                                                const signed char* arity, const int* nlayers,
                                                                const int* active, double* nuc, double2* env_out) {
-  __shared__ double2 M[GMM];
+  __shared__ xc M[2][GMM];
   __shared__ double2 env[16];
+  __shared__ double2 gold[GMAXSTEPS][16];   // the steps' gates, replaced one by one
+  __shared__ xc gx[GMAXSTEPS][16];          // the same in double-float
+  __shared__ int sk[GMAXSTEPS], sh[GMAXSTEPS], sl[GMAXSTEPS];
+  __shared__ int64_t sslot[GMAXSTEPS];
+  __shared__ WarpPolar wp;
+  const int tid = threadIdx.x, lane = tid & 31;
   for (int b = blockIdx.x; b < bd.B; b += gridDim.x) {
     if (active && !active[b]) continue;
     if (g >= gd.ngroups[b]) continue;
     const GroupEnt ge = gd.grp[(int64_t)b * gd.gmax + g];
     const int n = bd.n[b], L = nlayers[b], D = 1 << ge.u;
     const int c0 = gd.state_chunk0[b], nc = gd.state_nchunks[b];
+    const int cnt = ge.cnt < GMAXSTEPS ? ge.cnt : GMAXSTEPS;
+    const bool last = g + 1 == gd.ngroups[b];
     __syncthreads();
+    // the plan only groups valid steps; one that is not is never applied
+    if (tid < cnt * 16) {
+      const int s = tid >> 4, e = tid & 15;
+      int64_t slot = 0;
+      int q = 0, k = 0;
+      const bool ok = bwd_step(bd, arity, L, n, b, ge.j0 + s, &slot, &q, &k);
+      if (e == 0) {
+        sk[s] = ok ? k : 0;
+        sh[s] = __popc(ge.qmask >> (q + 1));
+        sl[s] = k == 2 ? __popc(ge.qmask >> (q + 2)) : 0;
+        sslot[s] = slot;
+      }
+      if (ok && e < (1 << (2 * k))) {
+        const double2 v = gates[bd.gate_off[b] + slot * 16 + e];
+        gold[s][e] = v;
+        gx[s][e] = xc_from_d(v);
+        gd.old_gates[((int64_t)b * GMAXSTEPS + s) * 16 + e] = v;
+      }
+    }
     // sum of the chunk partials in chunk order; eight chunks' loads are
     // issued together so the L2 latency overlaps
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
+    for (int e = tid; e < D * D; e += POLAR_THREADS) {
       const int i = e / D, k = e % D;
       const double2* src = gd.partials + (int64_t)c0 * GMM + i * GM + k;
       double2 s = czero();
@@ -990,67 +1003,59 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
         for (int u = 0; u < 8; ++u) s = cadd(s, v[u]);
       }
       for (; c < nc; ++c) s = cadd(s, src[(int64_t)c * GMM]);
-      M[i * GM + k] = s;
+      M[0][i * GM + k] = xc_from_d(s);
     }
     __syncthreads();
-    const double2* pend = nullptr;
-    int pk = 0, ph = 0, pl = 0;
-    for (int s = 0; s < ge.cnt && s < GMAXSTEPS; ++s) {
-      int64_t slot;
-      int q, k;
-      if (!bwd_step(bd, arity, L, n, b, ge.j0 + s, &slot, &q, &k)) continue;
-      double2* gptr = gates + bd.gate_off[b] + slot * 16;
-      const int h = __popc(ge.qmask >> (q + 1)), l = k == 2 ? __popc(ge.qmask >> (q + 2)) : 0;
-      if (pend) {
-        m_rows(M, D, pend, pk, ph, pl);
+    int cur = 0;
+    if (sk[0]) {
+      m_cols(M[0], M[1], D, gx[0], sk[0], sh[0], sl[0], tid, POLAR_THREADS);
+      cur = 1;
+      __syncthreads();
+    }
+    for (int s = 0; s < cnt; ++s) {
+      const int k = sk[s], k2 = s + 1 < cnt ? sk[s + 1] : 0;
+      if (tid < 32) {
+        const int m = 1 << k;
+        if (k) {
+          // E[r][c] = sum_o M[(r, o)][(c, o)], one part per lane
+          const int ent = lane >> 1, part = lane & 1;
+          if (ent < m * m) {
+            const int r = gate_place(ent / m, k, sh[s], sl[s]), c = gate_place(ent % m, k, sh[s], sl[s]);
+            double acc = 0.0;
+            for (int o = 0; o < D / m; ++o) {
+              const int ob = spread_bits(o, k, sh[s], sl[s]);
+              const xc v = M[cur][(r | ob) * GM + (c | ob)];
+              acc += part ? (double)v.y + (double)v.w : (double)v.x + (double)v.z;
+            }
+            reinterpret_cast<double*>(env)[lane] = acc;
+          }
+          __syncwarp();
+          bool finite = true;
+          const bool mine = lane < m * m;
+          const int64_t at = bd.gate_off[b] + sslot[s] * 16 + lane;
+          if (env_out) {   // environment at the fixed circuit: the gate stays
+            const double2 ev = mine ? env[lane] : czero();
+            finite = __all_sync(0xffffffffu, isfinite(ev.x) && isfinite(ev.y));
+            if (mine && finite) env_out[at] = ev;
+          } else {
+            const bool want = last && s + 1 == cnt;
+            const double nn = warp_polar(wp, env, gold[s], m, want, &finite);
+            if (finite && want && lane == 0) nuc[b] = nn;
+            if (finite && mine) gates[at] = gold[s][lane];
+          }
+          if (!finite && lane == 0) atomicOr(bd.err, KERR_NONFINITE);
+          if (mine) gx[s][lane] = xc_from_d(gold[s][lane]);
+        }
+      } else if (k2) {
+        m_cols(M[cur], M[cur ^ 1], D, gx[s + 1], k2, sh[s + 1], sl[s + 1], tid - 32, POLAR_THREADS - 32);
+      }
+      __syncthreads();
+      if (k2) cur ^= 1;
+      if (k && s + 1 < cnt) {
+        m_rows(M[cur], M[cur ^ 1], D, gx[s], k, sh[s], sl[s], tid, POLAR_THREADS);
+        cur ^= 1;
         __syncthreads();
       }
-      m_cols(M, D, gptr, k, h, l);
-      __syncthreads();
-      const int m = 1 << k;
-      if (threadIdx.x < m * m) {
-        const int r = threadIdx.x / m, c = threadIdx.x % m;
-        double2 acc = czero();
-        for (int o = 0; o < D / m; ++o) {
-          int ob = 0, kk = 0;
-          for (int bit = 0; (1 << bit) < D; ++bit) {
-            if (bit == h || (k == 2 && bit == l)) continue;
-            ob |= ((o >> kk) & 1) << bit;
-            ++kk;
-          }
-          const int ir = ob | (k == 2 ? (((r >> 1) & 1) << h) | ((r & 1) << l) : (r << h));
-          const int ic = ob | (k == 2 ? (((c >> 1) & 1) << h) | ((c & 1) << l) : (c << h));
-          acc = cadd(acc, M[ir * GM + ic]);
-        }
-        env[threadIdx.x] = acc;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double2 e[16], w[16], wprev[16];
-        bool finite = true;
-        for (int i = 0; i < m * m; ++i) {
-          e[i] = env[i];
-          finite = finite && isfinite(e[i].x) && isfinite(e[i].y);
-        }
-        double2* keep = gd.old_gates + ((int64_t)b * GMAXSTEPS + s) * 16;
-        for (int i = 0; i < m * m; ++i) keep[i] = gptr[i];
-        if (!finite) {
-          atomicOr(bd.err, KERR_NONFINITE);
-        } else if (env_out) {   // environment at the fixed circuit: the gate stays
-          double2* eo = env_out + bd.gate_off[b] + slot * 16;
-          for (int i = 0; i < m * m; ++i) eo[i] = e[i];
-        } else {
-          for (int i = 0; i < m * m; ++i) wprev[i] = cconj(gptr[i]);
-          const double nn = polar_sweep(e, m, w, wprev);
-          for (int i = 0; i < m * m; ++i) gptr[i] = cconj(w[i]);
-          nuc[b] = nn;
-        }
-      }
-      __syncthreads();
-      pend = gptr;
-      pk = k;
-      ph = h;
-      pl = l;
     }
   }
 }
