@@ -15,8 +15,8 @@
 // which keeps about 2^-46 of relative precision on the FP32 pipes.  The
 // small algebra is FP64: the eigensolvers of stage (a) and of the layer
 // cuts (shared with the fast mode), the closed-form gate construction, and
-// the sweep's polar factor (FP64 one-sided Jacobi, started from FP32
-// sweeps; the fast mode's FP32 polar is accurate to ~1e-7, which
+// the sweep's polar factor (FP64 one-sided Jacobi by one warp, started from
+// FP32 sweeps; the fast mode's FP32 polar is accurate to ~1e-7, which
 // rank-deficient environments carry into later steps at first order).
 //
 // Caller-facing statevector buffers of this mode are complex128; the plan
@@ -38,8 +38,10 @@
 //                             from the circuit state, reduce the gate's
 //                             environment, and (last tile of the state)
 //                             replace the gate by the conjugate of the
-//                             environment's polar factor
+//                             environment's polar factor (one warp,
+//                             warp_polar.cuh)
 #include "dfloat.cuh"
+#include "warp_polar.cuh"
 
 static int grid_for(const BatchDev& bd) {
   const int cap = 152 * 8;
@@ -527,6 +529,23 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_apply_gate(BatchDev bd, xc*
   }
 }
 
+// e[2 i], e[2 i + 1] += real and imaginary part of conj(u) v
+__device__ __forceinline__ void x_env_mac(DF (&e)[32], int i, xc u, xc v) {
+  df_mac(e[2 * i], u.x, u.z, v.x, v.z);
+  df_mac(e[2 * i], u.y, u.w, v.y, v.w);
+  df_mac(e[2 * i + 1], u.x, u.z, v.y, v.w);
+  df_mac(e[2 * i + 1], -u.y, -u.w, v.x, v.z);
+}
+
+// sum over the block's warps of part `lane`, in fixed order
+__device__ __forceinline__ double x_sum_warps(const double (*wred)[32], int lane) {
+  double v[WARPS];
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) v[w] = wred[w][lane];
+  return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+}
+static_assert(WARPS == 8, "the sum over the warps is written out for eight");
+
 // Backward sweep step `step` of every active state (the reference's
 // per-gate update, qmprs/synthesis/mps_encoding/sequential.py:452-505):
 //   psi <- G^H psi                      (peel the gate from the circuit state)
@@ -540,8 +559,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
                                                                 const int* nlayers, const int* active,
                                                                 double2* partials, double* nuc) {
   __shared__ xc gs[16];
-  __shared__ double2 wred[WARPS][16];
-  __shared__ double2 env[16];
+  __shared__ double wred[WARPS][32];
+  __shared__ double2 env[16], gd[16];
+  __shared__ WarpPolar wp;
   GateSel sel;
   sel.mode = SEL_SWEEP;
   sel.step = step;
@@ -551,7 +571,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
   sel.arity = arity;
   sel.nlayers = nlayers;
   sel.active = active;
-  const int warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     const int n = bd.n[b];
@@ -568,9 +588,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
     const int nt = bd.state_ntiles[b];
     int64_t lo, hi;
     tile_range(ipow2(n - k), bd.tile_idx[tile], nt, &lo, &hi);
-    XA e[16];
+    DF e[32];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) e[i] = xa_zero();
+    for (int i = 0; i < 32; ++i) e[i] = DF{0.f, 0.f};
     if (k == 2) {
       const int slo = n - 2 - q;
       const int64_t dlo = (int64_t)1 << slo, dhi = dlo << 1;
@@ -592,7 +612,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) xa_macc(e[a * 4 + c], tt[a], y[c]);
+          for (int c = 0; c < 4; ++c) x_env_mac(e, a * 4 + c, tt[a], y[c]);
       }
     } else {
       const int bit = n - 1 - q;
@@ -609,30 +629,19 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
         v[i0] = y0;
         v[i0 + d] = y1;
         const xc t0 = tv[i0], t1 = tv[i0 + d];
-        xa_macc(e[0], t0, y0);
-        xa_macc(e[1], t0, y1);
-        xa_macc(e[2], t1, y0);
-        xa_macc(e[3], t1, y1);
+        x_env_mac(e, 0, t0, y0);
+        x_env_mac(e, 1, t0, y1);
+        x_env_mac(e, 2, t1, y0);
+        x_env_mac(e, 3, t1, y1);
       }
     }
-    // per warp (fixed butterfly), then the block's warps in order
-    double acc[32];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const double2 d = xa_to_d(e[i]);
-      acc[2 * i] = d.x;
-      acc[2 * i + 1] = d.y;
-    }
-    warp_partial16_f64(acc, &wred[warp][0]);
+    // per warp (fixed exchange, double-float), then the block's warps in order
+    wred[warp][tid & 31] = warp_sum32_df(e);
     __syncthreads();
-    if (threadIdx.x < 16) {
-      double2 s = czero();
-      for (int w = 0; w < WARPS; ++w) s = cadd(s, wred[w][threadIdx.x]);
-      partials[(int64_t)tile * 16 + threadIdx.x] = s;
-    }
+    if (tid < 32) reinterpret_cast<double*>(partials + (int64_t)tile * 16)[tid] = x_sum_warps(wred, tid);
     __syncthreads();
     if (last_tile_ticket(bd.ticket, b, nt)) {
-      const int entry = threadIdx.x >> 4, l16 = threadIdx.x & 15;
+      const int entry = tid >> 4, l16 = tid & 15;
       const int t0 = bd.state_tile0[b];
       double2 s = czero();
       for (int tt = l16; tt < nt; tt += 16) s = cadd(s, ld_cg(&partials[(int64_t)(t0 + tt) * 16 + entry]));
@@ -642,26 +651,20 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
         s.y += __shfl_down_sync(0xffffffffu, s.y, o, 16);
       }
       if (l16 == 0) env[entry] = s;
+      if (tid < m * m) gd[tid] = gptr[tid];
       __syncthreads();
-      if (threadIdx.x == 0) {
-        double2 ee[16], w[16], wprev[16];
-        bool finite = true;
-        for (int i = 0; i < m * m; ++i) {
-          ee[i] = env[i];
-          finite = finite && isfinite(ee[i].x) && isfinite(ee[i].y);
+      if (tid < 32) {
+        // FP64 polar: rank-deficient environments leave null directions that
+        // follow the current gate, and an FP32 completion of them would
+        // enter the later steps at first order
+        bool finite;
+        const double nn = warp_polar_exact(wp, env, gd, m, &finite);
+        if (finite && tid < m * m) gptr[tid] = gd[tid];
+        if (tid == 0) {
+          if (finite) nuc[b] = nn;
+          else atomicOr(bd.err, KERR_NONFINITE);
+          bd.ticket[b] = 0;
         }
-        if (!finite) {
-          atomicOr(bd.err, KERR_NONFINITE);
-        } else {
-          // FP64 Hestenes polar: rank-deficient environments leave null
-          // directions that follow the current gate, and an FP32 completion
-          // of them would enter the later steps at first order
-          for (int i = 0; i < m * m; ++i) wprev[i] = cconj(gptr[i]);
-          const double nn = polar_jacobi_pre(ee, m, w, wprev);
-          for (int i = 0; i < m * m; ++i) gptr[i] = cconj(w[i]);
-          nuc[b] = nn;
-        }
-        bd.ticket[b] = 0;
       }
       __syncthreads();
     }
@@ -673,17 +676,19 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
 // the launch-per-step path (k_x_apply_gate / k_x_sweep_step /
 // k_sweep_finish): C|0> rebuilt gate by gate, t from the target, then per
 // gate (backward order) psi <- G^H psi, E = sum conj(t) psi, the FP64
-// polar factor by thread 0 (G <- conj(W)), t <- G^H t; after the sweep
+// polar factor by warp 0 (G <- conj(W)), t <- G^H t; after the sweep
 // the fidelity nuc / ||target||, the sweep count and the stop at
-// stop_fidelity.  The environment is reduced per warp (fixed butterfly)
-// and over the warps in order.
-__device__ __forceinline__ void x_fused_apply(xc* v, int n, int q, int k, const xc* gs) {
+// stop_fidelity.  The environment is reduced per warp (fixed exchange)
+// and over the warps in order.  As in k_sweep_fused the polar factor bounds
+// a step, and the other warps peel the next gate from psi meanwhile.
+// Measured (10 qubits, 15 layers, 2 sweeps, 300 steps): 51.2 ms with a
+// single-thread factor, 8.7 ms now (29 us a step).
+__device__ __forceinline__ void x_fused_apply(xc* v, int n, int q, int k, const xc* gs, int tid, int step) {
   if (k == 2) {
-    const int slo = n - 2 - q;
-    const int64_t dlo = (int64_t)1 << slo, dhi = dlo << 1;
-    for (int64_t r = threadIdx.x; r < ipow2(n - 2); r += blockDim.x) {
-      const int64_t i0 = quad_base(r, slo);
-      const int64_t idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
+    const int slo = n - 2 - q, dlo = 1 << slo, dhi = dlo << 1;
+    for (int r = tid; r < (1 << (n - 2)); r += step) {
+      const int i0 = (int)quad_base(r, slo);
+      const int idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
       xc x[4];
 #pragma unroll
       for (int a = 0; a < 4; ++a) x[a] = v[idx[a]];
@@ -696,10 +701,9 @@ __device__ __forceinline__ void x_fused_apply(xc* v, int n, int q, int k, const 
       }
     }
   } else {
-    const int bit = n - 1 - q;
-    const int64_t d = (int64_t)1 << bit;
-    for (int64_t r = threadIdx.x; r < ipow2(n - 1); r += blockDim.x) {
-      const int64_t i0 = pair_base(r, bit);
+    const int bit = n - 1 - q, d = 1 << bit;
+    for (int r = tid; r < (1 << (n - 1)); r += step) {
+      const int i0 = (int)pair_base(r, bit);
       const xc x0 = v[i0], x1 = v[i0 + d];
       XA s0 = xa_zero(), s1 = xa_zero();
       xa_mac(s0, gs[0], x0);
@@ -718,138 +722,140 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
                                                                  double stop_fid, double* sweep_fid,
                                                                  int* sweeps_done) {
   extern __shared__ xc xsm[];
-  __shared__ xc gs[16];
-  __shared__ double2 wred[WARPS][16];
+  __shared__ xc gs[2][16];           // the gate to apply (rebuild), or to peel
+  __shared__ xc gt[16];              // the new gate's adjoint
+  __shared__ double2 gd[2][16];      // the step's gate and the next step's
+  __shared__ double wred[WARPS][32];
   __shared__ double2 env[16];
-  __shared__ double s_nuc;
+  __shared__ WarpPolar wp;
   const int b = blockIdx.x;
   if (b >= bd.B) return;
   const int n = bd.n[b];
-  const int64_t N = ipow2(n);
+  const int N = 1 << n;
   xc* psi = xsm;
   xc* tt = xsm + N;
   const int L = nlayers[b];
   const int G = L * n;
-  const int warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const signed char* ar = arity + bd.gate_off[b] / 16;
   double2* gb = gates + bd.gate_off[b];
-  if (threadIdx.x == 0) s_nuc = 0.0;
+  double nuc = 0.0;   // warp 0
+  // the first step at or after j whose gate is valid (G if none); invalid
+  // slots raise the error flag and are skipped
+  auto next_step = [&](int j, bool forward, int& slot, int& site, int& k) {
+    for (; j < G; ++j) {
+      const int l = forward ? L - 1 - j / n : j / n;
+      site = forward ? j % n : n - 1 - j % n;
+      slot = l * n + site;
+      k = ar[slot];
+      if (k == 1 || (k == 2 && site <= n - 2)) break;
+      if (tid == 0) atomicOr(bd.err, KERR_BAD_GATE);
+    }
+    return j;
+  };
   for (int sw = 0; sw < num_sweeps; ++sw) {
     __syncthreads();
     if (!active[b]) break;
-    // C|0>
-    for (int64_t i = threadIdx.x; i < N; i += blockDim.x) psi[i] = make_float4(i == 0 ? 1.f : 0.f, 0.f, 0.f, 0.f);
-    for (int j = 0; j < G; ++j) {
-      const int l = L - 1 - j / n, sidx = j % n, k = ar[l * n + sidx];
-      if (!((k == 1) || (k == 2 && sidx <= n - 2))) {
-        if (threadIdx.x == 0) atomicOr(bd.err, KERR_BAD_GATE);
-        continue;
-      }
-      __syncthreads();
-      x_load_gate(gb + ((int64_t)l * n + sidx) * 16, 1 << k, 0, gs);
-      __syncthreads();
-      x_fused_apply(psi, n, sidx, k, gs);
+    for (int i = tid; i < N; i += BLOCK_THREADS) {
+      psi[i] = make_float4(i == 0 ? 1.f : 0.f, 0.f, 0.f, 0.f);
+      tt[i] = target[bd.vec_off[b] + i];
     }
-    for (int64_t i = threadIdx.x; i < N; i += blockDim.x) tt[i] = target[bd.vec_off[b] + i];
-    // backward sweep
-    for (int j = 0; j < G; ++j) {
-      const int l = j / n, sidx = n - 1 - j % n, k = ar[l * n + sidx];
-      if (!((k == 1) || (k == 2 && sidx <= n - 2))) {
-        if (threadIdx.x == 0) atomicOr(bd.err, KERR_BAD_GATE);
-        continue;
-      }
-      const int m = 1 << k;
-      double2* gptr = gb + ((int64_t)l * n + sidx) * 16;
+    // C|0>; the next gate is fetched while one is applied
+    int slot, site, k;
+    int j = next_step(0, true, slot, site, k);
+    if (j < G && tid < (1 << (2 * k))) gs[0][tid] = xc_from_d(gb[(int64_t)slot * 16 + tid]);
+    for (int buf = 0; j < G; buf ^= 1) {
       __syncthreads();
-      x_load_gate(gptr, m, 1, gs);
-      __syncthreads();
-      XA e[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) e[i] = xa_zero();
-      if (k == 2) {
-        const int slo = n - 2 - sidx;
-        const int64_t dlo = (int64_t)1 << slo, dhi = dlo << 1;
-        for (int64_t r = threadIdx.x; r < ipow2(n - 2); r += blockDim.x) {
-          const int64_t i0 = quad_base(r, slo);
-          const int64_t idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
-          xc x[4], y[4], tv[4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) x[a] = psi[idx[a]];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            XA acc = xa_zero();
-#pragma unroll
-            for (int c = 0; c < 4; ++c) xa_mac(acc, gs[a * 4 + c], x[c]);
-            y[a] = xa_round(acc);
-            psi[idx[a]] = y[a];
-            tv[a] = tt[idx[a]];
-          }
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) xa_macc(e[a * 4 + c], tv[a], y[c]);
-        }
-      } else {
-        const int bit = n - 1 - sidx;
-        const int64_t d = (int64_t)1 << bit;
-        for (int64_t r = threadIdx.x; r < ipow2(n - 1); r += blockDim.x) {
-          const int64_t i0 = pair_base(r, bit);
-          const xc x0 = psi[i0], x1 = psi[i0 + d];
-          XA s0 = xa_zero(), s1 = xa_zero();
-          xa_mac(s0, gs[0], x0);
-          xa_mac(s0, gs[1], x1);
-          xa_mac(s1, gs[2], x0);
-          xa_mac(s1, gs[3], x1);
-          const xc y0 = xa_round(s0), y1 = xa_round(s1);
-          psi[i0] = y0;
-          psi[i0 + d] = y1;
-          const xc t0 = tt[i0], t1 = tt[i0 + d];
-          xa_macc(e[0], t0, y0);
-          xa_macc(e[1], t0, y1);
-          xa_macc(e[2], t1, y0);
-          xa_macc(e[3], t1, y1);
-        }
-      }
-      double acc[32];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const double2 dv = xa_to_d(e[i]);
-        acc[2 * i] = dv.x;
-        acc[2 * i + 1] = dv.y;
-      }
-      warp_partial16_f64(acc, &wred[warp][0]);
-      __syncthreads();
-      if (threadIdx.x < 16) {
-        double2 sum = czero();
-        for (int w = 0; w < WARPS; ++w) sum = cadd(sum, wred[w][threadIdx.x]);
-        env[threadIdx.x] = sum;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double2 ee[16], w[16], wprev[16];
-        bool finite = true;
-        for (int i = 0; i < m * m; ++i) {
-          ee[i] = env[i];
-          finite = finite && isfinite(ee[i].x) && isfinite(ee[i].y);
-        }
-        if (!finite) {
-          atomicOr(bd.err, KERR_NONFINITE);
-        } else {
-          for (int i = 0; i < m * m; ++i) wprev[i] = cconj(gptr[i]);
-          const double nn = polar_jacobi_pre(ee, m, w, wprev);
-          for (int i = 0; i < m * m; ++i) gptr[i] = cconj(w[i]);
-          s_nuc = nn;
-        }
-      }
-      __syncthreads();
-      // t <- G_new^H t
-      x_load_gate(gptr, m, 1, gs);
-      __syncthreads();
-      x_fused_apply(tt, n, sidx, k, gs);
+      int slot2 = 0, site2 = 0, k2 = 0;
+      const int j2 = next_step(j + 1, true, slot2, site2, k2);
+      double2 pre = czero();
+      const bool fetch = j2 < G && tid < (1 << (2 * k2));
+      if (fetch) pre = gb[(int64_t)slot2 * 16 + tid];
+      x_fused_apply(psi, n, site, k, gs[buf], tid, BLOCK_THREADS);
+      if (fetch) gs[buf ^ 1][tid] = xc_from_d(pre);
+      j = j2;
+      slot = slot2;
+      site = site2;
+      k = k2;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      const double f = s_nuc / sqrt(tnorm2[b].x);
+    // backward sweep: the first gate is peeled here, every later one while
+    // its predecessor's polar factor is computed
+    j = next_step(0, false, slot, site, k);
+    if (j < G) {
+      if (tid < (1 << (2 * k))) {
+        const double2 v = gb[(int64_t)slot * 16 + tid];
+        gd[0][tid] = v;
+        gs[0][(tid % (1 << k)) * (1 << k) + tid / (1 << k)] = xc_from_d(cconj(v));
+      }
+      __syncthreads();
+      x_fused_apply(psi, n, site, k, gs[0], tid, BLOCK_THREADS);
+    }
+    for (int buf = 0; j < G; buf ^= 1) {
+      __syncthreads();
+      const int m = 1 << k;
+      int slot2 = 0, site2 = 0, k2 = 0;
+      const int j2 = next_step(j + 1, false, slot2, site2, k2);
+      double2 pre = czero();
+      const bool fetch = j2 < G && tid < (1 << (2 * k2));
+      if (fetch) pre = gb[(int64_t)slot2 * 16 + tid];
+      DF e[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) e[i] = DF{0.f, 0.f};
+      if (k == 2) {
+        const int slo = n - 2 - site, dlo = 1 << slo, dhi = dlo << 1;
+        for (int r = tid; r < (N >> 2); r += BLOCK_THREADS) {
+          const int i0 = (int)quad_base(r, slo);
+          const int idx[4] = {i0, i0 + dlo, i0 + dhi, i0 + dhi + dlo};
+          xc y[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) y[a] = psi[idx[a]];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const xc tv = tt[idx[a]];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x_env_mac(e, a * 4 + c, tv, y[c]);
+          }
+        }
+      } else {
+        const int bit = n - 1 - site, d = 1 << bit;
+        for (int r = tid; r < (N >> 1); r += BLOCK_THREADS) {
+          const int i0 = (int)pair_base(r, bit);
+          const xc y0 = psi[i0], y1 = psi[i0 + d], t0 = tt[i0], t1 = tt[i0 + d];
+          x_env_mac(e, 0, t0, y0);
+          x_env_mac(e, 1, t0, y1);
+          x_env_mac(e, 2, t1, y0);
+          x_env_mac(e, 3, t1, y1);
+        }
+      }
+      wred[warp][lane] = warp_sum32_df(e);
+      if (fetch) {
+        gd[buf ^ 1][tid] = pre;
+        gs[buf ^ 1][(tid % (1 << k2)) * (1 << k2) + tid / (1 << k2)] = xc_from_d(cconj(pre));
+      }
+      __syncthreads();
+      if (warp == 0) {
+        reinterpret_cast<double*>(env)[lane] = x_sum_warps(wred, lane);
+        __syncwarp();
+        bool finite;
+        double2* g = gd[buf];
+        const double nn = warp_polar_exact(wp, env, g, m, &finite);
+        if (finite) nuc = nn;
+        if (finite && lane < m * m) gb[(int64_t)slot * 16 + lane] = g[lane];
+        if (!finite && lane == 0) atomicOr(bd.err, KERR_NONFINITE);
+        if (lane < m * m) gt[(lane % m) * m + lane / m] = xc_from_d(cconj(g[lane]));
+      } else if (j2 < G) {
+        x_fused_apply(psi, n, site2, k2, gs[buf ^ 1], tid - 32, BLOCK_THREADS - 32);
+      }
+      __syncthreads();
+      if (j2 < G) x_fused_apply(tt, n, site, k, gt, tid, BLOCK_THREADS);   // t <- G_new^H t
+      j = j2;
+      slot = slot2;
+      site = site2;
+      k = k2;
+    }
+    if (tid == 0) {
+      const double f = nuc / sqrt(tnorm2[b].x);
       sweep_fid[(int64_t)b * num_sweeps + sw] = f;
       sweeps_done[b] = sw + 1;
       if (stop_fid > 0.0 && f >= stop_fid) active[b] = 0;

@@ -1,4 +1,5 @@
-// Unitary polar factor of a 4 x 4 (or 2 x 2) environment by one warp.
+// Unitary polar factor of a 4 x 4 (or 2 x 2) environment by one warp:
+// warp_polar for the fast mode, warp_polar_exact for the exact mode.
 //
 // The same definition as polar_sweep in small_linalg.h: W maximises
 // Re Tr(W^H E), singular values up to QM_POLAR_NULL_TOL of the largest
@@ -21,16 +22,22 @@
 // single-thread factor kept the FP32 error itself.  A null space on which
 // the current gate has no component either (rare) takes the single-thread
 // code.
+// The exact mode's factor (the definition of polar_jacobi_pre) starts the
+// same way, then finishes with Hestenes sweeps on FP64 columns.  Their
+// rotations take the angle from FP32 (FP64 square roots and divisions are
+// chains of about ten dependent operations each) as a complex tangent w, and
+// only c = 1 / sqrt(1 + |w|^2) in FP64, so every rotation is unitary to FP64
+// rounding and an inexact angle costs at most one more sweep.
 // Measured on a 10-qubit state (15 layers, one block): 48.5 us per sweep
 // step with the single-thread factor, 11.2 us with this one.
 #pragma once
 
-#include "device_common.cuh"
+#include "dfloat.cuh"
 
 struct WarpPolar {
   double2 E[16];          // the environment, scaled by a power of two, padded to 4 x 4
   double2 Wp[16];         // the current gate's conjugate, padded with the identity
-  double2 V[16], U[16], T[16];
+  double2 V[16], U[16], T[16], C[16];
   float sig[4], rsig[4];  // column norms of E V and their reciprocals; 0 for null columns
   int null_mask;
 };
@@ -296,6 +303,196 @@ static __device__ __noinline__ double warp_polar(WarpPolar& ws, const double2* e
   }
   __syncwarp();
   return tr;
+}
+
+__device__ __forceinline__ double quad_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v;
+}
+
+__device__ __forceinline__ double2 shfl_xor2(double2 v, int o) {
+  return cd(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+
+// 1 / sqrt(x) in FP64 for x in FP32's normal range: an FP32 seed and one
+// third-order step (relative error about 1e-20 before rounding).
+__device__ __forceinline__ double wp_rsqrt(double x) {
+  const double r = (double)rsqrtf((float)x), h = fma(-x * r, r, 1.0);
+  return fma(r * h, fma(0.375, h, 0.5), r);
+}
+
+#define WPX_TINY 1e-36f   // column norms^2 (of entries at most 1) below this are zero
+
+// Hestenes sweeps on FP64 columns: lane bits 0-1 row, 2 pair, 3 matrix (A or
+// V); the upper half warp repeats the lower one.  A pair rotates while the
+// cosine of its columns is above 1e-15 (as jacobi_pair).
+__device__ __forceinline__ void wx_sweeps(double2& xp, double2& xq, int& fp, int& fq, bool masked) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = (lane & 4) != 0;
+  for (int sweep = 0; sweep < 60; ++sweep) {
+    bool rot = false;
+#pragma unroll
+    for (int rd = 0; rd < 3; ++rd) {
+      const double al = quad_sum(fma(xp.x, xp.x, xp.y * xp.y)), be = quad_sum(fma(xq.x, xq.x, xq.y * xq.y));
+      const double gx = quad_sum(fma(xp.x, xq.x, xp.y * xq.y)), gy = quad_sum(fma(xp.x, xq.y, -xp.y * xq.x));
+      const float fa = (float)al, fb = (float)be;
+      const bool live = fa > WPX_TINY && fb > WPX_TINY && (!masked || (fp && fq));
+      const float rr = rsqrtf(live ? fa : 1.f) * rsqrtf(live ? fb : 1.f);
+      const float cx = (float)gx * rr, cy = (float)gy * rr, c2 = fmaf(cx, cx, cy * cy);
+      const bool go = live && c2 > 1e-30f && !(lane & 8);
+      const float ri = rsqrtf(go ? c2 : 1.f);
+      const float zeta = 0.5f * (float)(be - al) * rr * ri, az = fabsf(zeta);
+      const float s1 = fmaf(az, az, 1.f);
+      float t = az > 1e4f ? __fdividef(0.5f, az) : __fdividef(1.f, az + s1 * rsqrtf(s1));
+      t = go ? copysignf(t, zeta) * ri : 0.f;
+      // the columns of V follow those of A
+      const double wx = (double)__shfl_sync(0xffffffffu, cx * t, lane & 7);
+      const double wy = (double)__shfl_sync(0xffffffffu, cy * t, lane & 7);
+      rot |= go && t != 0.f;
+      if (__any_sync(0xffffffffu, go)) {
+        const double c = wp_rsqrt(fma(wx, wx, fma(wy, wy, 1.0))), sx = c * wx, sy = c * wy;
+        const double2 np = cd(fma(c, xp.x, -fma(sx, xq.x, sy * xq.y)), fma(c, xp.y, -fma(sx, xq.y, -sy * xq.x)));
+        const double2 nq = cd(fma(c, xq.x, fma(sx, xp.x, -sy * xp.y)), fma(c, xq.y, fma(sx, xp.y, sy * xp.x)));
+        xp = np;
+        xq = nq;
+      }
+      const bool give_p = rd != 1 && hi;   // next pairing, as in wh_sweeps
+      const double2 o = shfl_xor2(give_p ? xp : xq, 4);
+      const int fo = masked ? __shfl_xor_sync(0xffffffffu, give_p ? fp : fq, 4) : 0;
+      if (give_p) {
+        xp = o;
+        fp = fo;
+      } else {
+        xq = o;
+        fq = fo;
+      }
+    }
+    if (!__any_sync(0xffffffffu, rot)) break;
+  }
+}
+
+static __device__ __noinline__ double wp_single_thread_exact(const WarpPolar& ws, double2* gate, int m) {
+  double2 e[16], w[16], wprev[16];
+  for (int i = 0; i < m * m; ++i) {
+    e[i] = ws.E[(i / m) * 4 + i % m];
+    wprev[i] = ws.Wp[(i / m) * 4 + i % m];
+  }
+  const double nn = polar_jacobi_pre(e, m, w, wprev);
+  for (int i = 0; i < m * m; ++i) gate[i] = cconj(w[i]);
+  return nn;
+}
+
+// As warp_polar, to FP64 accuracy; returns the nuclear norm of env.
+static __device__ __noinline__ double warp_polar_exact(WarpPolar& ws, const double2* env, double2* gate, int m,
+                                                       bool* finite) {
+  const int lane = threadIdx.x & 31;
+  const int ex = wp_load(ws, env, gate, m, lane, finite);
+  if (!*finite) return 0.0;
+  const double unscale = __hiloint2double((1023 + ex) << 20, 0);
+  const int row = lane & 3, pr = (lane >> 2) & 1, ip = row * 4 + 2 * pr, iq = ip + 1;
+  const int ent = lane >> 1, i = ent >> 2, j = ent & 3, part = lane & 1;
+  const double eye = i == j && part == 0 ? 1.0 : 0.0;
+  int fp = 0, fq = 0;
+  {
+    float2 ap = cf((float)ws.E[ip].x, (float)ws.E[ip].y), aq = cf((float)ws.E[iq].x, (float)ws.E[iq].y);
+    float2 vp = cf(row == 2 * pr ? 1.f : 0.f, 0.f), vq = cf(row == 2 * pr + 1 ? 1.f : 0.f, 0.f);
+    wh_sweeps(ap, aq, vp, vq, fp, fq, false);
+    if (lane < 8) {
+      ws.V[ip] = f2d(vp);
+      ws.V[iq] = f2d(vq);
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int step = 0; step < 2; ++step) {   // V <- V (3I - V^H V) / 2: 1e-6, 1e-12, rounding
+    double v = wmm_part<true, false>(ws.V, ws.V, i, j, part);
+    wmm_store(ws.T, lane, 1.5 * eye - 0.5 * v);
+    __syncwarp();
+    v = wmm_part<false, false>(ws.V, ws.T, i, j, part);
+    __syncwarp();
+    wmm_store(ws.V, lane, v);
+    __syncwarp();
+  }
+  wmm_store(ws.U, lane, wmm_part<false, false>(ws.E, ws.V, i, j, part));
+  __syncwarp();
+  double2* mine = (lane & 8) ? ws.V : ws.U;
+  double2 xp = mine[ip], xq = mine[iq];
+  wx_sweeps(xp, xq, fp, fq, false);
+  // norms of A's columns, in every lane of their pair
+  double al = quad_sum(cnorm2(xp)), be = quad_sum(cnorm2(xq));
+  al = __shfl_sync(0xffffffffu, al, lane & 7);
+  be = __shfl_sync(0xffffffffu, be, lane & 7);
+  double m2 = fmax(al, be);
+  m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, 4));
+  const double thr = fmax(QM_POLAR_NULL_TOL * QM_POLAR_NULL_TOL * m2, (double)WPX_TINY);
+  fp = !(al > thr);
+  fq = !(be > thr);
+  const double ra = wp_rsqrt(al > WPX_TINY ? al : 1.0), rb = wp_rsqrt(be > WPX_TINY ? be : 1.0);
+  double nuc = (al > WPX_TINY ? al * ra : 0.0) + (be > WPX_TINY ? be * rb : 0.0);
+  nuc += __shfl_xor_sync(0xffffffffu, nuc, 4);
+  if (m == 2) nuc -= 2.0 * ws.E[10].x;   // the padding's two singular values
+  const bool any_null = __any_sync(0xffffffffu, fp || fq);
+  if (lane < 16) {
+    const bool a = lane < 8;
+    mine[ip] = a ? (fp ? czero() : cscale(xp, ra)) : xp;
+    mine[iq] = a ? (fq ? czero() : cscale(xq, rb)) : xq;
+  }
+  __syncwarp();
+  if (any_null) {
+    // null columns of U: X = (I - U_s U_s^H) Wp V_N rotated to orthogonal columns
+    wmm_store(ws.T, lane, wmm_part<false, false>(ws.Wp, ws.V, i, j, part));
+    __syncwarp();
+    wmm_store(ws.C, lane, wmm_part<true, false>(ws.U, ws.T, i, j, part));
+    __syncwarp();
+    const double x = reinterpret_cast<double*>(ws.T)[lane] - wmm_part<false, false>(ws.U, ws.C, i, j, part);
+    __syncwarp();
+    wmm_store(ws.T, lane, x);
+    __syncwarp();
+    if (!(lane & 8)) {
+      xp = fp ? ws.T[ip] : ws.U[ip];
+      xq = fq ? ws.T[iq] : ws.U[iq];
+    }
+    wx_sweeps(xp, xq, fp, fq, true);
+    al = quad_sum(cnorm2(xp));
+    be = quad_sum(cnorm2(xq));
+    if (!__all_sync(0xffffffffu, (lane & 8) || ((!fp || al > 1e-16) && (!fq || be > 1e-16)))) {
+      const double nn = lane == 0 ? wp_single_thread_exact(ws, gate, m) : 0.0;
+      __syncwarp();
+      return __shfl_sync(0xffffffffu, nn, 0) * unscale;
+    }
+    if (lane < 16) {
+      const bool a = lane < 8;
+      mine[ip] = a && fp ? cscale(xp, wp_rsqrt(al)) : xp;
+      mine[iq] = a && fq ? cscale(xq, wp_rsqrt(be)) : xq;
+    }
+    __syncwarp();
+  }
+  const double v = wmm_part<false, true>(ws.U, ws.V, i, j, part);
+  if (i < m && j < m) reinterpret_cast<double*>(gate)[2 * (i * m + j) + part] = part ? -v : v;
+  __syncwarp();
+  return nuc * unscale;
+}
+
+// Sum of 32 double-float values per lane over the warp: lane l returns the
+// total of value l (exchange as warp_sum32).
+__device__ __forceinline__ double warp_sum32_df(DF (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const DF give = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      const float gh = __shfl_xor_sync(0xffffffffu, give.hi, o), gl = __shfl_xor_sync(0xffffffffu, give.lo, o);
+      const float t = __fadd_rn(keep.hi, gh);
+      const float bv = __fsub_rn(t, keep.hi);
+      const float err = __fadd_rn(__fsub_rn(keep.hi, __fsub_rn(t, bv)), __fsub_rn(gh, bv));
+      v[i].hi = t;
+      v[i].lo = __fadd_rn(__fadd_rn(keep.lo, gl), err);
+    }
+  }
+  return (double)v[0].hi + (double)v[0].lo;
 }
 
 // Sum of 32 values per lane over the warp: lane l returns the total of

@@ -6,7 +6,9 @@ Bounds: in the fast mode an amplitude passes each of the G gates at most
 three times (rebuild, peel, target) at a relative rounding of at most 2^-22
 (complex FP32 products; the split-FP16 products of states above 13 qubits
 2^-20 with their accumulation), so a sweep's fidelity is within 3 G times
-that of the oracle's; the new gates are unitary to FP64 rounding.
+that of the oracle's; the new gates are unitary to FP64 rounding.  The exact
+mode's double-float products round at 2^-44 and its gates are compared too,
+where no choice of a null direction is left to rounding.
 """
 
 import copy
@@ -57,16 +59,18 @@ def _target(rng, n, kind):
 
 @pytest.mark.parametrize("kind", ["random", "product", "zero"])
 @pytest.mark.parametrize("ns", [[2], [3, 2, 4], [5, 13], [4, 14]])
-def test_sweep_gates_and_fidelity(eng, ns, kind):
+@pytest.mark.parametrize("precision", ["fast", "exact"])
+def test_sweep_gates_and_fidelity(eng, ns, kind, precision):
     L = 2
+    exact = precision == "exact"
     rng = np.random.default_rng(100 + sum(ns))
-    p = eng.plan(ns, L, 4)
+    p = eng.plan(ns, L, 4, precision)
     store = np.zeros(p.gate_elems, complex)
     arity = np.zeros(p.gate_elems // 16, np.int8)
     layers, targets = [], []
     for b, n in enumerate(ns):
         layers.append(_layers(rng, n, L, kind))
-        targets.append(_target(rng, n, kind).astype(np.complex64))
+        targets.append(_target(rng, n, kind).astype(p.npdtype))
         for l, layer in enumerate(reversed(layers[b])):
             for s, g in enumerate(layer[0][2]):
                 off = int(p.gate_off[b]) + (l * n + s) * 16
@@ -75,16 +79,19 @@ def test_sweep_gates_and_fidelity(eng, ns, kind):
     gates = torch.from_numpy(store.view(np.float64)).cuda()
     ar = torch.from_numpy(arity).cuda()
     nl = torch.full((len(ns),), L, dtype=torch.int32, device="cuda")
-    t = torch.from_numpy(np.concatenate(targets).view(np.float32)).cuda()
+    t = torch.from_numpy(np.concatenate(targets).view(np.float64 if exact else np.float32)).cuda()
     sf, sd = eng.stage_sweeps(p, t, gates, ar, nl, 1)
     got = gates.cpu().numpy().view(np.complex128)
     assert np.all(sd.cpu().numpy() == 1)
     for b, n in enumerate(ns):
-        _, f = D.sweep(targets[b].astype(np.complex128), n, copy.deepcopy(layers[b]))
-        eps = 2.0 ** -20 if max(ns) > 13 else 2.0 ** -22
+        ref, f = D.sweep(targets[b].astype(np.complex128), n, copy.deepcopy(layers[b]))
+        eps = 2.0 ** -44 if exact else 2.0 ** -20 if max(ns) > 13 else 2.0 ** -22
         assert abs(float(sf[b].cpu()) - f) <= 3 * n * L * eps, (n, kind)
         for i in range(L * n):
             m = 2 if (i + 1) % n == 0 else 4
             off = int(p.gate_off[b]) + i * 16
             u = got[off: off + m * m].reshape(m, m)
             assert np.max(np.abs(u @ u.conj().T - np.eye(m))) < 1e-13
+            if exact and kind == "random":
+                want = ref[L - 1 - i // n][0][2][i % n]
+                assert np.max(np.abs(u - want)) < 1e-8
