@@ -35,6 +35,9 @@ struct qmprs_plan {
       *d_state_ntiles = nullptr, *d_ticket = nullptr, *d_err = nullptr;
   int64_t *d_vec_off = nullptr, *d_gate_off = nullptr, *d_tensor_off = nullptr;
   int* d_bond_init = nullptr;
+  // layer stage: row units of every state, and how many of them (a prefix) each step needs
+  int *d_cut_state = nullptr, *d_cut_idx = nullptr;
+  std::vector<int> cut_count;
   // scratch
   float2 *S0 = nullptr, *S1 = nullptr, *S2 = nullptr;
   double2* partials = nullptr;
@@ -483,10 +486,8 @@ int exact_unitary_layers(qmprs_plan* p, const double2* target, int num_layers, d
     for (int l = 0; l < num_layers; ++l) {
       CK(cudaMemcpyAsync(p->bonds, p->d_bond_init, sizeof(int) * nb, cudaMemcpyDeviceToDevice, s2));
       for (int j = 0; j + 2 <= p->max_n; ++j) {
-        const xc* src = j == 0 ? work : buf[(j - 1) & 1];
-        launch_x_layer_gram(p->bd, j, work, src, p->bonds, p->partials, p->active, s2);
-        launch_layer_eig(p->bd, j, p->partials, p->vsel, p->bonds, p->site_t, p->active, s2);
-        launch_x_layer_project(p->bd, j, work, src, buf[j & 1], p->bonds, p->vsel, p->active, s2);
+        launch_x_layer_cut(p->bd, p->cut_count[j], j, work, buf[0], buf[1], p->bonds, p->vsel, p->site_t,
+                           p->partials, p->active, s2);
       }
       launch_x_layer_build(p->bd, l, buf[0], buf[1], p->bonds, p->site_t, gates, ar, p->active, s2);
       for (int st = 0; st < p->max_n; ++st) {
@@ -628,7 +629,7 @@ void qmprs_plan_destroy(qmprs_plan_t p) {
   if (p->cap) cudaStreamDestroy(p->cap);
   void* ptrs[] = {p->d_n,      p->d_tile_state, p->d_tile_idx, p->d_state_tile0, p->d_state_ntiles,
                   p->d_ticket, p->d_err,        p->d_vec_off,  p->d_gate_off,    p->d_tensor_off,
-                  p->d_bond_init, p->S0,        p->S1,         p->S2,            p->partials,
+                  p->d_bond_init, p->d_cut_state, p->d_cut_idx, p->S0, p->S1,         p->S2,            p->partials,
                   p->tt_partials, p->gram,      p->vsel,       p->vsel2,         p->site_t, p->vwork,
                   p->bonds,    p->active,       p->nlayers,    p->num_active,    p->nuc,
                   p->sq,       p->tnorm,        p->d_chunk_state, p->d_chunk_idx, p->d_state_chunk0,
@@ -705,6 +706,28 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
     }
   }
   p->nchunks = (int)chunk_state.size();
+  // layer stage: units of 2^CUT_ROW_BITS rows; unit i > 0 of a state is needed
+  // while its remainder has more than i units, unit 0 at every cut
+  struct Unit {
+    int state, idx, last;
+  };
+  std::vector<Unit> units;
+  for (int b = 0; b < num_states; ++b) {
+    const int n = p->n[b], rows = n - 1 - CUT_ROW_BITS;
+    units.push_back({b, 0, n - 2});
+    for (int i = 1, lg = 0; rows > 0 && i < (1 << rows); ++i) {
+      if (i >= (2 << lg)) ++lg;
+      units.push_back({b, i, rows - 1 - lg});
+    }
+  }
+  std::stable_sort(units.begin(), units.end(), [](const Unit& x, const Unit& y) { return x.last > y.last; });
+  p->cut_count.assign(p->max_n, 0);
+  std::vector<int> cut_state, cut_idx;
+  for (const Unit& u : units) {
+    cut_state.push_back(u.state);
+    cut_idx.push_back(u.idx);
+    for (int j = 0; j <= u.last; ++j) ++p->cut_count[j];
+  }
   std::vector<int> bond_init((size_t)num_states * (p->max_n + 1), 0);
   for (int b = 0; b < num_states; ++b) {
     bond_init[(size_t)b * (p->max_n + 1)] = 1;
@@ -731,6 +754,10 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   PC(dalloc(&p->d_ticket, B));
   PC(dalloc(&p->d_err, 1));
   PC(dalloc(&p->d_bond_init, (int64_t)bond_init.size()));
+  PC(dalloc(&p->d_cut_state, (int64_t)cut_state.size()));
+  PC(dalloc(&p->d_cut_idx, (int64_t)cut_idx.size()));
+  PC(cudaMemcpy(p->d_cut_state, cut_state.data(), sizeof(int) * cut_state.size(), cudaMemcpyHostToDevice));
+  PC(cudaMemcpy(p->d_cut_idx, cut_idx.data(), sizeof(int) * cut_idx.size(), cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_n, p->n.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_vec_off, p->vec_off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_gate_off, p->gate_off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice));
@@ -802,6 +829,8 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   bd.err = p->d_err;
   bd.tt_w = p->tt_w;
   bd.tt_b = p->tt_b;
+  bd.cut_state = p->d_cut_state;
+  bd.cut_idx = p->d_cut_idx;
   bd.eig_wmax = num_states <= BJ_SMALL_BATCH ? TT_MAXB : TT_MAXW;
   *out = p;
   return QMPRS_OK;
@@ -1045,10 +1074,8 @@ int qmprs_unitary_layers(qmprs_plan_t p, const void* target_, int num_layers, do
     for (int l = 0; l < num_layers; ++l) {
       CK(cudaMemcpyAsync(p->bonds, p->d_bond_init, sizeof(int) * nb, cudaMemcpyDeviceToDevice, st));
       for (int j = 0; j + 2 <= p->max_n; ++j) {
-        const float2* src = j == 0 ? work : buf[(j - 1) & 1];
-        launch_layer_gram(p->bd, j, work, src, p->bonds, p->partials, p->vsel, p->bonds, p->site_t, p->active,
-                          st);
-        launch_layer_project(p->bd, j, work, src, buf[j & 1], p->bonds, p->vsel, p->active, st);
+        launch_layer_cut(p->bd, p->cut_count[j], j, work, buf[0], buf[1], p->bonds, p->vsel, p->site_t, p->partials,
+                         p->active, st);
       }
       launch_layer_build(p->bd, l, buf[0], buf[1], p->bonds, p->site_t, gates, ar, p->active, st);
       // inverse of the new layer: tile passes of two 4-qubit windows (up to

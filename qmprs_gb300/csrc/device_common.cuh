@@ -48,41 +48,6 @@ __device__ __forceinline__ void block_sum(double (&vals)[K]) {
 #define WARPS WARPS_PER_BLOCK
 static_assert(WARPS_PER_BLOCK * 32 == BLOCK_THREADS, "per-warp partials assume BLOCK_THREADS / 32 warps");
 
-// Per-warp partial of 16 complex fp32 accumulators: promoted to fp64 and
-// summed over the warp with a fixed butterfly; lane i < 16 writes entry i.
-__device__ __forceinline__ void warp_partial16(const float2 (&e)[16], double2* out) {
-  const int lane = threadIdx.x & 31;
-  double2 mine = czero();
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    double re = (double)e[i].x, im = (double)e[i].y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      re += __shfl_xor_sync(0xffffffffu, re, o);
-      im += __shfl_xor_sync(0xffffffffu, im, o);
-    }
-    if (lane == i) mine = cd(re, im);
-  }
-  if (lane < 16) out[lane] = mine;
-}
-
-// Same for 16 complex fp64 accumulators held as 32 doubles.
-__device__ __forceinline__ void warp_partial16_f64(const double (&acc)[32], double2* out) {
-  const int lane = threadIdx.x & 31;
-  double2 mine = czero();
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    double re = acc[2 * i], im = acc[2 * i + 1];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      re += __shfl_xor_sync(0xffffffffu, re, o);
-      im += __shfl_xor_sync(0xffffffffu, im, o);
-    }
-    if (lane == i) mine = cd(re, im);
-  }
-  if (lane < 16) out[lane] = mine;
-}
-
 // Thread 0 publishes its partial (already written) and takes a ticket.
 // Returns true in every thread of the block that finishes state b last.
 __device__ __forceinline__ bool last_tile_ticket(int* ticket, int b, int nt) {
@@ -99,15 +64,6 @@ __device__ __forceinline__ bool last_tile_ticket(int* ticket, int b, int nt) {
 }
 
 __device__ __forceinline__ double2 ld_cg(const double2* p) { return __ldcg(p); }
-
-// Tiles of a state that take part in the layer stage's Gram of a 2^c-row
-// remainder: at least 4096 rows (16 per thread) each, so a short remainder
-// is not spread over every tile of the state, each paying a full fp64 warp
-// reduction.  The eigen kernel sums the partials of exactly these tiles.
-__device__ __forceinline__ int layer_gram_tiles(int c, int nt) {
-  const int64_t want = ((((int64_t)1) << c) + 4095) >> 12;
-  return want < nt ? (int)want : nt;
-}
 
 // Index of amplitude for quad r on bits (hi, lo = hi - 1), with values (bh, bl).
 __device__ __forceinline__ int64_t quad_base(int64_t r, int lo) {

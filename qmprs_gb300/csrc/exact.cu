@@ -30,9 +30,9 @@
 //   k_x_gemm                  C = A B, A double-float, B complex128 (the
 //                             projection M V and the target contraction)
 //   k_x_site0                 site 0 from the last remainder
-//   k_x_layer_gram / _project / _build / _fidelity   the layer stage's
-//                             bond-2 cuts (the FP64 eigen kernel is shared
-//                             with the fast mode)
+//   k_layer_cut, k_layer_build, k_x_layer_fidelity   the layer stage's
+//                             bond-2 cuts (layer_cut.cuh, shared with the
+//                             fast mode)
 //   k_x_apply_gate            one gate per state
 //   k_x_sweep_step            a backward sweep step: peel the step's gate
 //                             from the circuit state, reduce the gate's
@@ -41,7 +41,7 @@
 //                             environment's polar factor (one warp,
 //                             warp_polar.cuh)
 #include "dfloat.cuh"
-#include "warp_polar.cuh"
+#include "layer_cut.cuh"
 
 static int grid_for(const BatchDev& bd) {
   const int cap = 152 * 8;
@@ -305,158 +305,7 @@ __global__ void k_x_from_d_flat(const double2* src, xc* dst, int64_t count) {
 
 // ---- (b) layer stage -----------------------------------------------------------------
 
-// Gram rows of width W (2 or 4) of the remainder: upper triangle in
-// double-float, flushed to fp64 every TT_FLUSH rows, mirrored into the
-// 4 x 4 layout of the fast mode's partials (entry a * 4 + e).
-template <int W>
-__device__ __forceinline__ void x_gram_rows(const xc* m, int64_t lo, int64_t hi, double (&acc)[32]) {
-  constexpr int NE = W * (W + 1) / 2;
-  int64_t row = lo + threadIdx.x;
-  while (row < hi) {
-    XA s[NE];
-#pragma unroll
-    for (int k = 0; k < NE; ++k) s[k] = xa_zero();
-    for (int f = 0; f < TT_FLUSH && row < hi; ++f, row += blockDim.x) {
-      xc x[W];
-#pragma unroll
-      for (int a = 0; a < W; ++a) x[a] = m[row * W + a];
-      int k = 0;
-#pragma unroll
-      for (int a = 0; a < W; ++a)
-#pragma unroll
-        for (int e = a; e < W; ++e, ++k) xa_macc(s[k], x[a], x[e]);
-    }
-    int k = 0;
-#pragma unroll
-    for (int a = 0; a < W; ++a)
-#pragma unroll
-      for (int e = a; e < W; ++e, ++k) {
-        const double2 v = xa_to_d(s[k]);
-        acc[2 * (a * 4 + e)] += v.x;
-        acc[2 * (a * 4 + e) + 1] += v.y;
-        if (e != a) {
-          acc[2 * (e * 4 + a)] += v.x;
-          acc[2 * (e * 4 + a) + 1] -= v.y;
-        }
-      }
-  }
-}
-
-// Same tiles and partial layout as the fast mode's k_layer_gram, so the
-// shared FP64 eigen kernel (k_layer_eig) reads them unchanged.
-__global__ void __launch_bounds__(BLOCK_THREADS) k_x_layer_gram(BatchDev bd, int step, const xc* work, const xc* src,
-                                                                const int* bonds, double2* partials,
-                                                                const int* active) {
-  for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
-    const int b = bd.tile_state[tile];
-    const int n = bd.n[b];
-    const int c = n - 1 - step;
-    if (c < 1 || (active && !active[b])) continue;
-    const int* bond = bonds + (int64_t)b * (bd.max_n + 1);
-    const int r = bond[c + 1];
-    if (r != 1 && r != 2) continue;
-    const xc* m = (step == 0 ? work : src) + bd.vec_off[b];
-    const int vnt = layer_gram_tiles(c, bd.state_ntiles[b]);
-    if (bd.tile_idx[tile] >= vnt) continue;
-    int64_t lo, hi;
-    tile_range(ipow2(c), bd.tile_idx[tile], vnt, &lo, &hi);
-    double acc[32];
-#pragma unroll
-    for (int e = 0; e < 32; ++e) acc[e] = 0.0;
-    if (r == 1) x_gram_rows<2>(m, lo, hi, acc);
-    else x_gram_rows<4>(m, lo, hi, acc);
-    warp_partial16_f64(acc, partials + ((int64_t)tile * WARPS + (threadIdx.x >> 5)) * 16);
-  }
-}
-
-template <int W, int K>
-__device__ __forceinline__ void x_project_rows(const xc* m, xc* o, const xc (&vm)[16], int64_t lo, int64_t hi) {
-  for (int64_t row = lo + threadIdx.x; row < hi; row += blockDim.x) {
-    xc x[W];
-#pragma unroll
-    for (int a = 0; a < W; ++a) x[a] = m[row * W + a];
-#pragma unroll
-    for (int col = 0; col < K; ++col) {
-      XA s = xa_zero();
-#pragma unroll
-      for (int a = 0; a < W; ++a) xa_mac(s, vm[a * 4 + col], x[a]);
-      o[row * K + col] = xa_round(s);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(BLOCK_THREADS) k_x_layer_project(BatchDev bd, int step, const xc* work,
-                                                                   const xc* src, xc* dst, const int* bonds,
-                                                                   const double2* vsel, const int* active) {
-  for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
-    const int b = bd.tile_state[tile];
-    const int n = bd.n[b];
-    const int c = n - 1 - step;
-    if (c < 1 || (active && !active[b])) continue;
-    const int* bond = bonds + (int64_t)b * (bd.max_n + 1);
-    const int r = bond[c + 1];
-    const int keep = bond[c];
-    if ((r != 1 && r != 2) || (keep != 1 && keep != 2)) continue;
-    xc vm[16];
-    const double2* vs = vsel + (int64_t)b * 16;
-#pragma unroll
-    for (int a = 0; a < 16; ++a) vm[a] = xc_from_d(vs[a]);
-    const xc* m = (step == 0 ? work : src) + bd.vec_off[b];
-    xc* o = dst + bd.vec_off[b];
-    int64_t lo, hi;
-    tile_range(ipow2(c), bd.tile_idx[tile], bd.state_ntiles[b], &lo, &hi);
-    if (r == 1) {
-      if (keep == 1) x_project_rows<2, 1>(m, o, vm, lo, hi);
-      else x_project_rows<2, 2>(m, o, vm, lo, hi);
-    } else {
-      if (keep == 1) x_project_rows<4, 1>(m, o, vm, lo, hi);
-      else x_project_rows<4, 2>(m, o, vm, lo, hi);
-    }
-  }
-}
-
-// One thread per state: site 0 from the last remainder, then the n gates
-// (Ran's completion in closed form, as the fast mode's k_layer_build).
-__global__ void k_x_layer_build(BatchDev bd, int layer, const xc* rem0, const xc* rem1, const int* bonds,
-                                double2* site_t, double2* gates, signed char* arity, const int* active) {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < bd.B; b += gridDim.x * blockDim.x) {
-    if (active && !active[b]) continue;
-    const int n = bd.n[b];
-    const int* bond = bonds + (int64_t)b * (bd.max_n + 1);
-    const xc* rem = (((n - 2) & 1) ? rem1 : rem0) + bd.vec_off[b];
-    const int r1 = bond[1];
-    double2* st = site_t + (int64_t)b * bd.max_n * 8;
-    double nrm = 0.0;
-    for (int i = 0; i < 2 * r1; ++i) nrm += cnorm2(xc_to_d(rem[i]));
-    nrm = sqrt(nrm);
-    for (int i = 0; i < 2 * r1; ++i) st[i] = cscale(xc_to_d(rem[i]), nrm > 0.0 ? 1.0 / nrm : 0.0);
-    double worst = 0.0;
-    for (int s = 0; s < n; ++s) {
-      const double2* d = st + s * 8;
-      const bool is_end = (s == n - 1) || bond[s + 1] == 1;
-      const bool is_start = (s == 0) || bond[s] == 1;
-      double2 g[16];
-      for (int i = 0; i < 16; ++i) g[i] = czero();
-      int k;
-      if (is_end) {
-        k = 1;
-        if (is_start) ran_gate_single(d, g);
-        else ran_gate_last(d, g);
-      } else {
-        k = 2;
-        if (is_start) ran_gate_first(d, g);
-        else ran_gate_middle(d, g);
-      }
-      const double err = unitarity_error(g, 1 << k);
-      if (!(err <= worst)) worst = err;
-      const int64_t slot = (int64_t)layer * n + s;
-      double2* out = gates + bd.gate_off[b] + slot * 16;
-      for (int i = 0; i < 16; ++i) out[i] = g[i];
-      arity[bd.gate_off[b] / 16 + slot] = (signed char)k;
-    }
-    if (!(worst <= 1e-6)) atomicOr(bd.err, KERR_NONUNITARY);
-  }
-}
+// The cuts and the gates are layer_cut.cuh's kernels on double-float rows.
 
 __global__ void k_x_layer_fidelity(BatchDev bd, int layer, const xc* work, int num_layers, double atol,
                                    double2* layer_fid, int* nlayers, int* active) {
@@ -943,22 +792,19 @@ void launch_x_from_d_flat(const double2* src, xc* dst, int64_t count, cudaStream
   k_x_from_d_flat<<<blocks, 256, 0, s>>>(src, dst, count);
 }
 
-void launch_x_layer_gram(const BatchDev& bd, int step, const xc* work, const xc* src, const int* bonds,
-                         double2* partials, const int* active, cudaStream_t s) {
+void launch_x_layer_cut(const BatchDev& bd, int units, int step, const xc* work, xc* buf0, xc* buf1, int* bonds,
+                        double2* vsel, double2* site_t, double2* partials, const int* active, cudaStream_t s) {
+  const xc* prev = (step & 1) ? buf1 : buf0;
+  xc* dst = (step & 1) ? buf0 : buf1;
   qm_note_launch();
-  k_x_layer_gram<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, work, src, bonds, partials, active);
-}
-
-void launch_x_layer_project(const BatchDev& bd, int step, const xc* work, const xc* src, xc* dst, const int* bonds,
-                            const double2* vsel, const int* active, cudaStream_t s) {
-  qm_note_launch();
-  k_x_layer_project<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, work, src, dst, bonds, vsel, active);
+  k_layer_cut<CutExact><<<units, BLOCK_THREADS, 0, s>>>(bd, step, work, prev, dst, bonds, vsel, site_t,
+                                                        reinterpret_cast<double*>(partials), buf0, buf1, active);
 }
 
 void launch_x_layer_build(const BatchDev& bd, int layer, const xc* rem0, const xc* rem1, const int* bonds,
                           double2* site_t, double2* gates, signed char* arity, const int* active, cudaStream_t s) {
   qm_note_launch();
-  k_x_layer_build<<<(bd.B + 127) / 128, 128, 0, s>>>(bd, layer, rem0, rem1, bonds, site_t, gates, arity, active);
+  k_layer_build<CutExact><<<bd.B, BUILD_THREADS, 0, s>>>(bd, layer, rem0, rem1, bonds, site_t, gates, arity, active);
 }
 
 void launch_x_layer_fidelity(const BatchDev& bd, int layer, const xc* work, int num_layers, double atol,

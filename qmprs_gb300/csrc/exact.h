@@ -29,11 +29,9 @@ void launch_x_site0(const xc* rem, int r1, double in_sq, double2* t0, double* f_
 void launch_x_scale_flat(const xc* src, xc* dst, int64_t count, const double* f, cudaStream_t s);
 void launch_x_from_d_flat(const double2* src, xc* dst, int64_t count, cudaStream_t s);
 
-// (b) layer stage (the FP64 eigen kernel is launch_layer_eig)
-void launch_x_layer_gram(const BatchDev& bd, int step, const xc* work, const xc* src, const int* bonds,
-                         double2* partials, const int* active, cudaStream_t s);
-void launch_x_layer_project(const BatchDev& bd, int step, const xc* work, const xc* src, xc* dst, const int* bonds,
-                            const double2* vsel, const int* active, cudaStream_t s);
+// (b) layer stage (as launch_layer_cut)
+void launch_x_layer_cut(const BatchDev& bd, int units, int step, const xc* work, xc* buf0, xc* buf1, int* bonds,
+                        double2* vsel, double2* site_t, double2* partials, const int* active, cudaStream_t s);
 void launch_x_layer_build(const BatchDev& bd, int layer, const xc* rem0, const xc* rem1, const int* bonds,
                           double2* site_t, double2* gates, signed char* arity, const int* active, cudaStream_t s);
 void launch_x_layer_fidelity(const BatchDev& bd, int layer, const xc* work, int num_layers, double atol,

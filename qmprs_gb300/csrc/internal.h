@@ -74,12 +74,17 @@ struct BatchDev {
   int* err;                // [1] error flag bits
   int tt_w;                // stage (a): Gram stride (>= TT_MAXW, 2 x the largest bond)
   int tt_b;                // stage (a): largest bond / selected-column stride (>= TT_MAXB)
+  const int* cut_state;    // layer stage: state and index of each row unit (layer_cut.cuh),
+  const int* cut_idx;      // sorted by the last step that needs it
   int eig_wmax;            // stage (a): widest Gram of the one-block eigensolver; wider ones
                            // take the blocked solver (ttsvd_wide.cu)
 };
 // Batches of at most this many states send Grams wider than 64 to the
 // blocked multi-SM solver: one block per state would leave the GPU idle
 #define BJ_SMALL_BATCH 8
+
+// Rows of a remainder that one block of the layer stage takes (layer_cut.cuh).
+#define CUT_ROW_BITS 12
 
 // Gate selection modes for the per-step gate launches.
 enum {
@@ -146,15 +151,11 @@ void launch_reduce_tiles(const BatchDev& bd, const double2* partials, double2* o
 void launch_copy_normalize(const BatchDev& bd, const float2* src, float2* dst, double2* partials,
                            double2* sq_norms, cudaStream_t s);
 
-// (b) layer generation
-void launch_layer_gram(const BatchDev& bd, int step, const float2* work, const float2* src,
-                       const int* bonds, double2* partials, double2* vsel, int* bonds_out,
-                       double2* site_t, const int* active, cudaStream_t s);
-void launch_layer_eig(const BatchDev& bd, int step, const double2* partials, double2* vsel, int* bonds,
-                      double2* site_t, const int* active, cudaStream_t s);
-void launch_layer_project(const BatchDev& bd, int step, const float2* work, const float2* src,
-                          float2* dst, const int* bonds, const double2* vsel, const int* active,
-                          cudaStream_t s);
+// (b) layer generation: one cut of every state (`units` blocks: the step's
+// prefix of bd.cut_state / cut_idx)
+void launch_layer_cut(const BatchDev& bd, int units, int step, const float2* work, float2* buf0, float2* buf1,
+                      int* bonds, double2* vsel, double2* site_t, double2* partials, const int* active,
+                      cudaStream_t s);
 void launch_layer_build(const BatchDev& bd, int layer, const float2* rem0, const float2* rem1,
                         const int* bonds, double2* site_t, double2* gates, signed char* arity,
                         const int* active, cudaStream_t s);

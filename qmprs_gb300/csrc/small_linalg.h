@@ -100,15 +100,15 @@ QM_HD void herm_eig_jacobi(double2* a, int n, double2* v, double* lam) {
 // `stride` walks a column of a row-major matrix; `used` (may be null) masks
 // indices that are excluded.
 QM_HD int pivot_index(const double2* x, int n, int stride, const int* used) {
-  double m = -1.0;
+  double m2 = -1.0;   // squared magnitudes: no square root per entry
   for (int i = 0; i < n; ++i) {
     if (used && used[i]) continue;
-    double a = cabs_(x[i * stride]);
-    if (a > m) m = a;
+    double a = cnorm2(x[i * stride]);
+    if (a > m2) m2 = a;
   }
   for (int i = 0; i < n; ++i) {
     if (used && used[i]) continue;
-    if (cabs_(x[i * stride]) >= (1.0 - QM_PIVOT_TOL) * m) return i;
+    if (cnorm2(x[i * stride]) >= (1.0 - QM_PIVOT_TOL) * (1.0 - QM_PIVOT_TOL) * m2) return i;
   }
   return 0;
 }

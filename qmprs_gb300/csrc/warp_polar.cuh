@@ -100,11 +100,14 @@ __device__ __forceinline__ void wh_apply(float2& p, float2& q, float c, float sx
 
 // FP32 Hestenes sweeps of the four columns (lane l & 7 = 4 pair + row holds
 // rows of columns p and q of A and V); with `masked` only pairs of flagged
-// columns rotate.  Flags move with their columns.
-__device__ __forceinline__ void wh_sweeps(float2& ap, float2& aq, float2& vp, float2& vq, int& fp, int& fq,
+// columns rotate.  Flags move with their columns.  Returns 1 after an odd
+// number of sweeps, which leaves columns 2 and 3 exchanged.
+__device__ __forceinline__ int wh_sweeps(float2& ap, float2& aq, float2& vp, float2& vq, int& fp, int& fq,
                                           bool masked) {
   const bool hi = (threadIdx.x & 4) != 0;   // the second pair's lanes
+  int odd = 0;
   for (int sweep = 0; sweep < 30; ++sweep) {
+    odd ^= 1;
     bool rot = false;
 #pragma unroll
     for (int rd = 0; rd < 3; ++rd) {
@@ -131,6 +134,7 @@ __device__ __forceinline__ void wh_sweeps(float2& ap, float2& aq, float2& vp, fl
     }
     if (!__any_sync(0xffffffffu, rot)) break;
   }
+  return odd;
 }
 
 // Scale ws.E (m x m, stride m, unscaled in `env`) into the 4 x 4 workspace:
@@ -326,11 +330,14 @@ __device__ __forceinline__ double wp_rsqrt(double x) {
 
 // Hestenes sweeps on FP64 columns: lane bits 0-1 row, 2 pair, 3 matrix (A or
 // V); the upper half warp repeats the lower one.  A pair rotates while the
-// cosine of its columns is above 1e-15 (as jacobi_pair).
-__device__ __forceinline__ void wx_sweeps(double2& xp, double2& xq, int& fp, int& fq, bool masked) {
+// cosine of its columns is above 1e-15 (as jacobi_pair).  Returns 1 after an
+// odd number of sweeps.
+__device__ __forceinline__ int wx_sweeps(double2& xp, double2& xq, int& fp, int& fq, bool masked) {
   const int lane = threadIdx.x & 31;
   const bool hi = (lane & 4) != 0;
+  int odd = 0;
   for (int sweep = 0; sweep < 60; ++sweep) {
+    odd ^= 1;
     bool rot = false;
 #pragma unroll
     for (int rd = 0; rd < 3; ++rd) {
@@ -370,6 +377,7 @@ __device__ __forceinline__ void wx_sweeps(double2& xp, double2& xq, int& fp, int
     }
     if (!__any_sync(0xffffffffu, rot)) break;
   }
+  return odd;
 }
 
 static __device__ __noinline__ double wp_single_thread_exact(const WarpPolar& ws, double2* gate, int m) {
@@ -474,6 +482,16 @@ static __device__ __noinline__ double warp_polar_exact(WarpPolar& ws, const doub
   return nuc * unscale;
 }
 
+// s += the partner lane's `give` (lane ^ o), double-float
+__device__ __forceinline__ void df_shfl_add(DF& s, const DF& give, int o) {
+  const float gh = __shfl_xor_sync(0xffffffffu, give.hi, o), gl = __shfl_xor_sync(0xffffffffu, give.lo, o);
+  const float t = __fadd_rn(s.hi, gh);
+  const float bv = __fsub_rn(t, s.hi);
+  const float err = __fadd_rn(__fsub_rn(s.hi, __fsub_rn(t, bv)), __fsub_rn(gh, bv));
+  s.lo = __fadd_rn(__fadd_rn(s.lo, gl), err);
+  s.hi = t;
+}
+
 // Sum of 32 double-float values per lane over the warp: lane l returns the
 // total of value l (exchange as warp_sum32).
 __device__ __forceinline__ double warp_sum32_df(DF (&v)[32]) {
@@ -483,13 +501,9 @@ __device__ __forceinline__ double warp_sum32_df(DF (&v)[32]) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int i = 0; i < o; ++i) {
-      const DF give = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
-      const float gh = __shfl_xor_sync(0xffffffffu, give.hi, o), gl = __shfl_xor_sync(0xffffffffu, give.lo, o);
-      const float t = __fadd_rn(keep.hi, gh);
-      const float bv = __fsub_rn(t, keep.hi);
-      const float err = __fadd_rn(__fsub_rn(keep.hi, __fsub_rn(t, bv)), __fsub_rn(gh, bv));
-      v[i].hi = t;
-      v[i].lo = __fadd_rn(__fadd_rn(keep.lo, gl), err);
+      const DF give = up ? v[i] : v[i + o];
+      if (up) v[i] = v[i + o];
+      df_shfl_add(v[i], give, o);
     }
   }
   return (double)v[0].hi + (double)v[0].lo;
