@@ -147,7 +147,7 @@ int qmprs_plan_wide_stats(qmprs_plan_t p, int* grams, int* sweeps, int* refine_s
 
 /*
  * Autotuner of the sweep's tile passes (on by default).  The grouped sweep
- * and the circuit rebuild run grid-stride loops over chunks of 32 tiles of
+ * and the circuit rebuild run grid-stride loops over chunks of up to 32 tiles of
  * 2^11 amplitudes; how many blocks take them decides how evenly states of
  * uneven size and group count spread over the 152 SMs.  On a batch whose
  * signature (qubit-count histogram, bond dimension, layer count) the handle

@@ -58,7 +58,9 @@ struct qmprs_plan {
   int tt_w = TT_MAXW, tt_b = TT_MAXB;
   BJScratch bj, bj_sub;   // blocked eigensolver of Grams wider than TT_MAXW, its deflated subproblem
   BJStats bj_stats;
-  double2 *d_old_gates = nullptr, *d_gpartials = nullptr;
+  double2* d_old_gates = nullptr;
+  float4* d_gpartials = nullptr;
+  int chunk_tiles = GCHUNK;
   GroupDev gd;
   // profiling of the sweep kernels (kernel classes: 0 environment stream,
   // 1 target update, 2 circuit rebuild, 3 environment reduce + polar):
@@ -328,6 +330,27 @@ uint64_t plan_signature(const qmprs_plan* p) {
   mix((uint64_t)p->max_layers);
   return h;
 }
+// Tiles per chunk of the grouped sweep's passes: the largest power of two,
+// at most GCHUNK, that leaves the batch 240 chunks.  A chunk's set-up (offset
+// tables, composed gates) costs about one tile and every chunk adds a
+// partial to the polar kernel's sum, so chunks are long where there are
+// enough of them; a batch of few tiles needs all its tiles on different SMs.
+// Measured per pass of the case (tiles 32 / 16 / 8 / 4 / 2 / 1): one 20-qubit
+// state (512 tiles) 29.0 / 18.2 / 13.1 / 10.8 / 10.7 / 12.3 ms, environments
+// of 32 states of 13-16 qubits (480 tiles) 6.9 / 4.2 / 2.8 / 2.2 / 2.0 / 1.9
+// ms, 64 states of 12-20 qubits (6700 tiles) 24.9 / 18.2 / 18.4 / 18.6 / 21.6 /
+// 28.6 ms.
+#define CHUNKS_WANTED 240
+int choose_chunk_tiles(const std::vector<int>& n) {
+  int tiles = GCHUNK;
+  for (; tiles > 1; tiles /= 2) {
+    int64_t chunks = 0;
+    for (int q : n) chunks += q > GT ? (ipow2(q - GT) + tiles - 1) / tiles : 1;
+    if (chunks >= CHUNKS_WANTED) break;
+  }
+  return tiles;
+}
+
 inline uint64_t dbl_key(double v) {
   uint64_t u;
   std::memcpy(&u, &v, sizeof(u));
@@ -692,12 +715,13 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   p->ntiles = (int)tile_state.size();
   for (int b = 0; b < num_states; ++b) p->tt_b = std::max(p->tt_b, chi_eff_host(max_bond, p->n[b]));
   p->tt_w = std::max(TT_MAXW, 2 * p->tt_b);
-  // grouped sweep: tiles of 2^min(n, GT) amplitudes, GCHUNK tiles per chunk
+  // grouped sweep: tiles of 2^min(n, GT) amplitudes, chunk_tiles tiles per chunk
+  p->chunk_tiles = choose_chunk_tiles(p->n);
   std::vector<int> chunk_state, chunk_idx, state_chunk0(num_states), state_nchunks(num_states);
   for (int b = 0; b < num_states; ++b) {
     const int n = p->n[b];
     const int64_t tiles = n > GT ? ipow2(n - GT) : 1;
-    const int nc = (int)((tiles + GCHUNK - 1) / GCHUNK);
+    const int nc = (int)((tiles + p->chunk_tiles - 1) / p->chunk_tiles);
     state_chunk0[b] = (int)chunk_state.size();
     state_nchunks[b] = nc;
     for (int c = 0; c < nc; ++c) {
@@ -797,7 +821,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   PC(cudaMemcpy(p->d_chunk_idx, chunk_idx.data(), sizeof(int) * p->nchunks, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_state_chunk0, state_chunk0.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_state_nchunks, state_nchunks.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
-  PC(cudaMemset(p->d_gpartials, 0, sizeof(double2) * (size_t)p->nchunks * GMM));
+  PC(cudaMemset(p->d_gpartials, 0, sizeof(float4) * (size_t)p->nchunks * GMM));
 #undef PC
   GroupDev& gd = p->gd;
   gd.nchunks = p->nchunks;
@@ -810,6 +834,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   gd.ngroups = p->d_ngroups;
   gd.old_gates = p->d_old_gates;
   gd.partials = p->d_gpartials;
+  gd.chunk_tiles = p->chunk_tiles;
   gd.rgrp = p->d_rgrp;
   gd.grid = 0;
   gd.nrgroups = p->d_nrgroups;

@@ -30,6 +30,15 @@ __device__ __forceinline__ void df_mac(DF& s, float ah, float al, float bh, floa
   s.lo = __fadd_rn(s.lo, __fadd_rn(err, __fmaf_rn(ah, bl, __fmaf_rn(al, bh, pl))));
 }
 
+// s += (h + l)
+__device__ __forceinline__ void df_add(DF& s, float h, float l) {
+  const float t = __fadd_rn(s.hi, h);
+  const float bv = __fsub_rn(t, s.hi);
+  const float err = __fadd_rn(__fsub_rn(s.hi, __fsub_rn(t, bv)), __fsub_rn(h, bv));
+  s.lo = __fadd_rn(__fadd_rn(s.lo, l), err);
+  s.hi = t;
+}
+
 struct XA {
   DF re, im;
 };

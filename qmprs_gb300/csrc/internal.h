@@ -108,12 +108,12 @@ struct GateSel {
 // Grouped backward sweep (sweep_group.cu): a group is a run of consecutive
 // backward steps whose qubits fit a window of GW qubits; one pass over the
 // vectors per group, shared-memory tiles of 2^GT amplitudes, one partial
-// cross matrix per chunk of GCHUNK tiles.
+// cross matrix per chunk of at most GCHUNK tiles.
 #define GW 4
 #define GM (1 << GW)
 #define GMM (GM * GM)
 #define GT 11
-#define GCHUNK 32
+#define GCHUNK 32   // most tiles per chunk
 #define GMAXSTEPS 8
 #define PASS_GRID_DEFAULT (4 * 152)   // resident blocks of the tile passes (4 per SM)
 
@@ -134,7 +134,8 @@ struct GroupDev {
   GroupEnt* grp;             // [B * gmax]
   int* ngroups;              // [B]
   double2* old_gates;        // [B * GMAXSTEPS * 16] gates replaced by the last group
-  double2* partials;         // [nchunks * GMM]
+  float4* partials;          // [nchunks * GMM] double-float
+  int chunk_tiles;           // tiles per chunk, at most GCHUNK (chosen by the plan)
   GroupEnt* rgrp;            // [B * gmax] forward-order groups (circuit rebuild)
   int* nrgroups;             // [B]
   int grid;                  // blocks of the tile-pass launches (0: min(nchunks, 4 per SM)); set by the autotuner

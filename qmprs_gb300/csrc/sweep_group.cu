@@ -22,7 +22,7 @@
 //                  previous group's peels to x and its new gates to z,
 //                  write both back, and reduce this group's M (both
 //                  products on the tensor cores, fp32 per warp over a
-//                  chunk of GCHUNK tiles, fp64 across the block, one
+//                  chunk of tiles, double-float across the block, one
 //                  partial per chunk)
 //   k_group_polar  one block per state: sum the chunk partials in chunk
 //                  order, then run the group's steps on M (target update,
@@ -220,7 +220,7 @@ __device__ __forceinline__ void pass_cross(const PassShared& sh, const float2* x
 // chunk's partial (row-major 16 x 16 entries of M).  `red` aliases the tile
 // buffers.
 template <int U>
-__device__ __forceinline__ void pass_flush(const float2 (&acc)[16], double2* red, double2* out) {
+__device__ __forceinline__ void pass_flush(const float2 (&acc)[16], double2* red, xc* out) {
   constexpr int D = 1 << U, NBK = D / 4, NB = NBK * NBK;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int blk = threadIdx.x % NB;
@@ -241,7 +241,7 @@ __device__ __forceinline__ void pass_flush(const float2 (&acc)[16], double2* red
     for (int w = 0; w < nwarps; ++w) s = cadd(s, red[(w * NB) * 16 + ent]);
     const int b = ent / 16, e = ent % 16;
     const int i = 4 * (b / NBK) + e / 4, k = 4 * (b % NBK) + e % 4;
-    out[i * GM + k] = s;
+    out[i * GM + k] = xc_from_d(s);
   }
   __syncthreads();
 }
@@ -453,10 +453,10 @@ __device__ __forceinline__ void compose_gates(const GateList (&gl)[2], int nmat,
   __syncthreads();
 }
 
-// Sum the warps' M (fixed order) into the chunk's partial, unscaled by
-// 1 / (sx sz) (exact).  `red` aliases the tile buffers (needs
-// nwarps * 256 double2).
-__device__ __forceinline__ void pass_flush_tc(const float (&acc)[2][4][4], double us, double2* red, double2* out) {
+// Sum the warps' M (fixed order, double-float: the FP64 units would take
+// about 2 us for it) into the chunk's partial, unscaled by us = 1 / (sx sz),
+// a power of two.  `red` aliases the tile buffers (needs nwarps * 256 xc).
+__device__ __forceinline__ void pass_flush_tc(const float (&acc)[2][4][4], float us, xc* red, xc* out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gq = lane >> 2, tq = lane & 3;
   __syncthreads();   // tile buffers free
@@ -465,14 +465,21 @@ __device__ __forceinline__ void pass_flush_tc(const float (&acc)[2][4][4], doubl
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int i = gq + (e >> 1) * 8, k = nt * 8 + 2 * tq + (e & 1);
-      red[warp * GMM + i * GM + k] =
-          cd(((double)acc[nt][0][e] + (double)acc[nt][3][e]) * us, ((double)acc[nt][1][e] - (double)acc[nt][2][e]) * us);
+      DF re = {acc[nt][0][e], 0.f}, im = {acc[nt][1][e], 0.f};
+      df_add(re, acc[nt][3][e], 0.f);
+      df_add(im, -acc[nt][2][e], 0.f);
+      red[warp * GMM + i * GM + k] = make_float4(re.hi, im.hi, re.lo, im.lo);
     }
   __syncthreads();
   for (int ent = threadIdx.x; ent < GMM; ent += blockDim.x) {
-    double2 s = czero();
-    for (int w = 0; w < nwarps; ++w) s = cadd(s, red[w * GMM + ent]);
-    out[ent] = s;
+    XA s = xa_zero();
+    for (int w = 0; w < nwarps; ++w) {
+      const xc v = red[w * GMM + ent];
+      df_add(s.re, v.x, v.z);
+      df_add(s.im, v.y, v.w);
+    }
+    const xc r = xa_round(s);
+    out[ent] = make_float4(r.x * us, r.y * us, r.z * us, r.w * us);
   }
   __syncthreads();
 }
@@ -562,8 +569,8 @@ __device__ __forceinline__ void pass_chunk(const BatchDev& bd, const GroupDev& g
   for (int e = 0; e < (TC ? 1 : 16); ++e) acc[e] = cf(0.f, 0.f);
 #pragma unroll
   for (int e = 0; e < 32; ++e) (&tacc[0][0][0])[e] = 0.f;
-  const int64_t t0 = (int64_t)gd.chunk_idx[chunk] * GCHUNK;
-  const int64_t t1 = t0 + GCHUNK < ntiles ? t0 + GCHUNK : ntiles;
+  const int64_t t0 = (int64_t)gd.chunk_idx[chunk] * gd.chunk_tiles;
+  const int64_t t1 = t0 + gd.chunk_tiles < ntiles ? t0 + gd.chunk_tiles : ntiles;
   int64_t base = deposit_bits(t0, rest_mask);
   for (int64_t tt = t0; tt < t1; ++tt) {
     pass_issue(sh, xv + base, zv_in + base, xs, zs);
@@ -582,8 +589,7 @@ __device__ __forceinline__ void pass_chunk(const BatchDev& bd, const GroupDev& g
     base = next_in_mask(base, rest_mask);
   }
   if constexpr (TC)
-    pass_flush_tc(tacc, 1.0 / ((double)sh.sx * (double)sh.sz), reinterpret_cast<double2*>(xs),
-                  gd.partials + (int64_t)chunk * GMM);
+    pass_flush_tc(tacc, 1.f / (sh.sx * sh.sz), reinterpret_cast<xc*>(xs), gd.partials + (int64_t)chunk * GMM);
   else pass_flush<U>(acc, reinterpret_cast<double2*>(xs), gd.partials + (int64_t)chunk * GMM);
 }
 
@@ -637,6 +643,8 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_group_pass
       sh.wml_c = wc;
       sh.wml_p = wp;   // the current window when g = 0
       sh.npk = g > 0 ? (prv.cnt < GMAXSTEPS ? prv.cnt : GMAXSTEPS) : 0;
+    }
+    if (threadIdx.x == 32) {   // an FP64 square root, beside the masks above
       sh.sx = vec_scale(n, 1.0);   // x = C|0> (or its peels) has unit norm
       sh.sz = vec_scale(n, znorm ? sqrt(fabs(znorm[b].x)) : 1.0);
     }
@@ -737,8 +745,8 @@ __device__ __forceinline__ void rebuild_chunk(const BatchDev& bd, const GroupDev
   const int64_t ntiles = (int64_t)1 << (n - sh.T);
   const int64_t rest_mask = (((int64_t)1 << n) - 1) & ~(int64_t)sh.pos_mask;
   float2* xv = psi + bd.vec_off[b];
-  const int64_t t0 = (int64_t)gd.chunk_idx[chunk] * GCHUNK;
-  const int64_t t1 = t0 + GCHUNK < ntiles ? t0 + GCHUNK : ntiles;
+  const int64_t t0 = (int64_t)gd.chunk_idx[chunk] * gd.chunk_tiles;
+  const int64_t t1 = t0 + gd.chunk_tiles < ntiles ? t0 + gd.chunk_tiles : ntiles;
   const int t = threadIdx.x, lo = sh.d0[t & 63], st = swz(t);
   // double-buffered: tile tt + 1 streams into the other buffer while tile
   // tt is processed (one commit group per tile)
@@ -992,18 +1000,25 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
     // issued together so the L2 latency overlaps
     for (int e = tid; e < D * D; e += POLAR_THREADS) {
       const int i = e / D, k = e % D;
-      const double2* src = gd.partials + (int64_t)c0 * GMM + i * GM + k;
-      double2 s = czero();
+      const xc* src = gd.partials + (int64_t)c0 * GMM + i * GM + k;
+      XA s = xa_zero();
       int c = 0;
       for (; c + 8 <= nc; c += 8) {
-        double2 v[8];
+        xc v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = src[(int64_t)(c + u) * GMM];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s = cadd(s, v[u]);
+        for (int u = 0; u < 8; ++u) {
+          df_add(s.re, v[u].x, v[u].z);
+          df_add(s.im, v[u].y, v[u].w);
+        }
       }
-      for (; c < nc; ++c) s = cadd(s, src[(int64_t)c * GMM]);
-      M[0][i * GM + k] = xc_from_d(s);
+      for (; c < nc; ++c) {
+        const xc v = src[(int64_t)c * GMM];
+        df_add(s.re, v.x, v.z);
+        df_add(s.im, v.y, v.w);
+      }
+      M[0][i * GM + k] = xa_round(s);
     }
     __syncthreads();
     int cur = 0;

@@ -484,12 +484,7 @@ static __device__ __noinline__ double warp_polar_exact(WarpPolar& ws, const doub
 
 // s += the partner lane's `give` (lane ^ o), double-float
 __device__ __forceinline__ void df_shfl_add(DF& s, const DF& give, int o) {
-  const float gh = __shfl_xor_sync(0xffffffffu, give.hi, o), gl = __shfl_xor_sync(0xffffffffu, give.lo, o);
-  const float t = __fadd_rn(s.hi, gh);
-  const float bv = __fsub_rn(t, s.hi);
-  const float err = __fadd_rn(__fsub_rn(s.hi, __fsub_rn(t, bv)), __fsub_rn(gh, bv));
-  s.lo = __fadd_rn(__fadd_rn(s.lo, gl), err);
-  s.hi = t;
+  df_add(s, __shfl_xor_sync(0xffffffffu, give.hi, o), __shfl_xor_sync(0xffffffffu, give.lo, o));
 }
 
 // Sum of 32 double-float values per lane over the warp: lane l returns the
