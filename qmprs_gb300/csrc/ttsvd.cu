@@ -8,9 +8,9 @@
 //   k_tt_gram     Gram matrix M^H M in fp64, split over at most TT_SPLIT
 //                 row ranges per state, partials reduced in order;
 //   k_tt_eig      one CTA per state: parallel cyclic Jacobi (round-robin
-//                 pairs) on the w x w Gram, fp64, working set in global
-//                 memory (L2 resident); sort, rsum2 cutoff + max_bond,
-//                 canonical phases; site tensor c;
+//                 pairs) on the w x w Gram, fp32 passes with double-float
+//                 products (w <= 64) or fp32 and fp64 sweeps; sort, rsum2
+//                 cutoff + max_bond, canonical phases; site tensor c;
 //   k_tt_project  next remainder M V (fp32).
 // k_tt_site0 stores site 0 (the last remainder, rescaled to the input norm,
 // as quimb's rsum2 renormalisation does) and k_mps_contract rebuilds the
@@ -22,10 +22,12 @@
 // capacity raises KERR_EIG_WIDTH and has its bond poisoned (-1); every
 // later kernel of the stage skips a state whose bonds are out of range, so
 // no access ever depends on an unset bond.
-#include "device_common.cuh"
+#include "dfloat.cuh"
 
 #define TT_CH 32
 #define TT_EIG_SMEM_W 64   // widest Gram diagonalised in shared memory (3 x 65 KB)
+#define TT_EIG_THREADS 512
+#define TT_EIG_PAD 2
 
 __host__ __device__ inline int chi_eff(int chi, int n) {
   const int cap = 1 << (n / 2);
@@ -292,31 +294,434 @@ __device__ void smem_matmul(const double2* A, const double2* B, double2* Cm, int
   }
 }
 
-// One CTA per state; G and V are row-major w x w.  For w <= TT_EIG_SMEM_W
-// they live in shared memory (copied from `gram`, written back to `gram`
-// and `vwork` at the end), otherwise in place in global memory: each
-// Jacobi round is four block-wide phases, and shared memory takes the
-// memory latency out of them.
+// ---- eigenvectors of a Gram in shared memory (w <= 64) -------------------------------
 //
-// The eigenvectors are found in two precisions.  FP32 Jacobi sweeps on a
-// float copy of G converge V to FP32 accuracy at the FP32 rate; V is then
-// made orthonormal in FP64 by one Newton-Schulz step V <- V (3I - V^H V) / 2
-// (its FP32 error of about 1e-7 leaves about 1e-14), G is replaced by the
-// similar, nearly diagonal V^H G V, and the FP64 Jacobi sweeps finish from
-// there, accumulating into the same V, down to `fine` of the trace.  On the
-// Grams of the benchmark family this cuts the FP64 rotations from about 8.4
-// sweeps' worth to about 2.2 (w = 64).  For 64 < w <= 128 the same steps
-// run in global memory (L2 resident): the float copies in `scratch32` (the
-// Gram partials, already reduced) and the FP64 scratch in the state's slot
-// of `vsel` (written only at the end).
-__global__ void __launch_bounds__(BLOCK_THREADS) k_tt_eig(BatchDev bd, int step, int* bonds, double2* gram,
+// GB300 runs an FP64 warp instruction in 64 cycles per SM quarter, so both
+// FP64 Jacobi sweeps and FP64 matrix products of a 64 x 64 Gram cost about a
+// millisecond each.  The vectors are found by passes instead: FP32 Jacobi
+// sweeps on the FP32 rounding of G give V_k, which is made orthonormal, and
+//   G <- V_k^H G V_k,  V <- V V_k
+// are double-float products on the FP32 pipes (2^-46).  G is then graded and
+// nearly diagonal, its small entries known to their own FP32 precision, so
+// the next pass resolves what FP32 could not see at G's scale (each pass
+// gains about seven digits), down to a rotation floor of 1e-13 of the trace
+// (ten times the products' rounding; the truncation decides at 1e-10).
+// Three or four passes; a pass whose rotations were all below 3e-7 is the
+// last.  Measured (48 states, w = 64): about 6 ms per cut with FP64 products
+// and FP64 finishing sweeps, 1.5 ms now, two thirds of it the FP32 sweeps
+// (shared-memory traffic: 128 KB a round).
+
+extern __shared__ double2 eig_sm[];
+__device__ __forceinline__ float2* tt_smf() { return reinterpret_cast<float2*>(eig_sm); }
+__device__ __forceinline__ xc* tt_smx() { return reinterpret_cast<xc*>(eig_sm); }
+
+#define JW (TT_EIG_THREADS / 32)
+static_assert(TT_EIG_SMEM_W / 2 <= 2 * JW, "two row pairs per warp");
+
+// p <- c p - conj(s) q, q <- s p + c q
+__device__ __forceinline__ void jacobi32_cols(float2& p, float2& q, float c, float sx, float sy) {
+  const float2 a = cf(c * p.x - fmaf(sx, q.x, sy * q.y), c * p.y - fmaf(sx, q.y, -sy * q.x));
+  const float2 b = cf(fmaf(c, q.x, fmaf(sx, p.x, -sy * p.y)), fmaf(c, q.y, fmaf(sx, p.y, sy * p.x)));
+  p = a;
+  q = b;
+}
+
+// FP32 Jacobi sweeps (round-robin pairing) on the Hermitian g (row-major,
+// stride ld), accumulating v <- v R; both double-buffered with g2, v2.
+// Columns (and rows of g) sit at their position of the tournament: a round
+// pairs position l with w - 1 - l and writes every entry one position on, so
+// a lane's pair is always columns l and w - 1 - l (distinct banks, where
+// indexing by pair met two to four conflicts) and a whole sweep brings every
+// column home.  A lane computes its pair's rotation; a warp takes row pairs
+// warp, warp + 16, so every thread updates 2 x 2 blocks of g and two
+// rows of v and a round takes one barrier.  A pair rotates when |g_pq| is
+// above rel sqrt(|g_pp g_qq|) and floor_abs; sweeps repeat while a rotation
+// was above 1e-4 of sqrt(|g_pp g_qq|) (convergence is quadratic).  *moved: a
+// rotation of tangent above 3e-7 was made.  Returns v or v2, whichever holds
+// the result.  Uniform over the block.  The matrices are offsets into the
+// dynamic shared memory, so that every access is a shared-memory one.
+__device__ int jacobi32_run(int g, int g2, int v, int v2, int w, int ld, float rel, float floor_abs, bool* moved) {
+  float2* S = tt_smf();
+  const int half = w / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool act = lane < half;
+  const int pc = act ? lane : 0, qc = w - 1 - pc;
+  auto next = [&](int x) { return x == 0 ? 0 : x == 1 ? w - 1 : x - 1; };
+  const int pn = next(pc), qn = next(qc);
+  bool mv = false;
+  for (int sweep = 0; sweep < 30; ++sweep) {
+    bool again = false;
+    for (int k = 0; k < w - 1; ++k) {
+      float cc = 1.f, sx = 0.f, sy = 0.f;
+      if (act) {
+        const float2 x = S[g + pc * ld + qc];
+        const float app = S[g + pc * ld + pc].x, aqq = S[g + qc * ld + qc].x;
+        const float g2n = fmaf(x.x, x.x, x.y * x.y), sc = fabsf(app) * fabsf(aqq);
+        if (g2n > rel * rel * sc && g2n > floor_abs * floor_abs) {
+          const float d = 0.5f * (aqq - app);
+          const float ri = rsqrtf(fmaf(d, d, g2n));
+          const float c2 = fmaf(0.5f * fabsf(d), ri, 0.5f), ci = rsqrtf(c2);
+          const float f = copysignf(0.5f * ri * ci, d);
+          cc = c2 * ci;
+          sx = x.x * f;
+          sy = x.y * f;
+          again |= g2n > 1e-8f * sc;
+          mv |= fmaf(sx, sx, sy * sy) > 9e-14f * c2;
+        }
+      }
+      // both row pairs' loads come first: the stores may not be moved past them
+      float2 x[2][4], y[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int pr = warp + u * JW;
+        if (pr >= half || !act) continue;
+        const float2 *gp = S + g + pr * ld, *gq = S + g + (w - 1 - pr) * ld;
+        x[u][0] = gp[pc];
+        x[u][1] = gp[qc];
+        x[u][2] = gq[pc];
+        x[u][3] = gq[qc];
+        const float2 *vp = S + v + pr * ld, *vq = S + v + (pr + half) * ld;
+        y[u][0] = vp[pc];
+        y[u][1] = vp[qc];
+        y[u][2] = vq[pc];
+        y[u][3] = vq[qc];
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int pr = warp + u * JW;
+        if (pr >= half) continue;
+        const float cr = __shfl_sync(0xffffffffu, cc, pr);
+        const float rx = __shfl_sync(0xffffffffu, sx, pr), ry = __shfl_sync(0xffffffffu, sy, pr);
+        if (!act) continue;
+        // columns: col_p <- c col_p - s conj(e) col_q ; col_q <- s e col_p + c col_q
+        jacobi32_cols(x[u][0], x[u][1], cc, sx, sy);
+        jacobi32_cols(x[u][2], x[u][3], cc, sx, sy);
+        // rows: row_p <- c row_p - s e row_q ; row_q <- s conj(e) row_p + c row_q
+        jacobi32_cols(x[u][0], x[u][2], cr, rx, -ry);
+        jacobi32_cols(x[u][1], x[u][3], cr, rx, -ry);
+        if (pr == lane) {   // the rotated pair: real diagonal, eliminated off-diagonal
+          x[u][0].y = 0.f;
+          x[u][3].y = 0.f;
+          if (sx != 0.f || sy != 0.f) x[u][1] = x[u][2] = cf(0.f, 0.f);
+        }
+        jacobi32_cols(y[u][0], y[u][1], cc, sx, sy);
+        jacobi32_cols(y[u][2], y[u][3], cc, sx, sy);
+        float2 *op = S + g2 + next(pr) * ld, *oq = S + g2 + next(w - 1 - pr) * ld;
+        op[pn] = x[u][0];
+        op[qn] = x[u][1];
+        oq[pn] = x[u][2];
+        oq[qn] = x[u][3];
+        float2 *vp = S + v2 + pr * ld, *vq = S + v2 + (pr + half) * ld;
+        vp[pn] = y[u][0];
+        vp[qn] = y[u][1];
+        vq[pn] = y[u][2];
+        vq[qn] = y[u][3];
+      }
+      __syncthreads();
+      int t = g;
+      g = g2;
+      g2 = t;
+      t = v;
+      v = v2;
+      v2 = t;
+    }
+    if (!__syncthreads_or(again)) break;
+  }
+  *moved = __syncthreads_or(mv);
+  return v;
+}
+
+// A 4 x 2 block of outputs of a w x w product: rows r0 .. (rows past w - 1
+// repeat the last one and are not used), columns c0, c0 + 1.  Block t of all
+// of them, or with `upper` of those that touch the upper triangle; false
+// past the last one.
+struct TTBlock {
+  int r0, c0, nr;
+  int rr[4];
+};
+__device__ __forceinline__ bool tt_block(int w, int t, bool upper, TTBlock& o) {
+  const int cp = w / 2, rq = (w + 3) / 4;
+  int i = 0, j = t;
+  if (upper) {
+    while (i < rq && j >= cp - 2 * i) {
+      j -= cp - 2 * i;
+      ++i;
+    }
+    j += 2 * i;
+  } else {
+    i = t / cp;
+    j = t % cp;
+  }
+  o.r0 = 4 * i;
+  o.c0 = 2 * j;
+  o.nr = min(4, w - o.r0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) o.rr[k] = min(o.r0 + k, w - 1);
+  return i < rq;
+}
+
+// out = op(A) B in double-float, op the adjoint with ADJ.
+template <bool ADJ>
+__device__ __forceinline__ void tt_df_block(const xc* A, const xc* B, int w, int ld, const TTBlock& o, XA (&acc)[4][2]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = xa_zero();
+  for (int k = 0; k < w; ++k) {
+    const xc b0 = B[k * ld + o.c0], b1 = B[k * ld + o.c0 + 1];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const xc a = ADJ ? A[k * ld + o.rr[i]] : A[o.rr[i] * ld + k];
+      if (ADJ) {
+        xa_macc(acc[i][0], a, b0);
+        xa_macc(acc[i][1], a, b1);
+      } else {
+        xa_mac(acc[i][0], a, b0);
+        xa_mac(acc[i][1], a, b1);
+      }
+    }
+  }
+}
+
+// out = op(A) B in FP32.
+template <bool ADJ>
+__device__ __forceinline__ void tt_f_block(const float2* A, const float2* B, int w, int ld, const TTBlock& o,
+                                           float2 (&acc)[4][2]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = cf(0.f, 0.f);
+  for (int k = 0; k < w; ++k) {
+    const float2 b0 = B[k * ld + o.c0], b1 = B[k * ld + o.c0 + 1];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 a = ADJ ? A[k * ld + o.rr[i]] : A[o.rr[i] * ld + k];
+      if (ADJ) a.y = -a.y;
+      acc[i][0] = fmac(acc[i][0], a, b0);
+      acc[i][1] = fmac(acc[i][1], a, b1);
+    }
+  }
+}
+
+// v + x in double-float
+__device__ __forceinline__ xc tt_plus(xc v, float2 x) {
+  DF re = {v.x, v.z}, im = {v.y, v.w};
+  df_add(re, x.x, 0.f);
+  df_add(im, x.y, 0.f);
+  const float2 r = df_norm(re), i = df_norm(im);
+  return make_float4(r.x, i.x, r.y, i.y);
+}
+static_assert(TT_EIG_SMEM_W / 2 * (TT_EIG_SMEM_W / 4) <= TT_EIG_THREADS, "one block of outputs per thread");
+
+// Diagonalise the w x w Gram G (double-float, shared memory, scaled to a
+// trace in [1/2, 1)): G's diagonal becomes the eigenvalues, Vg (double-float,
+// global memory, stride w) the vectors.  Shared memory holds G, V_k and a
+// work matrix, the FP32 copies in the last two.
+__device__ void tt_df_eig(xc* Vg, int w, int ld) {
+  xc *G = tt_smx(), *vk = tt_smx() + w * ld, *t = tt_smx() + 2 * w * ld;
+  float2 *v32 = tt_smf() + 2 * w * ld, *t32 = tt_smf() + 4 * w * ld;
+  TTBlock o, u;
+  const bool mine = tt_block(w, threadIdx.x, false, o), uppr = tt_block(w, threadIdx.x, true, u);
+  for (int pass = 0; pass < 6; ++pass) {
+    for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
+      const int i = e / w, j = e % w;
+      const xc g = G[i * ld + j];
+      t32[i * ld + j] = cf(g.x, i == j ? 0.f : g.y);
+      v32[i * ld + j] = cf(i == j ? 1.f : 0.f, 0.f);
+    }
+    __syncthreads();
+    bool moved;
+    const float2* vr = tt_smf() + jacobi32_run(4 * w * ld, 5 * w * ld, 2 * w * ld, 3 * w * ld, w, ld, 1e-7f,
+                                               pass == 0 ? 1e-7f : 1e-13f, &moved);
+    if (!moved) {
+      // V_k = I + X with X below 3e-7: D = -(X + X^H + X^H X) / 2 and the
+      // products with X or D are FP32, and G's diagonal stands (X changes it
+      // by less than 1e-13 of itself)
+      for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
+        const int i = e / w, j = e % w;
+        const float2 x = vr[i * ld + j];
+        t32[i * ld + j] = cf(i == j ? x.x - 1.f : x.x, x.y);
+      }
+      __syncthreads();
+      float2 acc[4][2];
+      if (mine) {
+        tt_f_block<true>(t32, t32, w, ld, o, acc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float2 x = t32[o.rr[i] * ld + o.c0 + j], y = t32[(o.c0 + j) * ld + o.rr[i]];
+            // X + D
+            acc[i][j] = cf(x.x - 0.5f * (x.x + y.x + acc[i][j].x), x.y - 0.5f * (x.y - y.y + acc[i][j].y));
+          }
+      }
+      __syncthreads();
+      float2* z = t32 + w * ld;
+      if (mine)
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (i >= o.nr) continue;
+          z[(o.r0 + i) * ld + o.c0] = acc[i][0];
+          z[(o.r0 + i) * ld + o.c0 + 1] = acc[i][1];
+        }
+      for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
+        const xc v = pass == 0 ? make_float4(e / w == e % w ? 1.f : 0.f, 0.f, 0.f, 0.f) : Vg[e];
+        t32[(e / w) * ld + e % w] = cf(v.x, v.y);
+      }
+      __syncthreads();
+      if (mine) {
+        tt_f_block<false>(t32, z, w, ld, o, acc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (i >= o.nr) continue;
+            const int e = (o.r0 + i) * w + o.c0 + j;
+            const xc v = pass == 0 ? make_float4(o.r0 + i == o.c0 + j ? 1.f : 0.f, 0.f, 0.f, 0.f) : Vg[e];
+            Vg[e] = tt_plus(v, acc[i][j]);
+          }
+      }
+      __syncthreads();
+      return;
+    }
+    // D = (I - V_k^H V_k) / 2 (Hermitian)
+    float2* d32 = t32;
+    if (uppr) {
+      DF acc[4][2][2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = DF{0.f, 0.f};
+      for (int k = 0; k < w; ++k) {
+        const float2 b[2] = {vr[k * ld + u.c0], vr[k * ld + u.c0 + 1]};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 a = vr[k * ld + u.rr[i]];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            df_add_prod(acc[i][j][0], a.x, b[j].x);
+            df_add_prod(acc[i][j][0], a.y, b[j].y);
+            df_add_prod(acc[i][j][1], a.x, b[j].y);
+            df_add_prod(acc[i][j][1], -a.y, b[j].x);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (i >= u.nr) continue;
+          const int r = u.r0 + i, c = u.c0 + j;
+          const float one = r == c ? 1.f : 0.f;
+          const float2 d = cf(0.5f * ((one - acc[i][j][0].hi) - acc[i][j][0].lo),
+                              -0.5f * (acc[i][j][1].hi + acc[i][j][1].lo));
+          if (r <= c) d32[r * ld + c] = d;
+          if (r < c) d32[c * ld + r] = cf(d.x, -d.y);
+        }
+    }
+    __syncthreads();
+    // V_k (I - 2D)^(-1/2) = V_k (I + D + 3/2 D^2 + ...): after many FP32 rotations D is a few
+    // 1e-6, whose square shows at 1e-12
+    float2* z32 = t32 + w * ld;
+    if (mine) {
+      float2 acc[4][2];
+      tt_f_block<false>(d32, d32, w, ld, o, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (i >= o.nr) continue;
+          const float2 d = d32[(o.r0 + i) * ld + o.c0 + j];
+          z32[(o.r0 + i) * ld + o.c0 + j] = cf(fmaf(1.5f, acc[i][j].x, d.x), fmaf(1.5f, acc[i][j].y, d.y));
+        }
+    }
+    __syncthreads();
+    xc nv[4][2];
+    if (mine) {
+      float2 acc[4][2];
+      tt_f_block<false>(vr, z32, w, ld, o, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float2 v = vr[o.rr[i] * ld + o.c0 + j];
+          nv[i][j] = tt_plus(make_float4(v.x, v.y, 0.f, 0.f), acc[i][j]);
+        }
+    }
+    __syncthreads();
+    if (mine)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= o.nr) continue;
+        vk[(o.r0 + i) * ld + o.c0] = nv[i][0];
+        vk[(o.r0 + i) * ld + o.c0 + 1] = nv[i][1];
+      }
+    __syncthreads();
+    // G <- V_k^H (G V_k), Hermitian
+    if (mine) {
+      XA acc[4][2];
+      tt_df_block<false>(G, vk, w, ld, o, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= o.nr) continue;
+        t[(o.r0 + i) * ld + o.c0] = xa_round(acc[i][0]);
+        t[(o.r0 + i) * ld + o.c0 + 1] = xa_round(acc[i][1]);
+      }
+    }
+    __syncthreads();
+    if (uppr) {
+      XA acc[4][2];
+      tt_df_block<true>(vk, t, w, ld, u, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (i >= u.nr) continue;
+          const int r = u.r0 + i, c = u.c0 + j;
+          const xc g = xa_round(acc[i][j]);
+          if (r <= c) G[r * ld + c] = r == c ? make_float4(g.x, 0.f, g.z, 0.f) : g;
+          if (r < c) G[c * ld + r] = xc_conj(g);
+        }
+    }
+    __syncthreads();
+    // V <- V V_k
+    if (pass == 0) {
+      for (int e = threadIdx.x; e < w * w; e += blockDim.x) Vg[e] = vk[(e / w) * ld + e % w];
+    } else {
+      for (int e = threadIdx.x; e < w * w; e += blockDim.x) t[(e / w) * ld + e % w] = Vg[e];
+      __syncthreads();
+      if (mine) {
+        XA acc[4][2];
+        tt_df_block<false>(t, vk, w, ld, o, acc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (i >= o.nr) continue;
+          Vg[(o.r0 + i) * w + o.c0] = xa_round(acc[i][0]);
+          Vg[(o.r0 + i) * w + o.c0 + 1] = xa_round(acc[i][1]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// an eigenvalue for sorting: NaN counts as negative, so that ranks stay a permutation
+__device__ __forceinline__ double tt_number(double v) { return v == v ? v : -1.0; }
+
+// One CTA per state; G and V are row-major w x w.  For w <= TT_EIG_SMEM_W
+// they are diagonalised in shared memory by the double-float passes above;
+// the exact mode (fine = 1e-15 of the trace) continues from those vectors
+// with one FP64 Newton-Schulz step and FP64 sweeps.  For 64 < w <= 128 the
+// vectors are found in global memory (L2 resident) in two precisions: FP32
+// Jacobi sweeps on a float copy of G in `scratch32` (the Gram partials,
+// already reduced), one Newton-Schulz step V <- V (3I - V^H V) / 2 in FP64
+// (its FP32 error of about 1e-7 leaves about 1e-14), G replaced by the
+// similar, nearly diagonal V^H G V, and FP64 sweeps down to `fine` of the
+// trace, with the FP64 scratch in the state's slot of `vsel` (written only
+// at the end).
+__global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step, int* bonds, double2* gram,
                                                           double2* vwork, int max_bond, double cutoff,
                                                           double2* vsel, double2* tensors, int chi,
                                                           float2* scratch32, double fine) {
   __shared__ JacobiShared<double2, double> js64;
   __shared__ JacobiShared<float2, float> js32;
   __shared__ double s_floor;
-  __shared__ double s_lam[TT_MAXW];
+  __shared__ double s_lam[TT_MAXW], s_sorted[TT_MAXW];
   __shared__ int s_perm[TT_MAXW];
   __shared__ int s_keep;
   const int64_t WW = (int64_t)bd.tt_w * bd.tt_w;
@@ -333,31 +738,47 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_eig(BatchDev bd, int step,
   }
   const int w = 2 * r;
   if (w > bd.eig_wmax) return;   // diagonalised by the blocked solver (ttsvd_wide.cu)
-  extern __shared__ double2 eig_sm[];
   double2* Gg = gram + (int64_t)b * WW;
   double2* Vg = vwork + (int64_t)b * WW;
   const bool in_smem = w <= TT_EIG_SMEM_W;
-  const int ld = in_smem ? w + 1 : w;   // padded rows: column walks hit distinct banks
+  const int ld = in_smem ? w + TT_EIG_PAD : w;   // padded rows: both diagonals hit distinct banks
   double2* G = in_smem ? eig_sm : Gg;
   double2* V = in_smem ? eig_sm + w * ld : Vg;
   double2* Sc = in_smem ? eig_sm + 2 * w * ld : vsel + (int64_t)b * WW;   // FP64 scratch
-  float2* G32 = in_smem ? reinterpret_cast<float2*>(Sc) : scratch32 + (int64_t)b * 2 * TT_SPLIT * WW;
-  float2* V32 = G32 + w * ld;
-  if (in_smem)
-    for (int e = threadIdx.x; e < w * w; e += blockDim.x) G[(e / w) * ld + e % w] = Gg[e];
-  __syncthreads();
-  // Absolute rotation floor: off-diagonals at most 1e-15 of the trace move
-  // no eigenvalue by more than that (five orders below the 1e-10
-  // truncation cutoff).  Without it the rounding-level null-space block of
-  // a rank-deficient Gram keeps rotating until the sweep limit.
-  if (threadIdx.x == 0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  if (warp == 0) {   // the trace (a positive semidefinite G: its scale)
     double tr = 0.0;
-    for (int i = 0; i < w; ++i) tr += fabs(G[i * ld + i].x);
-    s_floor = tr;
+    for (int i = lane; i < w; i += 32) tr += fabs(Gg[i * w + i].x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    if (lane == 0) s_floor = tr;
   }
   __syncthreads();
   const double tr = s_floor;
-  {
+  bool fp64 = !in_smem;   // FP64 sweeps to `fine`
+  if (in_smem) {
+    int ex = 0;
+    if (tr > 0.0 && isfinite(tr)) frexp(tr, &ex);
+    const double sc = ldexp(1.0, -ex);
+    xc* Gx = reinterpret_cast<xc*>(G);
+    xc* Vx = reinterpret_cast<xc*>(Vg);
+    for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
+      const double2 g = Gg[e];
+      Gx[(e / w) * ld + e % w] = xc_from_d(cd(g.x * sc, g.y * sc));
+    }
+    __syncthreads();
+    tt_df_eig(Vx, w, ld);
+    for (int i = threadIdx.x; i < w; i += blockDim.x) s_lam[i] = tt_number(xc_to_d(Gx[i * ld + i]).x);
+    for (int e = threadIdx.x; e < w * w; e += blockDim.x) V[(e / w) * ld + e % w] = xc_to_d(Vx[e]);
+    __syncthreads();
+    if (fine < 1e-14) {
+      for (int e = threadIdx.x; e < w * w; e += blockDim.x) G[(e / w) * ld + e % w] = Gg[e];
+      __syncthreads();
+      fp64 = true;
+    }
+  } else {
+    float2* G32 = scratch32 + (int64_t)b * 2 * TT_SPLIT * WW;
+    float2* V32 = G32 + w * ld;
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
       const int i = e / w, j = e % w;
       const double2 g = G[i * ld + j];
@@ -371,6 +792,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_eig(BatchDev bd, int step,
       V[i * ld + j] = f2d(V32[i * ld + j]);
     }
     __syncthreads();
+  }
+  if (fp64) {
     // Newton-Schulz: Sc = (3I - V^H V) / 2, then V <- V Sc row by row (a
     // warp per row, each lane up to four columns, written after the warp's reads)
     smem_matmul(V, V, Sc, w, ld, true);
@@ -381,23 +804,20 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_eig(BatchDev bd, int step,
       Sc[i * ld + j] = cd((i == j ? 1.5 : 0.0) - 0.5 * v.x, -0.5 * v.y);
     }
     __syncthreads();
-    {
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-      for (int row = warp; row < w; row += nwarps) {
-        double2 o[TT_MAXW / 32];
+    for (int row = warp; row < w; row += nwarps) {
+      double2 o[TT_MAXW / 32];
 #pragma unroll
-        for (int q = 0; q < TT_MAXW / 32; ++q) o[q] = czero();
-        for (int k = 0; k < w; ++k) {
-          const double2 v = V[row * ld + k];
-#pragma unroll
-          for (int q = 0; q < TT_MAXW / 32; ++q)
-            if (lane + 32 * q < w) o[q] = cadd(o[q], cmul(v, Sc[k * ld + lane + 32 * q]));
-        }
-        __syncwarp();
+      for (int q = 0; q < TT_MAXW / 32; ++q) o[q] = czero();
+      for (int k = 0; k < w; ++k) {
+        const double2 v = V[row * ld + k];
 #pragma unroll
         for (int q = 0; q < TT_MAXW / 32; ++q)
-          if (lane + 32 * q < w) V[row * ld + lane + 32 * q] = o[q];
+          if (lane + 32 * q < w) o[q] = cadd(o[q], cmul(v, Sc[k * ld + lane + 32 * q]));
       }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < TT_MAXW / 32; ++q)
+        if (lane + 32 * q < w) V[row * ld + lane + 32 * q] = o[q];
     }
     __syncthreads();
     // G <- V^H (G V)
@@ -406,24 +826,26 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_eig(BatchDev bd, int step,
     smem_matmul(V, Sc, G, w, ld, true);
     __syncthreads();
     for (int i = threadIdx.x; i < w; i += blockDim.x) G[i * ld + i].y = 0.0;
+    __syncthreads();
+    // Absolute rotation floor: off-diagonals at most `fine` of the trace move
+    // no eigenvalue by more than that (three to five orders below the 1e-10
+    // truncation cutoff).  Without it the rounding-level null-space block of
+    // a rank-deficient Gram keeps rotating until the sweep limit.
+    jacobi_run<double2, double>(G, V, w, ld, 1e-15, fine * tr, 40, js64);
+    for (int i = threadIdx.x; i < w; i += blockDim.x) s_lam[i] = tt_number(G[i * ld + i].x);
+    __syncthreads();
+  }
+  // descending order (ties by index)
+  for (int i = threadIdx.x; i < w; i += blockDim.x) {
+    const double li = s_lam[i];
+    int rank = 0;
+    for (int j = 0; j < w; ++j) rank += s_lam[j] > li || (s_lam[j] == li && j < i);
+    s_perm[rank] = i;
+    s_sorted[rank] = li;
   }
   __syncthreads();
-  // After the FP32 stage the FP64 sweeps stop at 1e-13 of the trace (three
-  // orders below the 1e-10 cutoff; eigenvalues move by about 1e-15 of the
-  // trace against 1e-15): the remaining rotations are the null-space
-  // cluster's rounding noise.
-  jacobi_run<double2, double>(G, V, w, ld, 1e-15, fine * tr, 40, js64);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < w; ++i) { s_perm[i] = i; s_lam[i] = G[i * ld + i].x; }
-    for (int i = 1; i < w; ++i) {
-      const int kk = s_perm[i];
-      const double key = s_lam[i];
-      int j = i - 1;
-      while (j >= 0 && s_lam[j] < key) { s_lam[j + 1] = s_lam[j]; s_perm[j + 1] = s_perm[j]; --j; }
-      s_lam[j + 1] = key;
-      s_perm[j + 1] = kk;
-    }
-    int keep = rank_by_cutoff(s_lam, w, cutoff, max_bond);
+    int keep = rank_by_cutoff(s_sorted, w, cutoff, max_bond);
     if (keep > bd.tt_b) keep = bd.tt_b;
     if (c < 30 && keep > (1 << c)) keep = 1 << c;   // M has 2^c rows: rank <= 2^c
     s_keep = keep;
@@ -431,7 +853,32 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_eig(BatchDev bd, int step,
   }
   __syncthreads();
   const int keep = s_keep;
-  if (threadIdx.x < keep) phase_fix_column(V, w, ld, s_perm[threadIdx.x]);
+  // canonical phases (the rule of phase_fix_column), a warp per kept column
+  for (int k = warp; k < keep; k += nwarps) {
+    const int col = s_perm[k];
+    double mag[TT_MAXW / 32], m2 = -1.0;
+#pragma unroll
+    for (int q = 0; q < TT_MAXW / 32; ++q) {
+      const int i = lane + 32 * q;
+      mag[q] = i < w ? cnorm2(V[i * ld + col]) : -1.0;
+      m2 = fmax(m2, mag[q]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    const double lim = (1.0 - QM_PIVOT_TOL) * (1.0 - QM_PIVOT_TOL) * m2;
+    int piv = w;
+#pragma unroll
+    for (int q = TT_MAXW / 32 - 1; q >= 0; --q)
+      if (lane + 32 * q < w && mag[q] >= lim) piv = lane + 32 * q;
+    piv = __reduce_min_sync(0xffffffffu, piv);
+    const double2 z = piv < w ? V[piv * ld + col] : czero();
+    const double az = sqrt(cnorm2(z));
+    __syncwarp();
+    if (az > 0.0) {
+      const double2 ph = cscale(cconj(z), 1.0 / az);
+      for (int i = lane; i < w; i += 32) V[i * ld + col] = cmul(V[i * ld + col], ph);
+    }
+  }
   __syncthreads();
   double2* vs = vsel + (int64_t)b * WW;
   for (int e = threadIdx.x; e < w * keep; e += blockDim.x) {
@@ -549,7 +996,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_mps_contract(BatchDev bd, int
   }
 }
 
-#define TT_EIG_SMEM ((size_t)3 * TT_EIG_SMEM_W * (TT_EIG_SMEM_W + 1) * sizeof(double2))   // G, V, scratch
+#define TT_EIG_SMEM ((size_t)3 * TT_EIG_SMEM_W * (TT_EIG_SMEM_W + TT_EIG_PAD) * sizeof(double2))   // G, V, scratch
 
 static int grid_for(const BatchDev& bd) {
   int g = bd.ntiles;
@@ -572,7 +1019,7 @@ void launch_tt_eig(const BatchDev& bd, int step, int* bonds, double2* gram, doub
     attr = true;
   }
   qm_note_launch();
-  k_tt_eig<<<bd.B, BLOCK_THREADS, TT_EIG_SMEM, s>>>(bd, step, bonds, gram, vwork, max_bond, cutoff, vsel, tensors,
+  k_tt_eig<<<bd.B, TT_EIG_THREADS, TT_EIG_SMEM, s>>>(bd, step, bonds, gram, vwork, max_bond, cutoff, vsel, tensors,
                                                     chi, reinterpret_cast<float2*>(scratch), fine);
 }
 
