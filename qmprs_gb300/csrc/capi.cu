@@ -360,7 +360,7 @@ inline uint64_t dbl_key(double v) {
 int ensure_tt_scratch(qmprs_plan* p) {
   if (p->tt_partials) return QMPRS_OK;
   const int64_t WW = (int64_t)p->tt_w * p->tt_w;
-  CK(dalloc(&p->tt_partials, (int64_t)p->B * TT_SPLIT * WW));
+  CK(dalloc(&p->tt_partials, (int64_t)p->B * p->bd.tt_region));
   CK(dalloc(&p->gram, (int64_t)p->B * WW));
   CK(dalloc(&p->vsel2, (int64_t)p->B * WW));
   CK(dalloc(&p->vwork, (int64_t)p->B * WW));
@@ -447,7 +447,7 @@ int exact_mps_from_statevector(qmprs_plan* p, const double2* sv, int max_bond, d
       if (c < 1) continue;
       const int r = hb[(size_t)b * stride + c + 1];
       if (r < 1 || r > p->tt_b) continue;
-      launch_x_gram(src + p->vec_off[b], ipow2(c), 2 * r, p->tt_partials + (int64_t)b * TT_SPLIT * WW, WW,
+      launch_x_gram(src + p->vec_off[b], ipow2(c), 2 * r, p->tt_partials + (int64_t)b * p->bd.tt_region, WW,
                     p->gram + (int64_t)b * WW, s);
       wide = wide || 2 * r > p->bd.eig_wmax;
     }
@@ -854,6 +854,10 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   bd.err = p->d_err;
   bd.tt_w = p->tt_w;
   bd.tt_b = p->tt_b;
+  // room for TT_SPLIT partials of the widest Gram, and for as many 64-wide
+  // ones as the largest state has tiles
+  const int most_tiles = *std::max_element(state_ntiles.begin(), state_ntiles.end());
+  bd.tt_region = std::max<int64_t>((int64_t)TT_SPLIT * p->tt_w * p->tt_w, (int64_t)std::min(most_tiles, TT_SPLIT_MAX) * 4096);
   bd.cut_state = p->d_cut_state;
   bd.cut_idx = p->d_cut_idx;
   bd.eig_wmax = num_states <= BJ_SMALL_BATCH ? TT_MAXB : TT_MAXW;

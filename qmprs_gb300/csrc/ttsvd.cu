@@ -5,8 +5,8 @@
 // whose density-matrix method truncates from the right and leaves a
 // right-canonical MPS.  Cut c (c = n-1 .. 1) of state b holds the remainder
 // M (2^c x w, w = 2 r, r = bond c+1).  Per cut:
-//   k_tt_gram     Gram matrix M^H M in fp64, split over at most TT_SPLIT
-//                 row ranges per state, partials reduced in order;
+//   k_tt_gram     Gram matrix M^H M in double-float, split over row ranges;
+//   k_tt_gram_sum the ranges' partials summed in order, in fp64;
 //   k_tt_eig      one CTA per state: parallel cyclic Jacobi (round-robin
 //                 pairs) on the w x w Gram, fp32 passes with double-float
 //                 products (w <= 64) or fp32 and fp64 sweeps; sort, rsum2
@@ -59,34 +59,46 @@ __device__ __forceinline__ int gram_nblocks(int w) {
   return t;
 }
 
-// Upper triangle of M^H M (M = the 2^c x w remainder) per state: up to
-// TT_SPLIT blocks per state take row ranges; in a block, thread t takes the
-// entry block (t mod nb) and every (256 / nb)-th row of the range, sums
-// exact fp32 products with compensation and flushes to fp64; the rest
-// groups are then summed in fixed order through shared memory.  The last
-// block of a state (ticket) sums the splits in order and mirrors the lower
-// triangle.
+// Row splits of a state's Gram: as many as it has tiles, at most
+// TT_SPLIT_MAX, at least 32 rows each, and as many w x w partials as its
+// slot holds.  A 20-qubit state's 64-wide Gram has 16384 rows and one chunk
+// of entry blocks, so eight splits kept 16 SMs busy.
+__device__ __forceinline__ int tt_splits(const BatchDev& bd, int b, int c, int w) {
+  int64_t n = bd.state_ntiles[b];
+  n = min(n, (int64_t)TT_SPLIT_MAX);
+  n = min(n, max((int64_t)1, ipow2(c) >> 5));
+  n = min(n, bd.tt_region / ((int64_t)w * w));
+  return (int)n;
+}
+
+__device__ __forceinline__ bool tt_gram_here(const BatchDev& bd, const int* bond, int c, int* w) {
+  if (c < 1 || !bond_ok(bond[c + 1], bd.tt_b)) return false;
+  *w = 2 * bond[c + 1];
+  return !(*w > bd.eig_wmax && ipow2(c) < (int64_t)*w);   // else the row Gram (ttsvd_wide.cu)
+}
+
+// Upper triangle of M^H M (M = the 2^c x w remainder) per state, row split
+// by row split; in a block, thread t takes the entry block (t mod nb) and
+// every (256 / nb)-th row of the split, sums exact fp32 products in
+// double-float over TT_FLUSH rows, those sums in double-float too, and the
+// rest groups are then summed in fixed order through shared memory
+// (k_tt_gram_sum adds the splits in order).
+// Measured (20 qubits, 64 wide): 1380 us with eight splits and FP64 sums,
+// 86 us now (512 wide, FP32 bound: 1630 -> 520 us).
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step, const float2* sv,
-                                                           const float2* src, const int* bonds,
-                                                           double2* partials, double2* gram) {
-  __shared__ double2 red[BLOCK_THREADS * TT_EPB];   // 32 KB
-  const int64_t WW = (int64_t)bd.tt_w * bd.tt_w;
+                                                           const float2* src, const int* bonds, xc* partials) {
+  __shared__ xc red[BLOCK_THREADS * TT_EPB];   // 32 KB
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     const int n = bd.n[b];
     const int c = n - 1 - step;
     if (c < 1) continue;
     const int* bond = bonds + (int64_t)b * (bd.max_n + 1);
-    const int r = bond[c + 1];
     const int idx = bd.tile_idx[tile];
-    if (!bond_ok(r, bd.tt_b)) {
-      if (r > bd.tt_b && idx == 0 && threadIdx.x == 0) atomicOr(bd.err, KERR_EIG_WIDTH);
-      continue;
-    }
-    const int w = 2 * r;
-    if (w > bd.eig_wmax && ipow2(c) < (int64_t)w) continue;   // the row Gram (ttsvd_wide.cu)
-    const int nt = bd.state_ntiles[b];
-    const int nsplit = nt < TT_SPLIT ? nt : TT_SPLIT;
+    if (bond[c + 1] > bd.tt_b && idx == 0 && threadIdx.x == 0) atomicOr(bd.err, KERR_EIG_WIDTH);
+    int w;
+    if (!tt_gram_here(bd, bond, c, &w)) continue;
+    const int nt = bd.state_ntiles[b], nsplit = tt_splits(bd, b, c, w);
     const float2* m = (step == 0 ? sv : src) + bd.vec_off[b];
     const int nb = gram_nblocks(w);
     // work units: (row split, chunk of BLOCK_THREADS entry blocks), taken by
@@ -94,11 +106,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
     const int nech = (nb + BLOCK_THREADS - 1) / BLOCK_THREADS;
     const int units = nsplit * nech;
     for (int unit = idx; unit < units; unit += nt) {
-    const int split = unit % nsplit;
-    int64_t lo, hi;
-    tile_range(ipow2(c), split, nsplit, &lo, &hi);
-    double2* part = partials + ((int64_t)b * TT_SPLIT + split) * WW;
-    {
+      const int split = unit % nsplit;
+      int64_t lo, hi;
+      tile_range(ipow2(c), split, nsplit, &lo, &hi);
+      xc* part = partials + (int64_t)b * bd.tt_region + (int64_t)split * w * w;
       const int e0 = (unit / nsplit) * BLOCK_THREADS;
       const int nbp = nb - e0 < BLOCK_THREADS ? nb - e0 : BLOCK_THREADS;
       const int nsub = BLOCK_THREADS / nbp;
@@ -107,70 +118,98 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
       int bi = 0, bj = 0;
       if (act) gram_block(e0 + eb, w, &bi, &bj);
       const int a0 = 2 * bi, c0 = 4 * bj;
-      double2 acc[TT_EPB];
+      XA acc[TT_EPB];
 #pragma unroll
-      for (int k = 0; k < TT_EPB; ++k) acc[k] = czero();
+      for (int k = 0; k < TT_EPB; ++k) acc[k] = xa_zero();
       if (act) {
         int64_t row = lo + sub;
         while (row < hi) {
-          DF re[TT_EPB], im[TT_EPB];
+          XA s[TT_EPB];
 #pragma unroll
-          for (int k = 0; k < TT_EPB; ++k) re[k] = im[k] = DF{0.f, 0.f};
+          for (int k = 0; k < TT_EPB; ++k) s[k] = xa_zero();
           for (int f = 0; f < TT_FLUSH && row < hi; ++f, row += nsub) {
             const float2* x = m + row * w;
-            float2 xa[2], xc[4];
+            float2 xa[2], xv[4];
 #pragma unroll
             for (int u = 0; u < 2; ++u) xa[u] = x[a0 + u];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) xc[v] = c0 + v < w ? x[c0 + v] : cf(0.f, 0.f);
+            for (int v = 0; v < 4; ++v) xv[v] = c0 + v < w ? x[c0 + v] : cf(0.f, 0.f);
 #pragma unroll
             for (int u = 0; u < 2; ++u)
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
-                // conj(xa) * xc
-                df_add_prod(re[u * 4 + v], xa[u].x, xc[v].x);
-                df_add_prod(re[u * 4 + v], xa[u].y, xc[v].y);
-                df_add_prod(im[u * 4 + v], xa[u].x, xc[v].y);
-                df_add_prod(im[u * 4 + v], -xa[u].y, xc[v].x);
+                // conj(xa) * xv
+                XA& o = s[u * 4 + v];
+                df_add_prod(o.re, xa[u].x, xv[v].x);
+                df_add_prod(o.re, xa[u].y, xv[v].y);
+                df_add_prod(o.im, xa[u].x, xv[v].y);
+                df_add_prod(o.im, -xa[u].y, xv[v].x);
               }
           }
 #pragma unroll
           for (int k = 0; k < TT_EPB; ++k) {
-            acc[k].x += (double)re[k].hi + (double)re[k].lo;
-            acc[k].y += (double)im[k].hi + (double)im[k].lo;
+            df_add(acc[k].re, s[k].re.hi, s[k].re.lo);
+            df_add(acc[k].im, s[k].im.hi, s[k].im.lo);
           }
         }
       }
       // sum the row groups of each entry block in fixed order
       __syncthreads();
 #pragma unroll
-      for (int k = 0; k < TT_EPB; ++k) red[threadIdx.x * TT_EPB + k] = acc[k];
+      for (int k = 0; k < TT_EPB; ++k) red[threadIdx.x * TT_EPB + k] = xa_round(acc[k]);
       __syncthreads();
       for (int o = threadIdx.x; o < nbp * TT_EPB; o += BLOCK_THREADS) {
         const int ebo = o / TT_EPB, k = o % TT_EPB;
-        double2 sacc = czero();
-        for (int sb = 0; sb < nsub; ++sb) sacc = cadd(sacc, red[(sb * nbp + ebo) * TT_EPB + k]);
+        XA sacc = xa_zero();
+        for (int sb = 0; sb < nsub; ++sb) {
+          const xc v = red[(sb * nbp + ebo) * TT_EPB + k];
+          df_add(sacc.re, v.x, v.z);
+          df_add(sacc.im, v.y, v.w);
+        }
         int gi, gj;
         gram_block(e0 + ebo, w, &gi, &gj);
         const int a = 2 * gi + k / 4, cc = 4 * gj + k % 4;
-        if (a <= cc && cc < w) part[(int64_t)a * w + cc] = sacc;
+        if (a <= cc && cc < w) part[(int64_t)a * w + cc] = xa_round(sacc);
       }
     }
-    __syncthreads();
-    if (last_tile_ticket(bd.ticket, b, units)) {
-      for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-        const int a = e / w, cc = e % w;
-        if (a > cc) continue;
-        double2 s = czero();
-        for (int t = 0; t < nsplit; ++t) s = cadd(s, ld_cg(&partials[((int64_t)b * TT_SPLIT + t) * WW + a * w + cc]));
-        gram[(int64_t)b * WW + (int64_t)a * w + cc] = s;
-        if (a != cc) gram[(int64_t)b * WW + (int64_t)cc * w + a] = cconj(s);
-        else gram[(int64_t)b * WW + (int64_t)a * w + a] = cd(s.x, 0.0);
+  }
+}
+
+// The Gram of every state: the splits' partials summed in a fixed order
+// (eight lanes per entry, each every eighth split, then the lanes), the lower
+// triangle mirrored.  Block x takes 32 entries at a time, block y a state.
+__global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram_sum(BatchDev bd, int step, const int* bonds,
+                                                               const xc* partials, double2* gram) {
+  const int l8 = threadIdx.x & 7;
+  for (int b = blockIdx.y; b < bd.B; b += gridDim.y) {
+    const int c = bd.n[b] - 1 - step;
+    int w;
+    if (!tt_gram_here(bd, bonds + (int64_t)b * (bd.max_n + 1), c, &w)) continue;
+    const int nsplit = tt_splits(bd, b, c, w), ww = w * w;
+    const xc* part = partials + (int64_t)b * bd.tt_region;
+    double2* g = gram + (int64_t)b * bd.tt_w * bd.tt_w;
+    for (int e0 = blockIdx.x * (BLOCK_THREADS / 8); e0 < ww; e0 += gridDim.x * (BLOCK_THREADS / 8)) {
+      const int e = e0 + (threadIdx.x >> 3), a = e / w, cc = e % w;
+      XA s = xa_zero();
+      if (e < ww && a <= cc) {
+#pragma unroll 4
+        for (int t = l8; t < nsplit; t += 8) {
+          const xc v = part[(int64_t)t * ww + e];
+          df_add(s.re, v.x, v.z);
+          df_add(s.im, v.y, v.w);
+        }
       }
-      __syncthreads();
-      if (threadIdx.x == 0) bd.ticket[b] = 0;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        df_add(s.re, __shfl_xor_sync(0xffffffffu, s.re.hi, o), __shfl_xor_sync(0xffffffffu, s.re.lo, o));
+        df_add(s.im, __shfl_xor_sync(0xffffffffu, s.im.hi, o), __shfl_xor_sync(0xffffffffu, s.im.lo, o));
+      }
+      if (l8 == 0 && e < ww && a <= cc) {
+        const double2 r = xa_to_d(s);
+        g[e] = a == cc ? cd(r.x, 0.0) : r;
+        if (a != cc) g[(int64_t)cc * w + a] = cconj(r);
+      }
     }
-    }   // units
   }
 }
 
@@ -777,7 +816,7 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
       fp64 = true;
     }
   } else {
-    float2* G32 = scratch32 + (int64_t)b * 2 * TT_SPLIT * WW;
+    float2* G32 = scratch32 + (int64_t)b * 2 * bd.tt_region;
     float2* V32 = G32 + w * ld;
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
       const int i = e / w, j = e % w;
@@ -1006,8 +1045,15 @@ static int grid_for(const BatchDev& bd) {
 
 void launch_tt_gram(const BatchDev& bd, int step, const float2* sv, const float2* src, const int* bonds,
                     double2* partials, double2* gram, cudaStream_t s) {
+  xc* part = reinterpret_cast<xc*>(partials);
   qm_note_launch();
-  k_tt_gram<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, sv, src, bonds, partials, gram);
+  k_tt_gram<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, sv, src, bonds, part);
+  // the widest Gram a state can have at this step
+  const int64_t wmax = step < 12 ? std::min<int64_t>(ipow2(step + 1), 2 * bd.tt_b) : 2 * bd.tt_b;
+  const int64_t gx = std::min<int64_t>((wmax * wmax + BLOCK_THREADS / 8 - 1) / (BLOCK_THREADS / 8), 2048);
+  qm_note_launch();
+  k_tt_gram_sum<<<dim3((unsigned)gx, (unsigned)std::min(bd.B, 65535)), BLOCK_THREADS, 0, s>>>(bd, step, bonds, part,
+                                                                                              gram);
 }
 
 void launch_tt_eig(const BatchDev& bd, int step, int* bonds, double2* gram, double2* vwork, int max_bond,

@@ -26,7 +26,7 @@ def eng(cuda_lib):
 
 @pytest.mark.parametrize("precision", ["fast", "exact"])
 @pytest.mark.parametrize("n,bonds,chi", [(2, [1, 2], 4), (5, [3], 3), (11, [1, 3, 5, 7], 16),
-                                         (12, [21, 31, 32], 32), (13, [17, 32, 29], 24)])
+                                         (12, [21, 31, 32], 32), (13, [17, 32, 29], 24), (16, [4, 9], 8)])
 def test_sites_and_target(eng, n, bonds, chi, precision):
     exact = precision == "exact"
     states = [S.random_mps(n, bd, 11 * n + bd) for bd in bonds]
