@@ -7,7 +7,7 @@
 //                5th-generation tensor cores: operands staged into shared
 //                memory in the canonical K-major no-swizzle layout (8-row x
 //                16-byte core matrices), one elected thread issues
-//                tcgen05.mma (kind::f16, M = 128, N <= 256, K = 16 per
+//                tcgen05.mma (kind::f16, M = 128, N <= 64, K = 16 per
 //                instruction) into an FP32 accumulator in tensor memory,
 //                tcgen05.commit arrives on an mbarrier, and all four warps
 //                read their 32 accumulator lanes back with tcgen05.ld.
@@ -37,12 +37,15 @@
 #define MLP_BK 64
 #define MLP_MAXN 256
 #define MLP_THREADS 128
-#define MLP_TMEM_COLS 256
-// A tile 128 x 64 BF16 (16 KB) + B tile 256 x 64 BF16 (32 KB); the request
-// is padded to 96 KB so at most two blocks share an SM (2 x 256 TMEM columns).
+#define MLP_BN 64            // columns of C per block
+#define MLP_TMEM_COLS 64
+// A stage: A tile 128 x 64 BF16 (16 KB) + B tile 64 x 64 BF16 (8 KB).  Four
+// stages are 96 KB, so two blocks share an SM.
+#define MLP_STAGES 4
 #define MLP_SMEM_A 16384
-#define MLP_SMEM_B 32768
-#define MLP_SMEM_REQ (96 * 1024)
+#define MLP_SMEM_B 8192
+#define MLP_SMEM_STAGE (MLP_SMEM_A + MLP_SMEM_B)
+#define MLP_SMEM_REQ (MLP_STAGES * MLP_SMEM_STAGE)
 #define MLP_WAIT_LIMIT (1 << 22)
 #define MLP_WAIT_NS 1000000000ull   // and at most one second of wall time
 
@@ -183,14 +186,34 @@ __device__ __forceinline__ void stage_tile(uint8_t* s, const __nv_bfloat16* g, i
   }
 }
 
-__global__ void __launch_bounds__(MLP_THREADS, 1) k_gemm_tc(GemmArgs g) {
+// One 128 x 64 tile of C per block.  Splitting N as well as M gives a layer
+// of 4096 rows 128 blocks instead of 32, and shortens the epilogue, which
+// bounds these shapes (K is 256 or 512: four to eight steps); every output
+// still sums its products in the same order.  The first four K steps are
+// staged at once, a later one into the stage whose product has completed.
+// Measured (mean over a training step of 4096 rows): 44.6 us with 32 blocks of
+// 128 x 256 and one stage, 9.8 us now.
+__global__ void __launch_bounds__(MLP_THREADS, 2) k_gemm_tc(GemmArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sA = smem;
-  uint8_t* sB = smem + MLP_SMEM_A;
-  __shared__ __align__(8) uint64_t mbar;
+  __shared__ __align__(8) uint64_t mbar[MLP_STAGES];
   __shared__ uint32_t tmem_sh;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * MLP_BM;
+  const int m0 = blockIdx.x * MLP_BM, n0 = blockIdx.y * MLP_BN;
+  const int nn = min(MLP_BN, g.N - n0);
+  const int kbeg = blockIdx.z * g.ksplit;
+  const int kend = min(kbeg + g.ksplit, g.K);
+  const int nk = (kend - kbeg + MLP_BK - 1) / MLP_BK;
+  auto stage = [&](int it) {   // K step `it` into its stage, one copy group
+    if (it < nk) {
+      uint8_t* s = smem + (it % MLP_STAGES) * MLP_SMEM_STAGE;
+      const int k0 = kbeg + it * MLP_BK, kc = min(kend - k0, MLP_BK);
+      stage_tile(s, g.A, g.lda, m0, MLP_BM, k0, kc);
+      stage_tile(s + MLP_SMEM_A, g.B, g.ldb, n0, nn, k0, kc);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll
+  for (int it = 0; it < MLP_STAGES; ++it) stage(it);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_sh)),
                  "r"(MLP_TMEM_COLS)
@@ -198,65 +221,132 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) k_gemm_tc(GemmArgs g) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   if (threadIdx.x == 0) {
-    mbar_init(&mbar, 1);
+    for (int i = 0; i < MLP_STAGES; ++i) mbar_init(&mbar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_sh;
-  const uint32_t idesc = make_idesc_bf16(MLP_BM, g.N);
-  const int kbeg = blockIdx.z * g.ksplit;
-  const int kend = kbeg + g.ksplit < g.K ? kbeg + g.ksplit : g.K;
-  uint32_t phase = 0;
+  const uint32_t idesc = make_idesc_bf16(MLP_BM, nn);
+  // step it's product arrives at mbar[it % STAGES], its (it / STAGES)-th phase
+  auto done = [&](int it) { return mbar_wait(&mbar[it % MLP_STAGES], (uint32_t)(it / MLP_STAGES) & 1u); };
   bool ok = true;
-  for (int k0 = kbeg; k0 < kend; k0 += MLP_BK) {
-    const int kc = kend - k0 < MLP_BK ? kend - k0 : MLP_BK;
-    stage_tile(sA, g.A, g.lda, m0, MLP_BM, k0, kc);
-    stage_tile(sB, g.B, g.ldb, 0, g.N, k0, kc);
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+  int issued = 0;
+  for (int it = 0; it < nk; ++it) {
+    // all copy groups but the newest STAGES - 2 have landed: step it's among them
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(MLP_STAGES - 2) : "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
       tc_fence_after();
-      for (int kk = 0; kk < kc / 16; ++kk) {
-        const uint64_t ad = make_desc(smem_u32(sA) + kk * 256, 128, 1024);
-        const uint64_t bd = make_desc(smem_u32(sB) + kk * 256, 128, 1024);
-        mma_bf16(tmem, ad, bd, idesc, (k0 > kbeg || kk > 0) ? 1 : 0);
-      }
-      mma_commit(&mbar);
+      const uint32_t sa = smem_u32(smem + (it % MLP_STAGES) * MLP_SMEM_STAGE), sb = sa + MLP_SMEM_A;
+      const int kc = min(kend - kbeg - it * MLP_BK, MLP_BK);
+      for (int kk = 0; kk < kc / 16; ++kk)
+        mma_bf16(tmem, make_desc(sa + kk * 256, 128, 1024), make_desc(sb + kk * 256, 128, 1024), idesc,
+                 (it > 0 || kk > 0) ? 1 : 0);
+      mma_commit(&mbar[it % MLP_STAGES]);
     }
-    ok = __syncthreads_and(mbar_wait(&mbar, phase) ? 1 : 0) != 0;   // uniform decision
-    phase ^= 1u;
-    if (!ok) break;
+    issued = it + 1;
+    if (it >= 1) {   // refill the stage of step it - 1 once its product has read it
+      if (it - 1 + MLP_STAGES < nk) {
+        ok = __syncthreads_and(done(it - 1) ? 1 : 0) != 0;   // uniform decision
+        if (!ok) break;
+      }
+      stage(it - 1 + MLP_STAGES);
+    }
   }
+  if (ok && issued > 0) ok = __syncthreads_and(done(issued - 1) ? 1 : 0) != 0;
   if (!ok) {
     if (threadIdx.x == 0) atomicOr(g.err, KERR_TC_TIMEOUT);
-    (void)mbar_wait(&mbar, phase ^ 1u);   // the outstanding commit, bounded
-  } else if (kend > kbeg) {
+    (void)done(issued - 1);   // the outstanding product, bounded
+  } else if (nk > 0) {
     tc_fence_after();
     const int row = m0 + warp * 32 + lane;
     const bool split = gridDim.z > 1;
-    for (int c0 = 0; c0 < g.N; c0 += 16) {
+    // 16-byte stores and loads where the rows allow them
+    const bool cf4 = g.Cf && g.ldc % 4 == 0 && ((uintptr_t)g.Cf & 15) == 0;
+    const bool cb8 = g.Cb && g.ldc % 8 == 0 && ((uintptr_t)g.Cb & 15) == 0;
+    const bool rs4 = g.resid && g.ldr % 4 == 0 && ((uintptr_t)g.resid & 15) == 0;
+    const bool pt4 = split && ((uintptr_t)g.part & 15) == 0;   // N is a multiple of 16
+    for (int c0 = 0; c0 < nn; c0 += 16) {
       uint32_t v[16];
       tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      const int col0 = n0 + c0;
+      float z[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int col = c0 + j;
-        float z = __uint_as_float(v[j]);
-        if (split) {
-          g.part[((int64_t)blockIdx.z * g.M + row) * g.N + col] = z;
-          continue;
+      for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(v[j]);
+      if (split) {
+        float* o = g.part + ((int64_t)blockIdx.z * g.M + row) * g.N + col0;
+        if (pt4) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4*>(o + j) = make_float4(z[j], z[j + 1], z[j + 2], z[j + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] = z[j];
         }
-        if (g.bias) z += g.bias[col];
-        if (g.resid) z += g.resid[(int64_t)row * g.ldr + col];
-        if (g.Cf) g.Cf[(int64_t)row * g.ldc + col] = z;
-        const float a = g.act == MLP_ACT_GELU ? gelu_f(z) : z;
-        if (g.Cb) g.Cb[(int64_t)row * g.ldc + col] = __float2bfloat16_rn(a);
-        if (g.CbT) g.CbT[(int64_t)col * g.ldt + row] = __float2bfloat16_rn(a);
+        continue;
+      }
+      if (g.bias) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) z[j] += g.bias[col0 + j];
+      }
+      if (g.resid) {
+        const float* r = g.resid + (int64_t)row * g.ldr + col0;
+        if (rs4) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(r + j);
+            z[j] += x.x;
+            z[j + 1] += x.y;
+            z[j + 2] += x.z;
+            z[j + 3] += x.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) z[j] += r[j];
+        }
+      }
+      if (g.Cf) {
+        float* o = g.Cf + (int64_t)row * g.ldc + col0;
+        if (cf4) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4*>(o + j) = make_float4(z[j], z[j + 1], z[j + 2], z[j + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] = z[j];
+        }
+      }
+      if (!g.Cb && !g.CbT) continue;
+      __nv_bfloat16 h[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(g.act == MLP_ACT_GELU ? gelu_f(z[j]) : z[j]);
+      if (g.Cb) {
+        __nv_bfloat16* o = g.Cb + (int64_t)row * g.ldc + col0;
+        if (cb8) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 8) {
+            uint32_t p[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              p[q] = (uint32_t)__bfloat16_as_ushort(h[j + 2 * q]) |
+                     ((uint32_t)__bfloat16_as_ushort(h[j + 2 * q + 1]) << 16);
+            *reinterpret_cast<uint4*>(o + j) = make_uint4(p[0], p[1], p[2], p[3]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] = h[j];
+        }
+      }
+      if (g.CbT) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) g.CbT[(int64_t)(col0 + j) * g.ldt + row] = h[j];
       }
     }
   }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -424,13 +514,26 @@ __global__ void k_act_back(const float* dH, const float* Z, int B, int N, float*
   }
 }
 
-// out[c] = sum_r X[r][c] over r < B, one thread per column, fixed order
-__global__ void k_col_sum(const float* X, int B, int N, float* out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
+// out[c] = sum_r X[r][c] over r < B in a fixed order: a block takes 32
+// columns, thread (rg, c) every 32nd row, then the 32 row groups in order.
+// One thread per column was a chain of B loads on two blocks (4096 rows:
+// 120 us, 9.7 us now).
+#define COL_GROUPS 32
+__global__ void __launch_bounds__(32 * COL_GROUPS) k_col_sum(const float* X, int B, int N, float* out) {
+  __shared__ float red[COL_GROUPS][33];
+  const int l = threadIdx.x & 31, rg = threadIdx.x >> 5, c = blockIdx.x * 32 + l;
   float s = 0.f;
-  for (int r = 0; r < B; ++r) s += X[(int64_t)r * N + c];
-  out[c] = s;
+  if (c < N) {
+#pragma unroll 8
+    for (int r = rg; r < B; r += COL_GROUPS) s += X[(int64_t)r * N + c];
+  }
+  red[rg][l] = s;
+  __syncthreads();
+  if (rg == 0 && c < N) {
+    float t = 0.f;
+    for (int k = 0; k < COL_GROUPS; ++k) t += red[k][l];
+    out[c] = t;
+  }
 }
 
 // Adam on master weights W [rows x cols]; gradient G in the same layout, or
@@ -540,7 +643,7 @@ int qmprs_gemm_bf16(const void* A, int lda, const void* B, int ldb, int M, int N
   g.resid = resid;
   g.ldr = ldr;
   g.err = err;
-  dim3 grid(M / MLP_BM, 1, S);
+  dim3 grid(M / MLP_BM, (N + MLP_BN - 1) / MLP_BN, S);
   qm_note_launch();
   k_gemm_tc<<<grid, MLP_THREADS, MLP_SMEM_REQ, s>>>(g);
   if (S > 1) {
@@ -572,7 +675,7 @@ int qmprs_mlp_act_back(const float* dH, const float* Z, int B, int N, float* dZ,
 int qmprs_mlp_col_sum(const float* X, int B, int N, float* out, void* stream) {
   if (!X || !out || B <= 0 || N <= 0) return QMPRS_ERR_INVALID;
   qm_note_launch();
-  k_col_sum<<<(N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(X, B, N, out);
+  k_col_sum<<<(N + 31) / 32, 32 * COL_GROUPS, 0, (cudaStream_t)stream>>>(X, B, N, out);
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
 
