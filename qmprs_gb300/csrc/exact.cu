@@ -386,15 +386,6 @@ __device__ __forceinline__ void x_env_mac(DF (&e)[32], int i, xc u, xc v) {
   df_mac(e[2 * i + 1], -u.y, -u.w, v.x, v.z);
 }
 
-// sum over the block's warps of part `lane`, in fixed order
-__device__ __forceinline__ double x_sum_warps(const double (*wred)[32], int lane) {
-  double v[WARPS];
-#pragma unroll
-  for (int w = 0; w < WARPS; ++w) v[w] = wred[w][lane];
-  return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-}
-static_assert(WARPS == 8, "the sum over the warps is written out for eight");
-
 // Backward sweep step `step` of every active state (the reference's
 // per-gate update, qmprs/synthesis/mps_encoding/sequential.py:452-505):
 //   psi <- G^H psi                      (peel the gate from the circuit state)
@@ -406,10 +397,11 @@ static_assert(WARPS == 8, "the sum over the warps is written out for eight");
 __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int step, xc* psi, const xc* t,
                                                                 double2* gates, const signed char* arity,
                                                                 const int* nlayers, const int* active,
-                                                                double2* partials, double* nuc) {
+                                                                xc* partials, double* nuc) {
   __shared__ xc gs[16];
-  __shared__ double wred[WARPS][32];
-  __shared__ double2 env[16], gd[16];
+  __shared__ float2 wred[WARPS][32];
+  __shared__ xc env[16];
+  __shared__ double2 gd[16];
   __shared__ WarpPolar wp;
   GateSel sel;
   sel.mode = SEL_SWEEP;
@@ -485,21 +477,28 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
       }
     }
     // per warp (fixed exchange, double-float), then the block's warps in order
-    wred[warp][tid & 31] = warp_sum32_df(e);
+    {
+      const DF v = warp_sum32_df(e);
+      wred[warp][tid & 31] = make_float2(v.hi, v.lo);
+    }
     __syncthreads();
-    if (tid < 32) reinterpret_cast<double*>(partials + (int64_t)tile * 16)[tid] = x_sum_warps(wred, tid);
+    if (tid < 32) env_sum_warps(wred, partials + (int64_t)tile * 16, tid);
     __syncthreads();
     if (last_tile_ticket(bd.ticket, b, nt)) {
       const int entry = tid >> 4, l16 = tid & 15;
       const int t0 = bd.state_tile0[b];
-      double2 s = czero();
-      for (int tt = l16; tt < nt; tt += 16) s = cadd(s, ld_cg(&partials[(int64_t)(t0 + tt) * 16 + entry]));
+      XA s = xa_zero();
+      for (int tt = l16; tt < nt; tt += 16) {
+        const xc v = __ldcg(&partials[(int64_t)(t0 + tt) * 16 + entry]);
+        df_add(s.re, v.x, v.z);
+        df_add(s.im, v.y, v.w);
+      }
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) {
-        s.x += __shfl_down_sync(0xffffffffu, s.x, o, 16);
-        s.y += __shfl_down_sync(0xffffffffu, s.y, o, 16);
+        df_shfl_add(s.re, s.re, o);
+        df_shfl_add(s.im, s.im, o);
       }
-      if (l16 == 0) env[entry] = s;
+      if (l16 == 0) env[entry] = xa_round(s);
       if (tid < m * m) gd[tid] = gptr[tid];
       __syncthreads();
       if (tid < 32) {
@@ -507,11 +506,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
         // follow the current gate, and an FP32 completion of them would
         // enter the later steps at first order
         bool finite;
-        const double nn = warp_polar_exact(wp, env, gd, m, &finite);
+        const bool last = step == nlayers[b] * n - 1;
+        const double nn = warp_polar_exact(wp, env, gd, m, last, &finite);
         if (finite && tid < m * m) gptr[tid] = gd[tid];
         if (tid == 0) {
-          if (finite) nuc[b] = nn;
-          else atomicOr(bd.err, KERR_NONFINITE);
+          if (finite && last) nuc[b] = nn;
+          if (!finite) atomicOr(bd.err, KERR_NONFINITE);
           bd.ticket[b] = 0;
         }
       }
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
 // and over the warps in order.  As in k_sweep_fused the polar factor bounds
 // a step, and the other warps peel the next gate from psi meanwhile.
 // Measured (10 qubits, 15 layers, 2 sweeps, 300 steps): 51.2 ms with a
-// single-thread factor, 8.7 ms now (29 us a step).
+// single-thread factor, 4.5 ms now (15 us a step).
 __device__ __forceinline__ void x_fused_apply(xc* v, int n, int q, int k, const xc* gs, int tid, int step) {
   if (k == 2) {
     const int slo = n - 2 - q, dlo = 1 << slo, dhi = dlo << 1;
@@ -574,8 +574,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
   __shared__ xc gs[2][16];           // the gate to apply (rebuild), or to peel
   __shared__ xc gt[16];              // the new gate's adjoint
   __shared__ double2 gd[2][16];      // the step's gate and the next step's
-  __shared__ double wred[WARPS][32];
-  __shared__ double2 env[16];
+  __shared__ float2 wred[WARPS][32];
+  __shared__ xc env[16];
   __shared__ WarpPolar wp;
   const int b = blockIdx.x;
   if (b >= bd.B) return;
@@ -677,19 +677,22 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
           x_env_mac(e, 3, t1, y1);
         }
       }
-      wred[warp][lane] = warp_sum32_df(e);
+      {
+        const DF v = warp_sum32_df(e);
+        wred[warp][lane] = make_float2(v.hi, v.lo);
+      }
       if (fetch) {
         gd[buf ^ 1][tid] = pre;
         gs[buf ^ 1][(tid % (1 << k2)) * (1 << k2) + tid / (1 << k2)] = xc_from_d(cconj(pre));
       }
       __syncthreads();
       if (warp == 0) {
-        reinterpret_cast<double*>(env)[lane] = x_sum_warps(wred, lane);
+        env_sum_warps(wred, env, lane);
         __syncwarp();
         bool finite;
         double2* g = gd[buf];
-        const double nn = warp_polar_exact(wp, env, g, m, &finite);
-        if (finite) nuc = nn;
+        const double nn = warp_polar_exact(wp, env, g, m, j2 >= G, &finite);
+        if (finite && j2 >= G) nuc = nn;
         if (finite && lane < m * m) gb[(int64_t)slot * 16 + lane] = g[lane];
         if (!finite && lane == 0) atomicOr(bd.err, KERR_NONFINITE);
         if (lane < m * m) gt[(lane % m) * m + lane / m] = xc_from_d(cconj(g[lane]));
@@ -822,8 +825,8 @@ void launch_x_apply_gate(const BatchDev& bd, xc* vec, const GateSel& sel, cudaSt
 void launch_x_sweep_step(const BatchDev& bd, int step, xc* psi, const xc* t, double2* gates, const signed char* arity,
                          const int* nlayers, const int* active, double2* partials, double* nuc, cudaStream_t s) {
   qm_note_launch();
-  k_x_sweep_step<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, psi, t, gates, arity, nlayers, active, partials,
-                                                        nuc);
+  k_x_sweep_step<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, psi, t, gates, arity, nlayers, active,
+                                                        reinterpret_cast<xc*>(partials), nuc);
 }
 
 int launch_x_sweep_fused(const BatchDev& bd, int max_n, const xc* target, double2* gates, const signed char* arity,

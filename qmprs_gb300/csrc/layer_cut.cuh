@@ -9,7 +9,7 @@
 // state's last block diagonalises it and stores the vectors, the bond and
 // the site tensor.  A separate projection read and a separate eigenvalue
 // launch are gone: a cut of a 20-qubit state took 215 us (Gram 24, FP64
-// Jacobi of one thread 187, projection 4.7) and takes 35 us now.
+// Jacobi of one thread 187, projection 4.7) and takes 22 us now.
 //
 // The Gram's sums are exact FP32 products in double-float over a thread's
 // at most 16 rows and over the warp's lanes, FP64 across the
@@ -128,77 +128,33 @@ __device__ __forceinline__ void cut_rows(const typename P::T* src, typename P::T
   }
 }
 
-// Eigenvectors of the w x w Hermitian positive semidefinite Gram in ws.E
-// (unscaled, zero padded to 4 x 4) by one warp: one-sided Jacobi on its
-// columns, G V = U Lambda, started from FP32 sweeps.  ws.V receives the
-// vectors as columns in descending order of the eigenvalues (ties in index
-// order), lam[0..3] the eigenvalues of the Gram scaled by a power of two.
-__device__ __forceinline__ void warp_gram_eig(WarpPolar& ws, double* lam) {
+// Eigenvectors of the Gram g (warp_gram_vectors) by one warp, in descending
+// order of the eigenvalues (ties in index order): ws.B's columns, lam[0..3]
+// the eigenvalues times a power of two.
+__device__ __forceinline__ void warp_gram_eig(WarpPolar& ws, double2 g, double* lam) {
   const int lane = threadIdx.x & 31;
-  const int row = lane & 3, pr = (lane >> 2) & 1, ip = row * 4 + 2 * pr, iq = ip + 1;
-  const int ent = lane >> 1, i = ent >> 2, j = ent & 3, part = lane & 1;
-  const double eye = i == j && part == 0 ? 1.0 : 0.0;
-  {
-    const double2 e = ws.E[lane & 15];
-    const float mag = fmaxf(fabsf((float)e.x), fabsf((float)e.y));
-    const int mbits = __reduce_max_sync(0xffffffffu, __float_as_int(mag));
-    const int ex = mbits == 0 ? 0 : (mbits >> 23) - 126;
-    const double sc = __hiloint2double((1023 - ex) << 20, 0);
-    __syncwarp();
-    if (lane < 16) ws.E[lane] = cd(e.x * sc, e.y * sc);
-    __syncwarp();
-  }
-  int fp = 0, fq = 0, odd;
-  {
-    float2 ap = cf((float)ws.E[ip].x, (float)ws.E[ip].y), aq = cf((float)ws.E[iq].x, (float)ws.E[iq].y);
-    float2 vp = cf(row == 2 * pr ? 1.f : 0.f, 0.f), vq = cf(row == 2 * pr + 1 ? 1.f : 0.f, 0.f);
-    odd = wh_sweeps(ap, aq, vp, vq, fp, fq, false);
-    if (lane < 8) {
-      ws.V[ip] = f2d(vp);
-      ws.V[iq] = f2d(vq);
-    }
-  }
-  __syncwarp();
-#pragma unroll 1
-  for (int step = 0; step < 2; ++step) {
-    double v = wmm_part<true, false>(ws.V, ws.V, i, j, part);
-    wmm_store(ws.T, lane, 1.5 * eye - 0.5 * v);
-    __syncwarp();
-    v = wmm_part<false, false>(ws.V, ws.T, i, j, part);
-    __syncwarp();
-    wmm_store(ws.V, lane, v);
-    __syncwarp();
-  }
-  wmm_store(ws.U, lane, wmm_part<false, false>(ws.E, ws.V, i, j, part));
-  __syncwarp();
-  const double2* mine = (lane & 8) ? ws.V : ws.U;
-  double2 xp = mine[ip], xq = mine[iq];
-  odd ^= wx_sweeps(xp, xq, fp, fq, false);
-  const double al = quad_sum(cnorm2(xp)), be = quad_sum(cnorm2(xq));
-  double lp = al > WPX_TINY ? al * wp_rsqrt(al) : 0.0, lq = be > WPX_TINY ? be * wp_rsqrt(be) : 0.0;
-  // V's lanes take A's eigenvalues; original index of the column at a
-  // position: an odd number of sweeps leaves columns 2 and 3 exchanged
-  double l[4];
+  double p[4], l[4];
+  int odd;
+  warp_gram_vectors(ws, g, p, &odd);
 #pragma unroll
-  for (int cidx = 0; cidx < 4; ++cidx) {
-    const int pos = cidx >= 2 && odd ? 5 - cidx : cidx;
-    const double a = __shfl_sync(0xffffffffu, lp, (pos >> 1) * 4), b = __shfl_sync(0xffffffffu, lq, (pos >> 1) * 4);
-    l[cidx] = (pos & 1) ? b : a;
-  }
+  for (int c = 0; c < 4; ++c) l[c] = p[c >= 2 && odd ? 5 - c : c];   // by original index
+  // ranks by the order of the bits (the values are not negative): an FP64
+  // comparison takes 64 cycles
   int rk[4];
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     rk[a] = 0;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) rk[a] += l[b] > l[a] || (l[b] == l[a] && b < a);
+    for (int b = 0; b < 4; ++b) {
+      const long long x = __double_as_longlong(l[b]), y = __double_as_longlong(l[a]);
+      rk[a] += x > y || (x == y && b < a);
+    }
     if (lane == 0) lam[rk[a]] = l[a];
   }
-  const int cp = odd && pr ? 3 : 2 * pr, cq = odd && pr ? 2 : 2 * pr + 1;
+  double2 v = ws.B[lane & 15];
+  const int pos = lane & 3, idx = pos >= 2 && odd ? 5 - pos : pos;
   __syncwarp();
-  if (lane >= 8 && lane < 16) {
-    ws.V[row * 4 + (cp == 0 ? rk[0] : cp == 2 ? rk[2] : rk[3])] = xp;
-    ws.V[row * 4 + (cq == 1 ? rk[1] : cq == 3 ? rk[3] : rk[2])] = xq;
-  }
+  if (lane < 16) ws.B[(lane & 12) + (idx == 0 ? rk[0] : idx == 1 ? rk[1] : idx == 2 ? rk[2] : rk[3])] = v;
   __syncwarp();
 }
 
@@ -313,9 +269,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int st
   __syncthreads();
   const int w = 2 * r;
   if (tid < 32) {
-    if (tid < 16) {
-      const int a = tid >> 2, e = tid & 3;
-      double2 g = czero();
+    double2 g = czero();
+    {
+      const int a = (tid >> 2) & 3, e = tid & 3;
       if (a < w && e < w) {
         if (a == e) {
           g = cd(wred[0][a], 0.0);
@@ -324,10 +280,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int st
           g = cd(wred[0][k], a < e ? wred[0][k + 1] : -wred[0][k + 1]);
         }
       }
-      ws.E[tid] = g;
     }
-    __syncwarp();
-    warp_gram_eig(ws, lam);
+    warp_gram_eig(ws, g, lam);
     if (lane == 0) {
       s_keep = rank_by_cutoff(lam, w, QM_CUTOFF, 2);
       bond[c] = s_keep;
@@ -335,10 +289,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int st
     }
     __syncwarp();
     const int keep = s_keep;
-    warp_phase_fix(ws.V, keep);
+    warp_phase_fix(ws.B, keep);
     if (lane < 16) {
       const int a = lane >> 2, col = lane & 3;
-      const double2 v = a < w && col < keep ? ws.V[lane] : czero();
+      const double2 v = a < w && col < keep ? ws.B[lane] : czero();
       vs[lane] = v;
       vm[lane] = P::load_v(v);
       if (a < w && col < keep) site_t[((int64_t)b * bd.max_n + c) * 8 + col * w + a] = cconj(v);

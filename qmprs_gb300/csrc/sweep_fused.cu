@@ -9,8 +9,8 @@
 //   per gate (backward circuit order)
 //     psi <- G^H psi   peel the gate from the circuit state,
 //     E = sum_rest conj(t[a, rest]) psi[c, rest]   (FP32 per thread and
-//                      across a warp's lanes, FP64 across the warps, in
-//                      fixed order),
+//                      across a warp's lanes, double-float across the warps,
+//                      in fixed order),
 //     W = polar(E)     warp 0 (warp_polar.cuh; null directions towards the
 //                      current gate), G <- conj(W),
 //     t <- G^H t;
@@ -26,7 +26,7 @@
 // bounds it: peeling the next gate from psi does not depend on the new
 // gate, so the other warps do it meanwhile.
 // Measured (10 qubits, 15 layers, 4 sweeps, 600 steps): 29.1 ms with
-// a single-thread factor and the peel on the chain, 6.7 ms now (11 us a step).
+// a single-thread factor and the peel on the chain, 4.2 ms now (6 us a step).
 #include "warp_polar.cuh"
 
 __device__ __forceinline__ bool fused_valid(int k, int site, int n) { return k == 1 || (k == 2 && site <= n - 2); }
@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_sweep_fused(BatchDev bd, cons
   __shared__ float2 gs[2][16];       // the gate to apply (rebuild), or to peel
   __shared__ float2 gt[16];          // the new gate's adjoint
   __shared__ double2 gd[2][16];      // the step's gate and the next step's
-  __shared__ double wred[WARPS][32];
-  __shared__ double2 env[16];
+  __shared__ float2 wred[WARPS][32];
+  __shared__ xc env[16];
   __shared__ WarpPolar wp;
   const int b = blockIdx.x;
   if (b >= bd.B) return;
@@ -186,25 +186,21 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_sweep_fused(BatchDev bd, cons
         }
       }
       // over a warp's lanes in FP32 (a lane holds one to eight quads), over
-      // the warps in FP64
-      wred[warp][lane] = (double)warp_sum32(e);
+      // the warps in double-float
+      wred[warp][lane] = make_float2(warp_sum32(e), 0.f);
       if (fetch) {
         gd[buf ^ 1][tid] = pre;
         gs[buf ^ 1][(tid % (1 << k2)) * (1 << k2) + tid / (1 << k2)] = cf((float)pre.x, -(float)pre.y);
       }
       __syncthreads();
       if (warp == 0) {
-        double v[WARPS];
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) v[w] = wred[w][lane];
-        reinterpret_cast<double*>(env)[lane] =
-            ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        env_sum_warps(wred, env, lane);
         __syncwarp();
         bool finite = true;
         double2* g = gd[buf];
         if (env_out) {
           const bool mine = lane < m * m;
-          const double2 ev = mine ? env[lane] : czero();
+          const double2 ev = mine ? xc_to_d(env[lane]) : czero();
           finite = __all_sync(0xffffffffu, isfinite(ev.x) && isfinite(ev.y));
           if (mine && finite) env_out[bd.gate_off[b] + (int64_t)slot * 16 + lane] = ev;
         } else {
@@ -232,8 +228,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_sweep_fused(BatchDev bd, cons
     }
   }
 }
-static_assert(WARPS == 8, "the environment's sum over the warps is written out for eight");
-
 int launch_sweep_fused(const BatchDev& bd, int max_n, const float2* target, double2* gates, const signed char* arity,
                        const int* nlayers, int* active, const double2* tnorm2, int num_sweeps, double stop_fid,
                        double* sweep_fid, int* sweeps_done, cudaStream_t s, double2* env_out) {

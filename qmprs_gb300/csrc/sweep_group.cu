@@ -954,14 +954,14 @@ __device__ __forceinline__ void m_cols(const xc* src, xc* dst, int D, const xc* 
 // next step commutes with the rows' and runs on the other warps while warp
 // 0 computes the polar factor.
 // Measured on a 20-qubit state (three steps per group): 170 us per launch with
-// a single-thread factor and FP64 updates by 64 threads, 39 us now.
+// a single-thread factor and FP64 updates by 64 threads, 36 us now.
 #define POLAR_THREADS 256
 
 __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, GroupDev gd, int g, double2* gates,
                                                                const signed char* arity, const int* nlayers,
                                                                const int* active, double* nuc, double2* env_out) {
   __shared__ xc M[2][GMM];
-  __shared__ double2 env[16];
+  __shared__ xc env[16];
   __shared__ double2 gold[GMAXSTEPS][16];   // the steps' gates, replaced one by one
   __shared__ xc gx[GMAXSTEPS][16];          // the same in double-float
   __shared__ int sk[GMAXSTEPS], sh[GMAXSTEPS], sl[GMAXSTEPS];
@@ -1036,20 +1036,20 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
           const int ent = lane >> 1, part = lane & 1;
           if (ent < m * m) {
             const int r = gate_place(ent / m, k, sh[s], sl[s]), c = gate_place(ent % m, k, sh[s], sl[s]);
-            double acc = 0.0;
+            DF acc = {0.f, 0.f};
             for (int o = 0; o < D / m; ++o) {
               const int ob = spread_bits(o, k, sh[s], sl[s]);
               const xc v = M[cur][(r | ob) * GM + (c | ob)];
-              acc += part ? (double)v.y + (double)v.w : (double)v.x + (double)v.z;
+              df_add(acc, part ? v.y : v.x, part ? v.w : v.z);
             }
-            reinterpret_cast<double*>(env)[lane] = acc;
+            wdf_store(env, lane, acc);
           }
           __syncwarp();
           bool finite = true;
           const bool mine = lane < m * m;
           const int64_t at = bd.gate_off[b] + sslot[s] * 16 + lane;
           if (env_out) {   // environment at the fixed circuit: the gate stays
-            const double2 ev = mine ? env[lane] : czero();
+            const double2 ev = mine ? xc_to_d(env[lane]) : czero();
             finite = __all_sync(0xffffffffu, isfinite(ev.x) && isfinite(ev.y));
             if (mine && finite) env_out[at] = ev;
           } else {

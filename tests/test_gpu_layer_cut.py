@@ -71,3 +71,27 @@ def test_layers_at_unit_edges(eng, ns, kind, precision):
                 start, gs = s + 1, []
         psi = D.circuit_state([blocks], n)
         assert abs(abs(np.vdot(psi, sv)) / np.linalg.norm(sv) - abs(fids[0])) <= tol
+
+
+@pytest.mark.parametrize("precision", ["fast", "exact"])
+@pytest.mark.parametrize("gap", [0.0, 1e-9, 1e-7, 1e-6, 1e-5, 1e-3])
+def test_nearly_equal_singular_values(eng, gap, precision):
+    """(|0..0> + (1 + gap) |1..1>) under a unitary on each qubit: bond two at
+    every cut, so one layer prepares it to the working precision whichever
+    basis the nearly equal singular values take."""
+    exact = precision == "exact"
+    ns = [2, 5, 13]
+    p = eng.plan(ns, 1, 2, precision)
+    rng = np.random.default_rng(17)
+    states = []
+    for n in ns:
+        v = np.zeros([2] * n, complex)
+        v[(0,) * n], v[(1,) * n] = 1.0, 1.0 + gap
+        for k in range(n):
+            u = np.linalg.qr(rng.standard_normal((2, 2)) + 1j * rng.standard_normal((2, 2)))[0]
+            v = np.moveaxis(np.tensordot(u, v, (1, k)), 0, k)
+        states.append(v.reshape(-1) / np.linalg.norm(v))
+    t = torch.from_numpy(np.concatenate(states).astype(p.npdtype).view(np.float64 if exact else np.float32)).cuda()
+    lf = eng.stage_layers(p, t, 1, 1.0)[3].cpu().numpy().view(np.complex128)
+    for b, n in enumerate(ns):
+        assert abs(abs(lf[b]) - 1.0) <= 2 * n * (2.0 ** -44 if exact else 2.0 ** -23), n
