@@ -347,15 +347,15 @@ __device__ void smem_matmul(const double2* A, const double2* B, double2* Cm, int
 // (ten times the products' rounding; the truncation decides at 1e-10).
 // Three or four passes; a pass whose rotations were all below 3e-7 is the
 // last.  Measured (48 states, w = 64): about 6 ms per cut with FP64 products
-// and FP64 finishing sweeps, 1.5 ms now, two thirds of it the FP32 sweeps
-// (shared-memory traffic: 128 KB a round).
+// and FP64 finishing sweeps, 1.4 ms now, half of it the FP32 sweeps and half
+// the double-float products (three quarters of the FP32 pipes' rate).
 
 extern __shared__ double2 eig_sm[];
 __device__ __forceinline__ float2* tt_smf() { return reinterpret_cast<float2*>(eig_sm); }
 __device__ __forceinline__ xc* tt_smx() { return reinterpret_cast<xc*>(eig_sm); }
 
 #define JW (TT_EIG_THREADS / 32)
-static_assert(TT_EIG_SMEM_W / 2 <= 2 * JW, "two row pairs per warp");
+static_assert(JW == 16, "the Jacobi sweeps' warp roles");
 
 // p <- c p - conj(s) q, q <- s p + c q
 __device__ __forceinline__ void jacobi32_cols(float2& p, float2& q, float c, float sx, float sy) {
@@ -365,108 +365,256 @@ __device__ __forceinline__ void jacobi32_cols(float2& p, float2& q, float c, flo
   q = b;
 }
 
-// FP32 Jacobi sweeps (round-robin pairing) on the Hermitian g (row-major,
-// stride ld), accumulating v <- v R; both double-buffered with g2, v2.
-// Columns (and rows of g) sit at their position of the tournament: a round
-// pairs position l with w - 1 - l and writes every entry one position on, so
-// a lane's pair is always columns l and w - 1 - l (distinct banks, where
-// indexing by pair met two to four conflicts) and a whole sweep brings every
-// column home.  A lane computes its pair's rotation; a warp takes row pairs
-// warp, warp + 16, so every thread updates 2 x 2 blocks of g and two
-// rows of v and a round takes one barrier.  A pair rotates when |g_pq| is
-// above rel sqrt(|g_pp g_qq|) and floor_abs; sweeps repeat while a rotation
-// was above 1e-4 of sqrt(|g_pp g_qq|) (convergence is quadratic).  *moved: a
-// rotation of tangent above 3e-7 was made.  Returns v or v2, whichever holds
-// the result.  Uniform over the block.  The matrices are offsets into the
-// dynamic shared memory, so that every access is a shared-memory one.
-__device__ int jacobi32_run(int g, int g2, int v, int v2, int w, int ld, float rel, float floor_abs, bool* moved) {
-  float2* S = tt_smf();
-  const int half = w / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool act = lane < half;
-  const int pc = act ? lane : 0, qc = w - 1 - pc;
-  auto next = [&](int x) { return x == 0 ? 0 : x == 1 ? w - 1 : x - 1; };
-  const int pn = next(pc), qn = next(qc);
-  bool mv = false;
-  for (int sweep = 0; sweep < 30; ++sweep) {
-    bool again = false;
-    for (int k = 0; k < w - 1; ++k) {
-      float cc = 1.f, sx = 0.f, sy = 0.f;
-      if (act) {
-        const float2 x = S[g + pc * ld + qc];
-        const float app = S[g + pc * ld + pc].x, aqq = S[g + qc * ld + qc].x;
-        const float g2n = fmaf(x.x, x.x, x.y * x.y), sc = fabsf(app) * fabsf(aqq);
-        if (g2n > rel * rel * sc && g2n > floor_abs * floor_abs) {
-          const float d = 0.5f * (aqq - app);
-          const float ri = rsqrtf(fmaf(d, d, g2n));
-          const float c2 = fmaf(0.5f * fabsf(d), ri, 0.5f), ci = rsqrtf(c2);
-          const float f = copysignf(0.5f * ri * ci, d);
-          cc = c2 * ci;
-          sx = x.x * f;
-          sy = x.y * f;
-          again |= g2n > 1e-8f * sc;
-          mv |= fmaf(sx, sx, sy * sy) > 9e-14f * c2;
-        }
-      }
-      // both row pairs' loads come first: the stores may not be moved past them
-      float2 x[2][4], y[2][4];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int pr = warp + u * JW;
-        if (pr >= half || !act) continue;
-        const float2 *gp = S + g + pr * ld, *gq = S + g + (w - 1 - pr) * ld;
-        x[u][0] = gp[pc];
-        x[u][1] = gp[qc];
-        x[u][2] = gq[pc];
-        x[u][3] = gq[qc];
-        const float2 *vp = S + v + pr * ld, *vq = S + v + (pr + half) * ld;
-        y[u][0] = vp[pc];
-        y[u][1] = vp[qc];
-        y[u][2] = vq[pc];
-        y[u][3] = vq[qc];
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int pr = warp + u * JW;
-        if (pr >= half) continue;
-        const float cr = __shfl_sync(0xffffffffu, cc, pr);
-        const float rx = __shfl_sync(0xffffffffu, sx, pr), ry = __shfl_sync(0xffffffffu, sy, pr);
-        if (!act) continue;
-        // columns: col_p <- c col_p - s conj(e) col_q ; col_q <- s e col_p + c col_q
-        jacobi32_cols(x[u][0], x[u][1], cc, sx, sy);
-        jacobi32_cols(x[u][2], x[u][3], cc, sx, sy);
-        // rows: row_p <- c row_p - s e row_q ; row_q <- s conj(e) row_p + c row_q
-        jacobi32_cols(x[u][0], x[u][2], cr, rx, -ry);
-        jacobi32_cols(x[u][1], x[u][3], cr, rx, -ry);
-        if (pr == lane) {   // the rotated pair: real diagonal, eliminated off-diagonal
-          x[u][0].y = 0.f;
-          x[u][3].y = 0.f;
-          if (sx != 0.f || sy != 0.f) x[u][1] = x[u][2] = cf(0.f, 0.f);
-        }
-        jacobi32_cols(y[u][0], y[u][1], cc, sx, sy);
-        jacobi32_cols(y[u][2], y[u][3], cc, sx, sy);
-        float2 *op = S + g2 + next(pr) * ld, *oq = S + g2 + next(w - 1 - pr) * ld;
-        op[pn] = x[u][0];
-        op[qn] = x[u][1];
-        oq[pn] = x[u][2];
-        oq[qn] = x[u][3];
-        float2 *vp = S + v2 + pr * ld, *vq = S + v2 + (pr + half) * ld;
-        vp[pn] = y[u][0];
-        vp[qn] = y[u][1];
-        vq[pn] = y[u][2];
-        vq[qn] = y[u][3];
-      }
-      __syncthreads();
-      int t = g;
-      g = g2;
-      g2 = t;
-      t = v;
-      v = v2;
-      v2 = t;
-    }
-    if (!__syncthreads_or(again)) break;
+// ---- FP32 Jacobi sweeps in one block (w <= 64) ----
+//
+// Round-robin pairing by position: a round pairs position x with pw - 1 - x
+// (pair l: p = l, q = pw - 1 - l), and every column then moves to next(x),
+// so a sweep of pw - 1 rounds brings each one home.  pw is w rounded
+// up; the padding is zero and never rotates.  The block's warps take roles:
+//   warp 0        the rotations, one round ahead: lane l keeps pair l's
+//                 diagonal in registers and rotates the one entry the next
+//                 round's pair needs by itself, so that the angles of round
+//                 k + 1 are ready when the others finish round k;
+//   warps 1 - 8   v <- v R in registers: a lane holds a quarter of a row (a
+//                 warp one quarter of 32 rows, so that every angle is one
+//                 broadcast), whose columns change place by register, and
+//                 from quarter to quarter through shared memory;
+//   the others    G <- R^H G R on the 2 x 2 blocks of pairs R < C (G is
+//                 Hermitian; an entry is kept in the row of the smaller
+//                 pair), double-buffered in shared memory, the blocks of
+//                 pair rows P and half - 1 - P sharing a warp's lanes.
+// One barrier a round.  A pair rotates when |g_pq| is above rel sqrt(|g_pp
+// g_qq|) and floor_abs, and its entry counts as zero from then on; sweeps
+// repeat while a rotation was above 1e-4 of sqrt(|g_pp g_qq|) (convergence
+// is quadratic).  *moved: a rotation of tangent above 3e-7 was made.
+// With v in shared memory, both halves of G and the angles on the chain, a
+// round at w = 64 took 2800 cycles (128 KB of shared-memory traffic, 920 of
+// issue), 1050 now; the chain through warp 0 is about 500, which narrow
+// Grams take.
+#define JAC_G(buf) ((4 + (buf)) * TT_EIG_SMEM_W * (TT_EIG_SMEM_W + TT_EIG_PAD))
+#define JAC_SHARED (3 * TT_EIG_SMEM_W * (TT_EIG_SMEM_W + TT_EIG_PAD))
+struct JacShared {
+  float4 rot[2][TT_EIG_SMEM_W / 2];   // (c, Re s, Im s, 0) per pair
+  float2 edge[2][2][TT_EIG_SMEM_W / 16][TT_EIG_SMEM_W];   // columns between quarters: to the lower, to the upper
+  int again;
+};
+
+__device__ __forceinline__ int jac_next(int x, int pw) { return x == 0 ? 0 : x == 1 ? pw - 1 : x - 1; }
+
+static_assert(sizeof(JacShared) <= TT_EIG_SMEM_W * (TT_EIG_SMEM_W + TT_EIG_PAD) * sizeof(float2), "below JAC_G(0)");
+
+// Rotation of a pair with diagonal app, aqq and entry g: (c, Re s, Im s) and
+// the diagonal's shift.
+struct JacRot {
+  float c, sx, sy, shift;
+  bool again, moved;
+};
+__device__ __forceinline__ JacRot jac_rotation(float app, float aqq, float2 g, float rel, float floor_abs) {
+  JacRot o = {1.f, 0.f, 0.f, 0.f, false, false};
+  const float g2n = fmaf(g.x, g.x, g.y * g.y), sc = fabsf(app) * fabsf(aqq);
+  if (g2n > rel * rel * sc && g2n > floor_abs * floor_abs) {
+    const float d = 0.5f * (aqq - app);
+    const float ri = rsqrtf(fmaf(d, d, g2n));
+    const float c2 = fmaf(0.5f * fabsf(d), ri, 0.5f), ci = rsqrtf(c2);
+    const float h = copysignf(0.5f * ri * ci, d);
+    const float c = c2 * ci, sx = g.x * h, sy = g.y * h;
+    // unitary to rounding: rsqrtf's own errors would add up over the sweeps
+    const float e = 0.5f * fmaf(-sy, sy, fmaf(-sx, sx, fmaf(-c, c, 1.f)));
+    o.c = fmaf(c, e, c);
+    o.sx = fmaf(sx, e, sx);
+    o.sy = fmaf(sy, e, sy);
+    o.shift = h * ci * g2n;
+    o.again = g2n > 1e-8f * sc;
+    o.moved = fmaf(o.sx, o.sx, o.sy * o.sy) > 9e-14f * c2;
   }
-  *moved = __syncthreads_or(mv);
-  return v;
+  return o;
+}
+
+// NG groups of NP pairs to a row of v
+// (not inlined: the caller's values would leave the roles too few registers)
+template <int NP, int NG>
+__device__ __noinline__ bool jacobi32_sweeps(int vout, int w, int ld, float rel, float floor_abs) {
+  constexpr int PW = 2 * NP * NG, HALF = NP * NG, LJ = PW + 1, SPARE = PW * LJ;
+  constexpr int GWARP = 9, GWARPS = JW - GWARP, GIT = (HALF / 2 + GWARPS - 1) / GWARPS;
+  static_assert(SPARE + 32 <= TT_EIG_SMEM_W * (TT_EIG_SMEM_W + TT_EIG_PAD), "spare slots behind the matrix");
+  float2* S = tt_smf();
+  JacShared& js = *reinterpret_cast<JacShared*>(S + JAC_SHARED);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int buf = 0;
+  bool mv = false;
+  if (warp == 0) {
+    const bool act = lane < HALF;
+    const int l = act ? lane : HALF - 1;
+    const int R = l == 0 ? 0 : l == HALF - 1 ? HALF - 2 : l - 1, C = l == 0 ? 1 : l == HALF - 1 ? HALF - 1 : l + 1;
+    const int o00 = R * LJ + C, o01 = R * LJ + PW - 1 - C, o10 = (PW - 1 - R) * LJ + C,
+              o11 = (PW - 1 - R) * LJ + PW - 1 - C;
+    const bool rowq = l != 0, colq = l == HALF - 1;
+    // where the pair's own entry, now zero, goes
+    const int zero = jac_next(l, PW) * LJ + jac_next(PW - 1 - l, PW);
+    float app = S[JAC_G(0) + l * LJ + l].x, aqq = S[JAC_G(0) + (PW - 1 - l) * (LJ + 1)].x;
+    JacRot r = jac_rotation(app, aqq, S[JAC_G(0) + l * LJ + PW - 1 - l], rel, floor_abs);
+    if (act) js.rot[0][l] = make_float4(r.c, r.sx, r.sy, 0.f);
+    bool again = act && r.again, pend = act && r.moved;
+    __syncthreads();
+    for (int sweep = 0; sweep < 30; ++sweep) {
+      mv |= pend;
+      for (int k = 0; k < PW - 1; ++k) {
+        if (k == PW - 2) {
+          const bool any = __any_sync(0xffffffffu, again);
+          if (lane == 0) js.again = any;
+          again = false;
+        }
+        const float2* g = S + JAC_G(buf);
+        const float2 x00 = g[o00], x01 = g[o01], x10 = g[o10], x11 = g[o11];
+        const float4 rr = js.rot[buf][R], rc = js.rot[buf][C];
+        // the diagonals after this round, at their new pairs
+        const float np = app - r.shift, nq = aqq + r.shift;
+        const float dn = __shfl_down_sync(0xffffffffu, np, 1), up = __shfl_up_sync(0xffffffffu, nq, 1);
+        app = l == 0 ? np : l == HALF - 1 ? nq : dn;
+        aqq = l == 0 ? dn : up;
+        // columns (c, -conj(s)) or (s, c), rows (c, -s) or (conj(s), c)
+        const float2 ca = colq ? cf(rc.y, rc.z) : cf(rc.x, 0.f), cb = colq ? cf(rc.x, 0.f) : cf(-rc.y, rc.z);
+        const float2 ra = rowq ? cf(rr.y, -rr.z) : cf(rr.x, 0.f), rb = rowq ? cf(rr.x, 0.f) : cf(-rr.y, -rr.z);
+        float2 top = fmac(fmac(cf(0.f, 0.f), ca, x00), cb, x01);
+        float2 bot = fmac(fmac(cf(0.f, 0.f), ca, x10), cb, x11);
+        float2 e = fmac(fmac(cf(0.f, 0.f), ra, top), rb, bot);
+        if (l != 0) e.y = -e.y;
+        r = jac_rotation(app, aqq, e, rel, floor_abs);
+        if (act) {
+          js.rot[buf ^ 1][l] = make_float4(r.c, r.sx, r.sy, 0.f);
+          S[JAC_G(buf ^ 1) + zero] = cf(0.f, 0.f);
+        }
+        again |= act && r.again;
+        pend = act && r.moved;
+        if (k < PW - 2) mv |= pend;
+        __syncthreads();
+        buf ^= 1;
+      }
+      if (!js.again) break;
+    }
+  } else if (warp < GWARP) {
+    const int h = (warp - 1) & 3, row = ((warp - 1) >> 2) * 32 + lane;
+    const bool idle = h >= NG || row - lane >= w;
+    float2 p[NP], q[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int l = h * NP + i;
+      p[i] = cf(row == l ? 1.f : 0.f, 0.f);
+      q[i] = cf(row == PW - 1 - l ? 1.f : 0.f, 0.f);
+    }
+    __syncthreads();
+    for (int sweep = 0; sweep < 30; ++sweep) {
+      for (int k = 0; k < PW - 1; ++k) {
+        if (!idle) {
+          if (k + sweep > 0) {
+            if (h > 0) q[0] = js.edge[buf ^ 1][1][h - 1][row];
+            if (h < NG - 1) (NP == 1 && h == 0 ? q[0] : p[NP - 1]) = js.edge[buf ^ 1][0][h + 1][row];
+          }
+          const float4* rot = js.rot[buf] + h * NP;
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            const float4 r = rot[i];
+            jacobi32_cols(p[i], q[i], r.x, r.y, r.z);
+          }
+          // every column one position on; the ends go by shared memory
+          const float2 p0 = p[0], p1 = p[NP > 1 ? 1 : 0], q0 = q[NP - 1];
+          if (h > 0) js.edge[buf][0][h][row] = p0;
+          if (h < NG - 1) js.edge[buf][1][h][row] = q0;
+#pragma unroll
+          for (int i = NP - 1; i > 0; --i) q[i] = q[i - 1];
+#pragma unroll
+          for (int i = 0; i < NP - 1; ++i) p[i] = p[i + 1];
+          if (h == 0) p[0] = p0, q[0] = p1;
+          if (h == NG - 1) p[NP - 1] = q0;
+        }
+        __syncthreads();
+        buf ^= 1;
+      }
+      if (!js.again) break;
+    }
+    if (!idle) {   // the last round's exchange
+      if (h > 0) q[0] = js.edge[buf ^ 1][1][h - 1][row];
+      if (h < NG - 1) (NP == 1 && h == 0 ? q[0] : p[NP - 1]) = js.edge[buf ^ 1][0][h + 1][row];
+    }
+    if (!idle && row < w)
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const int l = h * NP + i;
+        if (l < w) S[vout + row * ld + l] = p[i];
+        if (PW - 1 - l < w) S[vout + row * ld + PW - 1 - l] = q[i];
+      }
+  } else {
+    int R[GIT], C[GIT], st[GIT][4];
+    bool act[GIT], flip[GIT];
+#pragma unroll
+    for (int u = 0; u < GIT; ++u) {
+      const int P = warp - GWARP + u * GWARPS;
+      act[u] = P < HALF / 2 && lane < HALF && lane != P;
+      R[u] = lane > P ? P : HALF - 1 - P;
+      C[u] = lane > P ? lane : HALF - 1 - lane;
+      if (!act[u]) R[u] = 0, C[u] = 1;
+      flip[u] = false;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int x = jac_next(e & 2 ? PW - 1 - R[u] : R[u], PW), y = jac_next(e & 1 ? PW - 1 - C[u] : C[u], PW);
+        const int px = min(x, PW - 1 - x), py = min(y, PW - 1 - y);
+        st[u][e] = px < py ? x * LJ + y : px > py ? y * LJ + x : SPARE + lane;   // the next pair's own: warp 0 has it
+        if (e == 2) flip[u] = px > py;
+      }
+    }
+    __syncthreads();
+    for (int sweep = 0; sweep < 30; ++sweep) {
+      for (int k = 0; k < PW - 1; ++k) {
+        const float2* g = S + JAC_G(buf);
+        float2* o = S + JAC_G(buf ^ 1);
+#pragma unroll
+        for (int u = 0; u < GIT; ++u) {
+          if (!act[u]) continue;
+          const float4 rc = js.rot[buf][C[u]], rr = js.rot[buf][R[u]];
+          const float2 *g0 = g + R[u] * LJ, *g1 = g + (PW - 1 - R[u]) * LJ;
+          float2 x00 = g0[C[u]], x01 = g0[PW - 1 - C[u]], x10 = g1[C[u]], x11 = g1[PW - 1 - C[u]];
+          // columns: col_p <- c col_p - conj(s) col_q ; col_q <- s col_p + c col_q
+          jacobi32_cols(x00, x01, rc.x, rc.y, rc.z);
+          jacobi32_cols(x10, x11, rc.x, rc.y, rc.z);
+          // rows: row_p <- c row_p - s row_q ; row_q <- conj(s) row_p + c row_q
+          jacobi32_cols(x00, x10, rr.x, rr.y, -rr.z);
+          jacobi32_cols(x01, x11, rr.x, rr.y, -rr.z);
+          if (flip[u]) x10.y = -x10.y;
+          o[st[u][0]] = x00;
+          o[st[u][1]] = x01;
+          o[st[u][2]] = x10;
+          o[st[u][3]] = x11;
+        }
+        __syncthreads();
+        buf ^= 1;
+      }
+      if (!js.again) break;
+    }
+  }
+  return __syncthreads_or(mv);
+}
+
+// V (stride ld, at offset vout of the shared memory) of the Hermitian w x w
+// matrix g(i, j).
+template <class F>
+__device__ bool jacobi32_run(F g, int vout, int w, int ld, float rel, float floor_abs) {
+  // pw: 4, 8, 16, 24, 32, 48 or 64
+  const int pw = w <= 4 ? 4 : w <= 8 ? 8 : w <= 32 ? (w + 7) / 8 * 8 : (w + 15) / 16 * 16;
+  float2* S = tt_smf() + JAC_G(0);
+  for (int e = threadIdx.x; e < pw * pw; e += blockDim.x) {
+    const int i = e / pw, j = e % pw;
+    S[i * (pw + 1) + j] = i < w && j < w ? g(i, j) : cf(0.f, 0.f);
+  }
+  __syncthreads();
+  switch (pw) {
+    case 4: return jacobi32_sweeps<1, 2>(vout, w, ld, rel, floor_abs);
+    case 8: return jacobi32_sweeps<1, 4>(vout, w, ld, rel, floor_abs);
+    case 16: return jacobi32_sweeps<2, 4>(vout, w, ld, rel, floor_abs);
+    case 24: return jacobi32_sweeps<3, 4>(vout, w, ld, rel, floor_abs);
+    case 32: return jacobi32_sweeps<4, 4>(vout, w, ld, rel, floor_abs);
+    case 48: return jacobi32_sweeps<6, 4>(vout, w, ld, rel, floor_abs);
+    default: return jacobi32_sweeps<8, 4>(vout, w, ld, rel, floor_abs);
+  }
 }
 
 // A 4 x 2 block of outputs of a w x w product: rows r0 .. (rows past w - 1
@@ -553,20 +701,21 @@ static_assert(TT_EIG_SMEM_W / 2 * (TT_EIG_SMEM_W / 4) <= TT_EIG_THREADS, "one bl
 // work matrix, the FP32 copies in the last two.
 __device__ void tt_df_eig(xc* Vg, int w, int ld) {
   xc *G = tt_smx(), *vk = tt_smx() + w * ld, *t = tt_smx() + 2 * w * ld;
-  float2 *v32 = tt_smf() + 2 * w * ld, *t32 = tt_smf() + 4 * w * ld;
-  TTBlock o, u;
-  const bool mine = tt_block(w, threadIdx.x, false, o), uppr = tt_block(w, threadIdx.x, true, u);
+  float2* t32 = tt_smf() + 4 * w * ld;
   for (int pass = 0; pass < 6; ++pass) {
-    for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-      const int i = e / w, j = e % w;
-      const xc g = G[i * ld + j];
-      t32[i * ld + j] = cf(g.x, i == j ? 0.f : g.y);
-      v32[i * ld + j] = cf(i == j ? 1.f : 0.f, 0.f);
-    }
-    __syncthreads();
-    bool moved;
-    const float2* vr = tt_smf() + jacobi32_run(4 * w * ld, 5 * w * ld, 2 * w * ld, 3 * w * ld, w, ld, 1e-7f,
-                                               pass == 0 ? 1e-7f : 1e-13f, &moved);
+    const bool moved = jacobi32_run(
+        [&](int i, int j) {
+          const xc g = G[i * ld + j];
+          return cf(g.x, i == j ? 0.f : g.y);
+        },
+        2 * w * ld, w, ld, 1e-7f, pass == 0 ? 1e-7f : 1e-13f);
+    const float2* vr = tt_smf() + 2 * w * ld;
+    // the thread's blocks, computed anew in every pass: kept over the sweeps
+    // they would be spilled
+    int tid;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    TTBlock o, u;
+    const bool mine = tt_block(w, tid, false, o), uppr = tt_block(w, tid, true, u);
     if (!moved) {
       // V_k = I + X with X below 3e-7: D = -(X + X^H + X^H X) / 2 and the
       // products with X or D are FP32, and G's diagonal stands (X changes it

@@ -26,7 +26,8 @@ def eng(cuda_lib):
 
 @pytest.mark.parametrize("precision", ["fast", "exact"])
 @pytest.mark.parametrize("n,bonds,chi", [(2, [1, 2], 4), (5, [3], 3), (11, [1, 3, 5, 7], 16),
-                                         (12, [21, 31, 32], 32), (13, [17, 32, 29], 24), (16, [4, 9], 8)])
+                                         (12, [21, 31, 32], 32), (13, [17, 32, 29], 24), (16, [4, 9], 8),
+                                         (9, [9, 11, 12], 12)])
 def test_sites_and_target(eng, n, bonds, chi, precision):
     exact = precision == "exact"
     states = [S.random_mps(n, bd, 11 * n + bd) for bd in bonds]
@@ -49,3 +50,39 @@ def test_sites_and_target(eng, n, bonds, chi, precision):
         got = tv[p.vec_off[b]: p.vec_off[b] + 2 ** n]
         tol = 4 * n * (2.0 ** -44 if exact else 2.0 ** -23) * 1e2
         assert np.linalg.norm(got - D.mps_to_dense(ref)) <= tol
+
+
+@pytest.mark.parametrize("kind", ["rank_one", "two_blocks", "flat"])
+@pytest.mark.parametrize("n,chi", [(4, 4), (8, 12), (10, 20), (11, 32)])
+def test_spectra_at_padded_widths(eng, n, chi, kind):
+    """Spectra the Jacobi sweeps meet at their edges: nothing to rotate, an
+    exact block structure with zero entries, all eigenvalues equal up to
+    rounding.  The bonds are within the capacity, so the target is the state
+    itself; the bound is test_sites_and_target's."""
+    rng = np.random.default_rng(n)
+    if kind == "rank_one":
+        v = np.ones(1)
+        for _ in range(n):
+            v = np.kron(v, rng.standard_normal(2) + 1j * rng.standard_normal(2))
+    elif kind == "two_blocks":   # (|0>|a> + |1>|b>) |0> |c>, a and b product states
+        a, b, c = np.ones(1), np.ones(1), np.ones(1)
+        for _ in range((n - 2) // 2):
+            a, b, c = (np.kron(x, rng.standard_normal(2) + 1j * rng.standard_normal(2)) for x in (a, b, c))
+        rest = n - 2 - (n - 2) // 2 * 2
+        v = np.kron(np.kron(np.concatenate([a, b]), [1.0, 0.0]), np.kron(c, [1.0] + [0.0] * (2 ** rest - 1)))
+    else:   # pairs (q, q + k) maximally entangled, k < chi's bits
+        k = int(np.log2(chi))
+        v = np.zeros([2] * n)
+        for bits in range(2 ** k):
+            idx = [0] * n
+            for j in range(k):
+                idx[j] = idx[n - k + j] = (bits >> j) & 1
+            v[tuple(idx)] = 1.0
+        v = v.reshape(-1).astype(complex)
+    v = v / np.linalg.norm(v)
+    p = eng.plan([n], 1, chi, "fast")
+    v32 = v.astype(p.npdtype)
+    _, bd, target = eng.stage_mps(p, torch.from_numpy(v32.view(np.float32)).cuda(), chi)
+    assert int(bd.cpu().max()) <= (1 if kind == "rank_one" else 2 if kind == "two_blocks" else chi)
+    got = target.cpu().numpy().view(p.npdtype)
+    assert np.linalg.norm(got - v32) <= 4 * n * 2.0 ** -23 * 1e2
