@@ -8,10 +8,11 @@
 //    32) is cut into blocks of 16 indices; a round pairs the blocks
 //    (round-robin tournament) and every pair is one 32 x 32 subproblem.
 //      k_bj_solve   one block per pair: the subproblem in shared memory,
-//                   one cyclic Jacobi sweep (31 rounds of 16 disjoint
-//                   rotations, each applied to 2 x 2 entry groups), the
-//                   accumulated 32 x 32 unitary J, and the rotated
-//                   diagonal tile written back;
+//                   cyclic Jacobi rounds of 16 disjoint rotations, each
+//                   applied to 2 x 2 entry groups (of all pairs in the
+//                   sweep's first round, of those between the two blocks in
+//                   the others), the accumulated 32 x 32 unitary J, and the
+//                   rotated diagonal tile written back;
 //      k_bj_update  A[P,Q] <- J_P^H A[P,Q] J_Q on every off-diagonal tile of
 //                   the round (upper triangle, mirrored) and V[:,Q] <- V J_Q.
 //    Sweeps run until one sweep makes no rotation larger than 1e-5 of
@@ -159,9 +160,14 @@ __device__ __forceinline__ void bj_rotate(float2& p, float2& q, float c, float s
   q = y;
 }
 
-// One block per pair of round k: one Jacobi sweep of the 32 x 32
-// subproblem; J (32 x 32, row-major) to Jbuf[pair]; the rotated diagonal
-// tile back into A.  count += 1 if a rotation was above 1e-5 relative.
+// One block per pair of round k: Jacobi rounds on the 32 x 32 subproblem; J
+// (32 x 32, row-major) to Jbuf[pair]; the rotated diagonal tile back into A.
+// count += 1 if a rotation was above 1e-5 relative.  The sweep's first round
+// takes all pairs of a subproblem (31 inner rounds), the others (CROSS) only
+// those between the two blocks (16 inner rounds), so that a sweep takes
+// every pair once: with all pairs in every round a Gram took as many sweeps
+// (random spectra: 132 and 133 over a state's nine cuts; Gaussian mixtures
+// 140 and 142), at twice the inner rounds.
 //
 // Rows and columns sit at their position of the inner tournament: a round
 // pairs position l with 31 - l and writes every entry one position on, so
@@ -170,16 +176,18 @@ __device__ __forceinline__ void bj_rotate(float2& p, float2& q, float c, float s
 // entry group of pairs (gr, gc); lane l of a warp computes the rotation of
 // pair l % 16 (its gc) and takes gr's from lane gr.  The subproblem and J are
 // double-buffered (read one copy, write the other), so an inner round takes
-// one barrier.  The 31 rounds are a chain of dependent rotations, so the
+// one barrier.  The inner rounds are a chain of dependent rotations, so the
 // rotation is built from three approximate reciprocals: the complex tangent
 // w = g / (|d| + sqrt(d^2 + |g|^2)), d half the diagonal's difference, then
 // c = 1 / sqrt(1 + |w|^2) (exactly 1 for a tiny w: no drift of the norms).
 // A pair rotates when |g| is above FP32 resolution (1e-7 relative, or
 // floor_abs).
 // Measured (W = 512, 16 blocks): 25.7 us with indexed pairs and correctly
-// rounded square roots and reciprocals, 12.7 us now (k_bj_update, whose
+// rounded square roots and reciprocals, 12.7 us without, 7.9 us over a sweep
+// whose later rounds take the crossing pairs only (k_bj_update, whose
 // indices took divisions too, 10.7 -> 6.9 us).
 #define BJ_LD (BJ_S + 2)
+template <bool CROSS>
 __global__ void __launch_bounds__(BJ_THREADS) k_bj_solve(float2* A, int W, int nb, int k, float2* Jbuf,
                                                          const double* stats, int* count) {
   __shared__ float2 a[2][BJ_S][BJ_LD];
@@ -199,11 +207,16 @@ __global__ void __launch_bounds__(BJ_THREADS) k_bj_solve(float2* A, int W, int n
   __syncthreads();
   const int gr = tid / (BJ_S / 2), gc = tid % (BJ_S / 2);
   const int pr = gr, qr = BJ_S - 1 - gr, pc = gc, qc = BJ_S - 1 - gc;
-  // position x moves to x - 1, 1 to 31; 0 stays
-  const int prn = pr == 0 ? 0 : pr == 1 ? BJ_S - 1 : pr - 1, qrn = qr - 1;
-  const int pcn = pc == 0 ? 0 : pc == 1 ? BJ_S - 1 : pc - 1, qcn = qc - 1;
+  // all pairs: position x moves to x - 1, 1 to 31, 0 stays; between the
+  // blocks: the first 16 stay, the others turn
+  auto next = [&](int x) {
+    if (CROSS) return x < BJ_B ? x : x == BJ_B ? BJ_S - 1 : x - 1;
+    return x == 0 ? 0 : x == 1 ? BJ_S - 1 : x - 1;
+  };
+  const int prn = next(pr), qrn = next(qr), pcn = next(pc), qcn = next(qc);
+  constexpr int rounds = CROSS ? BJ_B : BJ_S - 1;
   bool big = false;
-  for (int ir = 0; ir < BJ_S - 1; ++ir) {
+  for (int ir = 0; ir < rounds; ++ir) {
     const float2 (*cur)[BJ_LD] = a[ir & 1];
     float2 (*nxt)[BJ_LD] = a[(ir + 1) & 1];
     const float2 (*jc)[BJ_LD] = j[ir & 1];
@@ -250,11 +263,11 @@ __global__ void __launch_bounds__(BJ_THREADS) k_bj_solve(float2* A, int W, int n
     __syncthreads();
   }
   const int any_big = __syncthreads_or(big);
-  const float2 (*fin)[BJ_LD] = a[(BJ_S - 1) & 1];
+  const float2 (*fin)[BJ_LD] = a[rounds & 1];
   float2* jo = Jbuf + (int64_t)pair * BJ_S * BJ_S;
   for (int e = tid; e < BJ_S * BJ_S; e += BJ_THREADS) {
     const int r = e / BJ_S, c = e % BJ_S;
-    jo[e] = j[(BJ_S - 1) & 1][r][c];
+    jo[e] = j[rounds & 1][r][c];
     // Hermitian diagonal tile: the upper triangle and its mirror
     const float2 v = r <= c ? fin[r][c] : cf(fin[c][r].x, -fin[c][r].y);
     A[(int64_t)at(r) * W + at(c)] = v;
@@ -995,7 +1008,10 @@ static int bj_fp32(const double2* H, int n, BJScratch& sc, cudaStream_t s, int* 
     if (e != cudaSuccess) return (int)e;
     for (int k = 0; k < nb - 1; ++k) {
       qm_note_launch();
-      k_bj_solve<<<np, BJ_THREADS, 0, s>>>(sc.A, W, nb, k, sc.J, sc.stats, sc.count);
+      if (k > 0)
+        k_bj_solve<true><<<np, BJ_THREADS, 0, s>>>(sc.A, W, nb, k, sc.J, sc.stats, sc.count);
+      else
+        k_bj_solve<false><<<np, BJ_THREADS, 0, s>>>(sc.A, W, nb, k, sc.J, sc.stats, sc.count);
       if (nA + nV > 0) {
         qm_note_launch();
         k_bj_update<<<nA + nV, BJU_THREADS, 0, s>>>(sc.A, sc.V, W, nb, k, sc.J, nA);
