@@ -1,5 +1,6 @@
 """The tile passes over chunks of every length the plan picks: one tile per
-chunk (a few tiles), two, four, eight, and several states sharing a launch.
+chunk (a few tiles), two, four, eight, three (a last chunk of two), and several
+states sharing a launch.
 
 Every gate's environment against the oracle.  An environment is a sum of
 products of amplitudes that passed each gate at most twice through
@@ -28,7 +29,7 @@ def _unitary(rng, m):
     return q * (np.diag(r) / np.abs(np.diag(r)))
 
 
-@pytest.mark.parametrize("ns", [[14], [15, 12, 11, 3], [20], [21, 16], [22]])
+@pytest.mark.parametrize("ns", [[14], [15, 12, 11, 3], [20], [21, 16], [22], [16] * 40])
 def test_environments_over_chunk_lengths(eng, ns):
     L = 1
     rng = np.random.default_rng(sum(ns))
