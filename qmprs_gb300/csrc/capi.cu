@@ -330,9 +330,9 @@ uint64_t plan_signature(const qmprs_plan* p) {
   mix((uint64_t)p->max_layers);
   return h;
 }
-// Tiles per chunk of the grouped sweep's passes: the fewest, at most GCHUNK,
-// that leave the batch one wave of blocks (four per SM) and its largest state
-// 256 chunks.  The passes wait on memory, so every SM should have all its
+// Tiles per chunk of the grouped sweep's passes: the fewest, up to 16 and else
+// GCHUNK, that leave the batch one wave of blocks (four per SM) and its
+// largest state 256 chunks.  The passes wait on memory, so every SM should have all its
 // blocks; a chunk's set-up (offset tables, composed gates) costs about one
 // tile, so a second wave does not pay, and every chunk adds a partial to the
 // polar kernel's sum over its state.
@@ -343,17 +343,16 @@ uint64_t plan_signature(const qmprs_plan* p) {
 // 28.6 ms, and later 17.0 ms with 16 tiles (432 chunks), 16.0 ms with 12 (one wave).
 #define CHUNKS_PER_STATE 256
 int choose_chunk_tiles(const std::vector<int>& n) {
-  int tiles = 1;
-  for (; tiles < GCHUNK; ++tiles) {
+  for (int tiles = 1; tiles <= 16; ++tiles) {
     int64_t chunks = 0, most = 0;
     for (int q : n) {
       const int64_t c = q > GT ? (ipow2(q - GT) + tiles - 1) / tiles : 1;
       chunks += c;
       most = std::max(most, c);
     }
-    if (chunks <= PASS_GRID_DEFAULT && most <= CHUNKS_PER_STATE) break;
+    if (chunks <= PASS_GRID_DEFAULT && most <= CHUNKS_PER_STATE) return tiles;
   }
-  return tiles;
+  return GCHUNK;
 }
 
 inline uint64_t dbl_key(double v) {
