@@ -834,6 +834,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   gd.chunk_idx = p->d_chunk_idx;
   gd.state_chunk0 = p->d_state_chunk0;
   gd.state_nchunks = p->d_state_nchunks;
+  gd.most_chunks = *std::max_element(state_nchunks.begin(), state_nchunks.end());
   gd.grp = p->d_grp;
   gd.ngroups = p->d_ngroups;
   gd.old_gates = p->d_old_gates;

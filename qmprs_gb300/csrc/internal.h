@@ -132,6 +132,7 @@ struct GroupDev {
   const int* chunk_idx;      // [nchunks] chunk index within its state
   const int* state_chunk0;   // [B]
   const int* state_nchunks;  // [B]
+  int most_chunks;           // of one state
   GroupEnt* grp;             // [B * gmax]
   int* ngroups;              // [B]
   double2* old_gates;        // [B * GMAXSTEPS * 16] gates replaced by the last group

@@ -33,10 +33,14 @@
 // vectors are not needed: the sweep's fidelity is the last step's trace.
 #include <cuda_fp16.h>
 
+#include <cooperative_groups.h>
+
 #include "dfloat.cuh"
 #include "tile_layout.h"
 #include "warp_polar.cuh"
 #include "window.cuh"
+
+namespace cg = cooperative_groups;
 
 // Gate of state b at backward step j: generated layer j / n, site
 // n - 1 - j % n.
@@ -915,28 +919,36 @@ __device__ __forceinline__ int gate_place(int v, int k, int h, int l) {
 }
 
 // dst <- G^T src on the rows of gate bits (h, l): the target-side update
-// z <- P z with P = G^H maps M to conj(P) M = G^T M.
-__device__ __forceinline__ void m_rows(const xc* src, xc* dst, int D, const xc* G, int k, int h, int l, int tid,
+// z <- P z with P = G^H maps M to conj(P) M = G^T M.  M is 2^u x 2^u; the real
+// and the imaginary part of an entry are two threads'.
+__device__ __forceinline__ void m_rows(const xc* src, xc* dst, int u, const xc* G, int k, int h, int l, int tid,
                                        int step) {
   const int m = 1 << k, clear = ~gate_place(m - 1, k, h, l);
-  for (int e = tid; e < D * D; e += step) {
-    const int i = e / D, c = e % D, r = gate_bits(i, k, h, l), base = i & clear;
-    XA acc = xa_zero();
-    for (int rp = 0; rp < m; ++rp) xa_mac(acc, G[rp * m + r], src[(base | gate_place(rp, k, h, l)) * GM + c]);
-    dst[i * GM + c] = xa_round(acc);
+  for (int t = tid; t < 2 << (2 * u); t += step) {
+    const int part = t & 1, i = t >> (u + 1), c = (t >> 1) & ((1 << u) - 1), r = gate_bits(i, k, h, l), base = i & clear;
+    DF p = {0.f, 0.f}, q = {0.f, 0.f};   // two chains
+#pragma unroll
+    for (int rp = 0; rp < 4; ++rp) {
+      if (rp >= m) break;
+      const xc g = G[(rp << k) + r], x = src[(base | gate_place(rp, k, h, l)) * GM + c];
+      df_mac(p, g.x, g.z, part ? x.y : x.x, part ? x.w : x.z);
+      df_mac(q, part ? g.y : -g.y, part ? g.w : -g.w, part ? x.x : x.y, part ? x.z : x.w);
+    }
+    df_add(p, q.hi, q.lo);
+    wdf_store(dst, 2 * (i * GM + c) + part, p);
   }
 }
 
 // dst <- src Q^T on the columns of gate bits (h, l), Q = G^H: the
 // circuit-side peel x <- Q x.  (M Q^T)[i][c] = sum_c' M[i][c'] conj(G[c'][c]).
-__device__ __forceinline__ void m_cols(const xc* src, xc* dst, int D, const xc* G, int k, int h, int l, int tid,
+__device__ __forceinline__ void m_cols(const xc* src, xc* dst, int u, const xc* G, int k, int h, int l, int tid,
                                        int step) {
   const int m = 1 << k, clear = ~gate_place(m - 1, k, h, l);
-  for (int e = tid; e < D * D; e += step) {
-    const int i = e / D, c = e % D, r = gate_bits(c, k, h, l), base = c & clear;
+  for (int e = tid; e < 1 << (2 * u); e += step) {
+    const int i = e >> u, c = e & ((1 << u) - 1), r = gate_bits(c, k, h, l), base = c & clear;
     XA acc = xa_zero();
     for (int cp = 0; cp < m; ++cp)
-      xa_mac(acc, xc_conj(G[cp * m + r]), src[i * GM + (base | gate_place(cp, k, h, l))]);
+      xa_mac(acc, xc_conj(G[(cp << k) + r]), src[i * GM + (base | gate_place(cp, k, h, l))]);
     dst[i * GM + c] = xa_round(acc);
   }
 }
@@ -954,21 +966,28 @@ __device__ __forceinline__ void m_cols(const xc* src, xc* dst, int D, const xc* 
 // next step commutes with the rows' and runs on the other warps while warp
 // 0 computes the polar factor.
 // Measured on a 20-qubit state (three steps per group): 170 us per launch with
-// a single-thread factor and FP64 updates by 64 threads, 36 us now.
+// a single-thread factor and FP64 updates by 64 threads, 36 us with warp_polar.
+// The sum over the chunks' partials (256 x 4 KB for one 20-qubit state) took
+// 22000 cycles of the 36 us by 256 threads with eight loads in flight; it is
+// split over the blocks of a cluster, whose other blocks then leave
+// (launch_group_polar).  With the steps' index tables computed once and the
+// rows' update by parts, 26 us now, of which the three polar factors are 16.
 #define POLAR_THREADS 256
-
 __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, GroupDev gd, int g, double2* gates,
-                                                               const signed char* arity, const int* nlayers,
-                                                               const int* active, double* nuc, double2* env_out) {
+                                                    const signed char* arity, const int* nlayers, const int* active,
+                                                    double* nuc, double2* env_out) {
   __shared__ xc M[2][GMM];
   __shared__ xc env[16];
   __shared__ double2 gold[GMAXSTEPS][16];   // the steps' gates, replaced one by one
   __shared__ xc gx[GMAXSTEPS][16];          // the same in double-float
   __shared__ int sk[GMAXSTEPS], sh[GMAXSTEPS], sl[GMAXSTEPS];
+  __shared__ unsigned char so[GMAXSTEPS][8], sp[GMAXSTEPS][4];   // spread_bits, gate_place of each step
   __shared__ int64_t sslot[GMAXSTEPS];
   __shared__ WarpPolar wp;
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int b = blockIdx.x; b < bd.B; b += gridDim.x) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = cluster.num_blocks(), rank = cluster.block_rank();
+  for (int b = blockIdx.x / ranks; b < bd.B; b += gridDim.x / ranks) {
     if (active && !active[b]) continue;
     if (g >= gd.ngroups[b]) continue;
     const GroupEnt ge = gd.grp[(int64_t)b * gd.gmax + g];
@@ -978,17 +997,20 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
     const bool last = g + 1 == gd.ngroups[b];
     __syncthreads();
     // the plan only groups valid steps; one that is not is never applied
-    if (tid < cnt * 16) {
+    if (tid < cnt * 16 && rank == 0) {
       const int s = tid >> 4, e = tid & 15;
       int64_t slot = 0;
       int q = 0, k = 0;
       const bool ok = bwd_step(bd, arity, L, n, b, ge.j0 + s, &slot, &q, &k);
+      const int hi = __popc(ge.qmask >> (q + 1)), lo = k == 2 ? __popc(ge.qmask >> (q + 2)) : 0;
       if (e == 0) {
         sk[s] = ok ? k : 0;
-        sh[s] = __popc(ge.qmask >> (q + 1));
-        sl[s] = k == 2 ? __popc(ge.qmask >> (q + 2)) : 0;
+        sh[s] = hi;
+        sl[s] = lo;
         sslot[s] = slot;
       }
+      if (e < 8) so[s][e] = (unsigned char)spread_bits(e, k, hi, lo);
+      else if (e < 12) sp[s][e - 8] = (unsigned char)gate_place(e - 8, k, hi, lo);
       if (ok && e < (1 << (2 * k))) {
         const double2 v = gates[bd.gate_off[b] + slot * 16 + e];
         gold[s][e] = v;
@@ -996,34 +1018,67 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
         gd.old_gates[((int64_t)b * GMAXSTEPS + s) * 16 + e] = v;
       }
     }
-    // sum of the chunk partials in chunk order; eight chunks' loads are
-    // issued together so the L2 latency overlaps
-    for (int e = tid; e < D * D; e += POLAR_THREADS) {
-      const int i = e / D, k = e % D;
-      const xc* src = gd.partials + (int64_t)c0 * GMM + i * GM + k;
+    // sum of the chunk partials: each rank a range of the chunks in order;
+    // sixteen chunks' loads are issued together so the L2 latency overlaps
+    {
+      static_assert(POLAR_THREADS == GMM, "an entry of M per thread");
+      const int i = tid >> ge.u, k = tid & (D - 1);
+      const bool mine = tid < D * D;
       XA s = xa_zero();
-      int c = 0;
-      for (; c + 8 <= nc; c += 8) {
-        xc v[8];
+      if (mine) {
+        int c = (int)((int64_t)nc * rank / ranks);
+        const int c1 = (int)((int64_t)nc * (rank + 1) / ranks);
+        const xc* src = gd.partials + (int64_t)(c0 + c) * GMM + i * GM + k;
+        for (; c + 16 <= c1; c += 16, src += 16 * GMM) {
+          xc v[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = src[(int64_t)(c + u) * GMM];
+          for (int u = 0; u < 16; ++u) v[u] = src[u * GMM];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          df_add(s.re, v[u].x, v[u].z);
-          df_add(s.im, v[u].y, v[u].w);
+          for (int u = 0; u < 16; ++u) {
+            df_add(s.re, v[u].x, v[u].z);
+            df_add(s.im, v[u].y, v[u].w);
+          }
         }
+        for (; c + 4 <= c1; c += 4, src += 4 * GMM) {
+          xc v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u] = src[u * GMM];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            df_add(s.re, v[u].x, v[u].z);
+            df_add(s.im, v[u].y, v[u].w);
+          }
+        }
+        for (; c < c1; ++c, src += GMM) {
+          const xc v = *src;
+          df_add(s.re, v.x, v.z);
+          df_add(s.im, v.y, v.w);
+        }
+        M[0][i * GM + k] = xa_round(s);
       }
-      for (; c < nc; ++c) {
-        const xc v = src[(int64_t)c * GMM];
-        df_add(s.re, v.x, v.z);
-        df_add(s.im, v.y, v.w);
+      if (ranks > 1) {
+        cluster.sync();
+        xc v[8];
+        if (mine && rank == 0) {
+#pragma unroll
+          for (int r = 1; r < 8; ++r)
+            if (r < ranks) v[r] = cluster.map_shared_rank(&M[0][0], r)[i * GM + k];
+#pragma unroll
+          for (int r = 1; r < 8; ++r)
+            if (r < ranks) {
+              df_add(s.re, v[r].x, v[r].z);
+              df_add(s.im, v[r].y, v[r].w);
+            }
+          M[0][i * GM + k] = xa_round(s);
+        }
+        cluster.sync();   // the other blocks' M is read
+        if (rank > 0) continue;
       }
-      M[0][i * GM + k] = xa_round(s);
     }
     __syncthreads();
     int cur = 0;
     if (sk[0]) {
-      m_cols(M[0], M[1], D, gx[0], sk[0], sh[0], sl[0], tid, POLAR_THREADS);
+      m_cols(M[0], M[1], ge.u, gx[0], sk[0], sh[0], sl[0], tid, POLAR_THREADS);
       cur = 1;
       __syncthreads();
     }
@@ -1035,10 +1090,12 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
           // E[r][c] = sum_o M[(r, o)][(c, o)], one part per lane
           const int ent = lane >> 1, part = lane & 1;
           if (ent < m * m) {
-            const int r = gate_place(ent / m, k, sh[s], sl[s]), c = gate_place(ent % m, k, sh[s], sl[s]);
+            const int r = sp[s][ent >> k], c = sp[s][ent & (m - 1)], rest = 1 << (ge.u - k);
             DF acc = {0.f, 0.f};
-            for (int o = 0; o < D / m; ++o) {
-              const int ob = spread_bits(o, k, sh[s], sl[s]);
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+              if (o >= rest) break;
+              const int ob = so[s][o];
               const xc v = M[cur][(r | ob) * GM + (c | ob)];
               df_add(acc, part ? v.y : v.x, part ? v.w : v.z);
             }
@@ -1062,12 +1119,12 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
           if (mine) gx[s][lane] = xc_from_d(gold[s][lane]);
         }
       } else if (k2) {
-        m_cols(M[cur], M[cur ^ 1], D, gx[s + 1], k2, sh[s + 1], sl[s + 1], tid - 32, POLAR_THREADS - 32);
+        m_cols(M[cur], M[cur ^ 1], ge.u, gx[s + 1], k2, sh[s + 1], sl[s + 1], tid - 32, POLAR_THREADS - 32);
       }
       __syncthreads();
       if (k2) cur ^= 1;
       if (k && s + 1 < cnt) {
-        m_rows(M[cur], M[cur ^ 1], D, gx[s], k, sh[s], sl[s], tid, POLAR_THREADS);
+        m_rows(M[cur], M[cur ^ 1], ge.u, gx[s], k, sh[s], sl[s], tid, POLAR_THREADS);
         cur ^= 1;
         __syncthreads();
       }
@@ -1135,6 +1192,20 @@ int launch_group_pass(const BatchDev& bd, const GroupDev& gd, int g, float2* psi
 
 void launch_group_polar(const BatchDev& bd, const GroupDev& gd, int g, double2* gates, const signed char* arity,
                         const int* nlayers, const int* active, double* nuc, cudaStream_t s, double2* env_out) {
+  // Blocks of a cluster to a state: while every block has an SM and 32 chunks
+  // (fewer: the two cluster barriers cost what they save).
+  int ranks = 1;
+  while (ranks < 8 && bd.B * ranks * 2 <= 152 && gd.most_chunks >= 32 * ranks * 2) ranks *= 2;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ranks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(bd.B * ranks);
+  cfg.blockDim = dim3(POLAR_THREADS);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
   qm_note_launch();
-  k_group_polar<<<bd.B, POLAR_THREADS, 0, s>>>(bd, gd, g, gates, arity, nlayers, active, nuc, env_out);
+  cudaLaunchKernelEx(&cfg, k_group_polar, bd, gd, g, gates, arity, nlayers, active, nuc, env_out);
 }
