@@ -606,6 +606,7 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_group_pass
   float2* xs = reinterpret_cast<float2*>(dyn);
   float2* zs = xs + (1 << GT);
   __shared__ PassShared sh;
+  bool waited = false;   // uniform
   for (int chunk = blockIdx.x; chunk < gd.nchunks; chunk += gridDim.x) {
     const int b = gd.chunk_state[chunk];
     if (active && !active[b]) continue;
@@ -675,6 +676,8 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_group_pass
       sh.plp[r] = swz(U == 4 && T >= 8 ? apply_pos_offset(r, sh.wml_p, full & ~sh.wml_p)
                                         : deposit32(r, full & ~sh.wml_p));
     }
+    if (!waited) grid_wait();   // the gates are the last polar kernel's
+    waited = true;
     if (g > 0) {
       // stage P = (new gate)^H and Q = (replaced gate)^H of each previous
       // step, one thread per (step, entry)
@@ -703,6 +706,7 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_group_pass
     else if (U == 3) pass_chunk<3, false>(bd, gd, sh, xs, zs, g, b, chunk, psi, z_in, z_out);
     else pass_chunk<2, false>(bd, gd, sh, xs, zs, g, b, chunk, psi, z_in, z_out);
   }
+  if (!waited) grid_wait();
 }
 
 // ---- circuit rebuild ---------------------------------------------------------------
@@ -804,6 +808,8 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_rebuild_pa
   extern __shared__ __align__(16) unsigned char dyn[];
   float2* xs = reinterpret_cast<float2*>(dyn);
   __shared__ RebuildShared sh;
+  bool waited = pass == 0;   // uniform
+  if (waited) grid_wait();
   for (int chunk = blockIdx.x; chunk < gd.nchunks; chunk += gridDim.x) {
     const int b = gd.chunk_state[chunk];
     if (active && !active[b]) continue;
@@ -889,11 +895,15 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_rebuild_pa
       const GateList gl[2] = {{sh.pk[0], sh.phi[0], sh.plo[0], sh.gm[0], sh.nst[0]},
                               {sh.pk[1], sh.phi[1], sh.plo[1], sh.gm[1], sh.nst[1]}};
       compose_gates(gl, nw, xs, sh.gf);
-      rebuild_chunk<4, true>(bd, gd, sh, xs, b, chunk, psi);
-    } else if (U == 4) rebuild_chunk<4, false>(bd, gd, sh, xs, b, chunk, psi);
+    }
+    if (!waited) grid_wait();   // the tiles are the last pass's
+    waited = true;
+    if (U == 4 && T >= 8 && !exact) rebuild_chunk<4, true>(bd, gd, sh, xs, b, chunk, psi);
+    else if (U == 4) rebuild_chunk<4, false>(bd, gd, sh, xs, b, chunk, psi);
     else if (U == 3) rebuild_chunk<3, false>(bd, gd, sh, xs, b, chunk, psi);
     else rebuild_chunk<2, false>(bd, gd, sh, xs, b, chunk, psi);
   }
+  if (!waited) grid_wait();
 }
 
 // ---- per-group polar kernel ------------------------------------------------------
@@ -987,6 +997,7 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
   const int tid = threadIdx.x, lane = tid & 31;
   cg::cluster_group cluster = cg::this_cluster();
   const int ranks = cluster.num_blocks(), rank = cluster.block_rank();
+  bool waited = false;   // uniform
   for (int b = blockIdx.x / ranks; b < bd.B; b += gridDim.x / ranks) {
     if (active && !active[b]) continue;
     if (g >= gd.ngroups[b]) continue;
@@ -1015,9 +1026,14 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
         const double2 v = gates[bd.gate_off[b] + slot * 16 + e];
         gold[s][e] = v;
         gx[s][e] = xc_from_d(v);
-        gd.old_gates[((int64_t)b * GMAXSTEPS + s) * 16 + e] = v;
       }
     }
+    if (!waited) grid_wait();
+    waited = true;
+    __syncthreads();
+    // the pass that just ended read the previous group's
+    if (tid < cnt * 16 && rank == 0 && sk[tid >> 4] && (tid & 15) < (1 << (2 * sk[tid >> 4])))
+      gd.old_gates[((int64_t)b * GMAXSTEPS + (tid >> 4)) * 16 + (tid & 15)] = gold[tid >> 4][tid & 15];
     // sum of the chunk partials: each rank a range of the chunks in order;
     // sixteen chunks' loads are issued together so the L2 latency overlaps
     {
@@ -1130,6 +1146,7 @@ __global__ void __launch_bounds__(POLAR_THREADS) k_group_polar(BatchDev bd, Grou
       }
     }
   }
+  if (!waited) grid_wait();
 }
 
 // ---- launches ----------------------------------------------------------------------
@@ -1168,9 +1185,8 @@ void launch_rebuild_pass(const BatchDev& bd, const GroupDev& gd, int pass, float
                          const signed char* arity, const int* nlayers, const int* active, cudaStream_t s, int mode,
                          int layer, bool exact) {
   int grid = pass_grid(gd);
-  qm_note_launch();
-  k_rebuild_pass<<<grid, PASS_THREADS, (size_t)2 * sizeof(float2) << GT, s>>>(bd, gd, pass, psi, gates, arity,
-                                                                          nlayers, active, mode, layer, exact);
+  launch_after(k_rebuild_pass, pass > 0, grid, PASS_THREADS, (size_t)2 * sizeof(float2) << GT, 1, s, bd, gd, pass, psi,
+               gates, arity, nlayers, active, mode, layer, exact);
 }
 
 int launch_group_pass(const BatchDev& bd, const GroupDev& gd, int g, float2* psi, const float2* z_in, float2* z_out,
@@ -1184,9 +1200,8 @@ int launch_group_pass(const BatchDev& bd, const GroupDev& gd, int g, float2* psi
     attr_set = true;
   }
   int grid = pass_grid(gd);
-  qm_note_launch();
-  k_group_pass<<<grid, PASS_THREADS, PASS_DYN_SMEM, s>>>(bd, gd, g, psi, z_in, z_out, gates, gd.old_gates, arity,
-                                                          nlayers, active, znorm);
+  launch_after(k_group_pass, g > 0, grid, PASS_THREADS, PASS_DYN_SMEM, 1, s, bd, gd, g, psi, z_in, z_out, gates,
+               gd.old_gates, arity, nlayers, active, znorm);
   return 0;
 }
 
@@ -1196,16 +1211,6 @@ void launch_group_polar(const BatchDev& bd, const GroupDev& gd, int g, double2* 
   // (fewer: the two cluster barriers cost what they save).
   int ranks = 1;
   while (ranks < 8 && bd.B * ranks * 2 <= 152 && gd.most_chunks >= 32 * ranks * 2) ranks *= 2;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = ranks;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(bd.B * ranks);
-  cfg.blockDim = dim3(POLAR_THREADS);
-  cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  qm_note_launch();
-  cudaLaunchKernelEx(&cfg, k_group_polar, bd, gd, g, gates, arity, nlayers, active, nuc, env_out);
+  launch_after(k_group_polar, true, bd.B * ranks, POLAR_THREADS, 0, ranks, s, bd, gd, g, gates, arity, nlayers, active,
+               nuc, env_out);
 }
