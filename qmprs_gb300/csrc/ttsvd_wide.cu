@@ -196,8 +196,13 @@ __global__ void __launch_bounds__(BJ_THREADS) k_bj_solve(float2* A, int W, int n
   const BJPair at(nb, k, pair);
   for (int e = tid; e < BJ_S * BJ_S; e += BJ_THREADS) {
     const int r = e / BJ_S, c = e % BJ_S;
-    a[0][r][c] = A[(int64_t)at(r) * W + at(c)];
     j[0][r][c] = cf(r == c ? 1.f : 0.f, 0.f);
+  }
+  grid_wait();   // the last round's update
+#pragma unroll
+  for (int e = tid; e < BJ_S * BJ_S; e += BJ_THREADS) {
+    const int r = e / BJ_S, c = e % BJ_S;
+    a[0][r][c] = A[(int64_t)at(r) * W + at(c)];
   }
   // rotations below FP32 rounding of the entries are skipped: ||G||_F /
   // sqrt(W) is the entries' scale (||G||_F alone overstates it by up to
@@ -337,6 +342,7 @@ __global__ void __launch_bounds__(BJU_THREADS) k_bj_update(float2* A, float2* V,
     }
     const int Q = P + 1 + rem;
     const BJPair ip(nb, k, P), iq(nb, k, Q);
+    grid_wait();   // this round's solves
 #pragma unroll
     for (int e = tid; e < BJ_S * BJ_S; e += BJU_THREADS) {
       const int rr = e / BJ_S, cc = e % BJ_S;
@@ -364,6 +370,7 @@ __global__ void __launch_bounds__(BJU_THREADS) k_bj_update(float2* A, float2* V,
     const int tI = blockIdx.x - nA;
     const int R = tI / np, Q = tI % np;
     const BJPair iq(nb, k, Q);
+    grid_wait();
 #pragma unroll
     for (int e = tid; e < BJ_S * BJ_S; e += BJU_THREADS) {
       const int rr = e / BJ_S, cc = e % BJ_S;
@@ -1007,15 +1014,14 @@ static int bj_fp32(const double2* H, int n, BJScratch& sc, cudaStream_t s, int* 
     cudaError_t e = cudaMemsetAsync(sc.count, 0, sizeof(int), s);
     if (e != cudaSuccess) return (int)e;
     for (int k = 0; k < nb - 1; ++k) {
-      qm_note_launch();
+      // after the last round's update, which follows this kernel's own
+      // predecessor; a sweep's first round follows the counter's reset
       if (k > 0)
-        k_bj_solve<true><<<np, BJ_THREADS, 0, s>>>(sc.A, W, nb, k, sc.J, sc.stats, sc.count);
+        launch_after(k_bj_solve<true>, nA + nV > 0, np, BJ_THREADS, 0, 1, s, sc.A, W, nb, k, sc.J, sc.stats, sc.count);
       else
-        k_bj_solve<false><<<np, BJ_THREADS, 0, s>>>(sc.A, W, nb, k, sc.J, sc.stats, sc.count);
-      if (nA + nV > 0) {
-        qm_note_launch();
-        k_bj_update<<<nA + nV, BJU_THREADS, 0, s>>>(sc.A, sc.V, W, nb, k, sc.J, nA);
-      }
+        launch_after(k_bj_solve<false>, false, np, BJ_THREADS, 0, 1, s, sc.A, W, nb, k, sc.J, sc.stats, sc.count);
+      if (nA + nV > 0)
+        launch_after(k_bj_update, true, nA + nV, BJU_THREADS, 0, 1, s, sc.A, sc.V, W, nb, k, sc.J, nA);
     }
     ++sweeps;
     int cnt = 0;
