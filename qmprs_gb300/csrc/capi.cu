@@ -15,6 +15,7 @@
 
 #include "exact.h"
 #include "internal.h"
+#include "launch.cuh"
 #include "qmprs_gb300.h"
 
 struct qmprs_ctx {
@@ -188,16 +189,19 @@ struct ProfLog {
 };
 
 __global__ void k_fill_int(int* p, int64_t count, int value) {
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
     p[i] = value;
 }
 
 __global__ void k_check_norms(int B, const double2* sq, int* err) {
+  grid_wait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x)
     if (!(isfinite(sq[b].x) && sq[b].x > 0.0)) atomicOr(err, KERR_BAD_INPUT);
 }
 
 __global__ void k_count_active(int B, const int* active, int* num_active) {
+  grid_wait();
   __shared__ int cnt;
   if (threadIdx.x == 0) cnt = 0;
   __syncthreads();
@@ -213,17 +217,17 @@ void launch_fill_int(int* p, int64_t count, int value, cudaStream_t s) {
   int blocks = (int)std::min<int64_t>((count + 255) / 256, 1024);
   if (blocks < 1) blocks = 1;
   qm_note_launch();
-  k_fill_int<<<blocks, 256, 0, s>>>(p, count, value);
+  launch_after(k_fill_int, blocks, 256, 0, s, p, count, value);
 }
 
 void launch_check_norms(int B, const double2* sq, int* err, cudaStream_t s) {
   qm_note_launch();
-  k_check_norms<<<(B + 127) / 128, 128, 0, s>>>(B, sq, err);
+  launch_after(k_check_norms, (B + 127) / 128, 128, 0, s, B, sq, err);
 }
 
 void launch_count_active(int B, const int* active, int* num_active, cudaStream_t s) {
   qm_note_launch();
-  k_count_active<<<1, 256, 0, s>>>(B, active, num_active);
+  launch_after(k_count_active, 1, 256, 0, s, B, active, num_active);
 }
 
 // Left-to-right contraction steps of the dense target for states whose bond

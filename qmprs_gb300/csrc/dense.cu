@@ -3,6 +3,7 @@
 #include "device_common.cuh"
 
 __global__ void k_set_zero_state(BatchDev bd, float2* vec, const int* active) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     if (active && !active[b]) continue;
@@ -16,6 +17,7 @@ __global__ void k_set_zero_state(BatchDev bd, float2* vec, const int* active) {
 
 // Apply the selected gate of every state: y = G x on (q, q+1) or q.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_apply_gate(BatchDev bd, float2* vec, GateSel sel) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     const int n = bd.n[b];
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_apply_gate(BatchDev bd, float
 // <a|b> per state in fp64.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_overlap(BatchDev bd, const float2* a, const float2* bv,
                                                            double2* partials, double2* out) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     const int n = bd.n[b];
@@ -100,6 +103,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_overlap(BatchDev bd, const fl
 // One warp per state: partials summed in a fixed order (lane-strided, then a
 // fixed shuffle tree).
 __global__ void k_reduce_tiles(BatchDev bd, const double2* partials, double2* out) {
+  grid_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int b = warp; b < bd.B; b += nwarps) {
@@ -116,6 +120,7 @@ __global__ void k_reduce_tiles(BatchDev bd, const double2* partials, double2* ou
 }
 
 __global__ void k_scale_copy(BatchDev bd, const float2* src, float2* dst, const double2* sq) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     const int n = bd.n[b];
@@ -140,23 +145,23 @@ static int grid_for(const BatchDev& bd) {
 
 void launch_set_zero_state(const BatchDev& bd, float2* vec, const int* active, cudaStream_t s) {
   qm_note_launch();
-  k_set_zero_state<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, vec, active);
+  launch_after(k_set_zero_state, grid_for(bd), BLOCK_THREADS, 0, s, bd, vec, active);
 }
 
 void launch_apply_gate(const BatchDev& bd, float2* vec, const GateSel& sel, cudaStream_t s) {
   qm_note_launch();
-  k_apply_gate<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, vec, sel);
+  launch_after(k_apply_gate, grid_for(bd), BLOCK_THREADS, 0, s, bd, vec, sel);
 }
 
 void launch_reduce_tiles(const BatchDev& bd, const double2* partials, double2* out, cudaStream_t s) {
   qm_note_launch();
-  k_reduce_tiles<<<(bd.B + 7) / 8, 256, 0, s>>>(bd, partials, out);
+  launch_after(k_reduce_tiles, (bd.B + 7) / 8, 256, 0, s, bd, partials, out);
 }
 
 void launch_overlap(const BatchDev& bd, const float2* a, const float2* b, double2* partials,
                     double2* out, cudaStream_t s) {
   qm_note_launch();
-  k_overlap<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, a, b, partials, out);
+  launch_after(k_overlap, grid_for(bd), BLOCK_THREADS, 0, s, bd, a, b, partials, out);
   launch_reduce_tiles(bd, partials, out, s);
 }
 
@@ -165,7 +170,7 @@ void launch_copy_normalize(const BatchDev& bd, const float2* src, float2* dst, d
                            double2* sq, cudaStream_t s) {
   launch_overlap(bd, src, src, partials, sq, s);
   qm_note_launch();
-  k_scale_copy<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, src, dst, sq);
+  launch_after(k_scale_copy, grid_for(bd), BLOCK_THREADS, 0, s, bd, src, dst, sq);
 }
 
 // ---- input upload ---------------------------------------------------------------
@@ -175,6 +180,7 @@ void launch_copy_normalize(const BatchDev& bd, const float2* src, float2* dst, d
 // straight to host memory, with the address translations of many SMs in
 // flight at once instead of one copy engine's.  16-byte words.
 __global__ void k_upload(float4* __restrict__ dst, const float4* __restrict__ src, int64_t n16) {
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = src[i];
 }
@@ -185,5 +191,5 @@ void launch_upload(void* dst, const void* src_dev, int64_t bytes, cudaStream_t s
   if (grid > 152 * 8) grid = 152 * 8;
   if (grid < 1) grid = 1;
   qm_note_launch();
-  k_upload<<<(int)grid, 256, 0, s>>>((float4*)dst, (const float4*)src_dev, n16);
+  launch_after(k_upload, (int)grid, 256, 0, s, (float4*)dst, (const float4*)src_dev, n16);
 }

@@ -4,49 +4,8 @@
 #pragma once
 
 #include "internal.h"
+#include "launch.cuh"
 #include "small_linalg.h"
-
-// ---- programmatic launches ----
-//
-// Rebuild passes follow one another, and so do a group's pass and its polar
-// kernel, and the blocked eigensolver's rounds: each is launched while its
-// predecessor runs (launch_after), and does what does not depend on it
-// (offset tables, composed gates, the steps' gates) before grid_wait, which
-// returns when the predecessor is complete and its writes are visible.  Every block waits, also one without work, and only
-// then lets its own successor start: before its grid_wait a kernel may read
-// what its predecessor's predecessor wrote, and write no global memory.
-__device__ __forceinline__ void grid_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// Launch k, with `early` as the programmatic successor of the launch before it
-// in the stream (grid_wait), in clusters of `ranks` blocks.
-template <class... P, class... A>
-static void launch_after(void (*k)(P...), bool early, int grid, int block, size_t smem, int ranks, cudaStream_t s,
-                         A... args) {
-  cudaLaunchAttribute at[2] = {};
-  int na = 0;
-  if (early) {
-    at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[na++].val.programmaticStreamSerializationAllowed = 1;
-  }
-  if (ranks > 1) {
-    at[na].id = cudaLaunchAttributeClusterDimension;
-    at[na].val.clusterDim.x = ranks;
-    at[na].val.clusterDim.y = 1;
-    at[na++].val.clusterDim.z = 1;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = at;
-  cfg.numAttrs = na;
-  qm_note_launch();
-  cudaLaunchKernelEx(&cfg, k, args...);
-}
 
 __device__ __forceinline__ void tile_range(int64_t total, int idx, int nt, int64_t* lo, int64_t* hi) {
   int64_t per = (total + nt - 1) / nt;

@@ -51,6 +51,7 @@ static int grid_for(const BatchDev& bd) {
 // ---- conversions -------------------------------------------------------------------
 
 __global__ void k_x_from_d(BatchDev bd, const double2* src, xc* dst) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     int64_t lo, hi;
@@ -62,6 +63,7 @@ __global__ void k_x_from_d(BatchDev bd, const double2* src, xc* dst) {
 }
 
 __global__ void k_x_to_d(BatchDev bd, const xc* src, double2* dst) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     int64_t lo, hi;
@@ -73,6 +75,7 @@ __global__ void k_x_to_d(BatchDev bd, const xc* src, double2* dst) {
 }
 
 __global__ void k_x_copy(BatchDev bd, const xc* src, xc* dst, const int* active) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     if (active && !active[b]) continue;
@@ -85,6 +88,7 @@ __global__ void k_x_copy(BatchDev bd, const xc* src, xc* dst, const int* active)
 }
 
 __global__ void k_x_zero(BatchDev bd, xc* vec, const int* active) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     if (active && !active[b]) continue;
@@ -97,6 +101,7 @@ __global__ void k_x_zero(BatchDev bd, xc* vec, const int* active) {
 
 // dst = src / sqrt(sq[b].x) in double-float (the factor split once per tile).
 __global__ void k_x_scale(BatchDev bd, const xc* src, xc* dst, const double2* sq) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     int64_t lo, hi;
@@ -119,6 +124,7 @@ __global__ void k_x_scale(BatchDev bd, const xc* src, xc* dst, const double2* sq
 // <a|b> per tile: double-float accumulation flushed to fp64, block sum in
 // fixed order; k_reduce_tiles (dense.cu) sums the tiles of each state.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_x_dot(BatchDev bd, const xc* a, const xc* bv, double2* partials) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     int64_t lo, hi;
@@ -143,6 +149,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_dot(BatchDev bd, const xc* 
 // caller-facing overlaps of this mode).
 __global__ void __launch_bounds__(BLOCK_THREADS) k_d_dot(BatchDev bd, const double2* a, const double2* bv,
                                                          double2* partials) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     int64_t lo, hi;
@@ -172,6 +179,7 @@ __host__ __device__ inline int x_gram_nt(int w) { const int ti = x_gram_ti(w); r
 // part[split * WW + a * w + c] for the tile's entries with a <= c.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_tile(const xc* m, int64_t rows, int w, int nsplit,
                                                                double2* part, int64_t WW) {
+  grid_wait();
   __shared__ double2 red[BLOCK_THREADS * 4];
   const int TI = x_gram_ti(w), G = TI / 2, EG = G * G;
   const int RL = BLOCK_THREADS / EG;
@@ -220,6 +228,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_tile(const xc* m, int6
 
 // gram[a * w + c] = sum over splits (in order), mirrored to the lower triangle.
 __global__ void k_x_gram_reduce(const double2* part, int nsplit, int w, int64_t WW, double2* gram) {
+  grid_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)w * w; e += (int64_t)gridDim.x * blockDim.x) {
     const int a = (int)(e / w), c = (int)(e % w);
     if (a > c) continue;
@@ -242,6 +251,7 @@ __global__ void k_x_gram_reduce(const double2* part, int nsplit, int w, int64_t 
 // shared memory one K chunk at a time; sums flushed to fp64 per chunk.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gemm(const xc* A, int64_t lda, const double2* B, int64_t ldb,
                                                           xc* C, int64_t ldc, int64_t M, int N, int K, int TN) {
+  grid_wait();
   __shared__ xc Bs[XG_KC][32];
   const int TM = BLOCK_THREADS / TN;
   const int64_t row = (int64_t)blockIdx.x * TM + threadIdx.x / TN;
@@ -271,6 +281,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gemm(const xc* A, int64_t l
 // (quimb's rsum2 renormalisation), in FP64; the factor goes to *f_out.
 // One block.
 __global__ void k_x_site0(const xc* rem, int r1, double in_sq, double2* t0, double* f_out) {
+  grid_wait();
   __shared__ double s_nrm;
   if (threadIdx.x == 0) {
     double nrm = 0.0;
@@ -285,6 +296,7 @@ __global__ void k_x_site0(const xc* rem, int r1, double in_sq, double2* t0, doub
 
 // dst[i] = f * src[i] for count entries, f = *f_ptr (double-float product).
 __global__ void k_x_scale_flat(const xc* src, xc* dst, int64_t count, const double* f_ptr) {
+  grid_wait();
   const double f = *f_ptr;
   const float fh = __double2float_rn(f), fl = __double2float_rn(f - (double)fh);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
@@ -299,6 +311,7 @@ __global__ void k_x_scale_flat(const xc* src, xc* dst, int64_t count, const doub
 
 // Row-major complex128 -> double-float copy of count entries.
 __global__ void k_x_from_d_flat(const double2* src, xc* dst, int64_t count) {
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = xc_from_d(src[i]);
 }
@@ -309,6 +322,7 @@ __global__ void k_x_from_d_flat(const double2* src, xc* dst, int64_t count) {
 
 __global__ void k_x_layer_fidelity(BatchDev bd, int layer, const xc* work, int num_layers, double atol,
                                    double2* layer_fid, int* nlayers, int* active) {
+  grid_wait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < bd.B; b += gridDim.x * blockDim.x) {
     if (!active[b]) continue;
     const double2 f = cconj(xc_to_d(work[bd.vec_off[b]]));
@@ -330,6 +344,7 @@ __device__ __forceinline__ void x_load_gate(const double2* g, int m, int adjoint
 }
 
 __global__ void __launch_bounds__(BLOCK_THREADS) k_x_apply_gate(BatchDev bd, xc* vec, GateSel sel) {
+  grid_wait();
   __shared__ xc gs[16];
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
@@ -398,6 +413,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
                                                                 double2* gates, const signed char* arity,
                                                                 const int* nlayers, const int* active,
                                                                 xc* partials, double* nuc) {
+  grid_wait();
   __shared__ xc gs[16];
   __shared__ float2 wred[WARPS][32];
   __shared__ xc env[16];
@@ -570,6 +586,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
                                                                  int* active, const double2* tnorm2, int num_sweeps,
                                                                  double stop_fid, double* sweep_fid,
                                                                  int* sweeps_done) {
+  grid_wait();
   extern __shared__ xc xsm[];
   __shared__ xc gs[2][16];           // the gate to apply (rebuild), or to peel
   __shared__ xc gt[16];              // the new gate's adjoint
@@ -719,41 +736,41 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
 
 void launch_x_from_d(const BatchDev& bd, const double2* src, xc* dst, cudaStream_t s) {
   qm_note_launch();
-  k_x_from_d<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, src, dst);
+  launch_after(k_x_from_d, grid_for(bd), BLOCK_THREADS, 0, s, bd, src, dst);
 }
 
 void launch_x_to_d(const BatchDev& bd, const xc* src, double2* dst, cudaStream_t s) {
   qm_note_launch();
-  k_x_to_d<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, src, dst);
+  launch_after(k_x_to_d, grid_for(bd), BLOCK_THREADS, 0, s, bd, src, dst);
 }
 
 void launch_x_copy(const BatchDev& bd, const xc* src, xc* dst, const int* active, cudaStream_t s) {
   qm_note_launch();
-  k_x_copy<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, src, dst, active);
+  launch_after(k_x_copy, grid_for(bd), BLOCK_THREADS, 0, s, bd, src, dst, active);
 }
 
 void launch_x_zero(const BatchDev& bd, xc* vec, const int* active, cudaStream_t s) {
   qm_note_launch();
-  k_x_zero<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, vec, active);
+  launch_after(k_x_zero, grid_for(bd), BLOCK_THREADS, 0, s, bd, vec, active);
 }
 
 void launch_x_dot(const BatchDev& bd, const xc* a, const xc* b, double2* partials, double2* out, cudaStream_t s) {
   qm_note_launch();
-  k_x_dot<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, a, b, partials);
+  launch_after(k_x_dot, grid_for(bd), BLOCK_THREADS, 0, s, bd, a, b, partials);
   launch_reduce_tiles(bd, partials, out, s);
 }
 
 void launch_d_dot(const BatchDev& bd, const double2* a, const double2* b, double2* partials, double2* out,
                   cudaStream_t s) {
   qm_note_launch();
-  k_d_dot<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, a, b, partials);
+  launch_after(k_d_dot, grid_for(bd), BLOCK_THREADS, 0, s, bd, a, b, partials);
   launch_reduce_tiles(bd, partials, out, s);
 }
 
 void launch_x_normalize(const BatchDev& bd, const xc* src, xc* dst, double2* partials, double2* sq, cudaStream_t s) {
   launch_x_dot(bd, src, src, partials, sq, s);
   qm_note_launch();
-  k_x_scale<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, src, dst, sq);
+  launch_after(k_x_scale, grid_for(bd), BLOCK_THREADS, 0, s, bd, src, dst, sq);
 }
 
 void launch_x_gram(const xc* m, int64_t rows, int w, double2* part, int64_t WW, double2* gram, cudaStream_t s) {
@@ -761,11 +778,11 @@ void launch_x_gram(const xc* m, int64_t rows, int w, double2* part, int64_t WW, 
   const int nt = x_gram_nt(w);
   dim3 grid(nt * (nt + 1) / 2, nsplit);
   qm_note_launch();
-  k_x_gram_tile<<<grid, BLOCK_THREADS, 0, s>>>(m, rows, w, nsplit, part, WW);
+  launch_after(k_x_gram_tile, grid, BLOCK_THREADS, 0, s, m, rows, w, nsplit, part, WW);
   const int64_t ww = (int64_t)w * w;
   const int blocks = (int)std::min<int64_t>((ww + 255) / 256, 1024);
   qm_note_launch();
-  k_x_gram_reduce<<<blocks, 256, 0, s>>>(part, nsplit, w, WW, gram);
+  launch_after(k_x_gram_reduce, blocks, 256, 0, s, part, nsplit, w, WW, gram);
 }
 
 void launch_x_gemm(const xc* A, int64_t lda, const double2* B, int64_t ldb, xc* C, int64_t ldc, int64_t M, int N,
@@ -775,24 +792,24 @@ void launch_x_gemm(const xc* A, int64_t lda, const double2* B, int64_t ldb, xc* 
   const int TM = BLOCK_THREADS / TN;
   dim3 grid((unsigned)((M + TM - 1) / TM), (unsigned)((N + TN - 1) / TN));
   qm_note_launch();
-  k_x_gemm<<<grid, BLOCK_THREADS, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, TN);
+  launch_after(k_x_gemm, grid, BLOCK_THREADS, 0, s, A, lda, B, ldb, C, ldc, M, N, K, TN);
 }
 
 void launch_x_site0(const xc* rem, int r1, double in_sq, double2* t0, double* f_out, cudaStream_t s) {
   qm_note_launch();
-  k_x_site0<<<1, 64, 0, s>>>(rem, r1, in_sq, t0, f_out);
+  launch_after(k_x_site0, 1, 64, 0, s, rem, r1, in_sq, t0, f_out);
 }
 
 void launch_x_scale_flat(const xc* src, xc* dst, int64_t count, const double* f, cudaStream_t s) {
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((count + 255) / 256, 1024));
   qm_note_launch();
-  k_x_scale_flat<<<blocks, 256, 0, s>>>(src, dst, count, f);
+  launch_after(k_x_scale_flat, blocks, 256, 0, s, src, dst, count, f);
 }
 
 void launch_x_from_d_flat(const double2* src, xc* dst, int64_t count, cudaStream_t s) {
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((count + 255) / 256, 1024));
   qm_note_launch();
-  k_x_from_d_flat<<<blocks, 256, 0, s>>>(src, dst, count);
+  launch_after(k_x_from_d_flat, blocks, 256, 0, s, src, dst, count);
 }
 
 void launch_x_layer_cut(const BatchDev& bd, int units, int step, const xc* work, xc* buf0, xc* buf1, int* bonds,
@@ -800,33 +817,34 @@ void launch_x_layer_cut(const BatchDev& bd, int units, int step, const xc* work,
   const xc* prev = (step & 1) ? buf1 : buf0;
   xc* dst = (step & 1) ? buf0 : buf1;
   qm_note_launch();
-  k_layer_cut<CutExact><<<units, BLOCK_THREADS, 0, s>>>(bd, step, work, prev, dst, bonds, vsel, site_t,
-                                                        reinterpret_cast<double*>(partials), buf0, buf1, active);
+  launch_after(k_layer_cut<CutExact>, units, BLOCK_THREADS, 0, s, bd, step, work, prev, dst, bonds, vsel, site_t,
+               reinterpret_cast<double*>(partials), buf0, buf1, active);
 }
 
 void launch_x_layer_build(const BatchDev& bd, int layer, const xc* rem0, const xc* rem1, const int* bonds,
                           double2* site_t, double2* gates, signed char* arity, const int* active, cudaStream_t s) {
   qm_note_launch();
-  k_layer_build<CutExact><<<bd.B, BUILD_THREADS, 0, s>>>(bd, layer, rem0, rem1, bonds, site_t, gates, arity, active);
+  launch_after(k_layer_build<CutExact>, bd.B, BUILD_THREADS, 0, s, bd, layer, rem0, rem1, bonds, site_t, gates, arity,
+               active);
 }
 
 void launch_x_layer_fidelity(const BatchDev& bd, int layer, const xc* work, int num_layers, double atol,
                              double2* layer_fid, int* nlayers, int* active, cudaStream_t s) {
   qm_note_launch();
-  k_x_layer_fidelity<<<(bd.B + 127) / 128, 128, 0, s>>>(bd, layer, work, num_layers, atol, layer_fid, nlayers,
-                                                         active);
+  launch_after(k_x_layer_fidelity, (bd.B + 127) / 128, 128, 0, s, bd, layer, work, num_layers, atol, layer_fid,
+               nlayers, active);
 }
 
 void launch_x_apply_gate(const BatchDev& bd, xc* vec, const GateSel& sel, cudaStream_t s) {
   qm_note_launch();
-  k_x_apply_gate<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, vec, sel);
+  launch_after(k_x_apply_gate, grid_for(bd), BLOCK_THREADS, 0, s, bd, vec, sel);
 }
 
 void launch_x_sweep_step(const BatchDev& bd, int step, xc* psi, const xc* t, double2* gates, const signed char* arity,
                          const int* nlayers, const int* active, double2* partials, double* nuc, cudaStream_t s) {
   qm_note_launch();
-  k_x_sweep_step<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, psi, t, gates, arity, nlayers, active,
-                                                        reinterpret_cast<xc*>(partials), nuc);
+  launch_after(k_x_sweep_step, grid_for(bd), BLOCK_THREADS, 0, s, bd, step, psi, t, gates, arity, nlayers, active,
+               reinterpret_cast<xc*>(partials), nuc);
 }
 
 int launch_x_sweep_fused(const BatchDev& bd, int max_n, const xc* target, double2* gates, const signed char* arity,
@@ -836,7 +854,7 @@ int launch_x_sweep_fused(const BatchDev& bd, int max_n, const xc* target, double
   cudaError_t e = cudaFuncSetAttribute(k_x_sweep_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   qm_note_launch();
-  k_x_sweep_fused<<<bd.B, BLOCK_THREADS, smem, s>>>(bd, target, gates, arity, nlayers, active, tnorm2, num_sweeps,
-                                                    stop_fid, sweep_fid, sweeps_done);
+  launch_after(k_x_sweep_fused, bd.B, BLOCK_THREADS, smem, s, bd, target, gates, arity, nlayers, active, tnorm2,
+               num_sweeps, stop_fid, sweep_fid, sweeps_done);
   return (int)cudaGetLastError();
 }

@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int st
                                                              int* bonds, double2* vsel, double2* site_t,
                                                              double* partials, typename P::T* rem0,
                                                              typename P::T* rem1, const int* active) {
+  grid_wait();
   typedef typename P::T T;
   __shared__ T vm[16];
   __shared__ double wred[WARPS][16];
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(BUILD_THREADS) k_layer_build(BatchDev bd, int 
                                                                const typename P::T* rem1, const int* bonds,
                                                                double2* site_t, double2* gates, signed char* arity,
                                                                const int* active) {
+  grid_wait();
   __shared__ double2 g_s[MAX_QUBITS][16];
   __shared__ double2 st0[4];
   __shared__ signed char ks[MAX_QUBITS];

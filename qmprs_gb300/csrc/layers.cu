@@ -16,6 +16,7 @@
 // Sequential._get_unitary_layers (sequential.py:390): np.isclose(f, 1, atol).
 __global__ void k_layer_fidelity(BatchDev bd, int layer, const float2* work, int num_layers,
                                  double atol, double2* layer_fid, int* nlayers, int* active) {
+  grid_wait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < bd.B; b += gridDim.x * blockDim.x) {
     if (!active[b]) continue;
     const double2 f = cconj(f2d(work[bd.vec_off[b]]));
@@ -33,15 +34,16 @@ void launch_layer_cut(const BatchDev& bd, int units, int step, const float2* wor
   const float2* prev = (step & 1) ? buf1 : buf0;
   float2* dst = (step & 1) ? buf0 : buf1;
   qm_note_launch();
-  k_layer_cut<CutFast><<<units, BLOCK_THREADS, 0, s>>>(bd, step, work, prev, dst, bonds, vsel, site_t,
-                                                       reinterpret_cast<double*>(partials), buf0, buf1, active);
+  launch_after(k_layer_cut<CutFast>, units, BLOCK_THREADS, 0, s, bd, step, work, prev, dst, bonds, vsel, site_t,
+               reinterpret_cast<double*>(partials), buf0, buf1, active);
 }
 
 void launch_layer_build(const BatchDev& bd, int layer, const float2* rem0, const float2* rem1,
                         const int* bonds, double2* site_t, double2* gates, signed char* arity,
                         const int* active, cudaStream_t s) {
   qm_note_launch();
-  k_layer_build<CutFast><<<bd.B, BUILD_THREADS, 0, s>>>(bd, layer, rem0, rem1, bonds, site_t, gates, arity, active);
+  launch_after(k_layer_build<CutFast>, bd.B, BUILD_THREADS, 0, s, bd, layer, rem0, rem1, bonds, site_t, gates, arity,
+               active);
 }
 
 void launch_layer_fidelity(const BatchDev& bd, int layer, const float2* work, int num_layers,
@@ -49,5 +51,5 @@ void launch_layer_fidelity(const BatchDev& bd, int layer, const float2* work, in
                            cudaStream_t s) {
   int blocks = (bd.B + 127) / 128;
   qm_note_launch();
-  k_layer_fidelity<<<blocks, 128, 0, s>>>(bd, layer, work, num_layers, atol, layer_fid, nlayers, active);
+  launch_after(k_layer_fidelity, blocks, 128, 0, s, bd, layer, work, num_layers, atol, layer_fid, nlayers, active);
 }

@@ -30,6 +30,7 @@
 #include <stdint.h>
 
 #include "internal.h"
+#include "launch.cuh"
 #include "qmprs_gb300.h"
 #include "small_linalg.h"
 
@@ -194,6 +195,7 @@ __device__ __forceinline__ void stage_tile(uint8_t* s, const __nv_bfloat16* g, i
 // Measured (mean over a training step of 4096 rows): 44.6 us with 32 blocks of
 // 128 x 256 and one stage, 9.8 us now.
 __global__ void __launch_bounds__(MLP_THREADS, 2) k_gemm_tc(GemmArgs g) {
+  grid_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t mbar[MLP_STAGES];
   __shared__ uint32_t tmem_sh;
@@ -391,6 +393,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) k_tc_wait_selftest(int* err) {
 // part [S][M][N] -> C (+bias, act), fixed order over S
 __global__ void k_splitk_sum(const float* part, int S, int M, int N, const float* bias, const float* resid, int ldr,
                              int act, float* Cf, int ldc, __nv_bfloat16* Cb, __nv_bfloat16* CbT, int ldt) {
+  grid_wait();
   const int64_t total = (int64_t)M * N;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int row = (int)(i / N), col = (int)(i % N);
@@ -413,6 +416,7 @@ __global__ void k_splitk_sum(const float* part, int S, int M, int N, const float
 // dY = w (2 M - 2 e^{i phi*} U) / sum(w), phi* = arg Tr(U^H M).
 __global__ void k_mlp_loss(const float* Y, const float* U, const float* w, int B, float inv_wsum, float* loss,
                            float* dY, __nv_bfloat16* dYb, __nv_bfloat16* dYT, int ldt) {
+  grid_wait();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < B; s += gridDim.x * blockDim.x) {
     const float* y = Y + (int64_t)s * 32;
     const float* u = U + (int64_t)s * 32;
@@ -455,6 +459,7 @@ __global__ void k_mlp_loss(const float* Y, const float* U, const float* w, int B
 __global__ void k_mlp_overlap_grad(const double2* env, const double2* gates, const int64_t* slots,
                                    const signed char* kind, const float* tinv, int rows, int B, float gscale,
                                    float* fid, float* dY, __nv_bfloat16* dYb, __nv_bfloat16* dYT, int ldt) {
+  grid_wait();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < B; s += gridDim.x * blockDim.x) {
     float out[32];
 #pragma unroll
@@ -504,6 +509,7 @@ __global__ void k_mlp_overlap_grad(const double2* env, const double2* gates, con
 // dZ = dH * GELU'(Z) for [B x N]; BF16 copy and transposed BF16 copy [N x ldt]
 __global__ void k_act_back(const float* dH, const float* Z, int B, int N, float* dZ, __nv_bfloat16* dZb,
                            __nv_bfloat16* dZT, int ldt) {
+  grid_wait();
   const int64_t total = (int64_t)B * N;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int row = (int)(i / N), col = (int)(i % N);
@@ -520,6 +526,7 @@ __global__ void k_act_back(const float* dH, const float* Z, int B, int N, float*
 // 120 us, 9.7 us now).
 #define COL_GROUPS 32
 __global__ void __launch_bounds__(32 * COL_GROUPS) k_col_sum(const float* X, int B, int N, float* out) {
+  grid_wait();
   __shared__ float red[COL_GROUPS][33];
   const int l = threadIdx.x & 31, rg = threadIdx.x >> 5, c = blockIdx.x * 32 + l;
   float s = 0.f;
@@ -540,6 +547,7 @@ __global__ void __launch_bounds__(32 * COL_GROUPS) k_col_sum(const float* X, int
 // transposed ([cols x rows]) when gT != 0.  Writes BF16 W and W^T.
 __global__ void k_adam(float* W, const float* G, int gT, float* m, float* v, int rows, int cols, float lr, float b1,
                        float b2, float eps, float bc1, float bc2, float wd, __nv_bfloat16* Wb, __nv_bfloat16* WTb) {
+  grid_wait();
   const int64_t total = (int64_t)rows * cols;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(i / cols), c = (int)(i % cols);
@@ -558,6 +566,7 @@ __global__ void k_adam(float* W, const float* G, int gT, float* m, float* v, int
 
 __global__ void k_adam_vec(float* W, const float* G, float* m, float* v, int n, float lr, float b1, float b2,
                            float eps, float bc1, float bc2) {
+  grid_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gr = G[i];
     const float mm = b1 * m[i] + (1.f - b1) * gr;
@@ -573,6 +582,7 @@ __global__ void k_adam_vec(float* W, const float* G, float* m, float* v, int n, 
 // threshold are completed towards the gate already in the slot.
 __global__ void k_mlp_project(const float* Y, int rows, const int64_t* slots, const signed char* kind,
                               double2* gates) {
+  grid_wait();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
     const int m = kind[r] == 1 ? 2 : 4;
     double2 e[16], w[16], prev[16];
@@ -645,11 +655,11 @@ int qmprs_gemm_bf16(const void* A, int lda, const void* B, int ldb, int M, int N
   g.err = err;
   dim3 grid(M / MLP_BM, (N + MLP_BN - 1) / MLP_BN, S);
   qm_note_launch();
-  k_gemm_tc<<<grid, MLP_THREADS, MLP_SMEM_REQ, s>>>(g);
+  launch_after(k_gemm_tc, grid, MLP_THREADS, MLP_SMEM_REQ, s, g);
   if (S > 1) {
     qm_note_launch();
-    k_splitk_sum<<<grid1((int64_t)M * N, 256), 256, 0, s>>>(part, S, M, N, bias, resid, ldr, act, Cf, ldc,
-                                                             (__nv_bfloat16*)Cb, (__nv_bfloat16*)CbT, ldt);
+    launch_after(k_splitk_sum, grid1((int64_t)M * N, 256), 256, 0, s, part, S, M, N, bias, resid, ldr, act, Cf, ldc,
+                 (__nv_bfloat16*)Cb, (__nv_bfloat16*)CbT, ldt);
   }
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
@@ -658,8 +668,8 @@ int qmprs_mlp_loss(const float* Y, const float* U, const float* w, int B, float 
                    void* dYb, void* dYT, int ldt, void* stream) {
   if (!Y || !U || !w || !loss || !dY || !dYb || !dYT || B <= 0) return QMPRS_ERR_INVALID;
   qm_note_launch();
-  k_mlp_loss<<<grid1(B, 128), 128, 0, (cudaStream_t)stream>>>(Y, U, w, B, inv_wsum, loss, dY, (__nv_bfloat16*)dYb,
-                                                               (__nv_bfloat16*)dYT, ldt);
+  launch_after(k_mlp_loss, grid1(B, 128), 128, 0, (cudaStream_t)stream, Y, U, w, B, inv_wsum, loss, dY,
+               (__nv_bfloat16*)dYb, (__nv_bfloat16*)dYT, ldt);
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
 
@@ -667,15 +677,15 @@ int qmprs_mlp_act_back(const float* dH, const float* Z, int B, int N, float* dZ,
                        void* stream) {
   if (!dH || !Z || !dZ || !dZb || !dZT || B <= 0 || N <= 0) return QMPRS_ERR_INVALID;
   qm_note_launch();
-  k_act_back<<<grid1((int64_t)B * N, 256), 256, 0, (cudaStream_t)stream>>>(dH, Z, B, N, dZ, (__nv_bfloat16*)dZb,
-                                                                          (__nv_bfloat16*)dZT, ldt);
+  launch_after(k_act_back, grid1((int64_t)B * N, 256), 256, 0, (cudaStream_t)stream, dH, Z, B, N, dZ,
+               (__nv_bfloat16*)dZb, (__nv_bfloat16*)dZT, ldt);
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
 
 int qmprs_mlp_col_sum(const float* X, int B, int N, float* out, void* stream) {
   if (!X || !out || B <= 0 || N <= 0) return QMPRS_ERR_INVALID;
   qm_note_launch();
-  k_col_sum<<<(N + 31) / 32, 32 * COL_GROUPS, 0, (cudaStream_t)stream>>>(X, B, N, out);
+  launch_after(k_col_sum, (N + 31) / 32, 32 * COL_GROUPS, 0, (cudaStream_t)stream, X, B, N, out);
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
 
@@ -685,10 +695,11 @@ int qmprs_mlp_adam(float* W, const float* G, int gT, float* m, float* v, int row
   const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
   qm_note_launch();
   if (cols == 1 && !Wb && !WTb) {
-    k_adam_vec<<<grid1(rows, 256), 256, 0, (cudaStream_t)stream>>>(W, G, m, v, rows, lr, b1, b2, eps, bc1, bc2);
+    launch_after(k_adam_vec, grid1(rows, 256), 256, 0, (cudaStream_t)stream, W, G, m, v, rows, lr, b1, b2, eps, bc1,
+                 bc2);
   } else {
-    k_adam<<<grid1((int64_t)rows * cols, 256), 256, 0, (cudaStream_t)stream>>>(
-        W, G, gT, m, v, rows, cols, lr, b1, b2, eps, bc1, bc2, wd, (__nv_bfloat16*)Wb, (__nv_bfloat16*)WTb);
+    launch_after(k_adam, grid1((int64_t)rows * cols, 256), 256, 0, (cudaStream_t)stream, W, G, gT, m, v, rows, cols,
+                 lr, b1, b2, eps, bc1, bc2, wd, (__nv_bfloat16*)Wb, (__nv_bfloat16*)WTb);
   }
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
@@ -707,9 +718,9 @@ int qmprs_mlp_overlap_grad(const void* env, const void* gates, const int64_t* sl
       B <= 0 || ldt < B)
     return QMPRS_ERR_INVALID;
   qm_note_launch();
-  k_mlp_overlap_grad<<<grid1(B, 128), 128, 0, (cudaStream_t)stream>>>(
-      (const double2*)env, (const double2*)gates, slots, (const signed char*)kind, tinv, rows, B, gscale, fid, dY,
-      (__nv_bfloat16*)dYb, (__nv_bfloat16*)dYT, ldt);
+  launch_after(k_mlp_overlap_grad, grid1(B, 128), 128, 0, (cudaStream_t)stream, (const double2*)env,
+               (const double2*)gates, slots, (const signed char*)kind, tinv, rows, B, gscale, fid, dY,
+               (__nv_bfloat16*)dYb, (__nv_bfloat16*)dYT, ldt);
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
 
@@ -718,8 +729,8 @@ int qmprs_mlp_project(const float* Y, int rows, const int64_t* slots, const int8
   if (!Y || !slots || !kind || !gates || rows < 0) return QMPRS_ERR_INVALID;
   if (rows == 0) return QMPRS_OK;
   qm_note_launch();
-  k_mlp_project<<<grid1(rows, 64), 64, 0, (cudaStream_t)stream>>>(Y, rows, slots, (const signed char*)kind,
-                                                                   (double2*)gates);
+  launch_after(k_mlp_project, grid1(rows, 64), 64, 0, (cudaStream_t)stream, Y, rows, slots, (const signed char*)kind,
+               (double2*)gates);
   return cudaGetLastError() == cudaSuccess ? QMPRS_OK : QMPRS_ERR_CUDA;
 }
 

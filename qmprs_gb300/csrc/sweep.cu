@@ -10,6 +10,7 @@
 __global__ void k_sweep_finish(int B, int sweep, int num_sweeps, const double* nuc, const double2* tnorm2,
                                double* sweep_fid, int* sweeps_done, int* active, double stop_fid,
                                int* num_active) {
+  grid_wait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) {
     if (!active[b]) continue;
     const double f = nuc[b] / sqrt(tnorm2[b].x);
@@ -24,6 +25,6 @@ void launch_sweep_finish(int B, int sweep, int num_sweeps, const double* nuc, co
                          double* sweep_fid, int* sweeps_done, int* active, double stop_fid,
                          int* num_active, cudaStream_t s) {
   qm_note_launch();
-  k_sweep_finish<<<(B + 127) / 128, 128, 0, s>>>(B, sweep, num_sweeps, nuc, tnorm2, sweep_fid,
-                                                 sweeps_done, active, stop_fid, num_active);
+  launch_after(k_sweep_finish, (B + 127) / 128, 128, 0, s, B, sweep, num_sweeps, nuc, tnorm2, sweep_fid, sweeps_done,
+               active, stop_fid, num_active);
 }

@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_sweep_fused(BatchDev bd, cons
                                                                int* active, const double2* tnorm2, int num_sweeps,
                                                                double stop_fid, double* sweep_fid,
                                                                int* sweeps_done, double2* env_out) {
+  grid_wait();
   extern __shared__ float2 fsm[];
   __shared__ float2 gs[2][16];       // the gate to apply (rebuild), or to peel
   __shared__ float2 gt[16];          // the new gate's adjoint
@@ -235,7 +236,7 @@ int launch_sweep_fused(const BatchDev& bd, int max_n, const float2* target, doub
   cudaError_t e = cudaFuncSetAttribute(k_sweep_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   qm_note_launch();
-  k_sweep_fused<<<bd.B, BLOCK_THREADS, smem, s>>>(bd, target, gates, arity, nlayers, active, tnorm2, num_sweeps,
-                                                  stop_fid, sweep_fid, sweeps_done, env_out);
+  launch_after(k_sweep_fused, bd.B, BLOCK_THREADS, smem, s, bd, target, gates, arity, nlayers, active, tnorm2,
+               num_sweeps, stop_fid, sweep_fid, sweeps_done, env_out);
   return (int)cudaGetLastError();
 }

@@ -101,6 +101,7 @@ __device__ __forceinline__ int64_t deposit_bits(int64_t v, int64_t mask) {
 // min(GW, n) qubits.  States outside `active` (when given) get no groups.
 __global__ void k_group_plan(BatchDev bd, GroupDev gd, const signed char* arity, const int* nlayers, int mode,
                              int layer, const int* active, GroupEnt* grp, int* ngroups) {
+  grid_wait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < bd.B; b += gridDim.x * blockDim.x) {
     if (active && !active[b]) {
       ngroups[b] = 0;
@@ -606,7 +607,8 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_group_pass
   float2* xs = reinterpret_cast<float2*>(dyn);
   float2* zs = xs + (1 << GT);
   __shared__ PassShared sh;
-  bool waited = false;   // uniform
+  bool waited = g == 0;   // uniform
+  if (waited) grid_wait();
   for (int chunk = blockIdx.x; chunk < gd.nchunks; chunk += gridDim.x) {
     const int b = gd.chunk_state[chunk];
     if (active && !active[b]) continue;
@@ -1155,16 +1157,16 @@ void launch_group_plan(const BatchDev& bd, const GroupDev& gd, const signed char
                        cudaStream_t s) {
   const int blocks = (bd.B + 127) / 128;
   qm_note_launch();
-  k_group_plan<<<blocks, 128, 0, s>>>(bd, gd, arity, nlayers, ORDER_BWD, 0, nullptr, gd.grp, gd.ngroups);
+  launch_after(k_group_plan, blocks, 128, 0, s, bd, gd, arity, nlayers, ORDER_BWD, 0, nullptr, gd.grp, gd.ngroups);
   qm_note_launch();
-  k_group_plan<<<blocks, 128, 0, s>>>(bd, gd, arity, nlayers, ORDER_FWD, 0, nullptr, gd.rgrp, gd.nrgroups);
+  launch_after(k_group_plan, blocks, 128, 0, s, bd, gd, arity, nlayers, ORDER_FWD, 0, nullptr, gd.rgrp, gd.nrgroups);
 }
 
 void launch_layer_plan(const BatchDev& bd, const GroupDev& gd, const signed char* arity, int mode, int layer,
                        const int* active, cudaStream_t s) {
   const int blocks = (bd.B + 127) / 128;
   qm_note_launch();
-  k_group_plan<<<blocks, 128, 0, s>>>(bd, gd, arity, nullptr, mode, layer, active, gd.rgrp, gd.nrgroups);
+  launch_after(k_group_plan, blocks, 128, 0, s, bd, gd, arity, nullptr, mode, layer, active, gd.rgrp, gd.nrgroups);
 }
 
 // Blocks of a tile-pass launch: the autotuned count, or at most the
@@ -1185,8 +1187,9 @@ void launch_rebuild_pass(const BatchDev& bd, const GroupDev& gd, int pass, float
                          const signed char* arity, const int* nlayers, const int* active, cudaStream_t s, int mode,
                          int layer, bool exact) {
   int grid = pass_grid(gd);
-  launch_after(k_rebuild_pass, pass > 0, grid, PASS_THREADS, (size_t)2 * sizeof(float2) << GT, 1, s, bd, gd, pass, psi,
-               gates, arity, nlayers, active, mode, layer, exact);
+  qm_note_launch();
+  launch_after(k_rebuild_pass, grid, PASS_THREADS, (size_t)2 * sizeof(float2) << GT, s, bd, gd, pass, psi, gates,
+               arity, nlayers, active, mode, layer, exact);
 }
 
 int launch_group_pass(const BatchDev& bd, const GroupDev& gd, int g, float2* psi, const float2* z_in, float2* z_out,
@@ -1200,8 +1203,9 @@ int launch_group_pass(const BatchDev& bd, const GroupDev& gd, int g, float2* psi
     attr_set = true;
   }
   int grid = pass_grid(gd);
-  launch_after(k_group_pass, g > 0, grid, PASS_THREADS, PASS_DYN_SMEM, 1, s, bd, gd, g, psi, z_in, z_out, gates,
-               gd.old_gates, arity, nlayers, active, znorm);
+  qm_note_launch();
+  launch_after(k_group_pass, grid, PASS_THREADS, PASS_DYN_SMEM, s, bd, gd, g, psi, z_in, z_out, gates, gd.old_gates,
+               arity, nlayers, active, znorm);
   return 0;
 }
 
@@ -1211,6 +1215,7 @@ void launch_group_polar(const BatchDev& bd, const GroupDev& gd, int g, double2* 
   // (fewer: the two cluster barriers cost what they save).
   int ranks = 1;
   while (ranks < 8 && bd.B * ranks * 2 <= 152 && gd.most_chunks >= 32 * ranks * 2) ranks *= 2;
-  launch_after(k_group_polar, true, bd.B * ranks, POLAR_THREADS, 0, ranks, s, bd, gd, g, gates, arity, nlayers, active,
-               nuc, env_out);
+  qm_note_launch();
+  launch_ranks_after(k_group_polar, ranks, bd.B * ranks, POLAR_THREADS, 0, s, bd, gd, g, gates, arity, nlayers,
+                     active, nuc, env_out);
 }

@@ -87,6 +87,7 @@ __device__ __forceinline__ bool tt_gram_here(const BatchDev& bd, const int* bond
 // 86 us now (512 wide, FP32 bound: 1630 -> 520 us).
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step, const float2* sv,
                                                            const float2* src, const int* bonds, xc* partials) {
+  grid_wait();
   __shared__ xc red[BLOCK_THREADS * TT_EPB];   // 32 KB
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
 // triangle mirrored.  Block x takes 32 entries at a time, block y a state.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram_sum(BatchDev bd, int step, const int* bonds,
                                                                const xc* partials, double2* gram) {
+  grid_wait();
   const int l8 = threadIdx.x & 7;
   for (int b = blockIdx.y; b < bd.B; b += gridDim.y) {
     const int c = bd.n[b] - 1 - step;
@@ -906,6 +908,7 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
                                                           double2* vwork, int max_bond, double cutoff,
                                                           double2* vsel, double2* tensors, int chi,
                                                           float2* scratch32, double fine) {
+  grid_wait();
   __shared__ JacobiShared<double2, double> js64;
   __shared__ JacobiShared<float2, float> js32;
   __shared__ double s_floor;
@@ -1085,6 +1088,7 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_project(BatchDev bd, int step, const float2* sv,
                                                               const float2* src, float2* dst,
                                                               const int* bonds, const double2* vsel) {
+  grid_wait();
   extern __shared__ float2 sh[];
   float2* vs = sh;
   float2* xs = sh + TT_MAXW * TT_MAXB;
@@ -1127,6 +1131,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_project(BatchDev bd, int s
 
 __global__ void k_tt_site0(BatchDev bd, const float2* rem0, const float2* rem1, const int* bonds,
                            double2* tensors, int chi, const double2* in_sq) {
+  grid_wait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < bd.B; b += gridDim.x * blockDim.x) {
     const int n = bd.n[b];
     const int* bond = bonds + (int64_t)b * (bd.max_n + 1);
@@ -1148,6 +1153,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_mps_contract(BatchDev bd, int
                                                                 const int* bonds, int chi,
                                                                 const float2* src, float2* dst_buf,
                                                                 float2* target) {
+  grid_wait();
   extern __shared__ float2 as[];
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
@@ -1196,13 +1202,13 @@ void launch_tt_gram(const BatchDev& bd, int step, const float2* sv, const float2
                     double2* partials, double2* gram, cudaStream_t s) {
   xc* part = reinterpret_cast<xc*>(partials);
   qm_note_launch();
-  k_tt_gram<<<grid_for(bd), BLOCK_THREADS, 0, s>>>(bd, step, sv, src, bonds, part);
+  launch_after(k_tt_gram, grid_for(bd), BLOCK_THREADS, 0, s, bd, step, sv, src, bonds, part);
   // the widest Gram a state can have at this step
   const int64_t wmax = step < 12 ? std::min<int64_t>(ipow2(step + 1), 2 * bd.tt_b) : 2 * bd.tt_b;
   const int64_t gx = std::min<int64_t>((wmax * wmax + BLOCK_THREADS / 8 - 1) / (BLOCK_THREADS / 8), 2048);
   qm_note_launch();
-  k_tt_gram_sum<<<dim3((unsigned)gx, (unsigned)std::min(bd.B, 65535)), BLOCK_THREADS, 0, s>>>(bd, step, bonds, part,
-                                                                                              gram);
+  launch_after(k_tt_gram_sum, dim3((unsigned)gx, (unsigned)std::min(bd.B, 65535)), BLOCK_THREADS, 0, s, bd, step,
+               bonds, part, gram);
 }
 
 void launch_tt_eig(const BatchDev& bd, int step, int* bonds, double2* gram, double2* vwork, int max_bond,
@@ -1214,8 +1220,8 @@ void launch_tt_eig(const BatchDev& bd, int step, int* bonds, double2* gram, doub
     attr = true;
   }
   qm_note_launch();
-  k_tt_eig<<<bd.B, TT_EIG_THREADS, TT_EIG_SMEM, s>>>(bd, step, bonds, gram, vwork, max_bond, cutoff, vsel, tensors,
-                                                    chi, reinterpret_cast<float2*>(scratch), fine);
+  launch_after(k_tt_eig, bd.B, TT_EIG_THREADS, TT_EIG_SMEM, s, bd, step, bonds, gram, vwork, max_bond, cutoff, vsel,
+               tensors, chi, reinterpret_cast<float2*>(scratch), fine);
 }
 
 void launch_tt_project(const BatchDev& bd, int step, const float2* sv, const float2* src, float2* dst,
@@ -1227,13 +1233,13 @@ void launch_tt_project(const BatchDev& bd, int step, const float2* sv, const flo
     configured = true;
   }
   qm_note_launch();
-  k_tt_project<<<grid_for(bd), BLOCK_THREADS, smem, s>>>(bd, step, sv, src, dst, bonds, vsel);
+  launch_after(k_tt_project, grid_for(bd), BLOCK_THREADS, smem, s, bd, step, sv, src, dst, bonds, vsel);
 }
 
 void launch_tt_site0(const BatchDev& bd, const float2* rem0, const float2* rem1, const int* bonds,
                      double2* tensors, int chi, const double2* in_sq, cudaStream_t s) {
   qm_note_launch();
-  k_tt_site0<<<(bd.B + 127) / 128, 128, 0, s>>>(bd, rem0, rem1, bonds, tensors, chi, in_sq);
+  launch_after(k_tt_site0, (bd.B + 127) / 128, 128, 0, s, bd, rem0, rem1, bonds, tensors, chi, in_sq);
 }
 
 void launch_mps_contract(const BatchDev& bd, int step, const double2* tensors, const int* bonds, int chi,
@@ -1245,5 +1251,6 @@ void launch_mps_contract(const BatchDev& bd, int step, const double2* tensors, c
     configured = true;
   }
   qm_note_launch();
-  k_mps_contract<<<grid_for(bd), BLOCK_THREADS, smem, s>>>(bd, step, tensors, bonds, chi, src, dst_buf, target);
+  launch_after(k_mps_contract, grid_for(bd), BLOCK_THREADS, smem, s, bd, step, tensors, bonds, chi, src, dst_buf,
+               target);
 }

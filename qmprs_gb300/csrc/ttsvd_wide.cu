@@ -122,6 +122,7 @@ __device__ __forceinline__ float2 fcfmac(float2 acc, float2 a, float2 b) {   // 
 // A <- G (FP32, padded with zeros to W), V <- I; per-block partial sums of
 // |G_ij|^2 in FP64.
 __global__ void k_bj_load(const double2* G, int w, float2* A, float2* V, int W, double* part) {
+  grid_wait();
   double acc = 0.0;
   const int64_t total = (int64_t)W * W;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -142,6 +143,7 @@ __global__ void k_bj_load(const double2* G, int w, float2* A, float2* V, int W, 
 
 // stats[0] = ||G||_F, stats[1] = trace (fixed-order sums).
 __global__ void k_bj_stats(const double* part, int nparts, const double2* G, int w, double* stats) {
+  grid_wait();
   double v[2] = {0.0, 0.0};
   for (int i = threadIdx.x; i < nparts; i += blockDim.x) v[0] += part[i];
   for (int i = threadIdx.x; i < w; i += blockDim.x) v[1] += G[(int64_t)i * w + i].x;
@@ -393,6 +395,7 @@ __global__ void __launch_bounds__(BJU_THREADS) k_bj_update(float2* A, float2* V,
 // Descending order of the FP32 eigenvalues (diagonal of A, ties by index):
 // perm[rank] = index, lamA[rank] = value.  One block.
 __global__ void __launch_bounds__(1024) k_bj_sort(const float2* A, int W, int n, int* perm, double* lamA) {
+  grid_wait();
   extern __shared__ float dg[];
   for (int i = threadIdx.x; i < n; i += blockDim.x) dg[i] = A[(int64_t)i * W + i].x;
   __syncthreads();
@@ -410,6 +413,7 @@ __global__ void __launch_bounds__(1024) k_bj_sort(const float2* A, int W, int n,
 
 // X[r][j] = V[r][perm[j]] (r, j < n) in FP64.
 __global__ void k_bj_basis(const float2* V, int W, int n, const int* perm, double2* X) {
+  grid_wait();
   const int64_t total = (int64_t)n * n;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(e / n), jc = (int)(e % n);
@@ -428,6 +432,7 @@ template <bool CONJ>
 __global__ void __launch_bounds__(256) k_zgemm(const double2* A, int64_t lda, const double2* B, int64_t ldb,
                                                const double2* D, int64_t ldd, double2* C, int64_t ldc, int M, int N,
                                                int K, double alpha) {
+  grid_wait();
   __shared__ double2 As[ZG_K][ZG_T + 1];
   __shared__ double2 Bs[ZG_K][ZG_T];
   const int m0 = blockIdx.x * ZG_T, n0 = blockIdx.y * ZG_T;
@@ -504,6 +509,7 @@ __global__ void __launch_bounds__(T * T / (4 * CO)) k_zgemm_df(const double2* A,
                                                                int64_t ldb, const double2* D, int64_t ldd,
                                                                double2* C, int64_t ldc, int M, int N, int K,
                                                                double alpha) {
+  grid_wait();
   constexpr int TC = T / CO, NT = T * T / (4 * CO);
   __shared__ xc As[ZG_K][T + 1];
   __shared__ xc Bs[ZG_K][T];
@@ -572,6 +578,7 @@ __global__ void __launch_bounds__(T * T / (4 * CO)) k_zgemm_df(const double2* A,
 // 1e-10).  Same tiling as k_zgemm.
 __global__ void __launch_bounds__(256) k_zgemm_small(const double2* A, int64_t lda, const double2* B, int64_t ldb,
                                                      double2* C, int64_t ldc, int M, int N, int K) {
+  grid_wait();
   __shared__ float2 As[ZG_K][ZG_T + 1];
   __shared__ float2 Bs[ZG_K][ZG_T];
   const int m0 = blockIdx.x * ZG_T, n0 = blockIdx.y * ZG_T;
@@ -621,6 +628,7 @@ __global__ void __launch_bounds__(256) k_zgemm_small(const double2* A, int64_t l
 
 // dst[r][c] = src[r][c] for r < rows, c < cols (row strides lds, ldd).
 __global__ void k_bj_copy(const double2* src, int64_t lds, double2* dst, int64_t ldd, int rows, int cols) {
+  grid_wait();
   const int64_t total = (int64_t)rows * cols;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(e / cols), c = (int)(e % cols);
@@ -631,6 +639,7 @@ __global__ void k_bj_copy(const double2* src, int64_t lds, double2* dst, int64_t
 // l_j = S_jj / (1 - R_jj) for the Kc refined columns; SR holds [S | X^H X_K]
 // (row stride 2 Kc), so 1 - R_jj is the (j, Kc + j) entry.
 __global__ void k_bj_lam(const double2* SR, int Kc, double* lamK) {
+  grid_wait();
   const int jc = blockIdx.x * blockDim.x + threadIdx.x;
   if (jc >= Kc) return;
   const int64_t o = (int64_t)jc * 2 * Kc;
@@ -651,6 +660,7 @@ __global__ void k_bj_lam(const double2* SR, int Kc, double* lamK) {
 // a fixed-order block reduction.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_bj_correct(double2* SR, int n, int Kc, const double* lamK,
                                                               const double* lamA, double tiny_rel, unsigned* emax) {
+  grid_wait();
   const int jc = blockIdx.x;
   const double top = fabs(lamA[0]);
   const double noise = BJ_NOISE * top, tiny = tiny_rel * top;
@@ -713,6 +723,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_bj_correct(double2* SR, int n
 // per column, fixed-order reduction.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_bj_rq(const double2* X, int n, const double2* T, int ldt, int c0,
                                                          double* lamA) {
+  grid_wait();
   const int i = c0 + blockIdx.x;
   double v[2] = {0.0, 0.0};
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
@@ -726,6 +737,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_bj_rq(const double2* X, int n
 
 // T <- (3 I - T) / 2 (m x m): one Newton-Schulz step's factor.
 __global__ void k_bj_ns(double2* T, int m) {
+  grid_wait();
   const int64_t total = (int64_t)m * m;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(e / m), c = (int)(e % m);
@@ -750,6 +762,7 @@ __global__ void __launch_bounds__(1024) k_bj_finalize(BatchDev bd, int b, int c,
                                                       const double* lamK, const double* stats, const double* tr_sub,
                                                       int* bonds, int max_bond, double cutoff, int* order,
                                                       double* lsort) {
+  grid_wait();
   for (int i = threadIdx.x; i < Kr; i += blockDim.x) {
     const double li = lamK[i];
     int rank = 0;
@@ -787,6 +800,7 @@ __global__ void __launch_bounds__(1024) k_bj_finalize(BatchDev bd, int b, int c,
 __global__ void __launch_bounds__(BLOCK_THREADS) k_bj_emit(BatchDev bd, int b, int c, const double2* X, int ldx,
                                                            int w, const int* bonds, const int* order, double2* vsel,
                                                            int vstride, double2* tensors, int chi) {
+  grid_wait();
   __shared__ double s_m[BLOCK_THREADS / 32];
   __shared__ int s_j[BLOCK_THREADS / 32];
   __shared__ double2 s_ph;
@@ -835,6 +849,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_bj_emit(BatchDev bd, int b, i
 // Row-Gram path.  Mt = M^H (w x rows, FP64) of the complex64 remainder M
 // (rows x w): 32 x 32 tiles transposed through shared memory.
 __global__ void k_bj_mt(const float2* M, int rows, int w, double2* Mt) {
+  grid_wait();
   __shared__ float2 t[32][33];
   const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
   for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
@@ -850,6 +865,7 @@ __global__ void k_bj_mt(const float2* M, int rows, int w, double2* Mt) {
 
 // dst = src in FP64 (count complex entries).
 __global__ void k_bj_f2d(const float2* src, int64_t count, double2* dst) {
+  grid_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x)
     dst[e] = f2d(src[e]);
 }
@@ -858,6 +874,7 @@ __global__ void k_bj_f2d(const float2* src, int64_t count, double2* dst) {
 // square root of the l-th eigenvalue (descending); then V = M^H U holds the
 // right singular vectors of the kept values.
 __global__ void k_bj_gather(const double2* X, int n, const int* order, const double* lsort, int K, double2* U) {
+  grid_wait();
   const int64_t total = (int64_t)n * K;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(e / K), l = (int)(e % K);
@@ -873,6 +890,7 @@ __global__ void k_bj_gather(const double2* X, int n, const int* order, const dou
 #define CG_K 16
 __global__ void __launch_bounds__(256) k_cgemm(const float2* A, int64_t lda, const double2* B, int64_t ldb,
                                                float2* C, int64_t ldc, int64_t M, int N, int K) {
+  grid_wait();
   __shared__ float2 As[CG_K][CG_T + 1];
   __shared__ float2 Bs[CG_K][CG_T];
   const int64_t m0 = (int64_t)blockIdx.x * CG_T;
@@ -981,19 +999,19 @@ static void zgemm(bool conj, const double2* A, int64_t lda, const double2* B, in
   qm_note_launch();
   if (df && g.x * g.y >= 2 * 152) {
     if (conj)
-      k_zgemm_df<true, 64, 4><<<g, 256, 0, s>>>(A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<true, 64, 4>), g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
     else
-      k_zgemm_df<false, 64, 4><<<g, 256, 0, s>>>(A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<false, 64, 4>), g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   } else if (df) {
     const dim3 h((M + 31) / 32, (N + 31) / 32);
     if (conj)
-      k_zgemm_df<true, 32, 2><<<h, 128, 0, s>>>(A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<true, 32, 2>), h, 128, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
     else
-      k_zgemm_df<false, 32, 2><<<h, 128, 0, s>>>(A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<false, 32, 2>), h, 128, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   } else if (conj) {
-    k_zgemm<true><<<g, 256, 0, s>>>(A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+    launch_after(k_zgemm<true>, g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   } else {
-    k_zgemm<false><<<g, 256, 0, s>>>(A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+    launch_after(k_zgemm<false>, g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   }
 }
 
@@ -1005,23 +1023,24 @@ static int bj_fp32(const double2* H, int n, BJScratch& sc, cudaStream_t s, int* 
   if (W > sc.W) return (int)cudaErrorInvalidValue;
   const int nb = W / BJ_B, np = nb / 2;
   qm_note_launch();
-  k_bj_load<<<BJ_PARTS, BLOCK_THREADS, 0, s>>>(H, n, sc.A, sc.V, W, sc.part);
+  launch_after(k_bj_load, BJ_PARTS, BLOCK_THREADS, 0, s, H, n, sc.A, sc.V, W, sc.part);
   qm_note_launch();
-  k_bj_stats<<<1, BLOCK_THREADS, 0, s>>>(sc.part, BJ_PARTS, H, n, sc.stats);
+  launch_after(k_bj_stats, 1, BLOCK_THREADS, 0, s, sc.part, BJ_PARTS, H, n, sc.stats);
   const int nA = np * (np - 1) / 2, nV = (W / BJ_S) * np;
   int sweeps = 0;
   for (int sweep = 0; sweep < BJ_MAX_SWEEPS; ++sweep) {
     cudaError_t e = cudaMemsetAsync(sc.count, 0, sizeof(int), s);
     if (e != cudaSuccess) return (int)e;
     for (int k = 0; k < nb - 1; ++k) {
-      // after the last round's update, which follows this kernel's own
-      // predecessor; a sweep's first round follows the counter's reset
+      qm_note_launch();
       if (k > 0)
-        launch_after(k_bj_solve<true>, nA + nV > 0, np, BJ_THREADS, 0, 1, s, sc.A, W, nb, k, sc.J, sc.stats, sc.count);
+        launch_after(k_bj_solve<true>, np, BJ_THREADS, 0, s, sc.A, W, nb, k, sc.J, sc.stats, sc.count);
       else
-        launch_after(k_bj_solve<false>, false, np, BJ_THREADS, 0, 1, s, sc.A, W, nb, k, sc.J, sc.stats, sc.count);
-      if (nA + nV > 0)
-        launch_after(k_bj_update, true, nA + nV, BJU_THREADS, 0, 1, s, sc.A, sc.V, W, nb, k, sc.J, nA);
+        launch_after(k_bj_solve<false>, np, BJ_THREADS, 0, s, sc.A, W, nb, k, sc.J, sc.stats, sc.count);
+      if (nA + nV > 0) {
+        qm_note_launch();
+        launch_after(k_bj_update, nA + nV, BJU_THREADS, 0, s, sc.A, sc.V, W, nb, k, sc.J, nA);
+      }
     }
     ++sweeps;
     int cnt = 0;
@@ -1031,9 +1050,9 @@ static int bj_fp32(const double2* H, int n, BJScratch& sc, cudaStream_t s, int* 
     if (cnt == 0) break;
   }
   qm_note_launch();
-  k_bj_sort<<<1, 1024, sizeof(float) * W, s>>>(sc.A, W, n, sc.perm, sc.lamA);
+  launch_after(k_bj_sort, 1, 1024, sizeof(float) * W, s, sc.A, W, n, sc.perm, sc.lamA);
   qm_note_launch();
-  k_bj_basis<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.V, W, n, sc.perm, sc.X);
+  launch_after(k_bj_basis, BJ_EB, BLOCK_THREADS, 0, s, sc.V, W, n, sc.perm, sc.X);
   *sweeps_out += sweeps;
   return (int)cudaGetLastError();
 }
@@ -1048,32 +1067,32 @@ static int bj_refine(const double2* H, int n, BJScratch& sc, int Kc, double tol,
   if (Kc < n) {   // eigenvalue estimates of the columns that stay
     zgemm(false, H, n, sc.X + Kc, n, nullptr, 0, sc.T2, n - Kc, n, n - Kc, n, 1.0, s, df);
     qm_note_launch();
-    k_bj_rq<<<n - Kc, BLOCK_THREADS, 0, s>>>(sc.X, n, sc.T2, n - Kc, Kc, sc.lamA);
+    launch_after(k_bj_rq, n - Kc, BLOCK_THREADS, 0, s, sc.X, n, sc.T2, n - Kc, Kc, sc.lamA);
   }
   double2* Xk = sc.YX + Kc;   // row stride 2 Kc
   qm_note_launch();
-  k_bj_copy<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.X, n, Xk, 2 * Kc, n, Kc);
+  launch_after(k_bj_copy, BJ_EB, BLOCK_THREADS, 0, s, sc.X, n, Xk, 2 * Kc, n, Kc);
   float emax = 0.f;
   for (int it = 0; it < BJ_MAX_REFINE; ++it) {
     // Y = H X_K into YX[:, :Kc]; [S | X^H X_K] = X^H YX
     zgemm(false, H, n, Xk, 2 * Kc, nullptr, 0, sc.YX, 2 * Kc, n, Kc, n, 1.0, s, df);
     zgemm(true, sc.X, n, sc.YX, 2 * Kc, nullptr, 0, sc.SR, 2 * Kc, n, 2 * Kc, n, 1.0, s, df);
     qm_note_launch();
-    k_bj_lam<<<(Kc + 255) / 256, 256, 0, s>>>(sc.SR, Kc, sc.lamK);
+    launch_after(k_bj_lam, (Kc + 255) / 256, 256, 0, s, sc.SR, Kc, sc.lamK);
     cudaError_t e = cudaMemsetAsync(sc.emax, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return (int)e;
     qm_note_launch();
-    k_bj_correct<<<Kc, BLOCK_THREADS, 0, s>>>(sc.SR, n, Kc, sc.lamK, sc.lamA, df ? 1e-12 : 1e-14, sc.emax);
+    launch_after(k_bj_correct, Kc, BLOCK_THREADS, 0, s, sc.SR, n, Kc, sc.lamK, sc.lamA, df ? 1e-12 : 1e-14, sc.emax);
     // X_K += X E
     if (df) {
       const dim3 g1((n + ZG_T - 1) / ZG_T, (Kc + ZG_T - 1) / ZG_T);
       qm_note_launch();
-      k_zgemm_small<<<g1, 256, 0, s>>>(sc.X, n, sc.SR, 2 * Kc, Xk, 2 * Kc, n, Kc, n);
+      launch_after(k_zgemm_small, g1, 256, 0, s, sc.X, n, sc.SR, 2 * Kc, Xk, 2 * Kc, n, Kc, n);
     } else {   // the exact mode: large first corrections need their own low-order bits
       zgemm(false, sc.X, n, sc.SR, 2 * Kc, Xk, 2 * Kc, Xk, 2 * Kc, n, Kc, n, 1.0, s, true);
     }
     qm_note_launch();
-    k_bj_copy<<<BJ_EB, BLOCK_THREADS, 0, s>>>(Xk, 2 * Kc, sc.X, n, n, Kc);
+    launch_after(k_bj_copy, BJ_EB, BLOCK_THREADS, 0, s, Xk, 2 * Kc, sc.X, n, n, Kc);
     ++*steps_out;
     unsigned bits = 0;
     e = cudaMemcpyAsync(&bits, sc.emax, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
@@ -1110,7 +1129,7 @@ int tt_block_eig(const BatchDev& bd, int b, int c, int wv, double2* gram, const 
   if (rowsrc) {
     if (w > sc.W || wv > sc.W) return (int)cudaErrorInvalidValue;
     qm_note_launch();
-    k_bj_mt<<<dim3((wv + 31) / 32, (w + 31) / 32), BLOCK_THREADS, 0, s>>>(rowsrc, w, wv, sc.Mt);
+    launch_after(k_bj_mt, dim3((wv + 31) / 32, (w + 31) / 32), BLOCK_THREADS, 0, s, rowsrc, w, wv, sc.Mt);
     zgemm(true, sc.Mt, w, sc.Mt, w, nullptr, 0, G, w, w, w, wv, 1.0, s, true);
   }
   int sweeps = 0, steps = 0;
@@ -1146,7 +1165,7 @@ int tt_block_eig(const BatchDev& bd, int b, int c, int wv, double2* gram, const 
     // same remainder, M^H M, in double-float products
     if (rowsrc && Kr > r) {
       qm_note_launch();
-      k_bj_f2d<<<BJ_EB, BLOCK_THREADS, 0, s>>>(rowsrc, (int64_t)w * wv, sc.T);
+      launch_after(k_bj_f2d, BJ_EB, BLOCK_THREADS, 0, s, rowsrc, (int64_t)w * wv, sc.T);
       zgemm(true, sc.T, wv, sc.T, wv, nullptr, 0, G, wv, wv, wv, w, 1.0, s, true);
       rowsrc = nullptr;
       w = wv;
@@ -1172,11 +1191,11 @@ int tt_block_eig(const BatchDev& bd, int b, int c, int wv, double2* gram, const 
     for (int ns = 0; ns < 4; ++ns) {
       zgemm(true, sc.T2, m, sc.T2, m, nullptr, 0, sc.T, m, m, m, w, 1.0, s, df);
       qm_note_launch();
-      k_bj_ns<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.T, m);
+      launch_after(k_bj_ns, BJ_EB, BLOCK_THREADS, 0, s, sc.T, m);
       zgemm(false, sc.T2, m, sc.T, m, nullptr, 0, ns == 3 ? Xn : sc.YX, ns == 3 ? w : m, w, m, m, 1.0, s, df);
       if (ns < 3) {
         qm_note_launch();
-        k_bj_copy<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.YX, m, sc.T2, m, w, m);
+        launch_after(k_bj_copy, BJ_EB, BLOCK_THREADS, 0, s, sc.YX, m, sc.T2, m, w, m);
       }
     }
     // Gram of the unresolved subspace, solved in `sub`
@@ -1187,16 +1206,16 @@ int tt_block_eig(const BatchDev& bd, int b, int c, int wv, double2* gram, const 
     // X_N <- X_N U, the refined eigenvalues after those of the resolved part
     zgemm(false, Xn, w, sub.X, m, nullptr, 0, sc.T2, m, w, m, m, 1.0, s, df);
     qm_note_launch();
-    k_bj_copy<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.T2, m, Xn, w, w, m);
+    launch_after(k_bj_copy, BJ_EB, BLOCK_THREADS, 0, s, sc.T2, m, Xn, w, w, m);
     ce = cudaMemcpyAsync(sc.lamK + r, sub.lamK, sizeof(double) * K1, cudaMemcpyDeviceToDevice, s);
     if (ce != cudaSuccess) return (int)ce;
   }
   qm_note_launch();
-  k_bj_finalize<<<1, 1024, 0, s>>>(bd, b, c, w, Kr, K, r, sc.lamK, sc.stats, deflated ? sub.stats + 1 : nullptr,
-                                    bonds, max_bond, cutoff, sc.order, sc.lsort);
+  launch_after(k_bj_finalize, 1, 1024, 0, s, bd, b, c, w, Kr, K, r, sc.lamK, sc.stats,
+               deflated ? sub.stats + 1 : nullptr, bonds, max_bond, cutoff, sc.order, sc.lsort);
   if (rowsrc) {   // V = M^H U Sigma^-1 (wv x K), then emitted in order
     qm_note_launch();
-    k_bj_gather<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.X, w, sc.order, sc.lsort, K, sc.T);
+    launch_after(k_bj_gather, BJ_EB, BLOCK_THREADS, 0, s, sc.X, w, sc.order, sc.lsort, K, sc.T);
     zgemm(false, sc.Mt, w, sc.T, K, nullptr, 0, sc.T2, K, wv, K, w, 1.0, s, true);
     // the division by sigma_l amplifies the eigenvector's error by
     // sigma_1 / sigma_l: two Newton-Schulz steps V <- V (3I - V^H V) / 2
@@ -1205,16 +1224,17 @@ int tt_block_eig(const BatchDev& bd, int b, int c, int wv, double2* gram, const 
     for (int ns = 0; ns < 2; ++ns) {
       zgemm(true, sc.T2, K, sc.T2, K, nullptr, 0, sc.H, K, K, K, wv, 1.0, s, true);
       qm_note_launch();
-      k_bj_ns<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.H, K);
+      launch_after(k_bj_ns, BJ_EB, BLOCK_THREADS, 0, s, sc.H, K);
       zgemm(false, sc.T2, K, sc.H, K, nullptr, 0, sc.T, K, wv, K, K, 1.0, s, true);
       qm_note_launch();
-      k_bj_copy<<<BJ_EB, BLOCK_THREADS, 0, s>>>(sc.T, K, sc.T2, K, wv, K);
+      launch_after(k_bj_copy, BJ_EB, BLOCK_THREADS, 0, s, sc.T, K, sc.T2, K, wv, K);
     }
     qm_note_launch();
-    k_bj_emit<<<K, BLOCK_THREADS, 0, s>>>(bd, b, c, sc.T2, K, wv, bonds, nullptr, vsel, bd.tt_b, tensors, chi);
+    launch_after(k_bj_emit, K, BLOCK_THREADS, 0, s, bd, b, c, sc.T2, K, wv, bonds, nullptr, vsel, bd.tt_b, tensors,
+                 chi);
   } else {
     qm_note_launch();
-    k_bj_emit<<<K, BLOCK_THREADS, 0, s>>>(bd, b, c, sc.X, w, w, bonds, sc.order, vsel, bd.tt_b, tensors, chi);
+    launch_after(k_bj_emit, K, BLOCK_THREADS, 0, s, bd, b, c, sc.X, w, w, bonds, sc.order, vsel, bd.tt_b, tensors, chi);
   }
   if (st) {
     st->sweeps += sweeps;
@@ -1230,5 +1250,5 @@ void launch_cgemm(const float2* A, int64_t lda, const double2* B, int64_t ldb, f
   if (M <= 0 || N <= 0 || K <= 0) return;
   dim3 grid((unsigned)((M + CG_T - 1) / CG_T), (unsigned)((N + CG_T - 1) / CG_T));
   qm_note_launch();
-  k_cgemm<<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
+  launch_after(k_cgemm, grid, 256, 0, s, A, lda, B, ldb, C, ldc, M, N, K);
 }
