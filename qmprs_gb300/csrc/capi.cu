@@ -403,30 +403,46 @@ int read_ints(qmprs_plan* p, const int* dev, std::vector<int>& host, cudaStream_
 void x_contract(qmprs_plan* p, const double2* tensors, const std::vector<int>& hb, xc* out, cudaStream_t s,
                 const std::vector<int>* start = nullptr, const xc* saved = nullptr, const double* scale = nullptr) {
   const int stride = p->max_n + 1;
+  std::vector<int> next(p->B, 0);   // the next site; 0: a state with invalid bonds
   for (int b = 0; b < p->B; ++b) {
     const int n = p->n[b];
     const int* bb = hb.data() + (size_t)b * stride;
     bool ok = true;
     for (int c = 0; c <= n; ++c) ok = ok && bb[c] >= 1 && bb[c] <= p->tt_b;
     if (!ok) continue;
-    const int ce = chi_eff_host(p->max_bond, n);
-    const double2* t0 = tensors + p->tensor_off[b];
     xc* cur = p->X0 + p->vec_off[b];
-    xc* nxt = p->X1 + p->vec_off[b];
-    int c_first = 1;
+    next[b] = 1;
     if (start && (*start)[b] >= 1) {
-      c_first = (*start)[b];
-      launch_x_scale_flat(saved + p->vec_off[b], cur, ipow2(c_first) * bb[c_first], scale + b, s);
+      next[b] = (*start)[b];
+      launch_x_scale_flat(saved + p->vec_off[b], cur, ipow2(next[b]) * bb[next[b]], scale + b, s);
     } else {
-      launch_x_from_d_flat(t0, cur, 2 * (int64_t)bb[1], s);
+      launch_x_from_d_flat(tensors + p->tensor_off[b], cur, 2 * (int64_t)bb[1], s);
     }
-    for (int c = c_first; c <= n - 1; ++c) {
-      const int rc = bb[c], rn = bb[c + 1];
-      const double2* a = t0 + (int64_t)c * 2 * ce * ce;
-      xc* o = c == n - 1 ? out + p->vec_off[b] : nxt;
-      launch_x_gemm(cur, rc, a, 2 * rn, o, 2 * rn, ipow2(c), 2 * rn, rc, s);
-      std::swap(cur, nxt);
+  }
+  // the states' sites side by side, a site of each per step
+  std::vector<XGemmJob> jobs;
+  for (xc *cur = p->X0, *nxt = p->X1;; std::swap(cur, nxt)) {
+    jobs.clear();
+    for (int b = 0; b < p->B; ++b) {
+      const int n = p->n[b], c = next[b];
+      if (c < 1 || c > n - 1) continue;
+      const int* bb = hb.data() + (size_t)b * stride;
+      const int ce = chi_eff_host(p->max_bond, n), rc = bb[c], rn = bb[c + 1];
+      XGemmJob jb = {};
+      jb.A = cur + p->vec_off[b];
+      jb.lda = rc;
+      jb.B = tensors + p->tensor_off[b] + (int64_t)c * 2 * ce * ce;
+      jb.ldb = 2 * rn;
+      jb.C = (c == n - 1 ? out : nxt) + p->vec_off[b];
+      jb.ldc = 2 * rn;
+      jb.M = ipow2(c);
+      jb.N = 2 * rn;
+      jb.K = rc;
+      jobs.push_back(jb);
+      ++next[b];
     }
+    if (jobs.empty()) break;
+    launch_x_gemms(jobs.data(), (int)jobs.size(), s);
   }
 }
 
@@ -446,19 +462,28 @@ int exact_mps_from_statevector(qmprs_plan* p, const double2* sv, int max_bond, d
   CK(cudaMemcpyAsync(sq.data(), p->sq, sizeof(double2) * p->B, cudaMemcpyDeviceToHost, s));
   std::vector<int> hb((size_t)p->B * stride), start(p->B, -1);
   xc* buf[2] = {p->X1, p->X2};
+  std::vector<XGramJob> grams;
+  std::vector<XGemmJob> gemms;
+  if ((rc = read_ints(p, bonds, hb, s)) != QMPRS_OK) return rc;
   for (int j = 0; j + 2 <= p->max_n; ++j) {
-    if ((rc = read_ints(p, bonds, hb, s)) != QMPRS_OK) return rc;
     const xc* src = j == 0 ? p->X0 : buf[(j - 1) & 1];
     bool wide = false;
+    grams.clear();
     for (int b = 0; b < p->B; ++b) {
       const int c = p->n[b] - 1 - j;
       if (c < 1) continue;
       const int r = hb[(size_t)b * stride + c + 1];
       if (r < 1 || r > p->tt_b) continue;
-      launch_x_gram(src + p->vec_off[b], ipow2(c), 2 * r, p->tt_partials + (int64_t)b * p->bd.tt_region, WW,
-                    p->gram + (int64_t)b * WW, s);
+      XGramJob jb = {};
+      jb.m = src + p->vec_off[b];
+      jb.rows = ipow2(c);
+      jb.w = 2 * r;
+      jb.part = p->tt_partials + (int64_t)b * p->bd.tt_region;
+      jb.gram = p->gram + (int64_t)b * WW;
+      grams.push_back(jb);
       wide = wide || 2 * r > p->bd.eig_wmax;
     }
+    launch_x_grams(grams.data(), (int)grams.size(), WW, s);
     launch_tt_eig(p->bd, j, bonds, p->gram, p->vwork, max_bond, cutoff, p->vsel2, tensors, p->max_bond,
                   p->tt_partials, 1e-15, s);
     if (wide) {
@@ -473,21 +498,31 @@ int exact_mps_from_statevector(qmprs_plan* p, const double2* sv, int max_bond, d
       }
     }
     if ((rc = read_ints(p, bonds, hb, s)) != QMPRS_OK) return rc;
+    gemms.clear();
     for (int b = 0; b < p->B; ++b) {
       const int c = p->n[b] - 1 - j;
       if (c < 1) continue;
       const int r = hb[(size_t)b * stride + c + 1], keep = hb[(size_t)b * stride + c];
       if (r < 1 || keep < 1 || r > p->tt_b || keep > p->tt_b) continue;
-      launch_x_gemm(src + p->vec_off[b], 2 * r, p->vsel2 + (int64_t)b * WW, p->tt_b, buf[j & 1] + p->vec_off[b],
-                    keep, ipow2(c), keep, 2 * r, s);
+      XGemmJob jb = {};
+      jb.A = src + p->vec_off[b];
+      jb.lda = 2 * r;
+      jb.B = p->vsel2 + (int64_t)b * WW;
+      jb.ldb = p->tt_b;
+      jb.C = buf[j & 1] + p->vec_off[b];
+      jb.ldc = keep;
+      jb.M = ipow2(c);
+      jb.N = keep;
+      jb.K = 2 * r;
       // the last cut (so far, right to left) that truncates, or the first
       // cut: the target's contraction starts from its projected remainder
       if (c == p->n[b] - 1 || keep < std::min<int64_t>(ipow2(c), 2 * r)) {
-        CK(cudaMemcpyAsync(p->XT + p->vec_off[b], buf[j & 1] + p->vec_off[b], sizeof(xc) * ipow2(c) * keep,
-                           cudaMemcpyDeviceToDevice, s));
+        jb.C2 = p->XT + p->vec_off[b];
         start[b] = c;
       }
+      gemms.push_back(jb);
     }
+    launch_x_gemms(gemms.data(), (int)gemms.size(), s);
   }
   for (int b = 0; b < p->B; ++b) {
     const int r1 = hb[(size_t)b * stride + 1];

@@ -175,17 +175,39 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_d_dot(BatchDev bd, const doub
 __host__ __device__ inline int x_gram_ti(int w) { return w < 32 ? w : 32; }
 __host__ __device__ inline int x_gram_nt(int w) { const int ti = x_gram_ti(w); return (w + ti - 1) / ti; }
 
-// Partial Gram sums of the rows of split blockIdx.y for tile blockIdx.x:
+template <class J>
+struct XJobs {
+  J job[X_JOBS];
+  int count;
+};
+// The job of block `block` (uniform): the last whose first block is at most that.
+template <class J>
+__device__ __forceinline__ const J& x_job(const XJobs<J>& jobs, int J::*first, int block) {
+  int k = 0;
+  while (k + 1 < jobs.count && jobs.job[k + 1].*first <= block) ++k;
+  return jobs.job[k];
+}
+
+// Partial Gram sums of one tile over one split of the rows:
 // part[split * WW + a * w + c] for the tile's entries with a <= c.
-__global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_tile(const xc* m, int64_t rows, int w, int nsplit,
-                                                               double2* part, int64_t WW) {
+// The states of a batch run side by side: one after another, every launch of
+// a few dozen blocks waited on its own rows (14 states of 8-14 qubits: 145
+// launches of 18.4 us, and 145 of 2 us to sum them).
+__global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_tile(const __grid_constant__ XJobs<XGramJob> jobs,
+                                                               int64_t WW) {
   grid_wait();
   __shared__ double2 red[BLOCK_THREADS * 4];
+  const XGramJob& jb = x_job(jobs, &XGramJob::block0, blockIdx.x);
+  const xc* m = jb.m;
+  const int64_t rows = jb.rows;
+  const int w = jb.w, nt = x_gram_nt(w), ntri = nt * (nt + 1) / 2;
+  const int tile = (blockIdx.x - jb.block0) % ntri, split = (blockIdx.x - jb.block0) / ntri;
+  double2* part = jb.part + (int64_t)split * WW;
   const int TI = x_gram_ti(w), G = TI / 2, EG = G * G;
   const int RL = BLOCK_THREADS / EG;
   int ti = 0, tj = 0;
   {
-    int t = blockIdx.x, j = 0;
+    int t = tile, j = 0;
     while (t > j) {
       t -= j + 1;
       ++j;
@@ -196,7 +218,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_tile(const xc* m, int6
   const int e = threadIdx.x % EG, rl = threadIdx.x / EG;
   const int a0 = ti * TI + 2 * (e / G), c0 = tj * TI + 2 * (e % G);
   int64_t lo, hi;
-  tile_range(rows, blockIdx.y, nsplit, &lo, &hi);
+  tile_range(rows, split, jb.nsplit, &lo, &hi);
   double2 acc[4] = {czero(), czero(), czero(), czero()};
   if (rl < RL && a0 < w && c0 < w) {
     int64_t r = lo + rl;
@@ -222,16 +244,22 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_tile(const xc* m, int6
     double2 s = czero();
     for (int l = 0; l < RL; ++l) s = cadd(s, red[(l * EG + eo) * 4 + k]);
     const int a = ti * TI + 2 * (eo / G) + k / 2, c = tj * TI + 2 * (eo % G) + k % 2;
-    if (a < w && c < w && a <= c) part[(int64_t)blockIdx.y * WW + (int64_t)a * w + c] = s;
+    if (a < w && c < w && a <= c) part[(int64_t)a * w + c] = s;
   }
 }
 
 // gram[a * w + c] = sum over splits (in order), mirrored to the lower triangle.
-__global__ void k_x_gram_reduce(const double2* part, int nsplit, int w, int64_t WW, double2* gram) {
+__global__ void __launch_bounds__(BLOCK_THREADS) k_x_gram_reduce(const __grid_constant__ XJobs<XGramJob> jobs,
+                                                                 int64_t WW) {
   grid_wait();
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)w * w; e += (int64_t)gridDim.x * blockDim.x) {
+  const XGramJob& jb = x_job(jobs, &XGramJob::rblock0, blockIdx.x);
+  const int w = jb.w, nsplit = jb.nsplit;
+  const double2* part = jb.part;
+  double2* gram = jb.gram;
+  const int64_t e = (int64_t)(blockIdx.x - jb.rblock0) * BLOCK_THREADS + threadIdx.x;
+  if (e < (int64_t)w * w) {
     const int a = (int)(e / w), c = (int)(e % w);
-    if (a > c) continue;
+    if (a > c) return;
     double2 s = czero();
     for (int t = 0; t < nsplit; ++t) s = cadd(s, part[(int64_t)t * WW + e]);
     if (a == c) {
@@ -246,23 +274,28 @@ __global__ void k_x_gram_reduce(const double2* part, int nsplit, int w, int64_t 
 #define XG_KC 32   // K chunk of k_x_gemm
 
 // C (M x N, double-float, ldc) = A (M x K, double-float, lda) * B (K x N,
-// complex128, ldb).  Block tile: TN = min(N, 32) columns (a power of two) x
-// 256 / TN rows, one output per thread; B is split into double-float in
-// shared memory one K chunk at a time; sums flushed to fp64 per chunk.
-__global__ void __launch_bounds__(BLOCK_THREADS) k_x_gemm(const xc* A, int64_t lda, const double2* B, int64_t ldb,
-                                                          xc* C, int64_t ldc, int64_t M, int N, int K, int TN) {
+// complex128, ldb), the states of a batch side by side.  Block tile: tn =
+// min(N, 32) columns (a power of two) x 256 / tn rows, one output per thread;
+// B is split into double-float in shared memory one K chunk at a time; sums
+// flushed to fp64 per chunk.
+__global__ void __launch_bounds__(BLOCK_THREADS) k_x_gemm(const __grid_constant__ XJobs<XGemmJob> jobs) {
   grid_wait();
   __shared__ xc Bs[XG_KC][32];
-  const int TM = BLOCK_THREADS / TN;
-  const int64_t row = (int64_t)blockIdx.x * TM + threadIdx.x / TN;
-  const int col = blockIdx.y * TN + threadIdx.x % TN;
+  const XGemmJob& jb = x_job(jobs, &XGemmJob::block0, blockIdx.x);
+  const xc* A = jb.A;
+  const double2* B = jb.B;
+  const int64_t lda = jb.lda, ldb = jb.ldb, M = jb.M;
+  const int N = jb.N, K = jb.K, TN = jb.tn, TM = BLOCK_THREADS / TN;
+  const int gm = (int)((M + TM - 1) / TM), bx = (blockIdx.x - jb.block0) % gm, by = (blockIdx.x - jb.block0) / gm;
+  const int64_t row = (int64_t)bx * TM + threadIdx.x / TN;
+  const int col = by * TN + threadIdx.x % TN;
   const bool act = row < M && col < N;
   double2 acc = czero();
   for (int k0 = 0; k0 < K; k0 += XG_KC) {
     __syncthreads();
     for (int e = threadIdx.x; e < XG_KC * TN; e += blockDim.x) {
       const int kk = e / TN, nn = e % TN;
-      const int gk = k0 + kk, gn = blockIdx.y * TN + nn;
+      const int gk = k0 + kk, gn = by * TN + nn;
       Bs[kk][nn] = (gk < K && gn < N) ? xc_from_d(B[(int64_t)gk * ldb + gn]) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
@@ -274,7 +307,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_gemm(const xc* A, int64_t l
       acc = cadd(acc, xa_to_d(s));
     }
   }
-  if (act) C[row * ldc + col] = xc_from_d(acc);
+  if (act) {
+    const xc v = xc_from_d(acc);
+    jb.C[row * jb.ldc + col] = v;
+    if (jb.C2) jb.C2[row * jb.ldc + col] = v;
+  }
 }
 
 // Site 0 of state b: the last remainder (2 x r1) rescaled to the input norm
@@ -773,26 +810,45 @@ void launch_x_normalize(const BatchDev& bd, const xc* src, xc* dst, double2* par
   launch_after(k_x_scale, grid_for(bd), BLOCK_THREADS, 0, s, bd, src, dst, sq);
 }
 
-void launch_x_gram(const xc* m, int64_t rows, int w, double2* part, int64_t WW, double2* gram, cudaStream_t s) {
-  int nsplit = (int)std::min<int64_t>(TT_SPLIT, std::max<int64_t>(1, rows / 1024));
-  const int nt = x_gram_nt(w);
-  dim3 grid(nt * (nt + 1) / 2, nsplit);
-  qm_note_launch();
-  launch_after(k_x_gram_tile, grid, BLOCK_THREADS, 0, s, m, rows, w, nsplit, part, WW);
-  const int64_t ww = (int64_t)w * w;
-  const int blocks = (int)std::min<int64_t>((ww + 255) / 256, 1024);
-  qm_note_launch();
-  launch_after(k_x_gram_reduce, blocks, 256, 0, s, part, nsplit, w, WW, gram);
+void launch_x_grams(XGramJob* jobs, int count, int64_t WW, cudaStream_t s) {
+  for (int j0 = 0; j0 < count; j0 += X_JOBS) {
+    XJobs<XGramJob> js;
+    js.count = std::min(X_JOBS, count - j0);
+    int blocks = 0, rblocks = 0;
+    for (int k = 0; k < js.count; ++k) {
+      XGramJob& jb = js.job[k];
+      jb = jobs[j0 + k];
+      jb.nsplit = (int)std::min<int64_t>(TT_SPLIT, std::max<int64_t>(1, jb.rows / 1024));
+      jb.block0 = blocks;
+      jb.rblock0 = rblocks;
+      const int nt = x_gram_nt(jb.w);
+      blocks += nt * (nt + 1) / 2 * jb.nsplit;
+      rblocks += (int)(((int64_t)jb.w * jb.w + BLOCK_THREADS - 1) / BLOCK_THREADS);
+    }
+    qm_note_launch();
+    launch_after(k_x_gram_tile, blocks, BLOCK_THREADS, 0, s, js, WW);
+    qm_note_launch();
+    launch_after(k_x_gram_reduce, rblocks, BLOCK_THREADS, 0, s, js, WW);
+  }
 }
 
-void launch_x_gemm(const xc* A, int64_t lda, const double2* B, int64_t ldb, xc* C, int64_t ldc, int64_t M, int N,
-                   int K, cudaStream_t s) {
-  int TN = 1;
-  while (TN < N && TN < 32) TN <<= 1;
-  const int TM = BLOCK_THREADS / TN;
-  dim3 grid((unsigned)((M + TM - 1) / TM), (unsigned)((N + TN - 1) / TN));
-  qm_note_launch();
-  launch_after(k_x_gemm, grid, BLOCK_THREADS, 0, s, A, lda, B, ldb, C, ldc, M, N, K, TN);
+void launch_x_gemms(XGemmJob* jobs, int count, cudaStream_t s) {
+  for (int j0 = 0; j0 < count; j0 += X_JOBS) {
+    XJobs<XGemmJob> js;
+    js.count = std::min(X_JOBS, count - j0);
+    int64_t blocks = 0;
+    for (int k = 0; k < js.count; ++k) {
+      XGemmJob& jb = js.job[k];
+      jb = jobs[j0 + k];
+      jb.tn = 1;
+      while (jb.tn < jb.N && jb.tn < 32) jb.tn <<= 1;
+      const int tm = BLOCK_THREADS / jb.tn;
+      jb.block0 = (int)blocks;
+      blocks += (jb.M + tm - 1) / tm * ((jb.N + jb.tn - 1) / jb.tn);
+    }
+    qm_note_launch();
+    launch_after(k_x_gemm, (unsigned)blocks, BLOCK_THREADS, 0, s, js);
+  }
 }
 
 void launch_x_site0(const xc* rem, int r1, double in_sq, double2* t0, double* f_out, cudaStream_t s) {

@@ -19,12 +19,30 @@ void launch_d_dot(const BatchDev& bd, const double2* a, const double2* b, double
 // dst = src / ||src||, sq[b].x = ||src||^2
 void launch_x_normalize(const BatchDev& bd, const xc* src, xc* dst, double2* partials, double2* sq, cudaStream_t s);
 
-// stage (a), one state at a time: Gram of a rows x w remainder into gram
-// (row-major, stride w), through `part` (TT_SPLIT x WW complex128 partials)
-void launch_x_gram(const xc* m, int64_t rows, int w, double2* part, int64_t WW, double2* gram, cudaStream_t s);
-// C = A B (A double-float M x K, B complex128 K x N, C double-float M x N)
-void launch_x_gemm(const xc* A, int64_t lda, const double2* B, int64_t ldb, xc* C, int64_t ldc, int64_t M, int N,
-                   int K, cudaStream_t s);
+// stage (a)
+//
+// One state's Gram of m (rows x w) into gram, with partials of WW entries in
+// part, and one state's product C (M x N, ldc) = A B (also to C2 when given).
+// A step's jobs run side by side, X_JOBS of them to a launch; the launch
+// functions fill in the fields below the line.
+#define X_JOBS 24
+struct XGramJob {
+  const xc* m;
+  double2 *part, *gram;
+  int64_t rows;
+  int w;
+  int nsplit, block0, rblock0;   // splits of the rows; first block of the sums and of their reduction
+};
+struct XGemmJob {
+  const xc* A;
+  const double2* B;
+  xc *C, *C2;
+  int64_t lda, ldb, ldc, M;
+  int N, K;
+  int tn, block0;                // columns per block tile; first block
+};
+void launch_x_grams(XGramJob* jobs, int count, int64_t WW, cudaStream_t s);
+void launch_x_gemms(XGemmJob* jobs, int count, cudaStream_t s);
 void launch_x_site0(const xc* rem, int r1, double in_sq, double2* t0, double* f_out, cudaStream_t s);
 void launch_x_scale_flat(const xc* src, xc* dst, int64_t count, const double* f, cudaStream_t s);
 void launch_x_from_d_flat(const double2* src, xc* dst, int64_t count, cudaStream_t s);
