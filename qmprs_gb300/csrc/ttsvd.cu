@@ -890,13 +890,129 @@ __device__ void tt_df_eig(xc* Vg, int w, int ld) {
   }
 }
 
+// Entry t of the upper triangle, column by column: (i, j), i <= j.
+__device__ __forceinline__ void tt_upper(int t, int* i, int* j) {
+  int c = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+  while (c * (c + 1) / 2 > t) --c;
+  while ((c + 1) * (c + 2) / 2 <= t) ++c;
+  *j = c;
+  *i = t - c * (c + 1) / 2;
+}
+
+// FP64 finish of nearly exact vectors V of G (both w x w, stride ld, shared
+// memory), by one first-order step (Ogita & Aishima, as in ttsvd_wide.cu):
+// S = V^H G V and R = I - V^H V in FP64, l_j = S_jj / (1 - R_jj), E_ij =
+// (S_ij + l_j R_ij) / (l_j - l_i), E_jj = R_jj / 2, V <- V (I + E + E^2 / 2)
+// with FP32 products.  Pairs coupled by at most floor_abs only share their
+// defect, E_ij = R_ij / 2.  False, with G and V unchanged, if an entry of E is
+// above 2e-6 (its cube, or FP32's rounding of it, would show): FP64 sweeps
+// take it.  T is scratch.
+// FP64 instructions bound it (64 cycles each per SM quarter): two products
+// instead of the four, and the sweeps, that a Newton-Schulz step, the
+// similar matrix and Jacobi rotations took.  Measured over the 15 launches
+// of a batch of exact encodes (Grams up to 16 wide): 3.6 -> 1.5 ms with the passes before it.
+__device__ bool tt_refine(const double2* G, double2* V, double2* T, double* lam, int w, int ld, double floor_abs) {
+  const int nu = w * (w + 1) / 2;
+  float2* E = reinterpret_cast<float2*>(T);   // after its last use
+  float2* V32 = E + w * ld;   // E + E^2 / 2, then V
+  // upper triangles of S and R, two entries each per thread (w <= 64: up to five)
+  constexpr int PER = (TT_EIG_SMEM_W * (TT_EIG_SMEM_W + 1) / 2 + TT_EIG_THREADS - 1) / TT_EIG_THREADS;
+  for (int e = threadIdx.x; e < w * w; e += TT_EIG_THREADS) {   // T = G V
+    const int i = e / w, j = e % w;
+    double2 a = czero();
+    for (int k = 0; k < w; ++k) {
+      const double2 x = G[i * ld + k], y = V[k * ld + j];
+      a.x = fma(x.x, y.x, a.x);
+      a.y = fma(x.x, y.y, a.y);
+      a.x = fma(-x.y, y.y, a.x);
+      a.y = fma(x.y, y.x, a.y);
+    }
+    T[i * ld + j] = a;
+  }
+  __syncthreads();
+  double2 S[PER], R[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int t = threadIdx.x + u * TT_EIG_THREADS;
+    S[u] = R[u] = czero();
+    if (t >= nu) continue;
+    int i, j;
+    tt_upper(t, &i, &j);
+    double2 a = czero(), b = cd(i == j ? 1.0 : 0.0, 0.0);
+    for (int k = 0; k < w; ++k) {   // conj(v) (G V), - conj(v) v
+      const double2 v = V[k * ld + i], x = T[k * ld + j], y = V[k * ld + j];
+      a.x = fma(v.x, x.x, a.x);
+      a.y = fma(v.x, x.y, a.y);
+      b.x = fma(-v.x, y.x, b.x);
+      b.y = fma(-v.x, y.y, b.y);
+      a.x = fma(v.y, x.y, a.x);
+      a.y = fma(-v.y, x.x, a.y);
+      b.x = fma(-v.y, y.y, b.x);
+      b.y = fma(v.y, y.x, b.y);
+    }
+    S[u] = a;
+    R[u] = b;
+    if (i == j) lam[i] = a.x / (1.0 - b.x);
+  }
+  __syncthreads();   // lam; T is read
+  bool ok = true;
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int t = threadIdx.x + u * TT_EIG_THREADS;
+    if (t >= nu) continue;
+    int i, j;
+    tt_upper(t, &i, &j);
+    const float2 r = cf((float)R[u].x, (float)R[u].y);
+    float2 up = cf(0.5f * r.x, i == j ? 0.f : 0.5f * r.y), lo = cf(up.x, -up.y);
+    if (i != j) {
+      const float2 b = cf((float)fma(lam[j], R[u].x, S[u].x), (float)fma(lam[j], R[u].y, S[u].y));
+      if (fmaf(b.x, b.x, b.y * b.y) > (float)floor_abs * (float)floor_abs) {
+        const float d = (float)(lam[j] - lam[i]);
+        up = cf(__fdividef(b.x, d), __fdividef(b.y, d));
+        lo = cf(r.x - up.x, -(r.y - up.y));   // E + E^H = R
+      }
+      E[j * ld + i] = lo;
+    }
+    E[i * ld + j] = up;
+    ok = ok && fabsf(up.x) < 2e-6f && fabsf(up.y) < 2e-6f && fabsf(lo.x) < 2e-6f && fabsf(lo.y) < 2e-6f;
+  }
+  if (!__syncthreads_and(ok)) return false;
+  for (int e = threadIdx.x; e < w * w; e += TT_EIG_THREADS) {
+    const int i = e / w, j = e % w;
+    float2 a = cf(0.f, 0.f);
+    for (int k = 0; k < w; ++k) a = fmac(a, E[i * ld + k], E[k * ld + j]);
+    V32[i * ld + j] = cf(fmaf(0.5f, a.x, E[i * ld + j].x), fmaf(0.5f, a.y, E[i * ld + j].y));
+  }
+  __syncthreads();
+  {
+    float2* t = E;
+    E = V32;
+    V32 = t;
+  }
+  for (int e = threadIdx.x; e < w * w; e += TT_EIG_THREADS) {
+    const double2 v = V[e / w * ld + e % w];
+    V32[e / w * ld + e % w] = cf((float)v.x, (float)v.y);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < w * w; e += TT_EIG_THREADS) {
+    const int i = e / w, j = e % w;
+    float2 a = cf(0.f, 0.f);
+    for (int k = 0; k < w; ++k) a = fmac(a, V32[i * ld + k], E[k * ld + j]);
+    const double2 v = V[i * ld + j];
+    V[i * ld + j] = cd(v.x + (double)a.x, v.y + (double)a.y);
+  }
+  __syncthreads();
+  return true;
+}
+
 // an eigenvalue for sorting: NaN counts as negative, so that ranks stay a permutation
 __device__ __forceinline__ double tt_number(double v) { return v == v ? v : -1.0; }
 
 // One CTA per state; G and V are row-major w x w.  For w <= TT_EIG_SMEM_W
 // they are diagonalised in shared memory by the double-float passes above;
 // the exact mode (fine = 1e-15 of the trace) continues from those vectors
-// with one FP64 Newton-Schulz step and FP64 sweeps.  For 64 < w <= 128 the
+// with one FP64 step (tt_refine), or where that does not do with a
+// Newton-Schulz step and FP64 sweeps.  For 64 < w <= 128 the
 // vectors are found in global memory (L2 resident) in two precisions: FP32
 // Jacobi sweeps on a float copy of G in `scratch32` (the Gram partials,
 // already reduced), one Newton-Schulz step V <- V (3I - V^H V) / 2 in FP64
@@ -947,10 +1063,12 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
   __syncthreads();
   const double tr = s_floor;
   bool fp64 = !in_smem;   // FP64 sweeps to `fine`
+  double trg = tr;        // of the scaled G
   if (in_smem) {
     int ex = 0;
     if (tr > 0.0 && isfinite(tr)) frexp(tr, &ex);
     const double sc = ldexp(1.0, -ex);
+    trg = tr * sc;
     xc* Gx = reinterpret_cast<xc*>(G);
     xc* Vx = reinterpret_cast<xc*>(Vg);
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
@@ -963,9 +1081,13 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) V[(e / w) * ld + e % w] = xc_to_d(Vx[e]);
     __syncthreads();
     if (fine < 1e-14) {
-      for (int e = threadIdx.x; e < w * w; e += blockDim.x) G[(e / w) * ld + e % w] = Gg[e];
+      for (int e = threadIdx.x; e < w * w; e += blockDim.x) G[(e / w) * ld + e % w] = cscale(Gg[e], sc);
       __syncthreads();
-      fp64 = true;
+      fp64 = !tt_refine(G, V, Sc, s_lam, w, ld, fine * trg);
+      if (!fp64) {
+        for (int i = threadIdx.x; i < w; i += blockDim.x) s_lam[i] = tt_number(s_lam[i]);
+        __syncthreads();
+      }
     }
   } else {
     float2* G32 = scratch32 + (int64_t)b * 2 * bd.tt_region;
@@ -1022,7 +1144,7 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
     // no eigenvalue by more than that (three to five orders below the 1e-10
     // truncation cutoff).  Without it the rounding-level null-space block of
     // a rank-deficient Gram keeps rotating until the sweep limit.
-    jacobi_run<double2, double>(G, V, w, ld, 1e-15, fine * tr, 40, js64);
+    jacobi_run<double2, double>(G, V, w, ld, 1e-15, fine * trg, 40, js64);
     for (int i = threadIdx.x; i < w; i += blockDim.x) s_lam[i] = tt_number(G[i * ld + i].x);
     __syncthreads();
   }

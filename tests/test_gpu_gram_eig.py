@@ -86,3 +86,26 @@ def test_spectra_at_padded_widths(eng, n, chi, kind):
     assert int(bd.cpu().max()) <= (1 if kind == "rank_one" else 2 if kind == "two_blocks" else chi)
     got = target.cpu().numpy().view(p.npdtype)
     assert np.linalg.norm(got - v32) <= 4 * n * 2.0 ** -23 * 1e2
+
+
+@pytest.mark.parametrize("kind", ["mps", "mixture"])
+@pytest.mark.parametrize("n,chi", [(6, 8), (9, 9), (12, 20), (13, 32)])
+def test_exact_finish(eng, n, chi, kind):
+    """The exact mode's FP64 finish on spectra it takes in one step and on
+    decaying ones that go on to FP64 sweeps: right-isometric sites, and kept
+    weight as the oracle's.  Bounds: isometry as in test_sites_and_target; the
+    kept weight moves by the square of the vectors' error, so by the rounding
+    of its sum, 2^n terms at 2^-44."""
+    v = S.random_mps(n, 8, n) if kind == "mps" else S.gaussian_mixture(n, n)
+    v = (v / np.linalg.norm(v)).astype(complex)
+    p = eng.plan([n], 1, chi, "exact")
+    tensors, bonds, target = eng.stage_mps(p, torch.from_numpy(v.view(np.float64)).cuda(), chi)
+    t, tv = tensors.cpu().numpy().view(np.complex128), target.cpu().numpy().view(np.complex128)
+    bd = [int(x) for x in bonds.cpu().numpy()[: n + 1]]
+    ce, base = p.chi_eff(0), int(p.tensor_off[0])
+    for c in range(1, n):
+        keep, w = bd[c], 2 * bd[c + 1]
+        m = t[base + c * 2 * ce * ce:][: keep * w].reshape(keep, w)
+        assert np.max(np.abs(m @ m.conj().T - np.eye(keep))) <= w * 2.0 ** -44, c
+    ref = D.mps_to_dense(D.tt_svd_right(v, n, chi))
+    assert abs(abs(np.vdot(tv, v)) - abs(np.vdot(ref, v))) <= 2 ** (n / 2) * 2.0 ** -44
