@@ -166,8 +166,28 @@ struct PassShared {
 #define PASS_THREADS 128
 #define PASS_BLOCKS_PER_SM 4
 
-// tile-local bit of global position p (p must be in pos_mask)
-__device__ __forceinline__ int tile_bit(int pos_mask, int p) { return __popc(pos_mask & ((1 << p) - 1)); }
+// positions of the qubits in qmask (qubit q is position n - 1 - q)
+__device__ __forceinline__ int qubit_positions(int qmask, int n) { return (int)(__brev((unsigned)qmask) >> (32 - n)); }
+
+// A tile's T positions: those of two windows, and the lowest others.
+__device__ __forceinline__ int tile_positions(int windows, int T) {
+  int free = ~windows;
+  for (int c = T - __popc(windows); c > 0; --c) {
+    windows |= free & -free;
+    free &= free - 1;
+  }
+  return windows;
+}
+
+// tile-local mask of the positions in `window` (all in pos_mask)
+__device__ __forceinline__ int tile_mask(int pos_mask, int window) {
+  int m = 0;
+  while (window) {
+    m |= 1 << __popc(pos_mask & ((window & -window) - 1));
+    window &= window - 1;
+  }
+  return m;
+}
 
 // Previous group's peels on x and new gates on z, over the previous
 // window: a thread owns the 2^U amplitudes of one window position and
@@ -635,20 +655,11 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_group_pass
       }
     }
     if (threadIdx.x == 0) {
-      int pm = 0;
-      const int qm = cur.qmask | prv.qmask;
-      for (int q = 0; q < n; ++q)
-        if ((qm >> q) & 1) pm |= 1 << (n - 1 - q);
-      for (int p = 0; p < n && __popc(pm) < T; ++p) pm |= 1 << p;
-      int wc = 0, wp = 0;
-      for (int q = 0; q < n; ++q) {
-        if ((cur.qmask >> q) & 1) wc |= 1 << tile_bit(pm, n - 1 - q);
-        if ((prv.qmask >> q) & 1) wp |= 1 << tile_bit(pm, n - 1 - q);
-      }
+      const int pm = tile_positions(qubit_positions(cur.qmask | prv.qmask, n), T);
       sh.pos_mask = pm;
       sh.T = T;
-      sh.wml_c = wc;
-      sh.wml_p = wp;   // the current window when g = 0
+      sh.wml_c = tile_mask(pm, qubit_positions(cur.qmask, n));
+      sh.wml_p = tile_mask(pm, qubit_positions(prv.qmask, n));   // the current window when g = 0
       sh.npk = g > 0 ? (prv.cnt < GMAXSTEPS ? prv.cnt : GMAXSTEPS) : 0;
     }
     if (threadIdx.x == 32) {   // an FP64 square root, beside the masks above
@@ -839,23 +850,16 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_BLOCKS_PER_SM) k_rebuild_pa
         sh.pk[w][st] = 0;
       }
     }
+    if (threadIdx.x == 64) sh.sc = vec_scale(n, 1.0);   // C|0> and the normalised working vector of the layer stage
     if (threadIdx.x == 0) {
-      int pm = 0;
-      const int qm = ge[0].qmask | ge[1].qmask;
-      for (int q = 0; q < n; ++q)
-        if ((qm >> q) & 1) pm |= 1 << (n - 1 - q);
-      for (int p = 0; p < n && __popc(pm) < T; ++p) pm |= 1 << p;
+      const int pm = tile_positions(qubit_positions(ge[0].qmask | ge[1].qmask, n), T);
       for (int w = 0; w < 2; ++w) {
-        int m = 0;
-        for (int q = 0; q < n; ++q)
-          if ((ge[w].qmask >> q) & 1) m |= 1 << tile_bit(pm, n - 1 - q);
-        sh.wm[w] = m;
+        sh.wm[w] = tile_mask(pm, qubit_positions(ge[w].qmask, n));
         sh.nst[w] = ge[w].cnt < GMAXSTEPS ? ge[w].cnt : GMAXSTEPS;
       }
       sh.pos_mask = pm;
       sh.T = T;
       sh.nw = nw;
-      sh.sc = vec_scale(n, 1.0);   // C|0> and the normalised working vector of the layer stage
     }
     __syncthreads();
     const int full = (1 << T) - 1;
