@@ -552,8 +552,10 @@ int exact_unitary_layers(qmprs_plan* p, const double2* target, int num_layers, d
     for (int l = 0; l < num_layers; ++l) {
       CK(cudaMemcpyAsync(p->bonds, p->d_bond_init, sizeof(int) * nb, cudaMemcpyDeviceToDevice, s2));
       for (int j = 0; j + 2 <= p->max_n; ++j) {
-        launch_x_layer_cut(p->bd, p->cut_count[j], j, work, buf[0], buf[1], p->bonds, p->vsel, p->site_t,
+        const bool last = p->max_n - 1 - j <= CUT_ROW_BITS;
+        launch_x_layer_cut(p->bd, p->cut_count[j], j, last, work, buf[0], buf[1], p->bonds, p->vsel, p->site_t,
                            p->partials, p->active, s2);
+        if (last) break;
       }
       launch_x_layer_build(p->bd, l, buf[0], buf[1], p->bonds, p->site_t, gates, ar, p->active, s2);
       for (int st = 0; st < p->max_n; ++st) {
@@ -1147,8 +1149,10 @@ int qmprs_unitary_layers(qmprs_plan_t p, const void* target_, int num_layers, do
     for (int l = 0; l < num_layers; ++l) {
       CK(cudaMemcpyAsync(p->bonds, p->d_bond_init, sizeof(int) * nb, cudaMemcpyDeviceToDevice, st));
       for (int j = 0; j + 2 <= p->max_n; ++j) {
-        launch_layer_cut(p->bd, p->cut_count[j], j, work, buf[0], buf[1], p->bonds, p->vsel, p->site_t, p->partials,
-                         p->active, st);
+        const bool last = p->max_n - 1 - j <= CUT_ROW_BITS;   // one unit to every state: the launch does the other cuts too
+        launch_layer_cut(p->bd, p->cut_count[j], j, last, work, buf[0], buf[1], p->bonds, p->vsel, p->site_t,
+                         p->partials, p->active, st);
+        if (last) break;
       }
       launch_layer_build(p->bd, l, buf[0], buf[1], p->bonds, p->site_t, gates, ar, p->active, st);
       // inverse of the new layer: tile passes of two 4-qubit windows (up to

@@ -868,12 +868,10 @@ void launch_x_from_d_flat(const double2* src, xc* dst, int64_t count, cudaStream
   launch_after(k_x_from_d_flat, blocks, 256, 0, s, src, dst, count);
 }
 
-void launch_x_layer_cut(const BatchDev& bd, int units, int step, const xc* work, xc* buf0, xc* buf1, int* bonds,
+void launch_x_layer_cut(const BatchDev& bd, int units, int step, int last, const xc* work, xc* buf0, xc* buf1, int* bonds,
                         double2* vsel, double2* site_t, double2* partials, const int* active, cudaStream_t s) {
-  const xc* prev = (step & 1) ? buf1 : buf0;
-  xc* dst = (step & 1) ? buf0 : buf1;
   qm_note_launch();
-  launch_after(k_layer_cut<CutExact>, units, BLOCK_THREADS, 0, s, bd, step, work, prev, dst, bonds, vsel, site_t,
+  launch_after(k_layer_cut<CutExact>, units, BLOCK_THREADS, 0, s, bd, step, last, work, bonds, vsel, site_t,
                reinterpret_cast<double*>(partials), buf0, buf1, active);
 }
 

@@ -48,7 +48,7 @@ void launch_x_scale_flat(const xc* src, xc* dst, int64_t count, const double* f,
 void launch_x_from_d_flat(const double2* src, xc* dst, int64_t count, cudaStream_t s);
 
 // (b) layer stage (as launch_layer_cut)
-void launch_x_layer_cut(const BatchDev& bd, int units, int step, const xc* work, xc* buf0, xc* buf1, int* bonds,
+void launch_x_layer_cut(const BatchDev& bd, int units, int step, int last, const xc* work, xc* buf0, xc* buf1, int* bonds,
                         double2* vsel, double2* site_t, double2* partials, const int* active, cudaStream_t s);
 void launch_x_layer_build(const BatchDev& bd, int layer, const xc* rem0, const xc* rem1, const int* bonds,
                           double2* site_t, double2* gates, signed char* arity, const int* active, cudaStream_t s);

@@ -156,7 +156,7 @@ void launch_copy_normalize(const BatchDev& bd, const float2* src, float2* dst, d
 
 // (b) layer generation: one cut of every state (`units` blocks: the step's
 // prefix of bd.cut_state / cut_idx)
-void launch_layer_cut(const BatchDev& bd, int units, int step, const float2* work, float2* buf0, float2* buf1,
+void launch_layer_cut(const BatchDev& bd, int units, int step, int last, const float2* work, float2* buf0, float2* buf1,
                       int* bonds, double2* vsel, double2* site_t, double2* partials, const int* active,
                       cudaStream_t s);
 void launch_layer_build(const BatchDev& bd, int layer, const float2* rem0, const float2* rem1,

@@ -7,7 +7,11 @@
 // each of M_{c+1} times the kept vectors of the previous cut (step 0 reads
 // the working state as it is), stores them, and sums their Gram matrix; the
 // state's last block diagonalises it and stores the vectors, the bond and
-// the site tensor.  A separate projection read and a separate eigenvalue
+// the site tensor.  In the last launch, the first in which every state has
+// one unit, a block does all the cuts that are left: a launch each, with its
+// start and the reload of the state's tables, took as long as the cut (20
+// qubits: 19 launches, now 8; a state whose tail started in an earlier launch
+// would hold up the larger ones').  A separate projection read and a separate eigenvalue
 // launch are gone: a cut of a 20-qubit state took 215 us (Gram 24, FP64
 // Jacobi of one thread 187, projection 4.7) and takes 22 us now.
 //
@@ -185,8 +189,7 @@ __device__ __forceinline__ void warp_phase_fix(double2* v, int keep) {
 }
 
 template <class P>
-__global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int step, const typename P::T* work,
-                                                             const typename P::T* prev, typename P::T* dst,
+__global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int step, int last, const typename P::T* work,
                                                              int* bonds, double2* vsel, double2* site_t,
                                                              double* partials, typename P::T* rem0,
                                                              typename P::T* rem1, const int* active) {
@@ -198,118 +201,129 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int st
   __shared__ WarpPolar ws;
   __shared__ int s_keep;
   const int unit = blockIdx.x, b = bd.cut_state[unit], idx = bd.cut_idx[unit];
-  const int n = bd.n[b], c = n - 1 - step;
+  const int n = bd.n[b];
+  int c = n - 1 - step;
   if (c < 1 || (active && !active[b])) return;
   int* bond = bonds + (int64_t)b * (bd.max_n + 1);
-  const int r = bond[c + 1];
+  int r = bond[c + 1], rp = step > 0 ? bond[c + 2] : 0;
   if (r != 1 && r != 2) return;
   const int units = c > CUT_ROW_BITS ? 1 << (c - CUT_ROW_BITS) : 1;
   if (idx >= units) return;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int lo = idx * CUT_ROWS, hi = min(lo + CUT_ROWS, 1 << c);
   double2* vs = vsel + (int64_t)b * 16;
-  DF s[16];
+  if (step > 0 && tid < 16) vm[tid] = P::load_v(vs[tid]);
+  for (;; ++step, --c) {
+    const int lo = idx * CUT_ROWS, hi = min(lo + CUT_ROWS, 1 << c);
+    DF s[16];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) s[k] = DF{0.f, 0.f};
-  const T* m = work + bd.vec_off[b];   // this step's remainder (rows of 2 r)
-  if (step == 0) {
-    for (int row = lo + tid; row < hi; row += BLOCK_THREADS) {
-      T x[2];
-      P::template load<2>(m + (int64_t)row * 2, x);
-      cut_gram<P, 2>(s, x);
-    }
-  } else {
-    if (tid < 16) vm[tid] = P::load_v(vs[tid]);
-    __syncthreads();
-    const int rp = bond[c + 2];
-    const T* src = (step == 1 ? work : prev) + bd.vec_off[b];
-    T* o = dst + bd.vec_off[b];
-    m = o;
-    if (rp == 1) {
-      if (r == 1) cut_rows<P, 2, 1>(src, o, vm, lo, hi, s);
-      else cut_rows<P, 2, 2>(src, o, vm, lo, hi, s);
+    for (int k = 0; k < 16; ++k) s[k] = DF{0.f, 0.f};
+    const T* m = work + bd.vec_off[b];   // this step's remainder (rows of 2 r)
+    if (step == 0) {
+      for (int row = lo + tid; row < hi; row += BLOCK_THREADS) {
+        T x[2];
+        P::template load<2>(m + (int64_t)row * 2, x);
+        cut_gram<P, 2>(s, x);
+      }
     } else {
-      if (r == 1) cut_rows<P, 4, 1>(src, o, vm, lo, hi, s);
-      else cut_rows<P, 4, 2>(src, o, vm, lo, hi, s);
-    }
-  }
-  // 16 sums over the lanes (lane l holds value l mod 16), then the warps
-#pragma unroll
-  for (int k = 0; k < 16; ++k) df_shfl_add(s[k], s[k], 16);
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int k = 0; k < o; ++k) {
-      const DF give = up ? s[k] : s[k + o];
-      if (up) s[k] = s[k + o];
-      df_shfl_add(s[k], give, o);
-    }
-  }
-  if (lane < 16) wred[tid >> 5][lane] = (double)s[0].hi + (double)s[0].lo;
-  __syncthreads();
-  double* part = partials + (int64_t)bd.state_tile0[b] * WARPS * 32;   // 16 doubles per unit
-  if (tid < 16) {
-    double v[WARPS];
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) v[w] = wred[w][tid];
-    part[idx * 16 + tid] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-  }
-  __syncthreads();
-  if (units > 1 && !last_tile_ticket(bd.ticket, b, units)) return;
-  // the state's last block: Gram, eigenvectors, truncation
-  {
-    const int val = tid >> 4, l16 = tid & 15;
-    double v = 0.0;
-    for (int u = l16; u < units; u += 16) v += __ldcg(part + u * 16 + val);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
-    __syncthreads();
-    if (l16 == 0) wred[0][val] = v;
-  }
-  __syncthreads();
-  const int w = 2 * r;
-  if (tid < 32) {
-    double2 g = czero();
-    {
-      const int a = (tid >> 2) & 3, e = tid & 3;
-      if (a < w && e < w) {
-        if (a == e) {
-          g = cd(wred[0][a], 0.0);
-        } else {
-          const int k = 4 + 2 * cut_pair(min(a, e), max(a, e));
-          g = cd(wred[0][k], a < e ? wred[0][k + 1] : -wred[0][k + 1]);
-        }
+      __syncthreads();
+      // step j reads the remainder of step j - 1 and writes its own to the other buffer
+      const T* src = (step == 1 ? work : (step & 1) ? rem1 : rem0) + bd.vec_off[b];
+      T* o = ((step & 1) ? rem0 : rem1) + bd.vec_off[b];
+      m = o;
+      if (rp == 1) {
+        if (r == 1) cut_rows<P, 2, 1>(src, o, vm, lo, hi, s);
+        else cut_rows<P, 2, 2>(src, o, vm, lo, hi, s);
+      } else {
+        if (r == 1) cut_rows<P, 4, 1>(src, o, vm, lo, hi, s);
+        else cut_rows<P, 4, 2>(src, o, vm, lo, hi, s);
       }
     }
-    warp_gram_eig(ws, g, lam);
-    if (lane == 0) {
-      s_keep = rank_by_cutoff(lam, w, QM_CUTOFF, 2);
-      bond[c] = s_keep;
-      if (units > 1) bd.ticket[b] = 0;
-    }
-    __syncwarp();
-    const int keep = s_keep;
-    warp_phase_fix(ws.B, keep);
-    if (lane < 16) {
-      const int a = lane >> 2, col = lane & 3;
-      const double2 v = a < w && col < keep ? ws.B[lane] : czero();
-      vs[lane] = v;
-      vm[lane] = P::load_v(v);
-      if (a < w && col < keep) site_t[((int64_t)b * bd.max_n + c) * 8 + col * w + a] = cconj(v);
-    }
-  }
-  if (c > 1) return;
-  // the last remainder (2 rows) for site 0
-  __syncthreads();
-  if (tid < 2 * s_keep) {
-    const int row = tid / s_keep, col = tid % s_keep;
-    const T* x = m + row * w;
-    T xr[4];
+    // 16 sums over the lanes (lane l holds value l mod 16), then the warps
 #pragma unroll
-    for (int a = 0; a < 4; ++a) xr[a] = x[a < w ? a : 0];
-    const T y = w == 2 ? P::template project<2>(xr, vm, col) : P::template project<4>(xr, vm, col);
-    ((n & 1) ? rem1 : rem0)[bd.vec_off[b] + tid] = y;
+    for (int k = 0; k < 16; ++k) df_shfl_add(s[k], s[k], 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int k = 0; k < o; ++k) {
+        const DF give = up ? s[k] : s[k + o];
+        if (up) s[k] = s[k + o];
+        df_shfl_add(s[k], give, o);
+      }
+    }
+    if (lane < 16) wred[tid >> 5][lane] = (double)s[0].hi + (double)s[0].lo;
+    __syncthreads();
+    double* part = partials + (int64_t)bd.state_tile0[b] * WARPS * 32;   // 16 doubles per unit
+    if (tid < 16) {
+      double v[WARPS];
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) v[w] = wred[w][tid];
+      part[idx * 16 + tid] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
+    __syncthreads();
+    if (units > 1 && !last_tile_ticket(bd.ticket, b, units)) return;
+    // the state's last block: Gram, eigenvectors, truncation
+    {
+      const int val = tid >> 4, l16 = tid & 15;
+      double v = 0.0;
+      for (int u = l16; u < units; u += 16) v += __ldcg(part + u * 16 + val);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
+      __syncthreads();
+      if (l16 == 0) wred[0][val] = v;
+    }
+    __syncthreads();
+    const int w = 2 * r;
+    if (tid < 32) {
+      double2 g = czero();
+      {
+        const int a = (tid >> 2) & 3, e = tid & 3;
+        if (a < w && e < w) {
+          if (a == e) {
+            g = cd(wred[0][a], 0.0);
+          } else {
+            const int k = 4 + 2 * cut_pair(min(a, e), max(a, e));
+            g = cd(wred[0][k], a < e ? wred[0][k + 1] : -wred[0][k + 1]);
+          }
+        }
+      }
+      warp_gram_eig(ws, g, lam);
+      if (lane == 0) {
+        s_keep = rank_by_cutoff(lam, w, QM_CUTOFF, 2);
+        bond[c] = s_keep;
+        if (units > 1) bd.ticket[b] = 0;
+      }
+      __syncwarp();
+      const int keep = s_keep;
+      warp_phase_fix(ws.B, keep);
+      if (lane < 16) {
+        const int a = lane >> 2, col = lane & 3;
+        const double2 v = a < w && col < keep ? ws.B[lane] : czero();
+        vs[lane] = v;
+        vm[lane] = P::load_v(v);
+        if (a < w && col < keep) site_t[((int64_t)b * bd.max_n + c) * 8 + col * w + a] = cconj(v);
+      }
+    }
+    if (c > 1) {
+      if (!last) return;
+      __syncthreads();
+      rp = r;
+      r = s_keep;
+      if (r != 1 && r != 2) return;
+      continue;
+    }
+    // the last remainder (2 rows) for site 0
+    __syncthreads();
+    if (tid < 2 * s_keep) {
+      const int row = tid / s_keep, col = tid % s_keep;
+      const T* x = m + row * w;
+      T xr[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) xr[a] = x[a < w ? a : 0];
+      const T y = w == 2 ? P::template project<2>(xr, vm, col) : P::template project<4>(xr, vm, col);
+      ((n & 1) ? rem1 : rem0)[bd.vec_off[b] + tid] = y;
+    }
+    return;
   }
 }
 

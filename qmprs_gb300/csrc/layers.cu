@@ -27,14 +27,11 @@ __global__ void k_layer_fidelity(BatchDev bd, int layer, const float2* work, int
   }
 }
 
-void launch_layer_cut(const BatchDev& bd, int units, int step, const float2* work, float2* buf0, float2* buf1,
+void launch_layer_cut(const BatchDev& bd, int units, int step, int last, const float2* work, float2* buf0, float2* buf1,
                       int* bonds, double2* vsel, double2* site_t, double2* partials, const int* active,
                       cudaStream_t s) {
-  // step j reads the remainder of step j - 1 and writes its own to the other buffer
-  const float2* prev = (step & 1) ? buf1 : buf0;
-  float2* dst = (step & 1) ? buf0 : buf1;
   qm_note_launch();
-  launch_after(k_layer_cut<CutFast>, units, BLOCK_THREADS, 0, s, bd, step, work, prev, dst, bonds, vsel, site_t,
+  launch_after(k_layer_cut<CutFast>, units, BLOCK_THREADS, 0, s, bd, step, last, work, bonds, vsel, site_t,
                reinterpret_cast<double*>(partials), buf0, buf1, active);
 }
 
