@@ -504,17 +504,19 @@ __global__ void __launch_bounds__(256) k_zgemm(const double2* A, int64_t lda, co
 // threads): a 512 x 512 product has 64 large tiles, which leave 88 of 152
 // SMs idle.  Every output sums its terms in the same order in both.
 // Measured (512 x 512 x 512): 377 us a product with large tiles, 185 us.
-template <bool CONJ, int T, int CO>
-__global__ void __launch_bounds__(T * T / (4 * CO)) k_zgemm_df(const double2* A, int64_t lda, const double2* B,
+template <bool CONJ, int T, int CO, int KG>
+__global__ void __launch_bounds__(KG * T * T / (4 * CO)) k_zgemm_df(const double2* A, int64_t lda, const double2* B,
                                                                int64_t ldb, const double2* D, int64_t ldd,
                                                                double2* C, int64_t ldc, int M, int N, int K,
                                                                double alpha) {
   grid_wait();
-  constexpr int TC = T / CO, NT = T * T / (4 * CO);
+  constexpr int TC = T / CO, NG = T * T / (4 * CO), NT = KG * NG;
+  static_assert(KG == 1 || KG == 2, "one or two parts of K");
   __shared__ xc As[ZG_K][T + 1];
   __shared__ xc Bs[ZG_K][T];
+  __shared__ xc half[KG > 1 ? 4 * CO : 1][KG > 1 ? NG : 1];
   const int m0 = blockIdx.x * T, n0 = blockIdx.y * T;
-  const int tr = threadIdx.x / TC, tc = threadIdx.x % TC;
+  const int part = threadIdx.x / NG, tid = threadIdx.x % NG, tr = tid / TC, tc = tid % TC;
   XA acc[4][CO];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -541,7 +543,7 @@ __global__ void __launch_bounds__(T * T / (4 * CO)) k_zgemm_df(const double2* A,
     }
     __syncthreads();
 #pragma unroll 2
-    for (int kk = 0; kk < ZG_K; ++kk) {
+    for (int kk = part; kk < ZG_K; kk += KG) {
       xc av[4], bv[CO];
 #pragma unroll
       for (int i = 0; i < 4; ++i) av[i] = As[kk][tr * 4 + i];
@@ -556,6 +558,19 @@ __global__ void __launch_bounds__(T * T / (4 * CO)) k_zgemm_df(const double2* A,
           else
             xa_mac(acc[i][j2], av[i], bv[j2]);
         }
+    }
+  }
+  if (KG > 1) {
+    if (part == 1)
+#pragma unroll
+      for (int i = 0; i < 4 * CO; ++i) half[i][tid] = xa_round(acc[i / CO][i % CO]);
+    __syncthreads();
+    if (part == 1) return;
+#pragma unroll
+    for (int i = 0; i < 4 * CO; ++i) {
+      const xc v = half[i][tid];
+      df_add(acc[i / CO][i % CO].re, v.x, v.z);
+      df_add(acc[i / CO][i % CO].im, v.y, v.w);
     }
   }
 #pragma unroll
@@ -999,15 +1014,15 @@ static void zgemm(bool conj, const double2* A, int64_t lda, const double2* B, in
   qm_note_launch();
   if (df && g.x * g.y >= 2 * 152) {
     if (conj)
-      launch_after((k_zgemm_df<true, 64, 4>), g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<true, 64, 4, 1>), g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
     else
-      launch_after((k_zgemm_df<false, 64, 4>), g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<false, 64, 4, 1>), g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   } else if (df) {
     const dim3 h((M + 31) / 32, (N + 31) / 32);
     if (conj)
-      launch_after((k_zgemm_df<true, 32, 2>), h, 128, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<true, 32, 2, 2>), h, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
     else
-      launch_after((k_zgemm_df<false, 32, 2>), h, 128, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
+      launch_after((k_zgemm_df<false, 32, 2, 2>), h, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   } else if (conj) {
     launch_after(k_zgemm<true>, g, 256, 0, s, A, lda, B, ldb, D, ldd, C, ldc, M, N, K, alpha);
   } else {
