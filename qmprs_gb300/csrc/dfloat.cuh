@@ -17,6 +17,24 @@ __device__ __forceinline__ xc xc_from_d(double2 v) {
 
 __device__ __forceinline__ double2 xc_to_d(xc v) { return cd((double)v.x + (double)v.z, (double)v.y + (double)v.w); }
 
+// x = hi + lo as xc_from_d does, by integer operations: an FP64 subtraction
+// occupies an SM quarter's unit for 64 cycles.  hi is x rounded to 24 bits
+// (ties away from zero), lo the other 29 bits; values out of FP32's range
+// give what their conversion gives.
+__device__ __forceinline__ float2 df_split(double x) {
+  const int xh = __double2hiint(x), xl = __double2loint(x);
+  const int low = (int)((unsigned)(xl + 0x10000000) & 0x1fffffffu) - 0x10000000;   // x's bits below hi's, signed
+  const long long hb = (((long long)xh << 32) | (unsigned)xl) - low;
+  const float hi = __double2float_rn(__longlong_as_double(hb));
+  const int f = ((xh >> 20) & 0x7ff) - 895;   // exponent field of 2^(e + 1) in FP32
+  const float sc = f > 0 && f < 255 ? __int_as_float((f << 23) | (xh & 0x80000000)) : f < 255 ? 0.f : hi - hi;
+  return make_float2(hi, (float)low * 0x1p-53f * sc);
+}
+__device__ __forceinline__ xc xc_split(double2 v) {
+  const float2 r = df_split(v.x), i = df_split(v.y);
+  return make_float4(r.x, i.x, r.y, i.y);
+}
+
 // s += (ah + al)(bh + bl): the high product exactly (ph + pl), TwoSum into
 // s.hi, everything of lower order into s.lo.  Explicitly rounded
 // intrinsics keep the compiler from contracting the error terms.

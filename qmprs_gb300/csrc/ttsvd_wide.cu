@@ -502,8 +502,15 @@ __global__ void __launch_bounds__(256) k_zgemm(const double2* A, int64_t lda, co
 // T x T tiles, 4 x CO outputs per thread: 64 x 64 with 4 x 4 (256 threads)
 // for products with at least two tiles per SM, else 32 x 32 with 4 x 2 (128
 // threads): a 512 x 512 product has 64 large tiles, which leave 88 of 152
-// SMs idle.  Every output sums its terms in the same order in both.
-// Measured (512 x 512 x 512): 377 us a product with large tiles, 185 us.
+// SMs idle.
+// KG = 2: two groups of threads take a half of every K chunk, so that a block
+// of the small tiles gives every SM quarter two warps (one issues an
+// instruction every two to three cycles); they are summed at the end.  The
+// factors are split by integer operations (df_split): FP64 subtractions took
+// a sixth of the time.
+// Measured (512 x 512 x 512): 377 us a product with large tiles, 185 us with
+// small ones; the halves and the integer split took 1.8 and 2.1 ms off the 77
+// products of a 20-qubit truncation at bond 256 (14.1 ms before).
 template <bool CONJ, int T, int CO, int KG>
 __global__ void __launch_bounds__(KG * T * T / (4 * CO)) k_zgemm_df(const double2* A, int64_t lda, const double2* B,
                                                                int64_t ldb, const double2* D, int64_t ldd,
@@ -536,10 +543,10 @@ __global__ void __launch_bounds__(KG * T * T / (4 * CO)) k_zgemm_df(const double
       const int gm = m0 + mm, gk = k0 + kk;
       double2 v = czero();
       if (gm < M && gk < K) v = CONJ ? A[(int64_t)gk * lda + gm] : A[(int64_t)gm * lda + gk];
-      As[kk][mm] = xc_from_d(v);
+      As[kk][mm] = xc_split(v);
       const int kb = e / T, nn = e % T;
       const int gkb = k0 + kb, gn = n0 + nn;
-      Bs[kb][nn] = xc_from_d((gkb < K && gn < N) ? B[(int64_t)gkb * ldb + gn] : czero());
+      Bs[kb][nn] = xc_split((gkb < K && gn < N) ? B[(int64_t)gkb * ldb + gn] : czero());
     }
     __syncthreads();
 #pragma unroll 2
