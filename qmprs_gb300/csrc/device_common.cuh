@@ -64,8 +64,6 @@ __device__ __forceinline__ bool last_tile_ticket(int* ticket, int b, int nt) {
   return last;
 }
 
-__device__ __forceinline__ double2 ld_cg(const double2* p) { return __ldcg(p); }
-
 // Index of amplitude for quad r on bits (hi, lo = hi - 1), with values (bh, bl).
 __device__ __forceinline__ int64_t quad_base(int64_t r, int lo) {
   return ((r >> lo) << (lo + 2)) | (r & ((((int64_t)1) << lo) - 1));

@@ -906,20 +906,6 @@ QM_HD double polar_jacobi_ref(const double2* e, int m, double2* w_out, const dou
   return nuc;
 }
 
-// max |G G^H - I| over entries, G row-major m x m
-QM_HD double unitarity_error(const double2* g, int m) {
-  double err = 0.0;
-  for (int i = 0; i < m; ++i)
-    for (int j = 0; j < m; ++j) {
-      double2 acc = czero();
-      for (int k = 0; k < m; ++k) acc = cadd(acc, cmul(g[i * m + k], cconj(g[j * m + k])));
-      if (i == j) acc.x -= 1.0;
-      double a = cabs_(acc);
-      if (a > err) err = a;
-    }
-  return err;
-}
-
 // --------------------------------------------------------------------------
 // Ran's gate construction (reference qmprs/primitives/mps.py:565-744) in
 // closed form.  Gates are row-major 4x4 (two-qubit) or 2x2 (one-qubit); the
