@@ -461,7 +461,7 @@ def run_gpu(args, rank, world):
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "c64 (fp32 state, fp64 reductions/polar/eig)",
+        "dtype": "c64 (fp32 state, double-float and fp64 reductions/polar/eig)",
         "data": "synthetic",
         "config": {"workload": desc, "states_per_gpu": B, **cfg,
                    "path": "plain batched (analytic layers + sweeps); the warm-start arm is `warm_start`",
