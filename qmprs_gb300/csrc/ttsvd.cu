@@ -347,8 +347,8 @@ __device__ void smem_matmul(const double2* A, const double2* B, double2* Cm, int
 // the next pass resolves what FP32 could not see at G's scale (each pass
 // gains about seven digits), down to a rotation floor of 1e-13 of the trace
 // (ten times the products' rounding; the truncation decides at 1e-10).
-// Three or four passes; a pass whose rotations were all below 3e-7 is the
-// last.  Measured (48 states, w = 64): about 6 ms per cut with FP64 products
+// Three or four passes; a pass at that floor whose rotations were all below
+// 3e-7 is the last.  Measured (48 states, w = 64): about 6 ms per cut with FP64 products
 // and FP64 finishing sweeps, 1.4 ms now, half of it the FP32 sweeps and half
 // the double-float products (three quarters of the FP32 pipes' rate).
 
@@ -704,13 +704,20 @@ static_assert(TT_EIG_SMEM_W / 2 * (TT_EIG_SMEM_W / 4) <= TT_EIG_THREADS, "one bl
 __device__ void tt_df_eig(xc* Vg, int w, int ld) {
   xc *G = tt_smx(), *vk = tt_smx() + w * ld, *t = tt_smx() + 2 * w * ld;
   float2* t32 = tt_smf() + 4 * w * ld;
-  for (int pass = 0; pass < 6; ++pass) {
+  bool first = true;   // V is still I
+  float floor_abs = 1e-7f;
+  for (int pass = 0; pass < 7; ++pass) {
     const bool moved = jacobi32_run(
         [&](int i, int j) {
           const xc g = G[i * ld + j];
           return cf(g.x, i == j ? 0.f : g.y);
         },
-        2 * w * ld, w, ld, 1e-7f, pass == 0 ? 1e-7f : 1e-13f);
+        2 * w * ld, w, ld, 1e-7f, floor_abs);
+    // nothing above FP32's noise at G's scale: G is graded as it is, and the
+    // couplings among its small entries are resolved from it at once
+    const bool coarse = floor_abs > 1e-13f;
+    floor_abs = 1e-13f;
+    if (!moved && coarse) continue;
     const float2* vr = tt_smf() + 2 * w * ld;
     // the thread's blocks, computed anew in every pass: kept over the sweeps
     // they would be spilled
@@ -720,8 +727,9 @@ __device__ void tt_df_eig(xc* Vg, int w, int ld) {
     const bool mine = tt_block(w, tid, false, o), uppr = tt_block(w, tid, true, u);
     if (!moved) {
       // V_k = I + X with X below 3e-7: D = -(X + X^H + X^H X) / 2 and the
-      // products with X or D are FP32, and G's diagonal stands (X changes it
-      // by less than 1e-13 of itself)
+      // products with X or D are FP32, and G's diagonal stands: a tangent x
+      // moves its pair's eigenvalues by x^2 of their difference, together
+      // less than 1e-13 of the trace, the rotations' floor
       for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
         const int i = e / w, j = e % w;
         const float2 x = vr[i * ld + j];
@@ -750,7 +758,7 @@ __device__ void tt_df_eig(xc* Vg, int w, int ld) {
           z[(o.r0 + i) * ld + o.c0 + 1] = acc[i][1];
         }
       for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-        const xc v = pass == 0 ? make_float4(e / w == e % w ? 1.f : 0.f, 0.f, 0.f, 0.f) : Vg[e];
+        const xc v = first ? make_float4(e / w == e % w ? 1.f : 0.f, 0.f, 0.f, 0.f) : Vg[e];
         t32[(e / w) * ld + e % w] = cf(v.x, v.y);
       }
       __syncthreads();
@@ -762,7 +770,7 @@ __device__ void tt_df_eig(xc* Vg, int w, int ld) {
           for (int j = 0; j < 2; ++j) {
             if (i >= o.nr) continue;
             const int e = (o.r0 + i) * w + o.c0 + j;
-            const xc v = pass == 0 ? make_float4(o.r0 + i == o.c0 + j ? 1.f : 0.f, 0.f, 0.f, 0.f) : Vg[e];
+            const xc v = first ? make_float4(o.r0 + i == o.c0 + j ? 1.f : 0.f, 0.f, 0.f, 0.f) : Vg[e];
             Vg[e] = tt_plus(v, acc[i][j]);
           }
       }
@@ -870,7 +878,8 @@ __device__ void tt_df_eig(xc* Vg, int w, int ld) {
     }
     __syncthreads();
     // V <- V V_k
-    if (pass == 0) {
+    if (first) {
+      first = false;
       for (int e = threadIdx.x; e < w * w; e += blockDim.x) Vg[e] = vk[(e / w) * ld + e % w];
     } else {
       for (int e = threadIdx.x; e < w * w; e += blockDim.x) t[(e / w) * ld + e % w] = Vg[e];
