@@ -29,12 +29,12 @@ struct qmprs_plan {
   qmprs_ctx* h = nullptr;
   int B = 0, max_n = 0, max_layers = 0, max_bond = 0, ntiles = 0, tile_bits = 0;
   std::vector<int> n;
-  std::vector<int64_t> vec_off, gate_off, tensor_off;
+  std::vector<int64_t> vec_off, gate_off, tensor_off, tt_off;
   int64_t vec_total = 0, gate_total = 0, tensor_total = 0;
   // device tables
   int *d_n = nullptr, *d_tile_state = nullptr, *d_tile_idx = nullptr, *d_state_tile0 = nullptr,
       *d_state_ntiles = nullptr, *d_ticket = nullptr, *d_err = nullptr;
-  int64_t *d_vec_off = nullptr, *d_gate_off = nullptr, *d_tensor_off = nullptr;
+  int64_t *d_vec_off = nullptr, *d_gate_off = nullptr, *d_tensor_off = nullptr, *d_tt_off = nullptr;
   int* d_bond_init = nullptr;
   // layer stage: row units of every state, and how many of them (a prefix) each step needs
   int *d_cut_state = nullptr, *d_cut_idx = nullptr;
@@ -368,7 +368,7 @@ inline uint64_t dbl_key(double v) {
 int ensure_tt_scratch(qmprs_plan* p) {
   if (p->tt_partials) return QMPRS_OK;
   const int64_t WW = (int64_t)p->tt_w * p->tt_w;
-  CK(dalloc(&p->tt_partials, (int64_t)p->B * p->bd.tt_region));
+  CK(dalloc(&p->tt_partials, p->tt_off[p->B]));
   CK(dalloc(&p->gram, (int64_t)p->B * WW));
   CK(dalloc(&p->vsel2, (int64_t)p->B * WW));
   CK(dalloc(&p->vwork, (int64_t)p->B * WW));
@@ -478,7 +478,7 @@ int exact_mps_from_statevector(qmprs_plan* p, const double2* sv, int max_bond, d
       jb.m = src + p->vec_off[b];
       jb.rows = ipow2(c);
       jb.w = 2 * r;
-      jb.part = p->tt_partials + (int64_t)b * p->bd.tt_region;
+      jb.part = p->tt_partials + p->tt_off[b];
       jb.gram = p->gram + (int64_t)b * WW;
       grams.push_back(jb);
       wide = wide || 2 * r > p->bd.eig_wmax;
@@ -696,7 +696,7 @@ void qmprs_plan_destroy(qmprs_plan_t p) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
   if (p->cap) cudaStreamDestroy(p->cap);
   void* ptrs[] = {p->d_n,      p->d_tile_state, p->d_tile_idx, p->d_state_tile0, p->d_state_ntiles,
-                  p->d_ticket, p->d_err,        p->d_vec_off,  p->d_gate_off,    p->d_tensor_off,
+                  p->d_ticket, p->d_err,        p->d_vec_off,  p->d_gate_off,    p->d_tensor_off, p->d_tt_off,
                   p->d_bond_init, p->d_cut_state, p->d_cut_idx, p->S0, p->S1,         p->S2,            p->partials,
                   p->tt_partials, p->gram,      p->vsel,       p->vsel2,         p->site_t, p->vwork,
                   p->bonds,    p->active,       p->nlayers,    p->num_active,    p->nuc,
@@ -760,6 +760,20 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   p->ntiles = (int)tile_state.size();
   for (int b = 0; b < num_states; ++b) p->tt_b = std::max(p->tt_b, chi_eff_host(max_bond, p->n[b]));
   p->tt_w = std::max(TT_MAXW, 2 * p->tt_b);
+  // a state's Gram partials: TT_SPLIT of the widest Gram, and for a state of
+  // more tiles a 64-wide one per tile, as long as such states' row splits are
+  // what fills the GPU (a slot by the largest state's tiles for every state
+  // took four times the memory: 2.7 GB for 300 states of 8 qubits and one of
+  // 20, now 0.9 GB)
+  {
+    const int64_t least = (int64_t)TT_SPLIT * p->tt_w * p->tt_w, one = TT_EIG_SMEM_W * TT_EIG_SMEM_W;
+    int64_t many = 0;
+    for (int nt : state_ntiles) many += std::min(nt, TT_SPLIT_MAX) * one > least;
+    const int64_t most = many > 0 ? TT_SPLIT_BLOCKS / many : 0;
+    p->tt_off.assign(1, 0);
+    for (int nt : state_ntiles)
+      p->tt_off.push_back(p->tt_off.back() + std::max(least, std::min<int64_t>(std::min(nt, TT_SPLIT_MAX), most) * one));
+  }
   // grouped sweep: tiles of 2^min(n, GT) amplitudes, chunk_tiles tiles per chunk
   p->chunk_tiles = choose_chunk_tiles(p->n);
   std::vector<int> chunk_state, chunk_idx, state_chunk0(num_states), state_nchunks(num_states);
@@ -816,6 +830,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   PC(dalloc(&p->d_vec_off, B));
   PC(dalloc(&p->d_gate_off, B));
   PC(dalloc(&p->d_tensor_off, B));
+  PC(dalloc(&p->d_tt_off, B + 1));
   PC(dalloc(&p->d_tile_state, p->ntiles));
   PC(dalloc(&p->d_tile_idx, p->ntiles));
   PC(dalloc(&p->d_state_tile0, B));
@@ -831,6 +846,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   PC(cudaMemcpy(p->d_vec_off, p->vec_off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_gate_off, p->gate_off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_tensor_off, p->tensor_off.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice));
+  PC(cudaMemcpy(p->d_tt_off, p->tt_off.data(), sizeof(int64_t) * (B + 1), cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_tile_state, tile_state.data(), sizeof(int) * p->ntiles, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_tile_idx, tile_idx.data(), sizeof(int) * p->ntiles, cudaMemcpyHostToDevice));
   PC(cudaMemcpy(p->d_state_tile0, state_tile0.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
@@ -900,10 +916,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
   bd.err = p->d_err;
   bd.tt_w = p->tt_w;
   bd.tt_b = p->tt_b;
-  // room for TT_SPLIT partials of the widest Gram, and for as many 64-wide
-  // ones as the largest state has tiles
-  const int most_tiles = *std::max_element(state_ntiles.begin(), state_ntiles.end());
-  bd.tt_region = std::max<int64_t>((int64_t)TT_SPLIT * p->tt_w * p->tt_w, (int64_t)std::min(most_tiles, TT_SPLIT_MAX) * 4096);
+  bd.tt_off = p->d_tt_off;
   bd.cut_state = p->d_cut_state;
   bd.cut_idx = p->d_cut_idx;
   bd.eig_wmax = num_states <= BJ_SMALL_BATCH ? TT_MAXB : TT_MAXW;

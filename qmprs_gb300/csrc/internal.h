@@ -74,7 +74,7 @@ struct BatchDev {
   int* err;                // [1] error flag bits
   int tt_w;                // stage (a): Gram stride (>= TT_MAXW, 2 x the largest bond)
   int tt_b;                // stage (a): largest bond / selected-column stride (>= TT_MAXB)
-  int64_t tt_region;       // stage (a): entries of a state's slot of Gram partials
+  const int64_t* tt_off;   // [B + 1] stage (a): the states' slots of Gram partials (entries)
   const int* cut_state;    // layer stage: state and index of each row unit (layer_cut.cuh),
   const int* cut_idx;      // sorted by the last step that needs it
   int eig_wmax;            // stage (a): widest Gram of the one-block eigensolver; wider ones
@@ -254,8 +254,10 @@ void launch_count_active(int B, const int* active, int* num_active, cudaStream_t
 // raise KERR_BAD_INPUT unless every sq[b].x is finite and positive
 void launch_check_norms(int B, const double2* sq, int* err, cudaStream_t s);
 
+#define TT_EIG_SMEM_W 64    // widest Gram diagonalised in shared memory (3 x 65 KB)
 #define TT_SPLIT 8          // row splits of the widest Gram a plan can have
 #define TT_SPLIT_MAX 128    // row splits of a narrower one
+#define TT_SPLIT_BLOCKS (8 * 152)   // 64-wide partials, over TT_SPLIT widest ones a state, that a plan makes room for
 
 // helpers
 __host__ __device__ inline int64_t ipow2(int k) { return (int64_t)1 << k; }

@@ -25,7 +25,6 @@
 #include "dfloat.cuh"
 
 #define TT_CH 32
-#define TT_EIG_SMEM_W 64   // widest Gram diagonalised in shared memory (3 x 65 KB)
 #define TT_EIG_THREADS 512
 #define TT_EIG_PAD 2
 
@@ -67,7 +66,7 @@ __device__ __forceinline__ int tt_splits(const BatchDev& bd, int b, int c, int w
   int64_t n = bd.state_ntiles[b];
   n = min(n, (int64_t)TT_SPLIT_MAX);
   n = min(n, max((int64_t)1, ipow2(c) >> 5));
-  n = min(n, bd.tt_region / ((int64_t)w * w));
+  n = min(n, (bd.tt_off[b + 1] - bd.tt_off[b]) / ((int64_t)w * w));
   return (int)n;
 }
 
@@ -110,7 +109,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
       const int split = unit % nsplit;
       int64_t lo, hi;
       tile_range(ipow2(c), split, nsplit, &lo, &hi);
-      xc* part = partials + (int64_t)b * bd.tt_region + (int64_t)split * w * w;
+      xc* part = partials + bd.tt_off[b] + (int64_t)split * w * w;
       const int e0 = (unit / nsplit) * BLOCK_THREADS;
       const int nbp = nb - e0 < BLOCK_THREADS ? nb - e0 : BLOCK_THREADS;
       const int nsub = BLOCK_THREADS / nbp;
@@ -188,7 +187,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram_sum(BatchDev bd, int 
     int w;
     if (!tt_gram_here(bd, bonds + (int64_t)b * (bd.max_n + 1), c, &w)) continue;
     const int nsplit = tt_splits(bd, b, c, w), ww = w * w;
-    const xc* part = partials + (int64_t)b * bd.tt_region;
+    const xc* part = partials + bd.tt_off[b];
     double2* g = gram + (int64_t)b * bd.tt_w * bd.tt_w;
     for (int e0 = blockIdx.x * (BLOCK_THREADS / 8); e0 < ww; e0 += gridDim.x * (BLOCK_THREADS / 8)) {
       const int e = e0 + (threadIdx.x >> 3), a = e / w, cc = e % w;
@@ -1099,7 +1098,7 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
       }
     }
   } else {
-    float2* G32 = scratch32 + (int64_t)b * 2 * bd.tt_region;
+    float2* G32 = scratch32 + 2 * bd.tt_off[b];
     float2* V32 = G32 + w * ld;
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
       const int i = e / w, j = e % w;
