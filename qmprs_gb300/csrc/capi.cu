@@ -1047,7 +1047,7 @@ int qmprs_mps_from_statevector(qmprs_plan_t p, const void* sv_, int max_bond, do
   };
   for (int j = 0; j + 2 <= p->max_n; ++j) {
     const float2* src = j == 0 ? sv : buf[(j - 1) & 1];
-    launch_tt_gram(p->bd, j, sv, src, bonds, p->tt_partials, p->gram, s);
+    launch_tt_gram(p->bd, j, sv, src, bonds, p->sq, p->tt_partials, p->gram, s);
     launch_tt_eig(p->bd, j, bonds, p->gram, p->vwork, max_bond, cutoff, p->vsel2, tensors, p->max_bond,
                   p->tt_partials, 1e-13, s);
     launch_tt_project(p->bd, j, sv, src, buf[j & 1], bonds, p->vsel2, s);

@@ -192,7 +192,7 @@ void launch_sweep_finish(int B, int sweep, int num_sweeps, const double* nuc, co
 
 // (a) statevector -> MPS
 void launch_tt_gram(const BatchDev& bd, int step, const float2* sv, const float2* src, const int* bonds,
-                    double2* partials, double2* gram, cudaStream_t s);
+                    const double2* sq, double2* partials, double2* gram, cudaStream_t s);
 void launch_tt_eig(const BatchDev& bd, int step, int* bonds, double2* gram, double2* vwork, int max_bond,
                    double cutoff, double2* vsel, double2* tensors, int chi, double2* scratch, double fine,
                    cudaStream_t s);

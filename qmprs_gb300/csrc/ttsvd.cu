@@ -70,6 +70,11 @@ __device__ __forceinline__ int tt_splits(const BatchDev& bd, int b, int c, int w
   return (int)n;
 }
 
+// The sums over a state's rows are scaled where its norm^2 is near the end of
+// FP32's range, which holds a TT_FLUSH run of products but not their sum.
+#define TT_GRAM_DOWN 0x1p-40f
+__device__ __forceinline__ bool tt_gram_large(double2 sq) { return sq.x > 0x1p120; }
+
 __device__ __forceinline__ bool tt_gram_here(const BatchDev& bd, const int* bond, int c, int* w) {
   if (c < 1 || !bond_ok(bond[c + 1], bd.tt_b)) return false;
   *w = 2 * bond[c + 1];
@@ -85,9 +90,11 @@ __device__ __forceinline__ bool tt_gram_here(const BatchDev& bd, const int* bond
 // Measured (20 qubits, 64 wide): 1380 us with eight splits and FP64 sums,
 // 86 us now (512 wide, FP32 bound: 1630 -> 520 us).
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step, const float2* sv,
-                                                           const float2* src, const int* bonds, xc* partials) {
+                                                           const float2* src, const int* bonds, const double2* sq,
+                                                           xc* partials) {
   grid_wait();
   __shared__ xc red[BLOCK_THREADS * TT_EPB];   // 32 KB
+  __shared__ volatile int large;               // not a register over the rows
   for (int tile = blockIdx.x; tile < bd.ntiles; tile += gridDim.x) {
     const int b = bd.tile_state[tile];
     const int n = bd.n[b];
@@ -98,6 +105,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
     if (bond[c + 1] > bd.tt_b && idx == 0 && threadIdx.x == 0) atomicOr(bd.err, KERR_EIG_WIDTH);
     int w;
     if (!tt_gram_here(bd, bond, c, &w)) continue;
+    if (threadIdx.x == 0) large = tt_gram_large(sq[b]);
+    __syncthreads();
     const int nt = bd.state_ntiles[b], nsplit = tt_splits(bd, b, c, w);
     const float2* m = (step == 0 ? sv : src) + bd.vec_off[b];
     const int nb = gram_nblocks(w);
@@ -146,6 +155,13 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
                 df_add_prod(o.im, -xa[u].y, xv[v].x);
               }
           }
+          if (large) {
+#pragma unroll
+            for (int k = 0; k < TT_EPB; ++k) {
+              s[k].re = DF{s[k].re.hi * TT_GRAM_DOWN, s[k].re.lo * TT_GRAM_DOWN};
+              s[k].im = DF{s[k].im.hi * TT_GRAM_DOWN, s[k].im.lo * TT_GRAM_DOWN};
+            }
+          }
 #pragma unroll
           for (int k = 0; k < TT_EPB; ++k) {
             df_add(acc[k].re, s[k].re.hi, s[k].re.lo);
@@ -179,7 +195,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram(BatchDev bd, int step
 // (eight lanes per entry, each every eighth split, then the lanes), the lower
 // triangle mirrored.  Block x takes 32 entries at a time, block y a state.
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram_sum(BatchDev bd, int step, const int* bonds,
-                                                               const xc* partials, double2* gram) {
+                                                               const double2* sq, const xc* partials,
+                                                               double2* gram) {
   grid_wait();
   const int l8 = threadIdx.x & 7;
   for (int b = blockIdx.y; b < bd.B; b += gridDim.y) {
@@ -206,7 +223,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_gram_sum(BatchDev bd, int 
         df_add(s.im, __shfl_xor_sync(0xffffffffu, s.im.hi, o), __shfl_xor_sync(0xffffffffu, s.im.lo, o));
       }
       if (l8 == 0 && e < ww && a <= cc) {
-        const double2 r = xa_to_d(s);
+        double2 r = xa_to_d(s);
+        if (tt_gram_large(sq[b])) r = cscale(r, 1.0 / TT_GRAM_DOWN);
         g[e] = a == cc ? cd(r.x, 0.0) : r;
         if (a != cc) g[(int64_t)cc * w + a] = cconj(r);
       }
@@ -1329,16 +1347,16 @@ static int grid_for(const BatchDev& bd) {
 }
 
 void launch_tt_gram(const BatchDev& bd, int step, const float2* sv, const float2* src, const int* bonds,
-                    double2* partials, double2* gram, cudaStream_t s) {
+                    const double2* sq, double2* partials, double2* gram, cudaStream_t s) {
   xc* part = reinterpret_cast<xc*>(partials);
   qm_note_launch();
-  launch_after(k_tt_gram, grid_for(bd), BLOCK_THREADS, 0, s, bd, step, sv, src, bonds, part);
+  launch_after(k_tt_gram, grid_for(bd), BLOCK_THREADS, 0, s, bd, step, sv, src, bonds, sq, part);
   // the widest Gram a state can have at this step
   const int64_t wmax = step < 12 ? std::min<int64_t>(ipow2(step + 1), 2 * bd.tt_b) : 2 * bd.tt_b;
   const int64_t gx = std::min<int64_t>((wmax * wmax + BLOCK_THREADS / 8 - 1) / (BLOCK_THREADS / 8), 2048);
   qm_note_launch();
   launch_after(k_tt_gram_sum, dim3((unsigned)gx, (unsigned)std::min(bd.B, 65535)), BLOCK_THREADS, 0, s, bd, step,
-               bonds, part, gram);
+               bonds, sq, part, gram);
 }
 
 void launch_tt_eig(const BatchDev& bd, int step, int* bonds, double2* gram, double2* vwork, int max_bond,
