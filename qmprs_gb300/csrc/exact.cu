@@ -449,11 +449,11 @@ __device__ __forceinline__ void x_env_mac(DF (&e)[32], int i, xc u, xc v) {
 __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int step, xc* psi, const xc* t,
                                                                 double2* gates, const signed char* arity,
                                                                 const int* nlayers, const int* active,
-                                                                xc* partials, double* nuc) {
+                                                                double2* partials, double* nuc) {
   grid_wait();
   __shared__ xc gs[16];
-  __shared__ float2 wred[WARPS][32];
-  __shared__ xc env[16];
+  __shared__ double wred[WARPS][32];
+  __shared__ double2 env[16];
   __shared__ double2 gd[16];
   __shared__ WarpPolar wp;
   GateSel sel;
@@ -529,29 +529,22 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
         x_env_mac(e, 3, t1, y1);
       }
     }
-    // per warp (fixed exchange, double-float), then the block's warps in order
-    {
-      const DF v = warp_sum32_df(e);
-      wred[warp][tid & 31] = make_float2(v.hi, v.lo);
-    }
+    // per warp (fixed exchange), then the block's warps in a fixed order
+    wred[warp][tid & 31] = warp_sum32_d(e);
     __syncthreads();
     if (tid < 32) env_sum_warps(wred, partials + (int64_t)tile * 16, tid);
     __syncthreads();
     if (last_tile_ticket(bd.ticket, b, nt)) {
       const int entry = tid >> 4, l16 = tid & 15;
       const int t0 = bd.state_tile0[b];
-      XA s = xa_zero();
-      for (int tt = l16; tt < nt; tt += 16) {
-        const xc v = __ldcg(&partials[(int64_t)(t0 + tt) * 16 + entry]);
-        df_add(s.re, v.x, v.z);
-        df_add(s.im, v.y, v.w);
-      }
+      double2 s = czero();
+      for (int tt = l16; tt < nt; tt += 16) s = cadd(s, __ldcg(&partials[(int64_t)(t0 + tt) * 16 + entry]));
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) {
-        df_shfl_add(s.re, s.re, o);
-        df_shfl_add(s.im, s.im, o);
+        s.x += __shfl_down_sync(0xffffffffu, s.x, o, 16);
+        s.y += __shfl_down_sync(0xffffffffu, s.y, o, 16);
       }
-      if (l16 == 0) env[entry] = xa_round(s);
+      if (l16 == 0) env[entry] = s;
       if (tid < m * m) gd[tid] = gptr[tid];
       __syncthreads();
       if (tid < 32) {
@@ -584,7 +577,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
 // and over the warps in order.  As in k_sweep_fused the polar factor bounds
 // a step, and the other warps peel the next gate from psi meanwhile.
 // Measured (10 qubits, 15 layers, 2 sweeps, 300 steps): 51.2 ms with a
-// single-thread factor, 4.5 ms now (15 us a step).
+// single-thread factor, 4.8 ms now (16 us a step; environments summed in
+// double-float throughout took 1 us less and doubled the gates' error).
 __device__ __forceinline__ void x_fused_apply(xc* v, int n, int q, int k, const xc* gs, int tid, int step) {
   if (k == 2) {
     const int slo = n - 2 - q, dlo = 1 << slo, dhi = dlo << 1;
@@ -628,8 +622,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
   __shared__ xc gs[2][16];           // the gate to apply (rebuild), or to peel
   __shared__ xc gt[16];              // the new gate's adjoint
   __shared__ double2 gd[2][16];      // the step's gate and the next step's
-  __shared__ float2 wred[WARPS][32];
-  __shared__ xc env[16];
+  __shared__ double wred[WARPS][32];
+  __shared__ double2 env[16];
   __shared__ WarpPolar wp;
   const int b = blockIdx.x;
   if (b >= bd.B) return;
@@ -731,10 +725,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
           x_env_mac(e, 3, t1, y1);
         }
       }
-      {
-        const DF v = warp_sum32_df(e);
-        wred[warp][lane] = make_float2(v.hi, v.lo);
-      }
+      wred[warp][lane] = warp_sum32_d(e);
       if (fetch) {
         gd[buf ^ 1][tid] = pre;
         gs[buf ^ 1][(tid % (1 << k2)) * (1 << k2) + tid / (1 << k2)] = xc_from_d(cconj(pre));
@@ -898,7 +889,7 @@ void launch_x_sweep_step(const BatchDev& bd, int step, xc* psi, const xc* t, dou
                          const int* nlayers, const int* active, double2* partials, double* nuc, cudaStream_t s) {
   qm_note_launch();
   launch_after(k_x_sweep_step, grid_for(bd), BLOCK_THREADS, 0, s, bd, step, psi, t, gates, arity, nlayers, active,
-               reinterpret_cast<xc*>(partials), nuc);
+               partials, nuc);
 }
 
 int launch_x_sweep_fused(const BatchDev& bd, int max_n, const xc* target, double2* gates, const signed char* arity,

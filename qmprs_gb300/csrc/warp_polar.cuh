@@ -39,6 +39,7 @@
 struct WarpPolar {
   xc E[16];               // the matrix, scaled by a power of two, padded to 4 x 4
   xc V[16], U[16];
+  double2 D[16];          // the matrix in FP64 (exact mode, Grams)
   double2 A[16], B[16], C[16];
   float2 T[16];
   float sig[4], rsig[4];  // column norms of E V and their reciprocals; 0 for null columns
@@ -412,6 +413,27 @@ __device__ __forceinline__ int wp_load(WarpPolar& ws, const xc* env, int m, int 
   return ex;
 }
 
+// The same of an FP64 environment: ws.D, and its double-float rounding in
+// ws.E.
+__device__ __forceinline__ int wp_load(WarpPolar& ws, const double2* env, int m, int lane, bool* finite) {
+  const int r = (lane >> 2) & 3, c = lane & 3;
+  const bool in = r < m && c < m;
+  const double2 e = in ? env[r * m + c] : czero();
+  *finite = __all_sync(0xffffffffu, isfinite(e.x) && isfinite(e.y));
+  const int hx = __double2hiint(e.x) & 0x7fffffff, hy = __double2hiint(e.y) & 0x7fffffff;
+  const int mbits = __reduce_max_sync(0xffffffffu, max(hx, hy));
+  const int ex = mbits == 0 ? 0 : min(max((mbits >> 20) - 1022, -1000), 1000);
+  const double sc = __hiloint2double((1023 - ex) << 20, 0);
+  const double pad = r == c && m < 4 ? __hiloint2double(mbits, 0) * sc : 0.0;
+  const double2 d = in ? cd(e.x * sc, e.y * sc) : cd(pad, 0.0);
+  if (lane < 16) {
+    ws.D[lane] = d;
+    ws.E[lane] = xc_split(d);
+  }
+  __syncwarp();
+  return ex;
+}
+
 __device__ __forceinline__ double wp_unscale(int ex) { return __hiloint2double((1023 + ex) << 20, 0); }
 
 // Entry (r, c) of the current gate's conjugate, padded with the identity.
@@ -489,7 +511,7 @@ template <bool EXACT>
 __device__ __noinline__ double wp_single_thread(const WarpPolar& ws, double2* gate, int m) {
   double2 e[16], w[16], wprev[16];
   for (int i = 0; i < m * m; ++i) {
-    e[i] = xc_to_d(ws.E[(i / m) * 4 + i % m]);
+    e[i] = EXACT ? ws.D[(i / m) * 4 + i % m] : xc_to_d(ws.E[(i / m) * 4 + i % m]);
     wprev[i] = cconj(gate[i]);
   }
   const double nn = EXACT ? polar_jacobi_pre(e, m, w, wprev) : polar_sweep(e, m, w, wprev);
@@ -642,7 +664,7 @@ __device__ __forceinline__ void wp_norms(WarpPolar& ws, int lane, xc xp, xc xq, 
 }
 
 // FP64 from double-float: V (lanes 8-15 of vp, vq) orthonormal to rounding
-// in ws.B, E V in ws.A, E V's columns over their norms (ws.rs) in ws.C, and
+// in ws.B, D V in ws.A, its columns over their norms (ws.rs) in ws.C, and
 // T = (I - C^H C) / 2.
 __device__ __forceinline__ void wp_to_fp64(WarpPolar& ws, int lane, xc vp, xc vq) {
   const int ip = (lane & 3) * 4 + 2 * ((lane >> 2) & 1);
@@ -651,18 +673,13 @@ __device__ __forceinline__ void wp_to_fp64(WarpPolar& ws, int lane, xc vp, xc vq
     ws.B[ip] = xc_to_d(vp);
     ws.B[ip + 1] = xc_to_d(vq);
   }
-  {
-    const DF e = wdf_load(ws.E, lane);
-    wmm_store(ws.C, lane, (double)e.hi + (double)e.lo);
-  }
   __syncwarp();
   wp_gram_defect(ws.B, ws.T, lane);
   const double v = reinterpret_cast<const double*>(ws.B)[lane] + (double)wf_part(ws.B, ws.T, i, j, part);
   __syncwarp();
   wmm_store(ws.B, lane, v);
   __syncwarp();
-  const double a = wmm_part<false, false>(ws.C, ws.B, i, j, part);
-  __syncwarp();
+  const double a = wmm_part<false, false>(ws.D, ws.B, i, j, part);
   wmm_store(ws.A, lane, a);
   const DF r = ws.rs[j];
   wmm_store(ws.C, lane, a * ((double)r.hi + (double)r.lo));
@@ -693,11 +710,11 @@ __device__ __forceinline__ void wp_polar_weights(WarpPolar& ws, int lane, int nm
   __syncwarp();
 }
 
-// As warp_polar, to FP64 accuracy: with the columns orthogonal to
-// double-float, one first-order correction (defects of about 1e-13 from FP64
-// Grams, products with them in FP32) reaches FP64 rounding.  Returns the
+// As warp_polar, to FP64 accuracy and of an FP64 environment: with the columns
+// orthogonal to double-float, one first-order correction (defects of about
+// 1e-13 from FP64 Grams, products with them in FP32) reaches FP64 rounding.  Returns the
 // nuclear norm of env when `want_norm`.
-static __device__ __noinline__ double warp_polar_exact(WarpPolar& ws, const xc* env, double2* gate, int m,
+static __device__ __noinline__ double warp_polar_exact(WarpPolar& ws, const double2* env, double2* gate, int m,
                                                        bool want_norm, bool* finite) {
   const int lane = threadIdx.x & 31;
   const int ex = wp_load(ws, env, m, lane, finite);
@@ -855,6 +872,8 @@ __device__ __forceinline__ void warp_gram_vectors(WarpPolar& ws, double2 g, doub
   if (lane < 16) ws.U[lane] = xc_from_d(g);
   __syncwarp();
   wp_load(ws, ws.U, 4, lane, &finite);
+  const DF e = wdf_load(ws.E, lane);
+  wmm_store(ws.D, lane, (double)e.hi + (double)e.lo);
   xc yp, yq;
   int fp = 0, fq = 0;
   *odd = wp_df_columns(ws, lane, yp, yq);
@@ -907,11 +926,15 @@ __device__ __forceinline__ void warp_gram_vectors(WarpPolar& ws, double2 g, doub
 // ---- sums over a warp --------------------------------------------------------------------------
 
 // Sum of 32 double-float values per lane over the warp: lane l returns the
-// total of value l (exchange as warp_sum32).
-__device__ __forceinline__ DF warp_sum32_df(DF (&v)[32]) {
+// total of value l in FP64 (exchange as warp_sum32).  The first two steps
+// are double-float, whose roundings the 64 sums of four lanes of a block's
+// warps average out; from there on they would show beside those of the
+// amplitudes, so the high parts of the last seven additions are FP64 (31 of
+// them would take 4000 cycles of a block's step).
+__device__ __forceinline__ double warp_sum32_d(DF (&v)[32]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = 16; o > 4; o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int i = 0; i < o; ++i) {
@@ -920,7 +943,25 @@ __device__ __forceinline__ DF warp_sum32_df(DF (&v)[32]) {
       df_shfl_add(v[i], give, o);
     }
   }
-  return v[0];
+  double hi[8];
+  float lo[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    hi[i] = (double)v[i].hi;
+    lo[i] = v[i].lo;
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const double gh = up ? hi[i] : hi[i + o], kh = up ? hi[i + o] : hi[i];
+      const float gl = up ? lo[i] : lo[i + o], kl = up ? lo[i + o] : lo[i];
+      hi[i] = kh + __shfl_xor_sync(0xffffffffu, gh, o);
+      lo[i] = kl + __shfl_xor_sync(0xffffffffu, gl, o);
+    }
+  }
+  return hi[0] + (double)lo[0];
 }
 
 // Sum of 32 values per lane over the warp: lane l returns the total of
@@ -950,5 +991,12 @@ __device__ __forceinline__ void env_sum_warps(const float2 (*wred)[32], xc* env,
     df_add(s, v.x, v.y);
   }
   wdf_store(env, lane, s);
+}
+// The same of FP64 sums, as one part of an FP64 entry.
+__device__ __forceinline__ void env_sum_warps(const double (*wred)[32], double2* env, int lane) {
+  double v[WARPS];
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) v[w] = wred[w][lane];
+  wmm_store(env, lane, ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
 }
 static_assert(sizeof(xc) == sizeof(double2), "work matrices are shared between the precisions");
