@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
                                                                 double2* partials, double* nuc) {
   grid_wait();
   __shared__ xc gs[16];
-  __shared__ double wred[WARPS][32];
+  __shared__ TF wred[WARPS][32];
   __shared__ double2 env[16];
   __shared__ double2 gd[16];
   __shared__ WarpPolar wp;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
       }
     }
     // per warp (fixed exchange), then the block's warps in a fixed order
-    wred[warp][tid & 31] = warp_sum32_d(e);
+    wred[warp][tid & 31] = warp_sum32_tf(e);
     __syncthreads();
     if (tid < 32) env_sum_warps(wred, partials + (int64_t)tile * 16, tid);
     __syncthreads();
@@ -577,8 +577,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
 // and over the warps in order.  As in k_sweep_fused the polar factor bounds
 // a step, and the other warps peel the next gate from psi meanwhile.
 // Measured (10 qubits, 15 layers, 2 sweeps, 300 steps): 51.2 ms with a
-// single-thread factor, 4.8 ms now (16 us a step; environments summed in
-// double-float throughout took 1 us less and doubled the gates' error).
+// single-thread factor, 4.7 ms now (16 us a step; environments summed and
+// handed on in double-float took 0.5 us less and up to doubled the gates'
+// error, their last sums in FP64 half a microsecond more).
 __device__ __forceinline__ void x_fused_apply(xc* v, int n, int q, int k, const xc* gs, int tid, int step) {
   if (k == 2) {
     const int slo = n - 2 - q, dlo = 1 << slo, dhi = dlo << 1;
@@ -622,7 +623,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
   __shared__ xc gs[2][16];           // the gate to apply (rebuild), or to peel
   __shared__ xc gt[16];              // the new gate's adjoint
   __shared__ double2 gd[2][16];      // the step's gate and the next step's
-  __shared__ double wred[WARPS][32];
+  __shared__ TF wred[WARPS][32];
   __shared__ double2 env[16];
   __shared__ WarpPolar wp;
   const int b = blockIdx.x;
@@ -725,7 +726,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_fused(BatchDev bd, co
           x_env_mac(e, 3, t1, y1);
         }
       }
-      wred[warp][lane] = warp_sum32_d(e);
+      wred[warp][lane] = warp_sum32_tf(e);
       if (fetch) {
         gd[buf ^ 1][tid] = pre;
         gs[buf ^ 1][(tid % (1 << k2)) * (1 << k2) + tid / (1 << k2)] = xc_from_d(cconj(pre));

@@ -423,9 +423,14 @@ __device__ __forceinline__ int wp_load(WarpPolar& ws, const double2* env, int m,
   const int hx = __double2hiint(e.x) & 0x7fffffff, hy = __double2hiint(e.y) & 0x7fffffff;
   const int mbits = __reduce_max_sync(0xffffffffu, max(hx, hy));
   const int ex = mbits == 0 ? 0 : min(max((mbits >> 20) - 1022, -1000), 1000);
-  const double sc = __hiloint2double((1023 - ex) << 20, 0);
-  const double pad = r == c && m < 4 ? __hiloint2double(mbits, 0) * sc : 0.0;
-  const double2 d = in ? cd(e.x * sc, e.y * sc) : cd(pad, 0.0);
+  // times 2^-ex by the exponents (an FP64 product takes 64 cycles); what would
+  // leave the normal range is far below the others' rounding
+  auto scaled = [ex](double v) {
+    const int f = ((__double2hiint(v) >> 20) & 0x7ff) - ex;
+    return f > 0 && f > -ex ? __hiloint2double(__double2hiint(v) - (ex << 20), __double2loint(v)) : 0.0;
+  };
+  const double pad = r == c && m < 4 ? scaled(__hiloint2double(mbits, 0)) : 0.0;
+  const double2 d = in ? cd(scaled(e.x), scaled(e.y)) : cd(pad, 0.0);
   if (lane < 16) {
     ws.D[lane] = d;
     ws.E[lane] = xc_split(d);
@@ -925,43 +930,45 @@ __device__ __forceinline__ void warp_gram_vectors(WarpPolar& ws, double2 g, doub
 
 // ---- sums over a warp --------------------------------------------------------------------------
 
-// Sum of 32 double-float values per lane over the warp: lane l returns the
-// total of value l in FP64 (exchange as warp_sum32).  The first two steps
-// are double-float, whose roundings the 64 sums of four lanes of a block's
-// warps average out; from there on they would show beside those of the
-// amplitudes, so the high parts of the last seven additions are FP64 (31 of
-// them would take 4000 cycles of a block's step).
-__device__ __forceinline__ double warp_sum32_d(DF (&v)[32]) {
+// s += the partner lane's `give` (lane ^ o)
+__device__ __forceinline__ void tf_shfl_add(TF& s, const TF& give, int o) {
+  tf_add(s, TF{__shfl_xor_sync(0xffffffffu, give.h, o), __shfl_xor_sync(0xffffffffu, give.m, o),
+               __shfl_xor_sync(0xffffffffu, give.l, o)});
+}
+
+// Halving exchange over lanes N / 2, N / 4 .. 1: lane l returns the sum over
+// them of value l mod N.
+template <int N>
+__device__ __forceinline__ TF warp_fold_tf(TF (&v)[N]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16; o > 4; o >>= 1) {
+  for (int o = N / 2; o > 0; o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int i = 0; i < o; ++i) {
-      const DF give = up ? v[i] : v[i + o];
+      const TF give = up ? v[i] : v[i + o];
       if (up) v[i] = v[i + o];
-      df_shfl_add(v[i], give, o);
+      tf_shfl_add(v[i], give, o);
     }
   }
-  double hi[8];
-  float lo[8];
+  return v[0];
+}
+
+// Sum of 32 double-float values per lane over the warp: lane l returns the
+// total of value l (exchange as warp_sum32), as exact as FP64 sums but for the
+// first of five steps, whose roundings average out as those of the lanes' own
+// sums do.
+__device__ __forceinline__ TF warp_sum32_tf(DF (&v)[32]) {
+  TF t[16];
+  const bool up = (threadIdx.x & 16) != 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    hi[i] = (double)v[i].hi;
-    lo[i] = v[i].lo;
+  for (int i = 0; i < 16; ++i) {
+    const DF give = up ? v[i] : v[i + 16];
+    if (up) v[i] = v[i + 16];
+    df_shfl_add(v[i], give, 16);
+    t[i] = tf_from(v[i]);
   }
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const double gh = up ? hi[i] : hi[i + o], kh = up ? hi[i + o] : hi[i];
-      const float gl = up ? lo[i] : lo[i + o], kl = up ? lo[i + o] : lo[i];
-      hi[i] = kh + __shfl_xor_sync(0xffffffffu, gh, o);
-      lo[i] = kl + __shfl_xor_sync(0xffffffffu, gl, o);
-    }
-  }
-  return hi[0] + (double)lo[0];
+  return warp_fold_tf(t);
 }
 
 // Sum of 32 values per lane over the warp: lane l returns the total of
@@ -992,11 +999,15 @@ __device__ __forceinline__ void env_sum_warps(const float2 (*wred)[32], xc* env,
   }
   wdf_store(env, lane, s);
 }
-// The same of FP64 sums, as one part of an FP64 entry.
-__device__ __forceinline__ void env_sum_warps(const double (*wred)[32], double2* env, int lane) {
-  double v[WARPS];
+// The same of three-part sums, as one part of an FP64 entry.
+__device__ __forceinline__ void env_sum_warps(const TF (*wred)[32], double2* env, int lane) {
+  TF v[WARPS];
 #pragma unroll
   for (int w = 0; w < WARPS; ++w) v[w] = wred[w][lane];
-  wmm_store(env, lane, ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+#pragma unroll
+  for (int o = WARPS / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int w = 0; w < o; ++w) tf_add(v[w], v[w + o]);
+  wmm_store(env, lane, tf_to_d(v[0]));
 }
 static_assert(sizeof(xc) == sizeof(double2), "work matrices are shared between the precisions");
