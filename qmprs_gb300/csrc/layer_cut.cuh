@@ -16,8 +16,9 @@
 // Jacobi of one thread 187, projection 4.7) and takes 22 us now.
 //
 // The Gram's sums are exact FP32 products in double-float over a thread's
-// at most 16 rows and over the warp's lanes, FP64 across the
-// warps (fixed order) and the units.  4096 rows a unit keep the
+// at most 16 rows and over the warp's lanes (in three parts there for the
+// exact mode, whose rows carry 48 bits), FP64 across the warps (fixed order)
+// and the units; the eigensolver takes the FP64 sums.  4096 rows a unit keep the
 // double-float runs short and give a 20-qubit state 128 blocks; the table
 // of units is sorted by the last step that needs them, so a step's launch
 // holds only blocks with work.
@@ -29,6 +30,22 @@
 
 struct CutFast {
   typedef float2 T;
+  static __device__ __forceinline__ double lane_sums(DF (&s)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) df_shfl_add(s[k], s[k], 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int k = 0; k < o; ++k) {
+        const DF give = up ? s[k] : s[k + o];
+        if (up) s[k] = s[k + o];
+        df_shfl_add(s[k], give, o);
+      }
+    }
+    return (double)s[0].hi + (double)s[0].lo;
+  }
   static __device__ __forceinline__ T load_v(double2 v) { return cf((float)v.x, (float)v.y); }
   static __device__ __forceinline__ double2 to_d(T v) { return f2d(v); }
   template <int N>
@@ -68,6 +85,15 @@ struct CutFast {
 
 struct CutExact {
   typedef xc T;
+  static __device__ __forceinline__ double lane_sums(DF (&s)[16]) {
+    TF t[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      t[k] = tf_from(s[k]);
+      tf_shfl_add(t[k], t[k], 16);
+    }
+    return tf_to_d(warp_fold_tf(t));
+  }
   static __device__ __forceinline__ T load_v(double2 v) { return xc_from_d(v); }
   static __device__ __forceinline__ double2 to_d(T v) { return xc_to_d(v); }
   template <int N>
@@ -239,19 +265,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_layer_cut(BatchDev bd, int st
       }
     }
     // 16 sums over the lanes (lane l holds value l mod 16), then the warps
-#pragma unroll
-    for (int k = 0; k < 16; ++k) df_shfl_add(s[k], s[k], 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-      const bool up = (lane & o) != 0;
-#pragma unroll
-      for (int k = 0; k < o; ++k) {
-        const DF give = up ? s[k] : s[k + o];
-        if (up) s[k] = s[k + o];
-        df_shfl_add(s[k], give, o);
-      }
-    }
-    if (lane < 16) wred[tid >> 5][lane] = (double)s[0].hi + (double)s[0].lo;
+    const double sum = P::lane_sums(s);
+    if (lane < 16) wred[tid >> 5][lane] = sum;
     __syncthreads();
     double* part = partials + (int64_t)bd.state_tile0[b] * WARPS * 32;   // 16 doubles per unit
     if (tid < 16) {

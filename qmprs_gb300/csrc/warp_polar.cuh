@@ -874,11 +874,9 @@ __device__ __forceinline__ void warp_gram_vectors(WarpPolar& ws, double2 g, doub
   const int ip = (lane & 3) * 4 + 2 * ((lane >> 2) & 1);
   const int ent = lane >> 1, i = ent >> 2, j = ent & 3;
   bool finite;
-  if (lane < 16) ws.U[lane] = xc_from_d(g);
+  if (lane < 16) ws.A[lane] = g;
   __syncwarp();
-  wp_load(ws, ws.U, 4, lane, &finite);
-  const DF e = wdf_load(ws.E, lane);
-  wmm_store(ws.D, lane, (double)e.hi + (double)e.lo);
+  wp_load(ws, ws.A, 4, lane, &finite);
   xc yp, yq;
   int fp = 0, fq = 0;
   *odd = wp_df_columns(ws, lane, yp, yq);
