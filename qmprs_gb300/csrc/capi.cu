@@ -334,30 +334,6 @@ uint64_t plan_signature(const qmprs_plan* p) {
   mix((uint64_t)p->max_layers);
   return h;
 }
-// Tiles per chunk of the grouped sweep's passes: the fewest, up to 16 and else
-// GCHUNK, that leave the batch one wave of blocks (four per SM) and its
-// largest state 256 chunks.  The passes wait on memory, so every SM should have all its
-// blocks; a chunk's set-up (offset tables, composed gates) costs about one
-// tile, so a second wave does not pay, and every chunk adds a partial to the
-// polar kernel's sum over its state.
-// Measured per pass of the case (tiles 32 / 16 / 8 / 4 / 2 / 1): one 20-qubit
-// state (512 tiles) 29.0 / 18.2 / 13.1 / 10.8 / 10.7 / 12.3 ms, environments
-// of 32 states of 13-16 qubits (480 tiles) 6.9 / 4.2 / 2.8 / 2.2 / 2.0 / 1.9
-// ms, 64 states of 12-20 qubits (6700 tiles) 24.9 / 18.2 / 18.4 / 18.6 / 21.6 /
-// 28.6 ms, and later 17.0 ms with 16 tiles (432 chunks), 16.0 ms with 12 (one wave).
-#define CHUNKS_PER_STATE 256
-int choose_chunk_tiles(const std::vector<int>& n) {
-  for (int tiles = 1; tiles <= 16; ++tiles) {
-    int64_t chunks = 0, most = 0;
-    for (int q : n) {
-      const int64_t c = q > GT ? (ipow2(q - GT) + tiles - 1) / tiles : 1;
-      chunks += c;
-      most = std::max(most, c);
-    }
-    if (chunks <= PASS_GRID_DEFAULT && most <= CHUNKS_PER_STATE) return tiles;
-  }
-  return GCHUNK;
-}
 
 inline uint64_t dbl_key(double v) {
   uint64_t u;
@@ -775,7 +751,7 @@ int qmprs_plan_create(qmprs_handle_t h, int num_states, const int* num_qubits, i
       p->tt_off.push_back(p->tt_off.back() + std::max(least, std::min<int64_t>(std::min(nt, TT_SPLIT_MAX), most) * one));
   }
   // grouped sweep: tiles of 2^min(n, GT) amplitudes, chunk_tiles tiles per chunk
-  p->chunk_tiles = choose_chunk_tiles(p->n);
+  p->chunk_tiles = choose_chunk_tiles(p->n.data(), num_states);
   std::vector<int> chunk_state, chunk_idx, state_chunk0(num_states), state_nchunks(num_states);
   for (int b = 0; b < num_states; ++b) {
     const int n = p->n[b];

@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include "qm_complex.h"
+#include "tile_layout.h"
 
 #define TILE_BITS_MIN 12
 #define TILE_BITS_MAX 17
@@ -109,14 +110,11 @@ struct GateSel {
 // Grouped backward sweep (sweep_group.cu): a group is a run of consecutive
 // backward steps whose qubits fit a window of GW qubits; one pass over the
 // vectors per group, shared-memory tiles of 2^GT amplitudes, one partial
-// cross matrix per chunk of at most GCHUNK tiles.
+// cross matrix per chunk of at most GCHUNK tiles (tile_layout.h).
 #define GW 4
 #define GM (1 << GW)
 #define GMM (GM * GM)
-#define GT 11
-#define GCHUNK 32   // most tiles per chunk
 #define GMAXSTEPS 8
-#define PASS_GRID_DEFAULT (4 * 152)   // resident blocks of the tile passes (4 per SM)
 
 struct GroupEnt {
   int j0;     // first backward step

@@ -1,8 +1,8 @@
 // Shared-memory tile layout of the pass kernels: the swizzle, the bit
 // deposits, and the rest / position orders that keep the tensor-core
-// fragment loads on distinct banks.  Plain integer functions, compiled into
-// the CUDA library and into the host check build, so their bijectivity and
-// bank properties are tested on a CPU.
+// fragment loads on distinct banks; and how many tiles a block takes.  Plain
+// integer functions, compiled into the CUDA library and into the host check
+// build, so their bijectivity and bank properties are tested on a CPU.
 #pragma once
 
 #include "qm_complex.h"
@@ -96,4 +96,40 @@ QM_HD float vec_scale(int n, double nrm) {
   frexp(nrm, &e);   // nrm < 2^e
   const int top = n / 2 + 4 < 15 ? n / 2 + 4 : 15;
   return ldexpf(1.f, top - e);
+}
+
+#define GT 11                         // a tile of the pass kernels: 2^GT amplitudes
+#define GCHUNK 32                     // most tiles per chunk
+#define PASS_GRID_DEFAULT (4 * 152)   // resident blocks of the tile passes (4 per SM)
+#define CHUNKS_PER_STATE 256
+
+// Tiles per chunk of the grouped sweep's passes: the fewest, up to 16 and else
+// GCHUNK, that leave the batch's states of several tiles one wave of blocks
+// and the largest of them 256 chunks.  The passes wait on memory, so every SM
+// should have all its blocks; a chunk's set-up (offset tables, composed
+// gates) costs about one tile, so a second wave does not pay, and every chunk
+// adds a partial to the polar kernel's sum over its state.  A state of one
+// tile has one chunk whatever the length and is not counted: with 700 of 8
+// qubits beside one of 20 every length seemed to take two waves, and 32 tiles
+// were taken (two sweeps of four layers 11.1 ms, 5.5 ms with two).
+// Measured per pass of the case (tiles 32 / 16 / 8 / 4 / 2 / 1): one 20-qubit
+// state (512 tiles) 29.0 / 18.2 / 13.1 / 10.8 / 10.7 / 12.3 ms, environments
+// of 32 states of 13-16 qubits (480 tiles) 6.9 / 4.2 / 2.8 / 2.2 / 2.0 / 1.9
+// ms, 64 states of 12-20 qubits (6700 tiles) 24.9 / 18.2 / 18.4 / 18.6 / 21.6 /
+// 28.6 ms, and later 17.0 ms with 16 tiles (432 chunks), 16.0 ms with 12 (one wave).
+// Where one wave takes 17 to 31 tiles, or one state more than 256 chunks of 16,
+// the jump to 32 is not the fastest: 12 states of 21 qubits 18.4 ms, 15.1 with
+// 21 tiles; one of 24 qubits 9.4 ms, 6.8 with 14.
+inline int choose_chunk_tiles(const int* n, int count) {
+  for (int tiles = 1; tiles <= 16; ++tiles) {
+    long long chunks = 0, most = 0;
+    for (int b = 0; b < count; ++b) {
+      if (n[b] <= GT) continue;
+      const long long c = ((1ll << (n[b] - GT)) + tiles - 1) / tiles;
+      chunks += c;
+      most = c > most ? c : most;
+    }
+    if (chunks <= PASS_GRID_DEFAULT && most <= CHUNKS_PER_STATE) return tiles;
+  }
+  return GCHUNK;
 }
