@@ -22,9 +22,10 @@ __device__ __forceinline__ double2 xc_to_d(xc v) { return cd((double)v.x + (doub
 // (ties away from zero), lo the other 29 bits; values out of FP32's range
 // give what their conversion gives.
 __device__ __forceinline__ float2 df_split(double x) {
-  const int xh = __double2hiint(x), xl = __double2loint(x);
-  const int low = (int)((unsigned)(xl + 0x10000000) & 0x1fffffffu) - 0x10000000;   // x's bits below hi's, signed
-  const long long hb = (((long long)xh << 32) | (unsigned)xl) - low;
+  const int xh = __double2hiint(x);
+  const unsigned xl = (unsigned)__double2loint(x);
+  const int low = (int)((xl + 0x10000000u) & 0x1fffffffu) - 0x10000000;   // x's bits below hi's, signed
+  const long long hb = __double_as_longlong(x) - low;
   const float hi = __double2float_rn(__longlong_as_double(hb));
   const int f = ((xh >> 20) & 0x7ff) - 895;   // exponent field of 2^(e + 1) in FP32
   const float sc = f > 0 && f < 255 ? __int_as_float((f << 23) | (xh & 0x80000000)) : f < 255 ? 0.f : hi - hi;
