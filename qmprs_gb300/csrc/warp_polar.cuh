@@ -424,10 +424,12 @@ __device__ __forceinline__ int wp_load(WarpPolar& ws, const double2* env, int m,
   const int mbits = __reduce_max_sync(0xffffffffu, max(hx, hy));
   const int ex = mbits == 0 ? 0 : min(max((mbits >> 20) - 1022, -1000), 1000);
   // times 2^-ex by the exponents (an FP64 product takes 64 cycles); what would
-  // leave the normal range is far below the others' rounding
+  // leave the normal range is far below the others' rounding, and what is not
+  // finite stays so
   auto scaled = [ex](double v) {
-    const int f = ((__double2hiint(v) >> 20) & 0x7ff) - ex;
-    return f > 0 && f > -ex ? __hiloint2double(__double2hiint(v) - (ex << 20), __double2loint(v)) : 0.0;
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    if (e == 0x7ff) return v;
+    return e > 0 && e > ex ? __hiloint2double(__double2hiint(v) - ex * (1 << 20), __double2loint(v)) : 0.0;
   };
   const double pad = r == c && m < 4 ? scaled(__hiloint2double(mbits, 0)) : 0.0;
   const double2 d = in ? cd(scaled(e.x), scaled(e.y)) : cd(pad, 0.0);
