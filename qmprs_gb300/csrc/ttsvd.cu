@@ -1233,6 +1233,33 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
 }
 
 // Dynamic shared memory: V (TT_MAXW x TT_MAXB float2) then TT_CH rows.
+// Sum of `count` complex FP32 products x(k) v(k) in double-float, rounded once.
+// States of up to TT_DOT_QUBITS qubits take it in the projections and the
+// target's contraction: FP32 chains were most of the target's rounding there
+// (8 qubits: 3.3e-7 of its norm, 1.4e-7 so), which the layers multiply (the
+// prepared state of two layers and a sweep: error 0.60 times, 160 states).
+// A larger state's one block would show the ten times as many operations (12
+// qubits at bond 64: 3.7 -> 3.9 ms; 10 qubits at bond 32: within the spread).
+#define TT_DOT_QUBITS 10
+__device__ __forceinline__ void tt_dot_mac(DF& re, DF& im, float2 a, float2 b) {
+  df_add_prod(re, a.x, b.x);
+  df_add_prod(re, -a.y, b.y);
+  df_add_prod(im, a.x, b.y);
+  df_add_prod(im, a.y, b.x);
+}
+
+// o[row][col] = sum_a x[row][a] v[a][col] for nr x nc outputs (rows of x
+// ldx apart; not inlined: the larger states' loops keep their registers)
+__device__ __noinline__ void tt_small_product(const float2* x, int ldx, const float2* v, int w, int nr, int nc,
+                                              float2* o) {
+  for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
+    const int row = e / nc, col = e % nc;
+    DF re = {0.f, 0.f}, im = {0.f, 0.f};
+    for (int k = 0; k < w; ++k) tt_dot_mac(re, im, x[row * ldx + k], v[k * nc + col]);
+    o[e] = cf(re.hi + re.lo, im.hi + im.lo);
+  }
+}
+
 __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_project(BatchDev bd, int step, const float2* sv,
                                                               const float2* src, float2* dst,
                                                               const int* bonds, const double2* vsel) {
@@ -1266,6 +1293,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_tt_project(BatchDev bd, int s
       __syncthreads();
       for (int e = threadIdx.x; e < nr * w; e += blockDim.x) xs[(e / w) * TT_MAXW + e % w] = m[(r0 + e / w) * w + e % w];
       __syncthreads();
+      if (n <= TT_DOT_QUBITS) {
+        tt_small_product(xs, TT_MAXW, vs, w, nr, keep, o + r0 * keep);
+        continue;
+      }
       for (int e = threadIdx.x; e < nr * keep; e += blockDim.x) {
         const int rr = e / keep, col = e % keep;
         float2 acc = cf(0.f, 0.f);
@@ -1320,6 +1351,17 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_mps_contract(BatchDev bd, int
     const double2* t0 = tensors + bd.tensor_off[b];
     const float2* s = src + bd.vec_off[b];
     float2* o = (c == n - 1 ? target : dst_buf) + bd.vec_off[b];
+    if (n <= TT_DOT_QUBITS) {   // one tile
+      const float2* x = s;
+      if (step == 0) {          // site 0 (two rows), behind the site's entries
+        x = as + rc * 2 * rn;
+        __syncthreads();
+        for (int e = threadIdx.x; e < 2 * rc; e += blockDim.x) as[rc * 2 * rn + e] = cf((float)t0[e].x, (float)t0[e].y);
+        __syncthreads();
+      }
+      tt_small_product(x, rc, as, rc, (int)ipow2(c), 2 * rn, o);
+      continue;
+    }
     const int64_t total = ipow2(c + 1) * rn;
     int64_t lo, hi;
     tile_range(total, bd.tile_idx[tile], bd.state_ntiles[b], &lo, &hi);
