@@ -129,9 +129,12 @@ __device__ __forceinline__ float2 fmac(float2 acc, float2 a, float2 b) {
 
 // Compensated accumulation of exact products (double-float): p = u v is
 // split exactly into ph + pl (fma), ph enters (hi, lo) through a TwoSum and
-// pl and the TwoSum error land in lo.  Flushed to fp64 every TT_FLUSH rows,
-// the relative error of a Gram entry is about TT_FLUSH * 2^-48 of the sum of
-// |products|, far below the 1e-10 truncation cutoff the eigenvalues decide.
+// pl and the TwoSum error land in lo, whose own roundings grow with the run.
+// A run of TT_FLUSH = 32 squares is off by 2^-47 of its sum (root mean square;
+// 2^-44 the largest of 2000), 256 of them by 2^-44 (2^-42), 4096 by 2^-40, so
+// runs end after TT_FLUSH rows: in FP64, or in stage (a)'s fast Gram in
+// another double-float sum (16 runs 2^-47, 256 runs 2^-44).  The 1e-10 cutoff
+// that the eigenvalues decide is 2^-33.
 struct DF {
   float hi, lo;
 };
@@ -148,5 +151,5 @@ __device__ __forceinline__ void df_add_prod(DF& s, float u, float v) {
   s.hi = t;
 }
 
-// rows summed in double-float between fp64 flushes
+// rows summed in double-float before their sum is passed on
 #define TT_FLUSH 32

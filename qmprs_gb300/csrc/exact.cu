@@ -12,12 +12,16 @@
 //   products     a*b = ph + pl exactly (ph = fl(a*b), pl = fma(a, b, -ph));
 //   sums         TwoSum of the high parts, low parts and the cross terms
 //                a_hi*b_lo + a_lo*b_hi accumulated in FP32;
-// which keeps about 2^-46 of relative precision on the FP32 pipes.  The
-// small algebra is FP64: the eigensolvers of stage (a) and of the layer
-// cuts (shared with the fast mode), the closed-form gate construction, and
-// the sweep's polar factor (FP64 one-sided Jacobi by one warp, started from
-// FP32 sweeps; the fast mode's FP32 polar is accurate to ~1e-7, which
-// rank-deficient environments carry into later steps at first order).
+// which keeps about 2^-46 of relative precision on the FP32 pipes.  Sums
+// that end in a small matrix keep what FP64 would (Grams of stage (a) and of
+// the layer cuts, environments), and the small algebra ends in FP64: the
+// eigenvectors of stage (a) up to width 64 come from FP32 sweeps and
+// double-float products, those of a layer cut from FP32 and double-float
+// one-sided sweeps, the sweep's polar factor (one warp) from the same, each
+// with a first-order correction from FP64 products, or FP64 sweeps where that
+// does not do; the closed-form gate construction is FP64 throughout.  The
+// fast mode's polar factor is accurate to ~1e-7, which rank-deficient
+// environments carry into later steps at first order.
 //
 // Caller-facing statevector buffers of this mode are complex128; the plan
 // converts them to double-float scratch on entry and back on exit.
@@ -548,7 +552,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_x_sweep_step(BatchDev bd, int
       if (tid < m * m) gd[tid] = gptr[tid];
       __syncthreads();
       if (tid < 32) {
-        // FP64 polar: rank-deficient environments leave null directions that
+        // to FP64: rank-deficient environments leave null directions that
         // follow the current gate, and an FP32 completion of them would
         // enter the later steps at first order
         bool finite;

@@ -869,8 +869,11 @@ static __device__ __noinline__ double warp_polar_exact(WarpPolar& ws, const doub
 // 1 where columns 2 and 3 stand exchanged.
 // The columns are orthogonal to double-float; what is left is one
 // first-order rotation v_j += v_i g_ij / (l_j^2 - l_i^2) where that is below
-// 1e-8, else FP64 sweeps (eigenvalues that agree to about 1e-6).  Vectors of
-// eigenvalues below 1e-11 of the largest keep any rotation among themselves.
+// 1e-8, else FP64 sweeps (eigenvalues that agree to about 1e-6, and those
+// below 2e-7 of the largest, which the rounding of g to double-float for the
+// sweeps before turns by more; a cut of them takes no longer than when their
+// vectors stayed so).  Vectors of eigenvalues below 1e-11 of the largest keep
+// any rotation among themselves.
 __device__ __forceinline__ void warp_gram_vectors(WarpPolar& ws, double2 g, double (&l)[4], int* odd) {
   const int lane = threadIdx.x & 31;
   const int ip = (lane & 3) * 4 + 2 * ((lane >> 2) & 1);
