@@ -1241,6 +1241,7 @@ __global__ void __launch_bounds__(TT_EIG_THREADS) k_tt_eig(BatchDev bd, int step
 // A larger state's one block would show the ten times as many operations (12
 // qubits at bond 64: 3.7 -> 3.9 ms; 10 qubits at bond 32: within the spread).
 #define TT_DOT_QUBITS 10
+#define TT_DOT_BOND (1 << (TT_DOT_QUBITS / 2))   // their largest bond
 __device__ __forceinline__ void tt_dot_mac(DF& re, DF& im, float2 a, float2 b) {
   df_add_prod(re, a.x, b.x);
   df_add_prod(re, -a.y, b.y);
@@ -1351,9 +1352,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS) k_mps_contract(BatchDev bd, int
     const double2* t0 = tensors + bd.tensor_off[b];
     const float2* s = src + bd.vec_off[b];
     float2* o = (c == n - 1 ? target : dst_buf) + bd.vec_off[b];
-    if (n <= TT_DOT_QUBITS) {   // one tile
+    static_assert(TT_DOT_BOND * 2 * (TT_DOT_BOND + 1) <= TT_MAXB * 2 * TT_MAXB, "a site's entries and site 0");
+    if (n <= TT_DOT_QUBITS && rc <= TT_DOT_BOND && rn <= TT_DOT_BOND) {   // one tile; bonds are the caller's
       const float2* x = s;
-      if (step == 0) {          // site 0 (two rows), behind the site's entries
+      if (step == 0) {   // site 0 (two rows), behind the site's entries
         x = as + rc * 2 * rn;
         __syncthreads();
         for (int e = threadIdx.x; e < 2 * rc; e += blockDim.x) as[rc * 2 * rn + e] = cf((float)t0[e].x, (float)t0[e].y);
